@@ -1,4 +1,5 @@
-"""Builds the sm_100a kernel library in-tree: flashtensor_b200/libasuka_b200.so.
+"""Builds the sm_100a kernel library in-tree, flashtensor_b200/libasuka_b200.so, and the native front
+end of the operator layer over it, flashtensor_b200/_bind.so (csrc/bind.cpp, a CPython extension).
 
 Usage: python -m flashtensor_b200.build [--force] [--verbose]
 nvcc cross-compiles without a GPU; the result is loaded with ctypes by flashtensor_b200._lib.
@@ -7,11 +8,13 @@ import os
 import shutil
 import subprocess
 import sys
+import sysconfig
 
 PKG_DIR = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(PKG_DIR, "csrc")
 OBJ_DIR = os.path.join(PKG_DIR, "build")
 LIB_PATH = os.path.join(PKG_DIR, "libasuka_b200.so")
+BIND_PATH = os.path.join(PKG_DIR, "_bind.so")
 
 SOURCES = ["capi.cu", "attn_fwd.cu", "col_scores.cu", "select_topk.cu", "score_ops.cu", "sima.cu", "linattn32.cu"]
 NVCC_FLAGS = [
@@ -40,7 +43,8 @@ def _deps():
 
 
 def build(force=False, verbose=False):
-  """Compile every .cu under csrc/ for sm_100a and link the shared library.  Returns its path."""
+  """Compile every .cu under csrc/ for sm_100a, link the shared library and build the front end.
+  Returns the library's path."""
   nvcc = _nvcc()
   os.makedirs(OBJ_DIR, exist_ok=True)
   srcs = [s for s in SOURCES if os.path.exists(os.path.join(CSRC, s))]
@@ -63,12 +67,34 @@ def build(force=False, verbose=False):
         raise RuntimeError(f"nvcc failed on {s}")
       relink = True
   if relink or any(os.path.getmtime(o) > os.path.getmtime(LIB_PATH) for o in objs):
-    cmd = [nvcc, "-shared", "-o", LIB_PATH] + objs
+    cmd = [nvcc, "-shared", "-Xlinker", "-soname=libasuka_b200.so", "-o", LIB_PATH] + objs
     res = subprocess.run(cmd, capture_output=True, text=True)
     if res.returncode != 0:
       print(res.stdout + res.stderr, file=sys.stderr)
       raise RuntimeError("link failed")
+  _build_bind(nvcc, force)
   return LIB_PATH
+
+
+def _build_bind(nvcc, force):
+  """csrc/bind.cpp against torch's headers and the library above (found beside it at run time)."""
+  src = os.path.join(CSRC, "bind.cpp")
+  newest = max(os.path.getmtime(f) for f in (src, os.path.join(PKG_DIR, "..", "include", "asuka_b200.h")))
+  if not force and os.path.exists(BIND_PATH) and os.path.getmtime(BIND_PATH) > newest:
+    return
+  import torch
+  root = os.path.dirname(os.path.abspath(torch.__file__))
+  inc = os.path.join(root, "include")
+  cuda_inc = os.path.join(os.path.dirname(os.path.dirname(os.path.realpath(nvcc))), "include")
+  cmd = [shutil.which("g++") or "g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden", "-w",
+         f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+         f"-I{inc}", f"-I{os.path.join(inc, 'torch', 'csrc', 'api', 'include')}", f"-I{sysconfig.get_paths()['include']}",
+         f"-I{cuda_inc}", src, LIB_PATH, f"-L{os.path.join(root, 'lib')}", "-lc10", "-lc10_cuda", "-ltorch_cpu",
+         "-ltorch_cuda", "-ltorch_python", "-Wl,-rpath,$ORIGIN", "-o", BIND_PATH]
+  res = subprocess.run(cmd, capture_output=True, text=True)
+  if res.returncode != 0:
+    print(res.stdout + res.stderr, file=sys.stderr)
+    raise RuntimeError("building the native front end failed")
 
 
 if __name__ == "__main__":

@@ -46,7 +46,7 @@ class _Case:
     return self
 
   def _check(self, q):
-    if q.dim() == 4 and q.shape[2] != self.head_num:
+    if q.dim() == 4 and q.size(2) != self.head_num:
       raise RuntimeError(f"expected {self.head_num} heads, got {q.shape[2]}")
 
   def prepare(self, batch_size=1, q_len=4096, kv_len=4096, dtype=torch.float16, device=None):
