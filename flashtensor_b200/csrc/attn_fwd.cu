@@ -792,6 +792,7 @@ __global__ void __launch_bounds__(kMergeWarps * 32) attn_merge_kernel(const FwdP
 // S = 1024 to 4096: the partial results cost about as much L2 traffic again as the inputs); it
 // needs workspace for the parts' partial results.
 int attn_fwd_parts(const AttnShape& s, int num_sms, size_t ws_bytes) {
+  if (attn_decode_applies(s)) return 1;  // (attn_decode.cu splits the keys itself)
   const long long nq_blocks = (s.Sq + 2 * kTile - 1) / (2 * kTile);
   const long long n_items = nq_blocks * s.B * s.H;
   const int max_tiles = (s.Skv + kTile - 1) / kTile;

@@ -216,10 +216,15 @@ int attn_fwd_impl(const asuka_attn_params* p, float* lse_override, cudaStream_t 
     lse = static_cast<float*>(p->lse.ptr);
   }
   if ((r = check_arch()) != ASUKA_OK) return r;
-  CUtensorMap mq, mk, mv;
-  if ((r = make_map(&mq, p->q)) || (r = make_map(&mk, p->k)) || (r = make_map(&mv, p->v))) return r;
   const int sms = sm_count();
   if (sms <= 0) return ASUKA_ERR_CUDA;
+  CUtensorMap mq, mk, mv;
+  if (attn_decode_applies(c.s)) {
+    if ((r = make_map(&mk, p->k, 64)) || (r = make_map(&mv, p->v, 64))) return r;
+    return map_cuda(launch_attn_decode(mk, mv, p->q.ptr, p->q.stride[0], p->q.stride[1], p->q.stride[2], p->out.ptr,
+                                       p->out.stride[0], p->out.stride[1], p->out.stride[2], lse, c.s, sms, stream));
+  }
+  if ((r = make_map(&mq, p->q)) || (r = make_map(&mk, p->k)) || (r = make_map(&mv, p->v))) return r;
   size_t usable = 0;
   void* split_ws = align_ws(ws != nullptr ? ws : p->workspace, ws != nullptr ? ws_bytes : p->workspace_bytes, &usable);
   const int parts = attn_fwd_parts(c.s, sms, usable);

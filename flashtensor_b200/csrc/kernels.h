@@ -36,6 +36,27 @@ inline cudaError_t launch_dependent(void (*kernel)(Params...), dim3 grid, dim3 b
   return cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...);
 }
 
+// The same with thread-block clusters of `cluster` CTAs along x.
+template <typename... Params, typename... Args>
+inline cudaError_t launch_dependent_cluster(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem,
+                                            unsigned cluster, cudaStream_t stream, Args&&... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = cluster;
+  attr[1].val.clusterDim.y = 1;
+  attr[1].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 2;
+  return cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...);
+}
+
 struct AttnShape {
   int B, H, Sq, Skv;  // H: query heads
   int group;          // query heads per key/value head (1: multi-head attention)
@@ -55,6 +76,13 @@ cudaError_t launch_attn_fwd(const CUtensorMap& mq, const CUtensorMap& mk, const 
 // parts the key range is worth cutting into on `num_sms` SMs, limited by the workspace on offer
 int attn_fwd_parts(const AttnShape& s, int num_sms, size_t ws_bytes);
 size_t attn_fwd_split_bytes(const AttnShape& s, int parts);
+
+// Attention for a few query rows per key/value head (a decode step): K and V streamed once, all
+// query heads of a group together.  K and V maps with boxes of 64 rows.
+bool attn_decode_applies(const AttnShape& s);
+cudaError_t launch_attn_decode(const CUtensorMap& mk, const CUtensorMap& mv, const void* q, int64_t q_sb, int64_t q_ss,
+                               int64_t q_sh, void* out, int64_t o_sb, int64_t o_ss, int64_t o_sh, float* lse2,
+                               const AttnShape& s, int num_sms, cudaStream_t stream);
 
 struct ScoreArgs {
   const float* lse2;       // [B,H,Sq]

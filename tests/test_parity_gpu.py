@@ -164,6 +164,36 @@ def test_long_sequences_with_few_heads_vs_oracle(ops, shape):
 
 
 @pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("shape", [
+    # B, Sq, Skv, H, Hkv, causal: rows of a key/value head Sq * H / Hkv of 1 to 16, one above; keys
+    # around the 64-key stages and the cuts into parts
+    (1, 1, 63, 1, 1, True), (2, 1, 64, 2, 2, True), (1, 4, 65, 8, 2, True), (1, 16, 16, 1, 1, True),
+    (3, 2, 257, 6, 3, True), (1, 1, 4097, 8, 1, True), (40, 1, 700, 16, 8, True), (1, 3, 1000, 10, 2, False),
+    (1, 17, 400, 1, 1, True), (2, 5, 300, 4, 1, True),
+])
+def test_few_query_rows_vs_oracle(ops, shape, dtype):
+  B, Sq, Skv, H, Hkv, causal = shape
+  g = torch.Generator().manual_seed(Skv)
+  q = torch.randn(B, Sq, H, 128, generator=g).to(dtype)
+  k, v = (torch.randn(B, Skv, Hkv, 128, generator=g).to(dtype) for _ in range(2))
+  ref_out, ref_score = O.h2o_gqa(q, k, v, causal)
+  qd, kd, vd = q.cuda(), k.cuda(), v.cuda()
+  out, lse = ops.attn_fwd(qd, kd, vd, causal=causal, return_lse=True)
+  out2, score = ops.h2o(qd, kd, vd, causal=causal)
+  close(out, ref_out, "out")
+  close(score, ref_score, "score")
+  assert torch.equal(out, out2) and torch.equal(out, ops.attn_fwd(qd, kd, vd, causal=causal))
+  ke = k.float()[:, :, :, None].expand(-1, -1, -1, H // Hkv, -1).reshape(B, Skv, H, 128)
+  s = torch.einsum("bqhd,bkhd->bhqk", q.float(), ke) / 128 ** 0.5
+  if causal:
+    s = s + torch.triu(torch.full((Sq, Skv), float("-inf")), diagonal=Skv - Sq + 1)
+  torch.testing.assert_close(lse.cpu(), torch.logsumexp(s, -1) * 1.4426950408889634, rtol=1e-4, atol=2e-3)
+  ve = v.float()[:, :, :, None].expand(-1, -1, -1, H // Hkv, -1).reshape(B, Skv, H, 128)
+  close(ops.attn_fwd(qd, kd, vd, causal=causal, softcap=2.0), O.gemma2(q, ke, ve, 2.0, causal), "soft-capped out")
+  no_timeouts(ops)
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
 @pytest.mark.parametrize("shape", [(1, 384, 384, 2), (2, 1000, 1000, 3), (1, 200, 456, 2)])
 def test_roco_vs_oracle(ops, shape, dtype):
   B, Sq, Skv, H = shape
