@@ -4,10 +4,11 @@
 a fused QKV projection with bias (lines 3-5), split into heads of 32 features (lines 6-12), the
 linear-attention core (lines 13-17), and the output projection with bias (lines 18-22).
 
-The two projections are plain GEMMs with a bias and go to cuBLAS through ``torch.addmm``; the
-split / reshape / transpose between them and the core cost nothing, because the core kernel reads
-q, k, v as strided views of the projection's output and writes the layout the output projection
-reads.  The core is this library's kernel (``ops.linattn32_fwd``); there is no other path.
+Up to C = 128 (the files' own width) all of it is this library's: ``ops.linattn_block``, whose
+projections run with f32 accuracy on the tensor pipe.  Wider blocks send the two projections, plain
+GEMMs with a bias, to cuBLAS through ``torch.addmm``.  The split / reshape / transpose between the
+projections and the core cost nothing, because the core kernel reads q, k, v as strided views of the
+projection's output and writes the layout the output projection reads.
 """
 import torch
 
@@ -29,6 +30,8 @@ class LinearAttentionBlock:
     if C % HEAD_DIM or tuple(w_qkv.shape) != (3 * C, C) or tuple(b_qkv.shape) != (3 * C,) or \
        tuple(w_o.shape) != (C, C) or tuple(b_o.shape) != (C,):
       raise RuntimeError("expected w_qkv [3C, C], b_qkv [3C], w_o [C, C], b_o [C] with C a multiple of 32")
+    if C <= ops.LINEAR_MAX_K:
+      return ops.linattn_block(x, w_qkv, b_qkv, w_o, b_o, ea=self.ea)
     H = C // HEAD_DIM
     qkv = torch.addmm(b_qkv, x.reshape(B * N, C), w_qkv.t()).view(B, N, 3, H, HEAD_DIM)
     core = ops.linattn32_fwd(qkv[:, :, 0], qkv[:, :, 1], qkv[:, :, 2], ea=self.ea)   # [B, N, H, 32]

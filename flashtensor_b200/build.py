@@ -16,7 +16,7 @@ OBJ_DIR = os.path.join(PKG_DIR, "build")
 LIB_PATH = os.path.join(PKG_DIR, "libasuka_b200.so")
 BIND_PATH = os.path.join(PKG_DIR, "_bind.so")
 
-SOURCES = ["capi.cu", "attn_fwd.cu", "attn_decode.cu", "col_scores.cu", "select_topk.cu", "score_ops.cu", "sima.cu", "linattn32.cu"]
+SOURCES = ["capi.cu", "attn_fwd.cu", "attn_decode.cu", "col_scores.cu", "select_topk.cu", "score_ops.cu", "sima.cu", "linattn32.cu", "linear_f32.cu"]
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a", "-O3", "-lineinfo", "-std=c++17",
     "-Xcompiler", "-fPIC", "--use_fast_math", "-Xptxas", "-v",

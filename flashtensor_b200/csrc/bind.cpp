@@ -320,6 +320,64 @@ PyObject* linattn32_fwd(PyObject*, PyObject* const* a, Py_ssize_t n) {
   END_HANDLE_TH_ERRORS
 }
 
+// x w^T + bias into a new [M, N] tensor
+at::Tensor linear_f32(const at::Tensor& x, const at::Tensor& w, const at::Tensor& bias, asuka_stream stream) {
+  const at::Tensor out = empty({x.size(0), w.size(0)}, at::kFloat, x);
+  asuka_linear_params p;
+  p.x = desc(x);
+  p.w = desc(w);
+  p.bias = desc(bias);
+  p.out = desc(out);
+  call("asuka_b200_linear_f32", [&] { return asuka_b200_linear_f32(&p, stream); });
+  return out;
+}
+
+// (x [M, K], w [N, K], bias [N]) -> out [M, N]
+PyObject* linear(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  HANDLE_TH_ERRORS
+  try {
+    want_args(n, 3);
+    const at::Tensor &x = tensor_arg(a[0]), &w = tensor_arg(a[1]), &bias = tensor_arg(a[2]);
+    OnDevice on({&x, &w, &bias});
+    return wrap(linear_f32(x, w, bias, on.stream));
+  } catch (const BadArg&) {
+    return nullptr;
+  }
+  END_HANDLE_TH_ERRORS
+}
+
+// The whole block of bench/sima.mlir / bench/ea.mlir: (x [B, N, C], w_qkv, b_qkv, w_o, b_o, ea) -> [B, N, C];
+// the core reads q, k, v as strided views of the projection's output [B*N, 3, C/32, 32].
+PyObject* linattn_block(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  HANDLE_TH_ERRORS
+  try {
+    want_args(n, 6);
+    const at::Tensor x = tensor_arg(a[0]).contiguous(), w_qkv = tensor_arg(a[1]).contiguous(),
+                     b_qkv = tensor_arg(a[2]).contiguous(), w_o = tensor_arg(a[3]).contiguous(),
+                     b_o = tensor_arg(a[4]).contiguous();
+    OnDevice on({&x, &w_qkv, &b_qkv, &w_o, &b_o});
+    const int64_t B = x.size(0), N = x.size(1), C = x.size(2);
+    const at::Tensor qkv = linear_f32(x.view({B * N, C}), w_qkv, b_qkv, on.stream);
+    const at::Tensor core = empty({B, N, C / 32, 32}, at::kFloat, x);
+    asuka_linattn32_params p;
+    p.out = desc(core);
+    p.q = p.out;  // the same shape, strided over the fused rows
+    p.q.ptr = qkv.data_ptr();
+    p.q.stride[0] = N * 3 * C;
+    p.q.stride[1] = 3 * C;
+    p.k = p.q;
+    p.k.ptr = static_cast<float*>(p.q.ptr) + C;
+    p.v = p.q;
+    p.v.ptr = static_cast<float*>(p.q.ptr) + 2 * C;
+    p.ea = bool_arg(a[5]) ? 1 : 0;
+    call("asuka_b200_linattn32_fwd", [&] { return asuka_b200_linattn32_fwd(&p, on.stream); });
+    return wrap(linear_f32(core.view({B * N, C}), w_o, b_o, on.stream).view({B, N, C}));
+  } catch (const BadArg&) {
+    return nullptr;
+  }
+  END_HANDLE_TH_ERRORS
+}
+
 // (score, kernel_size) -> pooled score
 PyObject* pool_scores(PyObject*, PyObject* const* a, Py_ssize_t n) {
   HANDLE_TH_ERRORS
@@ -436,6 +494,7 @@ PyObject* select_topk(PyObject*, PyObject* const* a, Py_ssize_t n) {
 #define ENTRY(f) {#f, reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(f)), METH_FASTCALL, nullptr}
 PyMethodDef g_methods[] = {ENTRY(attn_fwd),    ENTRY(run_case),  ENTRY(linear_fwd), ENTRY(linattn32_fwd),
                            ENTRY(pool_scores), ENTRY(gather_kv), ENTRY(col_scores), ENTRY(select_topk),
+                           ENTRY(linear),      ENTRY(linattn_block),
                            {nullptr, nullptr, 0, nullptr}};
 PyModuleDef g_module = {PyModuleDef_HEAD_INIT, "_bind", nullptr, -1, g_methods, nullptr, nullptr, nullptr, nullptr};
 

@@ -462,6 +462,7 @@ size_t case_split_bytes(const asuka_case_params* p, CaseKind kind) {
   s.Sq = static_cast<int>(p->q.shape[1]);
   s.H = static_cast<int>(p->q.shape[2]);
   s.Skv = static_cast<int>(p->k.shape[1]);
+  s.group = p->k.shape[2] > 0 ? static_cast<int>(p->q.shape[2] / p->k.shape[2]) : 1;
   const int mode = kind == CASE_H2O ? ASUKA_SCORE_SUM : kind == CASE_ROCO ? ASUKA_SCORE_SUM_SQ : ASUKA_SCORE_PERTURBED;
   const size_t fwd = attn_fwd_split_bytes(s, attn_fwd_parts(s, sms, ~static_cast<size_t>(0)));
   const size_t col = col_scores_split_bytes(s, mode, col_scores_chunks(s, mode, sms, ~static_cast<size_t>(0)));
@@ -756,6 +757,28 @@ int asuka_b200_linattn32_fwd(const asuka_linattn32_params* p, asuka_stream strea
   a.v_sb = p->v.stride[0]; a.v_sn = p->v.stride[1]; a.v_sh = p->v.stride[2];
   a.o_sb = p->out.stride[0]; a.o_sn = p->out.stride[1]; a.o_sh = p->out.stride[2];
   return map_cuda(launch_linattn32(a, static_cast<cudaStream_t>(stream)));
+}
+
+int asuka_b200_linear_f32(const asuka_linear_params* p, asuka_stream stream) {
+  if (p == nullptr) return ASUKA_ERR_NULL_POINTER;
+  if (p->x.ptr == nullptr || p->w.ptr == nullptr) return ASUKA_ERR_NULL_POINTER;
+  if (p->x.ndim != 2 || p->w.ndim != 2) return ASUKA_ERR_BAD_SHAPE;
+  const int64_t M = p->x.shape[0], K = p->x.shape[1], N = p->w.shape[0];
+  if (M <= 0 || N <= 0 || K <= 0 || K % 8 != 0) return ASUKA_ERR_BAD_SHAPE;
+  if (K > ASUKA_LINEAR_MAX_K || M > 0x3fffffff || N > (1 << 14)) return ASUKA_ERR_TOO_LARGE;
+  const int64_t xs[2] = {M, K}, ws[2] = {N, K}, bs[1] = {N}, os[2] = {M, N};
+  int r;
+  if ((r = check_dense(p->x, ASUKA_F32, 2, xs)) != ASUKA_OK) return r;
+  if ((r = check_dense(p->w, ASUKA_F32, 2, ws)) != ASUKA_OK) return r;
+  if ((r = check_dense(p->bias, ASUKA_F32, 1, bs)) != ASUKA_OK) return r;
+  if ((r = check_dense(p->out, ASUKA_F32, 2, os)) != ASUKA_OK) return r;
+  if ((r = check_arch()) != ASUKA_OK) return r;
+  const int sms = sm_count();
+  if (sms <= 0) return ASUKA_ERR_CUDA;
+  return map_cuda(launch_linear_f32(static_cast<const float*>(p->x.ptr), static_cast<const float*>(p->w.ptr),
+                                    static_cast<const float*>(p->bias.ptr), static_cast<float*>(p->out.ptr),
+                                    static_cast<int>(M), static_cast<int>(N), static_cast<int>(K), sms,
+                                    static_cast<cudaStream_t>(stream)));
 }
 
 int asuka_b200_gather_kv(const asuka_gather_params* p, asuka_stream stream) {

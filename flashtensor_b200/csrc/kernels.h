@@ -165,6 +165,10 @@ struct LinAttn32Args {
 };
 cudaError_t launch_linattn32(const LinAttn32Args& a, cudaStream_t stream);
 
+// out[M, N] = x[M, K] w[N, K]^T + bias[N], contiguous f32, K a multiple of 8 and at most 128
+cudaError_t launch_linear_f32(const float* x, const float* w, const float* bias, float* out, int M, int N, int K,
+                              int num_sms, cudaStream_t stream);
+
 struct SimaShape {
   int B, H, S;
   bool bf16;

@@ -1,0 +1,335 @@
+// out[M, N] = x[M, K] w[N, K]^T + bias[N] in f32, for the projections around the linear-attention
+// core of the reference's SimA and EA benchmark programs (bench/sima.mlir:3-5,18-22: f32, C = 128).
+//
+// f32 accuracy on the bf16 tensor pipe: every operand is split into three bf16 terms,
+// x = h + m + l (8 significant bits each, what is left out is below 2^-26 |x|), and the six
+// products h.h, h.m, m.h, m.m, h.l, l.h are accumulated in f32 in TMEM; the dropped ones are below
+// 2^-26 of |x||w|, under the rounding of an f32 product.  The CUDA cores' 74 TFLOP/s would need
+// 66 us for the 4.9 GFLOP of the QKV projection at B64 N784 C128; six bf16 products at the tensor
+// pipe's rate need 15, and the 103 MB it moves 16.
+//
+// One persistent CTA per SM owns a block of 128 output columns and walks tiles of 128 rows of x.  The
+// product is formed transposed, out^T = w x^T: the split weights are the A operand and stay in TMEM
+// for the whole kernel, so the MMAs read only the x tile from shared memory (with both operands
+// there, a 128 x 128 MMA takes all of its bandwidth and the warps that write the next tile stall:
+// 38 us instead of the figure below), and an accumulator lane is an output column, so a warp's store
+// is one 128-byte line of an output row.
+//   warps 0-7    load x (a whole tile ahead), split it and store the three terms as swizzled K-major tiles
+//   warp 8       issues tcgen05.mma into one of two accumulators
+//   warps 9-12   split the weights into TMEM; then accumulator + bias to global memory
+// The small products of a tile are accumulated before any h.h: the tensor pipe truncates when it adds
+// to an accumulator, and forty small terms added to a large sum would each leave a bias there
+// (measured at K = 128: 4.1e-7 relative error in the natural order, against 1.5e-7 of an f32 GEMM on
+// the CUDA cores).
+// Measured at B64 N784 C128 (M = 50176, K = 128), bias included: N = 384 (QKV) 32 us, N = 128 (output)
+// 15 us; the f32 GEMM of the BLAS library with its bias pass takes 200 and 64.
+#include <cuda_bf16.h>
+
+#include "kernels.h"
+#include "sm100_ptx.cuh"
+#include "tma_host.h"
+
+namespace asuka {
+using namespace sm100;
+
+namespace {
+
+constexpr int kTile = 128;               // rows of x and output columns of a tile
+constexpr int kMaxK = 128;
+constexpr int kChunk = 64;               // reduction columns of one 128-byte swizzled row of bf16
+constexpr uint32_t kTermBytes = kTile * kChunk * 2;  // one bf16 term of a [128 x 64] piece
+constexpr uint32_t kPieceBytes = 3 * kTermBytes;
+constexpr uint32_t kStageBytes = (kMaxK / kChunk) * kPieceBytes;  // a tile of x: 96 KB
+constexpr int kSplitWarps = 8;
+constexpr int kThreads = (kSplitWarps + 1 + 4) * 32;
+constexpr uint32_t kOutBytes = 32 * 32 * 4;                       // one TMA store of a warp: 32 rows x 32 columns
+constexpr uint32_t kSmemBytes = 2 * kStageBytes + 4 * 2 * kOutBytes + 1024;
+constexpr uint32_t kTermCols = kMaxK / 2;  // TMEM columns of one term of the weights
+constexpr uint32_t kAccCol = 3 * kTermCols;
+
+struct LinParams {
+  const float* x;
+  const float* w;
+  const float* bias;
+  float* out;
+  int M, N, K;
+  int m_tiles, n_tiles, chunks;
+  int tma_out;  // rows of `out` can be described to TMA (N a multiple of 4)
+  uint32_t* status;
+};
+
+struct LinBars {
+  uint64_t x_full[2], x_empty[2];
+  uint64_t acc_full[2], acc_empty[2];
+};
+
+__device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
+  __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
+  return *reinterpret_cast<uint32_t*>(&v);
+}
+// eight f32 values to their three bf16 terms, eight values in 16 bytes each
+__device__ __forceinline__ void split8(const float (&v)[8], uint4 (&t)[3]) {
+  uint32_t w[3][4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    float a = v[2 * i], b = v[2 * i + 1];
+#pragma unroll
+    for (int s = 0; s < 3; ++s) {
+      const uint32_t p = pack_bf16(a, b);
+      w[s][i] = p;
+      const float ra = __uint_as_float(p << 16), rb = __uint_as_float(p & 0xffff0000u);
+      a -= ra;  // (exact; infinite values leave NaN, so a row with one gives NaN)
+      b -= rb;
+    }
+  }
+#pragma unroll
+  for (int s = 0; s < 3; ++s) t[s] = make_uint4(w[s][0], w[s][1], w[s][2], w[s][3]);
+}
+
+__device__ __forceinline__ void record_timeout(uint32_t* status, uint32_t site) {
+  atomicAdd(&status[0], 1u);
+  status[1] = site;
+}
+
+__global__ void __launch_bounds__(kThreads, 1) linear_f32_kernel(const __grid_constant__ CUtensorMap map_out, const LinParams p) {
+  extern __shared__ uint8_t smem_raw[];
+  __shared__ __align__(8) LinBars bars;
+  __shared__ uint32_t tmem_base_s;
+  __shared__ uint32_t abort_s;
+  const uint32_t sX = (smem_u32(smem_raw) + 1023u) & ~1023u;
+  uint8_t* const gX = smem_raw + (sX - smem_u32(smem_raw));
+
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  volatile uint32_t* abortp = &abort_s;
+  // CTAs are dealt out over the column blocks; those of one block share its row tiles
+  const int nb = static_cast<int>(blockIdx.x) % p.n_tiles;
+  const int m_first = static_cast<int>(blockIdx.x) / p.n_tiles;
+  const int m_step = (static_cast<int>(gridDim.x) - nb + p.n_tiles - 1) / p.n_tiles;  // CTAs of this column block
+  const int n0 = nb * kTile;
+
+  if (tid == 0) {
+    abort_s = 0;
+    for (int i = 0; i < 2; ++i) {
+      mbar_init(smem_u32(&bars.x_full[i]), kSplitWarps * 32);
+      mbar_init(smem_u32(&bars.x_empty[i]), 1);
+      mbar_init(smem_u32(&bars.acc_full[i]), 1);
+      mbar_init(smem_u32(&bars.acc_empty[i]), 128);
+    }
+    mbar_fence_init();
+  }
+  if (warp == kSplitWarps) {
+    __syncwarp();
+    tmem_alloc(smem_u32(&tmem_base_s), 512);
+    tmem_relinquish();
+  }
+  tc_fence_before_sync();
+  __syncthreads();
+  tc_fence_after_sync();
+  const uint32_t tbase = tmem_base_s;
+  const int wq = warp & 3;  // (epilogue warps) TMEM lane quarter
+  const uint32_t lane_base = static_cast<uint32_t>(wq * 32) << 16;
+  const int n = n0 + wq * 32 + lane;  // (epilogue warps) this thread's output column
+  griddep_wait();
+  griddep_launch_dependents();
+  if (warp > kSplitWarps) {
+    // the weights of this block of columns, split once: thread = output column = TMEM lane
+    const float* src = p.w + static_cast<int64_t>(min(n, p.N - 1)) * p.K;
+    for (int k0 = 0; k0 < p.chunks * kChunk; k0 += 32) {
+      uint32_t t[3][16];
+#pragma unroll
+      for (int g = 0; g < 4; ++g) {
+        const int k = k0 + g * 8;
+        const bool live = n < p.N && k < p.K;  // (K is a multiple of 8)
+        const float4 lo = live ? __ldg(reinterpret_cast<const float4*>(src + k)) : make_float4(0.f, 0.f, 0.f, 0.f);
+        const float4 hi = live ? __ldg(reinterpret_cast<const float4*>(src + k + 4)) : make_float4(0.f, 0.f, 0.f, 0.f);
+        const float v[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
+        uint4 q[3];
+        split8(v, q);
+#pragma unroll
+        for (int s = 0; s < 3; ++s) {
+          t[s][g * 4 + 0] = q[s].x;
+          t[s][g * 4 + 1] = q[s].y;
+          t[s][g * 4 + 2] = q[s].z;
+          t[s][g * 4 + 3] = q[s].w;
+        }
+      }
+#pragma unroll
+      for (int s = 0; s < 3; ++s) tmem_st16(tbase + lane_base + s * kTermCols + k0 / 2, t[s]);
+    }
+    tmem_wait_st();
+  }
+  tc_fence_before_sync();
+  __syncthreads();
+  tc_fence_after_sync();
+
+  if (warp < kSplitWarps) {
+    // ------------------------------------------------------------------ load and split x
+    // A thread takes 8 columns (32 bytes) of four rows of every 64-column piece; eight threads cover
+    // a row's 256 bytes.  The next tile's loads are in flight while this one is split.
+    const int c = tid & 7, row0 = tid >> 3;  // rows row0, +32, +64, +96
+    float4 v[2][4][2];
+    auto fetch = [&](int mt) {
+#pragma unroll
+      for (int ch = 0; ch < 2; ++ch) {
+        const int k = ch * kChunk + c * 8;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const int row = mt * kTile + row0 + i * 32;
+          const bool live = row < p.M && k < p.K;
+          const float4* src = reinterpret_cast<const float4*>(p.x + static_cast<int64_t>(row) * p.K + k);
+          v[ch][i][0] = live ? __ldg(src) : make_float4(0.f, 0.f, 0.f, 0.f);
+          v[ch][i][1] = live ? __ldg(src + 1) : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+      }
+    };
+    uint32_t t = 0;
+    if (m_first < p.m_tiles) fetch(m_first);
+    for (int mt = m_first; mt < p.m_tiles; mt += m_step, ++t) {
+      const int st = t & 1;
+      if (t >= 2 && !mbar_wait(smem_u32(&bars.x_empty[st]), ((t >> 1) - 1) & 1, abortp)) {
+        if (lane == 0) record_timeout(p.status, 81);
+        break;
+      }
+#pragma unroll
+      for (int ch = 0; ch < 2; ++ch) {
+        if (ch < p.chunks) {
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            const float4 lo = v[ch][i][0], hi = v[ch][i][1];
+            const float e[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
+            uint4 q[3];
+            split8(e, q);
+#pragma unroll
+            for (int s = 0; s < 3; ++s)
+              *reinterpret_cast<uint4*>(gX + st * kStageBytes + ch * kPieceBytes + s * kTermBytes +
+                                        sw128_offset(row0 + i * 32, c)) = q[s];
+          }
+        }
+      }
+      if (mt + m_step < p.m_tiles) fetch(mt + m_step);
+      fence_proxy_async_smem();
+      mbar_arrive(smem_u32(&bars.x_full[st]));
+    }
+  } else if (warp == kSplitWarps) {
+    // ------------------------------------------------------------------ MMA issuer
+    constexpr uint32_t idesc = umma_idesc_f16(UMMA_BF16, UMMA_K_MAJOR, UMMA_K_MAJOR, 128, 128);
+    auto wait_all = [&](uint64_t* bar, uint32_t parity, uint32_t site) -> bool {
+      const bool good = __all_sync(0xffffffffu, mbar_wait(smem_u32(bar), parity, abortp));
+      if (!good && lane == 0) record_timeout(p.status, site);
+      return good;
+    };
+    uint32_t t = 0;
+    for (int mt = m_first; mt < p.m_tiles; mt += m_step, ++t) {
+      const int st = t & 1;
+      if (t >= 2 && !wait_all(&bars.acc_empty[st], ((t >> 1) - 1) & 1, 82)) break;
+      if (!wait_all(&bars.x_full[st], (t >> 1) & 1, 83)) break;
+      tc_fence_after_sync();
+      if (elect_one()) {
+        constexpr int kW[6] = {2, 0, 1, 1, 0, 0}, kX[6] = {0, 2, 1, 0, 1, 0};
+        const uint32_t acc = tbase + kAccCol + st * 128;
+#pragma unroll
+        for (int pr = 0; pr < 6; ++pr) {
+          for (int ch = 0; ch < p.chunks; ++ch) {
+            const uint64_t xd =
+                umma_smem_desc_sw128(sX + st * kStageBytes + ch * kPieceBytes + kX[pr] * kTermBytes, 16, 1024);
+            const uint32_t wt = tbase + kW[pr] * kTermCols + ch * (kChunk / 2);
+#pragma unroll
+            for (int kk = 0; kk < 4; ++kk)
+              umma_ts(acc, wt + kk * 8, xd + kk * 2, idesc, (pr > 0 || ch > 0 || kk > 0) ? 1u : 0u);
+          }
+        }
+        umma_commit(smem_u32(&bars.x_empty[st]));
+        umma_commit(smem_u32(&bars.acc_full[st]));
+      }
+      __syncwarp();
+    }
+  } else {
+    // ------------------------------------------------------------------ epilogue
+    uint8_t* const stage = gX + 2 * kStageBytes + wq * 2 * kOutBytes;
+    const float bias = n < p.N ? __ldg(p.bias + n) : 0.f;
+    uint32_t t = 0;
+    for (int mt = m_first; mt < p.m_tiles; mt += m_step, ++t) {
+      const int st = t & 1;
+      if (!__all_sync(0xffffffffu, mbar_wait(smem_u32(&bars.acc_full[st]), (t >> 1) & 1, abortp))) {
+        if (lane == 0) record_timeout(p.status, 84);
+        break;
+      }
+      tc_fence_after_sync();
+      const int row_t = mt * kTile;
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        uint32_t u[32];
+        tmem_ld32(tbase + lane_base + kAccCol + st * 128 + q * 32, u);
+        uint8_t* const dst = stage + (q & 1) * kOutBytes;
+        if (lane == 0) tma_store_wait_read_n<1>();  // the store before last has left this half of the stage
+        __syncwarp();
+        tmem_wait_ld();
+        if (q == 3) {
+          tc_fence_before_sync();
+          mbar_arrive(smem_u32(&bars.acc_empty[st]));
+        }
+#pragma unroll
+        for (int r = 0; r < 32; ++r)
+          *reinterpret_cast<float*>(dst + sw128_offset(r, lane >> 2) + (lane & 3) * 4) = __uint_as_float(u[r]) + bias;
+        const int row_q = row_t + q * 32;
+        if (p.tma_out) {
+          fence_proxy_async_smem();
+          __syncwarp();
+          if (lane == 0) {
+            if (row_q < p.M && n < p.N) tma_store_4d(&map_out, smem_u32(dst), n, row_q, 0, 0);  // (lane 0: n is the block's first column)
+            tma_store_commit();
+          }
+        } else if (n < p.N) {  // (a thread reads back only what it wrote)
+          for (int r = 0; r < 32 && row_q + r < p.M; ++r)
+            p.out[static_cast<int64_t>(row_q + r) * p.N + n] =
+                *reinterpret_cast<const float*>(dst + sw128_offset(r, lane >> 2) + (lane & 3) * 4);
+        }
+      }
+    }
+    if (lane == 0) tma_store_wait_all();
+    __syncwarp();
+  }
+  tc_fence_before_sync();
+  __syncthreads();
+  if (warp == kSplitWarps) {
+    __syncwarp();
+    tmem_dealloc(tbase, 512);
+  }
+}
+
+}  // namespace
+
+cudaError_t launch_linear_f32(const float* x, const float* w, const float* bias, float* out, int M, int N, int K,
+                              int num_sms, cudaStream_t stream) {
+  LinParams p;
+  p.x = x;
+  p.w = w;
+  p.bias = bias;
+  p.out = out;
+  p.M = M;
+  p.N = N;
+  p.K = K;
+  p.m_tiles = (M + kTile - 1) / kTile;
+  p.n_tiles = (N + kTile - 1) / kTile;
+  p.chunks = (K + kChunk - 1) / kChunk;
+  p.status = device_status_words();
+  p.tma_out = N % 4 == 0 ? 1 : 0;
+  CUtensorMap mo = {};
+  if (p.tma_out) {
+    const uint64_t row_bytes = static_cast<uint64_t>(N) * 4;
+    const uint64_t dims[4] = {static_cast<uint64_t>(N), static_cast<uint64_t>(M), 1, 1};
+    const uint64_t strides[3] = {row_bytes, row_bytes, row_bytes};
+    const uint32_t box[4] = {32, 32, 1, 1};
+    if (tma_host::make_f32_map_sw128(&mo, out, dims, strides, box) != 0) return cudaErrorInvalidValue;
+  }
+  const int64_t tiles = static_cast<int64_t>(p.m_tiles) * p.n_tiles;
+  const int64_t most = num_sms > p.n_tiles ? num_sms : p.n_tiles;  // (every column block needs a CTA)
+  const unsigned grid = static_cast<unsigned>(tiles < most ? tiles : most);
+  cudaError_t e = ensure_dynamic_smem(reinterpret_cast<const void*>(linear_f32_kernel), kSmemBytes);
+  if (e != cudaSuccess) return e;
+  e = launch_dependent(linear_f32_kernel, dim3(grid), dim3(kThreads), kSmemBytes, stream, mo, p);
+  count_launch();
+  return e;
+}
+
+}  // namespace asuka

@@ -159,6 +159,21 @@ def linattn32_fwd(q, k, v, ea=False, out=None):
   return _bind().linattn32_fwd(q, k, v, ea, out)
 
 
+def linear_f32(x, w, bias):
+  """x w^T + bias with f32 accuracy on the tensor pipe: x [M, K], w [N, K], bias [N] -> [M, N], f32,
+  contiguous, K a multiple of 8 and at most LINEAR_MAX_K."""
+  return _bind().linear(x, w, bias)
+
+
+LINEAR_MAX_K = 128
+
+
+def linattn_block(x, w_qkv, b_qkv, w_o, b_o, ea=False):
+  """The whole block of bench/sima.mlir (ea=False) or bench/ea.mlir (ea=True), f32: QKV projection,
+  core, output projection in three launches.  x [B, N, C], C a multiple of 32 and at most LINEAR_MAX_K."""
+  return _bind().linattn_block(x, w_qkv, b_qkv, w_o, b_o, ea)
+
+
 _H2O, _ROCO, _KEYFORMER = 0, 1, 2   # case kinds of the native front end
 
 

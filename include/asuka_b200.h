@@ -211,6 +211,16 @@ typedef struct {
 } asuka_linattn32_params;
 int asuka_b200_linattn32_fwd(const asuka_linattn32_params* p, asuka_stream stream);
 
+/* ---- the projections around that core (bench/sima.mlir:3-5,18-22): out = x w^T + bias in f32 -------
+ * x [M, K], w [N, K], bias [N], out [M, N], f32, contiguous; K a multiple of 8, at most
+ * ASUKA_LINEAR_MAX_K.  The result has f32 accuracy (products of three-term bf16 splits on the tensor
+ * pipe, f32 accumulation). */
+#define ASUKA_LINEAR_MAX_K 128
+typedef struct {
+  asuka_tensor x, w, bias, out;
+} asuka_linear_params;
+int asuka_b200_linear_f32(const asuka_linear_params* p, asuka_stream stream);
+
 /* ---- fused cases: forward + column scores (+ selection) enqueued back to back on one stream.
  *      `workspace` holds the row statistics between the kernels: two arrays of B*H*Sq floats
  *      (unperturbed and Keyformer's perturbed one), each rounded up to 256 bytes, plus, when k

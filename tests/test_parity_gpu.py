@@ -343,6 +343,23 @@ def test_ea_keys_that_grow_along_the_sequence(ops, shape, dtype):
   no_timeouts(ops)
 
 
+@pytest.mark.parametrize("shape", [(1, 8, 8), (129, 97, 40), (128, 384, 128), (1000, 128, 64), (77, 130, 128), (40000, 96, 32)])
+def test_f32_projection_vs_float64(ops, shape):
+  # tile edges in rows and columns, both reduction lengths of a tile, more row tiles than CTAs; f32
+  # bound: K products rounded and added in f32, each step at most one unit of 2^-23 of sum |x||w|
+  M, N, K = shape
+  g = torch.Generator().manual_seed(M + N)
+  x, w, b = torch.randn(M, K, generator=g), torch.randn(N, K, generator=g), torch.randn(N, generator=g)
+  got = ops.linear_f32(x.cuda(), w.cuda(), b.cuda()).cpu().double()
+  ref = x.double() @ w.double().t() + b.double()
+  bound = (K + 2) * 2.0 ** -23 * (x.double().abs() @ w.double().abs().t() + b.double().abs())
+  assert ((got - ref).abs() <= bound).all()
+  x[0, 0] = float("inf")   # (spreads to its own row only)
+  bad = ops.linear_f32(x.cuda(), w.cuda(), b.cuda()).cpu()
+  assert not torch.isfinite(bad[0]).any() and torch.equal(bad[1:].double(), got[1:])
+  no_timeouts(ops)
+
+
 @pytest.mark.parametrize("ea", [False, True])
 def test_linear_attention_blocks_at_the_reference_bench_shapes(ops, ea):
   # bench/sima.mlir / bench/ea.mlir: x [B, 784, 128] f32, 4 heads of 32; B reduced from 64 for the CPU oracle
