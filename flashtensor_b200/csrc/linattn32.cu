@@ -6,28 +6,54 @@
 //   EA    out = softmax_d(Q)   . (softmax_n(K)^T . V)
 //
 // With 32 features the two products are 2 flops per byte moved, far too few for tensor-core tiles:
-// plain CUDA-core code with coalesced accesses.  One CTA per (batch, head); every warp streams
-// rows n = w, w + 8, ... of the [N, 32] slices with lane = feature (one 128-byte row per load,
-// sixteen rows in flight), three times: column statistics, the 32 x 32 product K'^T V, then the
-// output rows.  In the two products a lane keeps one column of the 32 x 32 matrix in registers and
-// the other operand's row is broadcast through a per-warp shared-memory buffer with 16-byte loads;
-// the multiply-adds are the packed two-wide f32 FMAs of sm_100.  Every sum runs in a fixed order,
-// so results are reproducible.  What bounds it is the latency of the row loads: a (batch, head) is
-// one dependent chain of three passes, and 256 of them give a B200 only 16 warps per SM, each one
-// step of eight rows ahead.  Splitting a (batch, head) over a cluster of 2 or 4 CTAs was measured
-// and is slower.
+// CUDA-core code, bound by how much of the [N, 32] slices (one 128-byte line per row and tensor) is
+// in flight.  One CTA per (batch, head), two to an SM; every tile of 64 rows comes and goes by TMA:
+//   pass A  K, V (and SimA's Q) through a ring of four stages; eight warps take eight rows of a
+//           stage each.  A lane keeps an 8 x 4 block of the 32 x 32 product K'^T V in registers, so a
+//           row costs it three 16-byte reads of shared memory (a whole column per lane needs eight
+//           for K's row alone, and shared memory was what the kernel waited for).  The statistics are gathered on the way: SimA's
+//           sums of |K| and |Q|; for EA each warp exponentiates K in place against a running
+//           reference of its own per column, raised (with its partial product rescaled) only when
+//           a value exceeds it by more than 8, so no pass over K precedes the product.
+//   pass B  Q through a ring of eight tiles; the output row is written over the row of Q it came
+//           from and leaves by TMA.
+// Multiply-adds are the packed two-wide f32 FMAs of sm_100; every sum runs in a fixed order.
+// Measured at B64 H4 N784 (SimA / EA): three passes of plain loads with sixteen rows of a warp in
+// flight 58 / 67 us, this kernel 37 / 47 us.
 #include "kernels.h"
+#include "sm100_ptx.cuh"
+#include "tma_host.h"
 
 namespace asuka {
+using namespace sm100;
+
 namespace {
 
 constexpr int kD = 32;
 constexpr int kWarps = 8;
-constexpr int kUnroll = 8;  // rows of a warp per step (twice as many are in flight)
+constexpr int kThreads = (kWarps + 1) * 32;  // + the producer warp
+constexpr int kRows = 64;                    // rows of a tile
+constexpr int kWarpRows = kRows / kWarps;
+constexpr uint32_t kTileBytes = kRows * kD * 4;
+constexpr int kStages = 4;                   // pass A: K, V, Q tiles
+constexpr int kQStages = 8;                  // pass B: Q tiles, in the part of the ring above the partial products
+constexpr uint32_t kPartBytes = kWarps * kD * kD * 4;
+constexpr uint32_t kSmemBytes = kStages * 3 * kTileBytes + 1024;
+static_assert(kPartBytes + kQStages * kTileBytes <= kStages * 3 * kTileBytes, "pass B's ring");
 
-__device__ __forceinline__ float exp_fast(float x) {  // e^x
+struct Lin32Params {
+  int N, H;
+  uint32_t* status;
+};
+
+struct Lin32Bars {
+  uint64_t a_full[kStages], a_empty[kStages];
+  uint64_t b_full[kQStages], b_empty[kQStages];
+};
+
+__device__ __forceinline__ float ex2(float x) {
   float y;
-  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x * 1.4426950408889634f));
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
 }
 __device__ __forceinline__ float warp_max(float x) {
@@ -40,198 +66,297 @@ __device__ __forceinline__ float warp_sum(float x) {
   for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
   return x;
 }
-
-// acc[d] += row[d] * x for d = 0..31 (acc as 16 pairs), `row` a 32-float shared-memory buffer
-__device__ __forceinline__ void axpy_row(float2 (&acc)[kD / 2], const float* row, float x) {
-  const float2 xx = make_float2(x, x);
-#pragma unroll
-  for (int g = 0; g < 8; ++g) {
-    const float4 r = *reinterpret_cast<const float4*>(row + g * 4);
-    acc[g * 2 + 0] = __ffma2_rn(make_float2(r.x, r.y), xx, acc[g * 2 + 0]);
-    acc[g * 2 + 1] = __ffma2_rn(make_float2(r.z, r.w), xx, acc[g * 2 + 1]);
-  }
+__device__ __forceinline__ void record_timeout(uint32_t* status, uint32_t site) {
+  atomicAdd(&status[0], 1u);
+  status[1] = site;
 }
 
 template <bool kEA>
-__global__ void __launch_bounds__(kWarps * 32) linattn32_kernel(const LinAttn32Args a) {
-  __shared__ __align__(16) float row_s[kWarps][kUnroll][kD];  // per warp: rows being broadcast
-  __shared__ __align__(16) float m_part[kWarps / 2][kD][kD];  // partial K'^T V, four warps at a time
-  __shared__ __align__(16) float m_s[kD][kD];                 // M' = normalised K'^T V, [d][e]
-  __shared__ float red[2][kWarps][kD];
-  __shared__ float col_a[kD], col_b[kD];  // EA: column maximum, denominator; SimA: sum|K|, sum|Q|
+__global__ void __launch_bounds__(kThreads, 2)
+linattn32_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
+                 const __grid_constant__ CUtensorMap map_v, const __grid_constant__ CUtensorMap map_out,
+                 const Lin32Params p) {
+  extern __shared__ uint8_t smem_raw[];
+  __shared__ __align__(8) Lin32Bars bars;
+  __shared__ __align__(16) float m_s[kD][kD];       // M' = normalised K'^T V, [d][e]
+  __shared__ __align__(16) float scale_s[kWarps][kD];  // EA: rescale factors of a warp's partial product
+  __shared__ float stat_s[2][kWarps][kD];           // SimA: sum|K|, sum|Q|; EA: reference, sum of K'
+  __shared__ uint32_t abort_s;
+  const uint32_t ring = (smem_u32(smem_raw) + 1023u) & ~1023u;
+  float* const ring_gen = reinterpret_cast<float*>(smem_raw + (ring - smem_u32(smem_raw)));
+  constexpr float kLog2e = 1.4426950408889634f;
 
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int b = blockIdx.x / a.H, h = blockIdx.x % a.H;
-  const float* q = a.q + static_cast<int64_t>(b) * a.q_sb + static_cast<int64_t>(h) * a.q_sh + lane;
-  const float* k = a.k + static_cast<int64_t>(b) * a.k_sb + static_cast<int64_t>(h) * a.k_sh + lane;
-  const float* v = a.v + static_cast<int64_t>(b) * a.v_sb + static_cast<int64_t>(h) * a.v_sh + lane;
-  float* out = a.out + static_cast<int64_t>(b) * a.o_sb + static_cast<int64_t>(h) * a.o_sh + lane;
-  constexpr int kStep = kWarps * kUnroll;  // rows all warps take per step
+  volatile uint32_t* abortp = &abort_s;
+  const int b = blockIdx.x / p.H, h = blockIdx.x % p.H;
+  const int n_tiles = (p.N + kRows - 1) / kRows;
 
-  // ---- pass 1: column statistics over the sequence
-  {
-    float s0 = kEA ? -INFINITY : 0.f, s1 = 0.f;
-    for (int n0 = warp; n0 < a.N; n0 += 2 * kStep) {
-      float kv[2 * kUnroll], qv[kEA ? 1 : 2 * kUnroll];
-#pragma unroll
-      for (int u = 0; u < 2 * kUnroll; ++u) {
-        const int n = n0 + u * kWarps;
-        kv[u] = n < a.N ? __ldg(k + static_cast<int64_t>(n) * a.k_sn) : (kEA ? -INFINITY : 0.f);
-        if constexpr (!kEA) qv[u] = n < a.N ? __ldg(q + static_cast<int64_t>(n) * a.q_sn) : 0.f;
-      }
-#pragma unroll
-      for (int u = 0; u < 2 * kUnroll; ++u) {
-        if constexpr (kEA) {
-          s0 = fmaxf(s0, kv[u]);
-        } else {
-          s0 += fabsf(kv[u]);
-          s1 += fabsf(qv[u]);
-        }
-      }
+  if (tid == 0) {
+    abort_s = 0;
+    for (int i = 0; i < kStages; ++i) {
+      mbar_init(smem_u32(&bars.a_full[i]), 1);
+      mbar_init(smem_u32(&bars.a_empty[i]), kWarps);
     }
-    red[0][warp][lane] = s0;
-    red[1][warp][lane] = s1;
-    __syncthreads();
-    if (tid < kD) {
-      float r0 = red[0][0][tid], r1 = red[1][0][tid];
-      for (int w = 1; w < kWarps; ++w) {
-        r0 = kEA ? fmaxf(r0, red[0][w][tid]) : r0 + red[0][w][tid];
-        r1 += red[1][w][tid];
-      }
-      col_a[tid] = r0;
-      col_b[tid] = r1;
+    for (int i = 0; i < kQStages; ++i) {
+      mbar_init(smem_u32(&bars.b_full[i]), 1);
+      mbar_init(smem_u32(&bars.b_empty[i]), kWarps);
     }
-    __syncthreads();
+    mbar_fence_init();
   }
+  __syncthreads();
+  griddep_wait();
+  griddep_launch_dependents();
 
-  // ---- pass 2: M[d][e] = sum_n K'[n][d] V[n][e], K' = exp(K - column maximum) (EA) or K (SimA).
-  // Lane e keeps column e of this warp's partial M; the K' row is broadcast through row_s.
-  {
-    float2 acc[kD / 2];
+  // ---- pass A
+  const int e0 = (lane & 7) * 4, d0 = (lane >> 3) * 8;  // this lane's block of a 32 x 32 product
+  float2 acc[4][4];  // [e][pair of d]
 #pragma unroll
-    for (int d = 0; d < kD / 2; ++d) acc[d] = make_float2(0.f, 0.f);
-    float zsum = 0.f;  // EA: column sum of K' for feature `lane` over this warp's rows
-    const float cm = kEA ? col_a[lane] : 0.f;
-    // software pipeline: the rows of the next step are in flight while this step's FMAs run
-    float kn[kUnroll], vn[kUnroll];
-    auto fetch = [&](int n0) {
+  for (int e = 0; e < 4; ++e)
 #pragma unroll
-      for (int u = 0; u < kUnroll; ++u) {
-        const int n = n0 + u * kWarps;
-        kn[u] = n < a.N ? __ldg(k + static_cast<int64_t>(n) * a.k_sn) : (kEA ? -INFINITY : 0.f);
-        vn[u] = n < a.N ? __ldg(v + static_cast<int64_t>(n) * a.v_sn) : 0.f;
-      }
-    };
-    fetch(warp);
-    for (int n0 = warp; n0 < a.N; n0 += kStep) {
-      float vv[kUnroll];
-#pragma unroll
-      for (int u = 0; u < kUnroll; ++u) {
-        float kv = kn[u];
-        vv[u] = vn[u];
-        if constexpr (kEA) {
-          kv = exp_fast(kv - cm);  // rows past the end were loaded as -inf: they give 0
-          zsum += kv;
+    for (int d = 0; d < 4; ++d) acc[e][d] = make_float2(0.f, 0.f);
+  float s0 = kEA ? -INFINITY : 0.f, s1 = 0.f;
+  if (warp == kWarps) {
+    if (lane == 0) {
+      int t = 0;
+      for (; t < n_tiles; ++t) {
+        const int st = t % kStages;
+        if (t >= kStages && !mbar_wait(smem_u32(&bars.a_empty[st]), (t / kStages - 1) & 1, abortp)) {
+          record_timeout(p.status, 91);
+          break;
         }
-        row_s[warp][u][lane] = kv;
+        const uint32_t bar = smem_u32(&bars.a_full[st]), dst = ring + st * 3 * kTileBytes;
+        mbar_expect_tx(bar, (kEA ? 2 : 3) * kTileBytes);
+        tma_load_4d(dst, &map_k, bar, 0, h, t * kRows, b);
+        tma_load_4d(dst + kTileBytes, &map_v, bar, 0, h, t * kRows, b);
+        if (!kEA) tma_load_4d(dst + 2 * kTileBytes, &map_q, bar, 0, h, t * kRows, b);
       }
-      fetch(n0 + kStep);
-      __syncwarp();
-#pragma unroll
-      for (int u = 0; u < kUnroll; ++u) axpy_row(acc, row_s[warp][u], vv[u]);
-      __syncwarp();
+      if (t < n_tiles) {  // gave up: let copies in flight land
+        volatile uint32_t none = 0;
+        for (int x = t > kStages ? t - kStages : 0; x < t; ++x)
+          mbar_wait(smem_u32(&bars.a_full[x % kStages]), (x / kStages) & 1, &none);
+      }
     }
-    // fixed-order reduction over the warps, four at a time through shared memory
-    red[0][warp][lane] = zsum;
-    float total[kD];
-#pragma unroll
-    for (int d = 0; d < kD; ++d) total[d] = 0.f;
-#pragma unroll
-    for (int round = 0; round < 2; ++round) {
-      if ((warp >> 2) == round) {
-#pragma unroll
-        for (int d = 0; d < kD / 2; ++d) {
-          m_part[warp & 3][2 * d][lane] = acc[d].x;
-          m_part[warp & 3][2 * d + 1][lane] = acc[d].y;
-        }
+    __syncwarp();
+  } else {
+    for (int t = 0; t < n_tiles; ++t) {
+      const int st = t % kStages;
+      if (!__all_sync(0xffffffffu, mbar_wait(smem_u32(&bars.a_full[st]), (t / kStages) & 1, abortp))) {
+        if (lane == 0) record_timeout(p.status, 92);
+        break;
       }
-      __syncthreads();
-      if (warp == 0) {
-#pragma unroll
-        for (int w = 0; w < kWarps / 2; ++w) {
-#pragma unroll
-          for (int d = 0; d < kD; ++d) total[d] += m_part[w][d][lane];
-        }
-      }
-      __syncthreads();
-    }
-    if (warp == 0) {
+      float* const kt = ring_gen + (st * 3 * kTileBytes) / 4 + warp * kWarpRows * kD;
+      const float* const vt = kt + kTileBytes / 4;
+      const float* const qt = vt + kTileBytes / 4;
       if constexpr (kEA) {
-        float z = 0.f;
-        for (int w = 0; w < kWarps; ++w) z += red[0][w][lane];
-        col_b[lane] = z;
+        float kv[kWarpRows];
+        float mx = -INFINITY;
+#pragma unroll
+        for (int u = 0; u < kWarpRows; ++u) {
+          const bool live = t * kRows + warp * kWarpRows + u < p.N;
+          kv[u] = live ? kt[u * kD + lane] * kLog2e : -INFINITY;
+          mx = fmaxf(mx, kv[u]);
+        }
+        // (a warp whose rows all lie past the end changes nothing)
+        const bool raise = mx > s0 + 8.f;
+        if (__any_sync(0xffffffffu, raise)) {
+          const float m_new = raise ? mx : s0;
+          const float f = m_new > -INFINITY ? ex2(s0 - m_new) : 1.f;
+          s0 = m_new;
+          s1 *= f;
+          scale_s[warp][lane] = f;
+          __syncwarp();
+          const float4 f0 = *reinterpret_cast<const float4*>(&scale_s[warp][d0]);
+          const float4 f1 = *reinterpret_cast<const float4*>(&scale_s[warp][d0 + 4]);
+          const float2 ff[4] = {make_float2(f0.x, f0.y), make_float2(f0.z, f0.w), make_float2(f1.x, f1.y), make_float2(f1.z, f1.w)};
+#pragma unroll
+          for (int e = 0; e < 4; ++e)
+#pragma unroll
+            for (int d = 0; d < 4; ++d) acc[e][d] = __fmul2_rn(acc[e][d], ff[d]);
+        }
+#pragma unroll
+        for (int u = 0; u < kWarpRows; ++u) {
+          const float e = kv[u] > -INFINITY ? ex2(kv[u] - s0) : 0.f;
+          s1 += e;
+          kt[u * kD + lane] = e;
+        }
+        __syncwarp();
+      } else {
+#pragma unroll
+        for (int u = 0; u < kWarpRows; ++u) {
+          s0 += fabsf(kt[u * kD + lane]);
+          s1 += fabsf(qt[u * kD + lane]);
+        }
+      }
+      // acc[e][d] += V[row][e] * K'[row][d]
+#pragma unroll
+      for (int u = 0; u < kWarpRows; ++u) {
+        const float4 v = *reinterpret_cast<const float4*>(vt + u * kD + e0);
+        const float4 k0 = *reinterpret_cast<const float4*>(kt + u * kD + d0);
+        const float4 k1 = *reinterpret_cast<const float4*>(kt + u * kD + d0 + 4);
+        const float ve[4] = {v.x, v.y, v.z, v.w};
+        const float2 kk[4] = {make_float2(k0.x, k0.y), make_float2(k0.z, k0.w), make_float2(k1.x, k1.y), make_float2(k1.z, k1.w)};
+#pragma unroll
+        for (int e = 0; e < 4; ++e)
+#pragma unroll
+          for (int d = 0; d < 4; ++d) acc[e][d] = __ffma2_rn(kk[d], make_float2(ve[e], ve[e]), acc[e][d]);
       }
       __syncwarp();
-#pragma unroll
-      for (int d = 0; d < kD; ++d) {
-        const float inv = kEA ? 1.f / col_b[d] : 1.f / (col_a[d] * col_b[d]);
-        m_s[d][lane] = total[d] * inv;
-      }
+      if (lane == 0) mbar_arrive(smem_u32(&bars.a_empty[st]));
     }
-    __syncthreads();
+    stat_s[0][warp][lane] = s0;
+    stat_s[1][warp][lane] = s1;
+  }
+  if constexpr (kEA) fence_proxy_async_smem();  // (K' was written over tiles that TMA refills below)
+  __syncthreads();
+
+  // ---- the warps' partial products to M', in warp order, while the first tiles of pass B arrive
+  float* const part = ring_gen;
+  const uint32_t qring = ring + kPartBytes;
+  if (warp < kWarps) {
+#pragma unroll
+    for (int d = 0; d < 4; ++d) {
+      *reinterpret_cast<float4*>(part + (warp * kD + d0 + 2 * d) * kD + e0) =
+          make_float4(acc[0][d].x, acc[1][d].x, acc[2][d].x, acc[3][d].x);
+      *reinterpret_cast<float4*>(part + (warp * kD + d0 + 2 * d + 1) * kD + e0) =
+          make_float4(acc[0][d].y, acc[1][d].y, acc[2][d].y, acc[3][d].y);
+    }
+    named_bar_sync(1, kWarps * 32);
+    for (int d = warp; d < kD; d += kWarps) {
+      float total = 0.f, inv;
+      if constexpr (kEA) {
+        float m = -INFINITY, z = 0.f;
+#pragma unroll
+        for (int w = 0; w < kWarps; ++w) m = fmaxf(m, stat_s[0][w][d]);
+#pragma unroll
+        for (int w = 0; w < kWarps; ++w) {
+          const float f = stat_s[0][w][d] > -INFINITY ? ex2(stat_s[0][w][d] - m) : 0.f;
+          z = fmaf(f, stat_s[1][w][d], z);
+          total = fmaf(f, part[(w * kD + d) * kD + lane], total);
+        }
+        inv = 1.f / z;
+      } else {
+        float ck = 0.f, cq = 0.f;
+#pragma unroll
+        for (int w = 0; w < kWarps; ++w) {
+          ck += stat_s[0][w][d];
+          cq += stat_s[1][w][d];
+          total += part[(w * kD + d) * kD + lane];
+        }
+        inv = 1.f / (ck * cq);
+      }
+      m_s[d][lane] = total * inv;
+    }
+    named_bar_sync(1, kWarps * 32);
   }
 
-  // ---- pass 3: out[n][e] = sum_d Qn[n][d] M'[d][e]; lane e keeps column e of M' in registers
-  {
-    float2 mcol[kD / 2];
-#pragma unroll
-    for (int d = 0; d < kD / 2; ++d) mcol[d] = make_float2(m_s[2 * d][lane], m_s[2 * d + 1][lane]);
-    float qn[kUnroll];
-    auto fetch_q = [&](int n0) {
-#pragma unroll
-      for (int u = 0; u < kUnroll; ++u) {
-        const int n = n0 + u * kWarps;
-        qn[u] = n < a.N ? __ldg(q + static_cast<int64_t>(n) * a.q_sn) : 0.f;
-      }
-    };
-    fetch_q(warp);
-    for (int n0 = warp; n0 < a.N; n0 += kStep) {
-#pragma unroll
-      for (int u = 0; u < kUnroll; ++u) {
-        float qv = qn[u];
-        if constexpr (kEA) {
-          const float e = exp_fast(qv - warp_max(qv));
-          qv = e / warp_sum(e);
+  // ---- pass B: out[n][e] = sum_d Qn[n][d] M'[d][e]; a lane keeps its 8 x 4 block of M' in registers,
+  // and the four lanes with the same columns e add their parts up
+  if (warp == kWarps) {
+    if (lane == 0) {
+      int t = 0;
+      for (; t < n_tiles; ++t) {
+        const int st = t % kQStages;
+        if (t >= kQStages && !mbar_wait(smem_u32(&bars.b_empty[st]), (t / kQStages - 1) & 1, abortp)) {
+          record_timeout(p.status, 93);
+          break;
         }
-        row_s[warp][u][lane] = qv;
+        const uint32_t bar = smem_u32(&bars.b_full[st]);
+        mbar_expect_tx(bar, kTileBytes);
+        tma_load_4d(qring + st * kTileBytes, &map_q, bar, 0, h, t * kRows, b);
       }
-      fetch_q(n0 + kStep);
+      if (t < n_tiles) {
+        volatile uint32_t none = 0;
+        for (int x = t > kQStages ? t - kQStages : 0; x < t; ++x)
+          mbar_wait(smem_u32(&bars.b_full[x % kQStages]), (x / kQStages) & 1, &none);
+      }
+    }
+    __syncwarp();
+  } else {
+    float2 mb[4][4];  // [e][pair of d]
+#pragma unroll
+    for (int e = 0; e < 4; ++e)
+#pragma unroll
+      for (int d = 0; d < 4; ++d) mb[e][d] = make_float2(m_s[d0 + 2 * d][e0 + e], m_s[d0 + 2 * d + 1][e0 + e]);
+    const bool hi16 = (lane & 16) != 0, hi8 = (lane & 8) != 0;
+    const int e_mine = e0 + (hi16 ? 2 : 0) + (hi8 ? 1 : 0);
+    for (int t = 0; t < n_tiles; ++t) {
+      const int st = t % kQStages;
+      if (!__all_sync(0xffffffffu, mbar_wait(smem_u32(&bars.b_full[st]), (t / kQStages) & 1, abortp))) {
+        if (lane == 0) record_timeout(p.status, 94);
+        break;
+      }
+      float* const qt = ring_gen + (kPartBytes + st * kTileBytes) / 4 + warp * kWarpRows * kD;
+      if constexpr (kEA) {
+#pragma unroll
+        for (int u = 0; u < kWarpRows; ++u) {
+          const float x = qt[u * kD + lane] * kLog2e;
+          const float e = ex2(x - warp_max(x));
+          qt[u * kD + lane] = e / warp_sum(e);
+        }
+        __syncwarp();
+      }
+      float y[kWarpRows];
+#pragma unroll
+      for (int u = 0; u < kWarpRows; ++u) {
+        const float4 q0 = *reinterpret_cast<const float4*>(qt + u * kD + d0);
+        const float4 q1 = *reinterpret_cast<const float4*>(qt + u * kD + d0 + 4);
+        const float2 qq[4] = {make_float2(q0.x, q0.y), make_float2(q0.z, q0.w), make_float2(q1.x, q1.y), make_float2(q1.z, q1.w)};
+        float o[4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          float2 o2 = __fmul2_rn(qq[0], mb[e][0]);
+#pragma unroll
+          for (int d = 1; d < 4; ++d) o2 = __ffma2_rn(qq[d], mb[e][d], o2);
+          o[e] = o2.x + o2.y;
+        }
+        const float a0 = __shfl_xor_sync(0xffffffffu, hi16 ? o[0] : o[2], 16) + (hi16 ? o[2] : o[0]);
+        const float a1 = __shfl_xor_sync(0xffffffffu, hi16 ? o[1] : o[3], 16) + (hi16 ? o[3] : o[1]);
+        y[u] = __shfl_xor_sync(0xffffffffu, hi8 ? a0 : a1, 8) + (hi8 ? a1 : a0);
+      }
       __syncwarp();
 #pragma unroll
-      for (int u = 0; u < kUnroll; ++u) {
-        const int n = n0 + u * kWarps;
-        float2 o2 = make_float2(0.f, 0.f);
-#pragma unroll
-        for (int g = 0; g < 8; ++g) {
-          const float4 r = *reinterpret_cast<const float4*>(&row_s[warp][u][g * 4]);
-          o2 = __ffma2_rn(make_float2(r.x, r.y), mcol[g * 2 + 0], o2);
-          o2 = __ffma2_rn(make_float2(r.z, r.w), mcol[g * 2 + 1], o2);
-        }
-        if (n < a.N) out[static_cast<int64_t>(n) * a.o_sn] = o2.x + o2.y;
+      for (int u = 0; u < kWarpRows; ++u) qt[u * kD + e_mine] = y[u];
+      fence_proxy_async_smem();
+      __syncwarp();
+      if (lane == 0) {
+        const int row = t * kRows + warp * kWarpRows;
+        if (row < p.N)
+          tma_store_4d(&map_out, qring + st * kTileBytes + warp * kWarpRows * kD * 4, 0, h, row, b);
+        tma_store_commit();
+        tma_store_wait_read_n<1>();  // the tile before has left: its buffer may be refilled
+        if (t > 0) mbar_arrive(smem_u32(&bars.b_empty[(t - 1) % kQStages]));
       }
       __syncwarp();
     }
+    if (lane == 0) tma_store_wait_all();
+    __syncwarp();
   }
+  __syncthreads();
 }
 
 }  // namespace
 
 cudaError_t launch_linattn32(const LinAttn32Args& a, cudaStream_t stream) {
-  const dim3 grid(static_cast<unsigned>(a.B) * a.H);
-  if (a.ea) linattn32_kernel<true><<<grid, kWarps * 32, 0, stream>>>(a);
-  else linattn32_kernel<false><<<grid, kWarps * 32, 0, stream>>>(a);
+  Lin32Params p;
+  p.N = a.N;
+  p.H = a.H;
+  p.status = device_status_words();
+  const uint64_t dims[4] = {kD, static_cast<uint64_t>(a.H), static_cast<uint64_t>(a.N), static_cast<uint64_t>(a.B)};
+  auto map = [&](CUtensorMap* m, const float* base, int64_t sh, int64_t sn, int64_t sb, uint32_t rows) {
+    const uint64_t strides[3] = {static_cast<uint64_t>(sh) * 4, static_cast<uint64_t>(sn) * 4, static_cast<uint64_t>(sb) * 4};
+    const uint32_t box[4] = {kD, 1, rows, 1};
+    return tma_host::make_f32_map(m, base, dims, strides, box, false) == 0;
+  };
+  CUtensorMap mq, mk, mv, mo;
+  if (!map(&mq, a.q, a.q_sh, a.q_sn, a.q_sb, kRows) || !map(&mk, a.k, a.k_sh, a.k_sn, a.k_sb, kRows) ||
+      !map(&mv, a.v, a.v_sh, a.v_sn, a.v_sb, kRows) || !map(&mo, a.out, a.o_sh, a.o_sn, a.o_sb, kWarpRows))
+    return cudaErrorInvalidValue;
+  auto kern = a.ea ? linattn32_kernel<true> : linattn32_kernel<false>;
+  cudaError_t e = ensure_dynamic_smem(reinterpret_cast<const void*>(kern), kSmemBytes);
+  if (e != cudaSuccess) return e;
+  e = launch_dependent(kern, dim3(static_cast<unsigned>(a.B) * a.H), dim3(kThreads), kSmemBytes, stream, mq, mk, mv, mo, p);
   count_launch();
-  return cudaGetLastError();
+  return e;
 }
 
 }  // namespace asuka
