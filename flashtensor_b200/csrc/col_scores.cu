@@ -10,14 +10,18 @@
 // Orientation is transposed: S^T = K Q^T, so TMEM lane = key and one thread owns one key.  A
 // key's sum over all query rows is then a serial f32 sum in one thread, in a fixed order: no
 // cross-thread or cross-CTA reduction exists, and results are bitwise reproducible.
-//   warp 0      producer: two resident K tiles (256 keys), Q tiles + their row statistics in a ring
-//   warp 1      tcgen05.mma issuer: S^T_t[buf] = K_t Q_i^T into one of two TMEM buffers per key tile
-//   warps 4-11  keys   0..127 of the block: exp2, mask, accumulate; two warps per 32 keys, one for
-//               queries 0..63 and one for queries 64..127 of every query tile
-//   warps 12-19 keys 128..255, likewise
-// Four key warps per scheduler, not two: one warp's stream of FFMA -> MUFU -> FADD chains stalls
-// on its own latencies about half the time, and its loads and barrier waits stall it outright, so
-// two warps leave the MUFU idle a third of the time.
+//   warp 0      producer: one resident K tile (128 keys), Q tiles and their row statistics in two rings
+//   warp 1      tcgen05.mma issuer: S^T[buf] = K Q_i^T into one of two TMEM buffers
+//   warps 2-9   exp2, mask, accumulate; two warps per 32 keys, one for queries 0..63 and one for
+//               queries 64..127 of every query tile
+// Two CTAs share an SM (96 KB and 256 TMEM columns each), so sixteen key warps run on it: one warp's
+// stream of FFMA -> MUFU -> FADD chains stalls on its own latencies about half the time, and its loads
+// and barrier waits stall it outright; with two warps per scheduler the MUFU idled a third of the time.
+// The two CTAs are at different points of their lives, so one's set-up (barriers, TMEM, the first K and
+// Q tiles) and tail run under the other's steps.  One CTA of 256 keys with the same sixteen warps, which
+// has nothing to run then, measured (this kernel in the middle of the case, us, before -> after): 500
+// rows over 5003 keys, 32/8 heads 45.6 -> 35.8; H2O S4096 H32 110.7 -> 96.8; RoCo B2 H40 S4096
+// 302 -> 272; seeded Keyformer B2 H32 S1501 108.6 -> 99.7.
 //
 // The Keyformer row pass (kf_rowstat) is the row-oriented counterpart: S = Q K^T, one thread per
 // query row, online max/sum of the perturbed logits, nothing else.
@@ -39,13 +43,13 @@ namespace {
 constexpr int kTile = 128;
 constexpr uint32_t kTileBytes = 128 * 128 * 2;
 constexpr uint32_t kHalfBytes = kTileBytes / 2;
-constexpr int kQStages = 4;
-#ifndef ASUKA_COL_UTIL_WARPS
-#define ASUKA_COL_UTIL_WARPS 2
-#endif
-constexpr int kUtilWarps = ASUKA_COL_UTIL_WARPS;  // producer and MMA issuer (no idle warps: their registers go to the key warps)
-constexpr int kThreads = (kUtilWarps + 16) * 32;  // + 16 key warps; 576 threads x 112 registers, no setmaxnreg
-constexpr uint32_t kSmemBytes = (2 + kQStages) * kTileBytes + 1024;
+constexpr int kUtilWarps = 2;                     // producer and MMA issuer
+constexpr int kKeyWarps = 8;                      // col_scores_kernel: two per 32 keys
+constexpr int kColThreads = (kUtilWarps + kKeyWarps) * 32;
+constexpr int kQStages = 2;                       // Q tiles; free again as soon as the MMA has read them
+constexpr int kLseStages = 4;                     // row statistics of the Q tiles; free when the key warps have read them
+constexpr uint32_t kSmemBytes = (1 + kQStages) * kTileBytes + 1024;
+constexpr int kThreads = (kUtilWarps + 16) * 32;  // kf_col_tma_kernel: 16 key warps
 
 struct ColParams {
   int B, H, Sq, Skv;
@@ -75,7 +79,8 @@ struct ColParams {
 struct ColBars {
   uint64_t k_full;
   uint64_t q_full[kQStages], q_empty[kQStages];
-  uint64_t s_full[2][2], s_empty[2][2];
+  uint64_t lse_empty[kLseStages];
+  uint64_t s_full[2], s_empty[2];
 };
 
 __device__ __forceinline__ float ex2(float x) {
@@ -190,19 +195,19 @@ __device__ __forceinline__ void record_timeout(uint32_t* status, uint32_t site) 
 // kMode: 0 sum, 1 sum + sum of squares, 2 perturbed (noise operand), 3 perturbed (seeded noise),
 //        4 CORM: any_i(p_ij >= mask_ij) with a [Sq, Skv] threshold operand (cases/kernels/corm.py:34-37)
 template <bool kBF16, int kMode>
-__global__ void __launch_bounds__(kThreads, 1)
+__global__ void __launch_bounds__(kColThreads, (kMode == 2 || kMode == 4) ? 1 : 2)
 col_scores_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                   const ColParams p) {
   extern __shared__ uint8_t smem_raw[];
   __shared__ __align__(8) ColBars bars;
-  __shared__ __align__(16) float lse_s[kQStages][kTile];  // minus the row statistic
-  __shared__ float part_s[2][2][2][kTile];  // [sum, sum of squares][query half][key tile][key]
+  __shared__ __align__(16) float lse_s[kLseStages][kTile];  // minus the row statistic
+  __shared__ float part_s[2][2][kTile];  // [sum, sum of squares][query half][key]
   __shared__ uint32_t tmem_base_s;
   __shared__ uint32_t abort_s;
 
   const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
-  const uint32_t sK = smem_base;                    // 2 tiles
-  const uint32_t sQ = smem_base + 2 * kTileBytes;   // kQStages tiles
+  const uint32_t sK = smem_base;
+  const uint32_t sQ = smem_base + kTileBytes;   // kQStages tiles
 
   const int tid = threadIdx.x;
   const int warp = tid >> 5;
@@ -211,26 +216,19 @@ col_scores_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
 
   const int bh_count = p.B * p.H;
   const int blk = static_cast<int>(blockIdx.x) / bh_count;
-  const int kvb = blk / p.n_qchunks;  // low key blocks are the long ones
+  const int kt = blk / p.n_qchunks;  // low key tiles are the long ones
   const int qc = p.n_qchunks - 1 - blk % p.n_qchunks;  // (late query ranges see the most keys)
   const int bh = static_cast<int>(blockIdx.x) % bh_count;
   const int b = bh / p.H, h = bh % p.H;
-  const int kv0[2] = {kvb * 2 * kTile, kvb * 2 * kTile + kTile};
-  const bool active[2] = {kv0[0] < p.Skv, kv0[1] < p.Skv};
-  // this CTA's query tiles [i_lo, i_end), and the first of them that can see the first key of
-  // each key tile
-  const int i_lo = qc * p.q_chunk;
-  const int i_end = min(p.nq_tiles, i_lo + p.q_chunk);
-  int i_start[2];
-#pragma unroll
-  for (int t = 0; t < 2; ++t) i_start[t] = max(i_lo, p.causal ? max(0, kv0[t] - p.diag_off) / kTile : 0);
-  const int i_begin = i_start[0];
-  const int n_active = (active[0] ? 1 : 0) + (active[1] ? 1 : 0);
+  const int kv0 = kt * kTile;
+  // this CTA's query tiles: its range, from the first tile that can see its first key
+  const int i_begin = max(qc * p.q_chunk, p.causal ? max(0, kv0 - p.diag_off) / kTile : 0);
+  const int i_end = min(p.nq_tiles, (qc + 1) * p.q_chunk);
 
   // Launched as a programmatic dependent: unless the caller vouches for the kernel ahead (the fused
   // case entry points, whose forward kernel writes only the output and the row statistic), q and k
   // may still be in the making, and everything waits.  Otherwise only the producer waits, before
-  // its first read of the row statistic, and the set-up and the K loads run under that kernel's tail.
+  // its first read of the row statistic, and the set-up and the K load run under that kernel's tail.
   if (!p.chained) griddep_wait();
   griddep_launch_dependents();
 
@@ -239,32 +237,26 @@ col_scores_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
     mbar_init(smem_u32(&bars.k_full), 1);
     for (int i = 0; i < kQStages; ++i) {
       mbar_init(smem_u32(&bars.q_full[i]), 1);
-      mbar_init(smem_u32(&bars.q_empty[i]), 1 + 8 * n_active);
+      mbar_init(smem_u32(&bars.q_empty[i]), 1);
     }
-    for (int t = 0; t < 2; ++t)
-      for (int i = 0; i < 2; ++i) {
-        mbar_init(smem_u32(&bars.s_full[t][i]), 1);
-        mbar_init(smem_u32(&bars.s_empty[t][i]), 256);
-      }
+    for (int i = 0; i < kLseStages; ++i) mbar_init(smem_u32(&bars.lse_empty[i]), kKeyWarps);
+    for (int i = 0; i < 2; ++i) {
+      mbar_init(smem_u32(&bars.s_full[i]), 1);
+      mbar_init(smem_u32(&bars.s_empty[i]), kKeyWarps * 32);
+    }
     mbar_fence_init();
     tma_prefetch_desc(&map_q);
     tma_prefetch_desc(&map_k);
-    // the K tiles are the first thing every role waits for: start them now, under the TMEM
-    // allocation and the CTA-wide barrier below (this thread initialised the barrier they signal)
-    {
-      const uint32_t bar = smem_u32(&bars.k_full);
-      mbar_expect_tx(bar, kTileBytes * n_active);
-      for (int t = 0; t < 2; ++t) {
-        if (active[t]) {
-          tma_load_4d(sK + t * kTileBytes, &map_k, bar, 0, h / p.group, kv0[t], b);
-          tma_load_4d(sK + t * kTileBytes + kHalfBytes, &map_k, bar, 64, h / p.group, kv0[t], b);
-        }
-      }
-    }
+    // the K tile is the first thing every role waits for: start it now, under the TMEM allocation
+    // and the CTA-wide barrier below (this thread initialised the barrier it signals)
+    const uint32_t bar = smem_u32(&bars.k_full);
+    mbar_expect_tx(bar, kTileBytes);
+    tma_load_4d(sK, &map_k, bar, 0, h / p.group, kv0, b);
+    tma_load_4d(sK + kHalfBytes, &map_k, bar, 64, h / p.group, kv0, b);
   }
   if (warp == 1) {
     __syncwarp();
-    tmem_alloc(smem_u32(&tmem_base_s), 512);
+    tmem_alloc(smem_u32(&tmem_base_s), 256);
     tmem_relinquish();
   }
   tc_fence_before_sync();
@@ -279,19 +271,21 @@ col_scores_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
     if (p.chained) griddep_wait();  // the row statistic is the output of the kernel ahead
     for (int i = i_begin; i < i_end; ++i) {
       const int c = i - i_begin;
-      const int st = c % kQStages;
-      const uint32_t use = static_cast<uint32_t>(c / kQStages);
-      if (use > 0) {
-        ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&bars.q_empty[st]), (use - 1) & 1, abortp));
-        if (!ok) { if (lane == 0) record_timeout(p.status, 21); break; }
-      }
+      const int st = c % kQStages, ls = c % kLseStages;
+      if (c >= kLseStages)
+        ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&bars.lse_empty[ls]), (c / kLseStages - 1) & 1, abortp));
       // NEGATED row statistics of this query tile (they are only ever subtracted); rows past the
       // end get -inf so that exp2 gives 0
+      if (ok) {
 #pragma unroll
-      for (int r = 0; r < 4; ++r) {
-        const int qi = i * kTile + r * 32 + lane;
-        lse_s[st][r * 32 + lane] = qi < p.Sq ? -__ldg(lse_row + qi) : -INFINITY;
+        for (int r = 0; r < 4; ++r) {
+          const int qi = i * kTile + r * 32 + lane;
+          lse_s[ls][r * 32 + lane] = qi < p.Sq ? -__ldg(lse_row + qi) : -INFINITY;
+        }
+        if (c >= kQStages)
+          ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&bars.q_empty[st]), (c / kQStages - 1) & 1, abortp));
       }
+      if (!ok) { if (lane == 0) record_timeout(p.status, 21); break; }
       __syncwarp();
       if (lane == 0) {
         const uint32_t bar = smem_u32(&bars.q_full[st]);
@@ -300,7 +294,7 @@ col_scores_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
         tma_load_4d(sQ + st * kTileBytes + kHalfBytes, &map_q, bar, 64, h, i * kTile, b);
       }
     }
-    if (!ok && lane == 0) {
+    if (lane == 0 && (!ok || i_begin >= i_end)) {  // nothing else waits for the K tile then
       volatile uint32_t none = 0;
       mbar_wait(smem_u32(&bars.k_full), 0, &none);
     }
@@ -308,57 +302,39 @@ col_scores_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
     // ------------------------------------------------------------------ MMA issuer
     // The whole warp walks the loop (warp-uniform descriptors, converged waits); one elected lane
     // issues the tcgen05.mma / commit instructions.
-    {
-      constexpr uint32_t kFmt = kBF16 ? UMMA_BF16 : UMMA_F16;
-      constexpr uint32_t idesc = umma_idesc_f16(kFmt, UMMA_K_MAJOR, UMMA_K_MAJOR, 128, 128);
-      auto wait_all = [&](uint64_t* bar, uint32_t parity, uint32_t site) -> bool {
-        const bool good = __all_sync(0xffffffffu, mbar_wait(smem_u32(bar), parity, abortp));
-        if (!good && lane == 0) record_timeout(p.status, site);
-        return good;
-      };
-      bool ok = wait_all(&bars.k_full, 0, 22);
-      for (int i = i_begin; i < i_end && ok; ++i) {
-        const int c = i - i_begin;
-        const int st = c % kQStages;
-        ok = wait_all(&bars.q_full[st], (c / kQStages) & 1, 23);
-        if (!ok) break;
-        tc_fence_after_sync();
-        const uint64_t qdesc = umma_smem_desc_sw128(sQ + st * kTileBytes, 16, 1024);
+    constexpr uint32_t kFmt = kBF16 ? UMMA_BF16 : UMMA_F16;
+    constexpr uint32_t idesc = umma_idesc_f16(kFmt, UMMA_K_MAJOR, UMMA_K_MAJOR, 128, 128);
+    auto wait_all = [&](uint64_t* bar, uint32_t parity, uint32_t site) -> bool {
+      const bool good = __all_sync(0xffffffffu, mbar_wait(smem_u32(bar), parity, abortp));
+      if (!good && lane == 0) record_timeout(p.status, site);
+      return good;
+    };
+    bool ok = wait_all(&bars.k_full, 0, 22);
+    const uint64_t kdesc = umma_smem_desc_sw128(sK, 16, 1024);
+    for (int i = i_begin; i < i_end && ok; ++i) {
+      const int c = i - i_begin;
+      const int st = c % kQStages, buf = c & 1;
+      ok = wait_all(&bars.q_full[st], (c / kQStages) & 1, 23);
+      if (ok && c >= 2) ok = wait_all(&bars.s_empty[buf], ((c >> 1) - 1) & 1, 24);
+      if (!ok) break;
+      tc_fence_after_sync();
+      const uint64_t qdesc = umma_smem_desc_sw128(sQ + st * kTileBytes, 16, 1024);
+      if (elect_one()) {
 #pragma unroll
-        for (int t = 0; t < 2; ++t) {
-          if (!active[t] || i < i_start[t]) continue;
-          const int ct = i - i_start[t];
-          const int buf = ct & 1;
-          if (ct >= 2) {
-            ok = wait_all(&bars.s_empty[t][buf], ((ct >> 1) - 1) & 1, 24);
-            if (!ok) break;
-            tc_fence_after_sync();
-          }
-          const uint64_t kdesc = umma_smem_desc_sw128(sK + t * kTileBytes, 16, 1024);
-          const uint32_t tS = tbase + (t * 2 + buf) * 128;
-          if (elect_one()) {
-#pragma unroll
-            for (int kk = 0; kk < 8; ++kk) {
-              const uint64_t off = static_cast<uint64_t>((kk & 3) * 2 + (kk >> 2) * (kHalfBytes >> 4));
-              umma_ss(tS, kdesc + off, qdesc + off, idesc, kk > 0 ? 1u : 0u);
-            }
-            umma_commit(smem_u32(&bars.s_full[t][buf]));
-          }
-          __syncwarp();
+        for (int kk = 0; kk < 8; ++kk) {
+          const uint64_t off = static_cast<uint64_t>((kk & 3) * 2 + (kk >> 2) * (kHalfBytes >> 4));
+          umma_ss(tbase + buf * 128, kdesc + off, qdesc + off, idesc, kk > 0 ? 1u : 0u);
         }
-        if (!ok) break;
-        if (elect_one()) umma_commit(smem_u32(&bars.q_empty[st]));
-        __syncwarp();
+        umma_commit(smem_u32(&bars.s_full[buf]));
+        umma_commit(smem_u32(&bars.q_empty[st]));
       }
+      __syncwarp();
     }
-  } else if (warp < kUtilWarps) {
   } else {
     // ------------------------------------------------------------------ one thread per (key, query half)
-    const int kw = warp - kUtilWarps;
-    const int t = kw >> 3;         // key tile
-    const int hq = (kw >> 2) & 1;  // which 64 queries of every query tile
+    const int hq = (warp - kUtilWarps) >> 2;  // which 64 queries of every query tile
     const int wq = warp & 3;       // TMEM lane quarter this warp may touch (every four consecutive key warps cover all four)
-    const int key = kv0[t] + wq * 32 + lane;
+    const int key = kv0 + wq * 32 + lane;
     const uint32_t lane_base = static_cast<uint32_t>(wq * 32) << 16;
     const float scale = p.scale_log2;
     float acc[4] = {0.f, 0.f, 0.f, 0.f};
@@ -372,25 +348,22 @@ col_scores_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
     }
     bool hit = false;
 
-    if (active[t]) {
+    {
       for (int i = i_begin; i < i_end; ++i) {
         const int c = i - i_begin;
-        const int st = c % kQStages;
-        if (i >= i_start[t]) {
-          const int ct = i - i_start[t];
-          const int buf = ct & 1;
+        const int ls = c % kLseStages, buf = c & 1;
+        {
           // S^T of this step is complete; its MMAs were issued after Q and the row statistics of
-          // the stage had landed, so this wait covers q_full as well
-          ok = __all_sync(0xffffffffu,
-                          mbar_wait(smem_u32(&bars.s_full[t][buf]), (ct >> 1) & 1, abortp));
+          // the stage had landed, so this wait covers them as well
+          ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&bars.s_full[buf]), (c >> 1) & 1, abortp));
           if (!ok) { if (lane == 0) record_timeout(p.status, 26); break; }
           tc_fence_after_sync();
-          const uint32_t tS = tbase + lane_base + (t * 2 + buf) * 128 + hq * 64;
+          const uint32_t tS = tbase + lane_base + buf * 128 + hq * 64;
           const int q_base = i * kTile + hq * 64;
           // query q of this tile sees `key` iff key <= q + diag_off
           const int first_visible = p.causal ? key - p.diag_off - q_base : 0;
-          const bool tile_has_mask = p.causal && (kv0[t] + kTile - 1 - p.diag_off > q_base);
-          const float4* lse4 = reinterpret_cast<const float4*>(lse_s[st]) + hq * 16;
+          const bool tile_has_mask = p.causal && (kv0 + kTile - 1 - p.diag_off > q_base);
+          const float4* lse4 = reinterpret_cast<const float4*>(lse_s[ls]) + hq * 16;
           // two chunks of 32 queries: every exponential of a chunk is in flight at once
 #pragma unroll
           for (int ch = 0; ch < 2; ++ch) {
@@ -418,7 +391,7 @@ col_scores_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
               // this thread's part of the tile is in registers; when all 256 have said so the MMA
               // warp may overwrite the TMEM buffer
               tc_fence_before_sync();
-              mbar_arrive(smem_u32(&bars.s_empty[t][buf]));
+              mbar_arrive(smem_u32(&bars.s_empty[buf]));
             }
 #pragma unroll
             for (int g = 0; g < 8; ++g) {
@@ -490,20 +463,15 @@ col_scores_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
               acc2[0] = q01.x; acc2[1] = q01.y; acc2[2] = q23.x; acc2[3] = q23.y;
             }
           }
-        } else {
-          // a step this key tile skips (its keys are invisible to the whole query tile): the stage
-          // may only be released once it has been filled
-          ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&bars.q_full[st]), (c / kQStages) & 1, abortp));
-          if (!ok) { if (lane == 0) record_timeout(p.status, 25); break; }
         }
         __syncwarp();
-        if (lane == 0) mbar_arrive(smem_u32(&bars.q_empty[st]));
+        if (lane == 0) mbar_arrive(smem_u32(&bars.lse_empty[ls]));
       }
     }
     // Both query halves leave their parts in shared memory; after the CTA-wide barrier below the
     // first half's thread adds the two in a fixed order and stores.
-    part_s[0][hq][t][wq * 32 + lane] = kMode == 4 ? (hit ? 1.f : 0.f) : (acc[0] + acc[1]) + (acc[2] + acc[3]);
-    part_s[1][hq][t][wq * 32 + lane] = (acc2[0] + acc2[1]) + (acc2[2] + acc2[3]);
+    part_s[0][hq][wq * 32 + lane] = kMode == 4 ? (hit ? 1.f : 0.f) : (acc[0] + acc[1]) + (acc[2] + acc[3]);
+    part_s[1][hq][wq * 32 + lane] = (acc2[0] + acc2[1]) + (acc2[2] + acc2[3]);
     if (!ok) *abortp = 1u;
   }
 
@@ -511,15 +479,14 @@ col_scores_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
   __syncthreads();
   if (warp == 1) {
     __syncwarp();
-    tmem_dealloc(tbase, 512);
+    tmem_dealloc(tbase, 256);
   }
-  if (warp >= kUtilWarps && ((warp - kUtilWarps) >> 2 & 1) == 0 && !*abortp) {
-    const int t = (warp - kUtilWarps) >> 3;
+  if (warp >= kUtilWarps && warp < kUtilWarps + 4 && !*abortp) {
     const int k_in_tile = (warp & 3) * 32 + lane;
-    const int key = kv0[t] + k_in_tile;
-    if (key < p.Skv) {  // (implies that this key tile is active)
+    const int key = kv0 + k_in_tile;
+    if (key < p.Skv) {
       const size_t o = (static_cast<size_t>(b) * p.H + h) * p.Skv + key;
-      const float v = part_s[0][0][t][k_in_tile] + part_s[0][1][t][k_in_tile];
+      const float v = part_s[0][0][k_in_tile] + part_s[0][1][k_in_tile];
       // with a query-range split the sums of this range go to its slab of the workspace (a range
       // that sees none of the keys leaves zeros there)
       const size_t slab = static_cast<size_t>(qc) * bh_count * p.Skv;
@@ -529,7 +496,7 @@ col_scores_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
         (p.n_qchunks > 1 ? p.part + slab : p.score)[o] = v;
       }
       if constexpr (kMode == 1)
-        (p.n_qchunks > 1 ? p.part_sq + slab : p.score_sq)[o] = part_s[1][0][t][k_in_tile] + part_s[1][1][t][k_in_tile];
+        (p.n_qchunks > 1 ? p.part_sq + slab : p.score_sq)[o] = part_s[1][0][k_in_tile] + part_s[1][1][k_in_tile];
     }
   }
 }
@@ -1278,8 +1245,8 @@ cudaError_t launch_col_scores(const CUtensorMap& mq, const CUtensorMap& mk, cons
   } else
 #endif
   {
-  const int n_kvb = (s.Skv + 2 * kTile - 1) / (2 * kTile);
-  const dim3 grid(static_cast<unsigned>(n_kvb) * p.n_qchunks * s.B * s.H);
+  const int n_kt = (s.Skv + kTile - 1) / kTile;
+  const dim3 grid(static_cast<unsigned>(n_kt) * p.n_qchunks * s.B * s.H);
   void (*kern)(CUtensorMap, CUtensorMap, ColParams) = nullptr;
   if (a.mode == ASUKA_SCORE_SUM) kern = s.bf16 ? col_scores_kernel<true, 0> : col_scores_kernel<false, 0>;
   else if (a.mode == ASUKA_SCORE_SUM_SQ) kern = s.bf16 ? col_scores_kernel<true, 1> : col_scores_kernel<false, 1>;
@@ -1288,7 +1255,7 @@ cudaError_t launch_col_scores(const CUtensorMap& mq, const CUtensorMap& mk, cons
   else kern = s.bf16 ? col_scores_kernel<true, 3> : col_scores_kernel<false, 3>;
   e = ensure_dynamic_smem(reinterpret_cast<const void*>(kern), kSmemBytes);
   if (e != cudaSuccess) return e;
-  e = launch_dependent(kern, grid, dim3(kThreads), kSmemBytes, stream, mq, mk, p);
+  e = launch_dependent(kern, grid, dim3(kColThreads), kSmemBytes, stream, mq, mk, p);
   count_launch();
   }
   if (e != cudaSuccess || p.n_qchunks == 1) return e;
