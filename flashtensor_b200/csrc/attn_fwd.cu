@@ -24,6 +24,7 @@
 #include <cuda_fp16.h>
 
 #include <cstdlib>
+#include <type_traits>
 
 #include "kernels.h"
 #include "sm100_ptx.cuh"
@@ -36,12 +37,22 @@ namespace {
 constexpr int kTile = 128;
 constexpr uint32_t kTileBytes = 128 * 128 * 2;  // one [128 x 128] 16-bit tile = two swizzled halves
 constexpr uint32_t kHalfBytes = kTileBytes / 2;
-constexpr int kKStages = 3;  // K(j) is needed one iteration before V(j): give it the deeper ring
-constexpr int kVStages = 2;
+// How the query tiles and keys of a launch are cut into work items (each its own instantiation: what
+// one mode needs per item costs the softmax warps of another registers they do not have).
+//   kPair   two query tiles, each over all its keys; a K/V tile serves both
+//   kSplit  two query tiles over a part of their keys; attn_merge_kernel combines the parts
+//   kSolo   ONE query tile, its even key tiles on the first softmax slot and its odd ones on the second,
+//           merged in the epilogue
+enum FwdMode { kPair = 0, kSplit = 1, kSolo = 2 };
+template <int kMode> struct Rings {
+  static constexpr int kQTiles = kMode == kSolo ? 1 : 2;
+  static constexpr int kK = 3;  // K(j) is needed one iteration before V(j): give it the deeper ring
+  static constexpr int kV = kMode == kSolo ? 3 : 2;
+};
 constexpr int kThreads = 384;
 constexpr int kUtilRegs = 96;      // 128 * 96 + 256 * 200 = 63488 <= 384 * 168
 constexpr int kSoftmaxRegs = 200;
-constexpr uint32_t kSmemBytes = (2 + kKStages + kVStages) * kTileBytes + 1024;
+constexpr uint32_t kSmemBytes = 7 * kTileBytes + 1024;
 constexpr float kRescaleLimit = 8192.0f;  // largest tile row sum tolerated under a stale reference:
                                           // bounds every exponential far below fp16's 65504
 
@@ -70,8 +81,8 @@ struct FwdParams {
 
 struct Bars {
   uint64_t q_full[2], q_empty[2];
-  uint64_t k_full[kKStages], k_empty[kKStages];
-  uint64_t v_full[kVStages], v_empty[kVStages];
+  uint64_t k_full[3], k_empty[3];
+  uint64_t v_full[3], v_empty[3];
   uint64_t s_full[2], p_ready[2], o_done[2], o_free[2];
 };
 
@@ -149,13 +160,24 @@ struct Item {
   int nparts[2];  // parts that serve each tile (1: this item writes the tile's final result)
 };
 
-// Item `idx` of the launch; items are numbered heaviest first.  kSplit = false is the common case
-// of one item per 256-row block, compiled without any of the key-range arithmetic (which costs
-// the softmax warps registers they do not have).
-template <bool kSplit>
+// Item `idx` of the launch; items are numbered heaviest first.
+template <int kMode>
 __device__ __forceinline__ void decode_item(int idx, const FwdParams& p, Item* item) {
   const int bh_count = p.B * p.H;
-  if constexpr (!kSplit) {
+  if constexpr (kMode == kSolo) {
+    const int bh = idx % bh_count, n = kv_tiles_for((p.nq_tiles - 1 - idx / bh_count) * kTile, p);
+    item->b = bh / p.H;
+    item->h = bh % p.H;
+    item->q0[0] = item->q0[1] = (p.nq_tiles - 1 - idx / bh_count) * kTile;
+    item->j0 = 0;
+    item->n_kv[0] = (n + 1) / 2;
+    item->n_kv[1] = n / 2;
+    item->n_max = item->n_kv[0];
+    item->part = 0;
+    item->nparts[0] = item->nparts[1] = 1;
+    return;
+  }
+  if constexpr (kMode == kPair) {
     // unit_major: the blocks of one (batch, head) follow each other, latest first, so that they
     // run at about the same time and K/V are in L2 for all but the first of them.  It is used
     // when K and V of the whole launch do not fit L2 (otherwise every wave of blocks would fetch
@@ -214,13 +236,13 @@ __device__ __forceinline__ void decode_item(int idx, const FwdParams& p, Item* i
 // backwards when it is odd, which evens out the totals (at 32 heads and S = 4096 the busiest CTA
 // gets 3 % more than the mean; assigning longest-first to the least-loaded CTA on the host would
 // get within 2.5 %, the items being as coarse as they are, and was not worth a table).
-template <bool kSplit>
+template <int kMode>
 __device__ __forceinline__ bool get_item(int it, const FwdParams& p, Item* item) {
   const int G = static_cast<int>(gridDim.x);
   const int r = static_cast<int>(blockIdx.x);
   const int idx = it * G + ((it & 1) ? G - 1 - r : r);
   if (idx >= p.n_items) return false;
-  decode_item<kSplit>(idx, p, item);
+  decode_item<kMode>(idx, p, item);
   return true;
 }
 // with an odd number of waves the last, backwards-dealt wave can skip a CTA that still has none
@@ -230,18 +252,21 @@ __device__ __forceinline__ int item_waves(const FwdParams& p) {
 
 // kCap: Gemma-2 style soft-capping, logits -> cap * tanh(logits / cap) before the mask
 // (cases/kernels/gemma2.py:30-33; the reference emits tanh.approx.f32 too, to_triton.cpp:351-369).
-template <bool kBF16, bool kCap, bool kSplit>
+template <bool kBF16, bool kCap, int kMode>
 __global__ void __launch_bounds__(kThreads, 1)
 attn_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                 const __grid_constant__ CUtensorMap map_v, const FwdParams p) {
   extern __shared__ uint8_t smem_raw[];
+  constexpr int kKStages = Rings<kMode>::kK, kVStages = Rings<kMode>::kV;
+  constexpr bool kOne = kMode == kSolo;  // one query tile, the two slots share its keys
   __shared__ __align__(8) Bars bars;
+  __shared__ float2 row_s[kOne ? kTile : 1];  // (kSolo) second slot's reference and row sum; then both slots' factors
   __shared__ uint32_t tmem_base_s;
   __shared__ uint32_t abort_s;
 
   const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
-  const uint32_t sQ = smem_base;                          // 2 tiles
-  const uint32_t sK = smem_base + 2 * kTileBytes;         // kKStages tiles
+  const uint32_t sQ = smem_base;                          // one or two tiles
+  const uint32_t sK = smem_base + Rings<kMode>::kQTiles * kTileBytes;  // kKStages tiles
   const uint32_t sV = sK + kKStages * kTileBytes;         // kVStages tiles
 
   const int tid = threadIdx.x;
@@ -258,7 +283,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
       mbar_init(smem_u32(&bars.s_full[i]), 1);
       mbar_init(smem_u32(&bars.p_ready[i]), 128);
       mbar_init(smem_u32(&bars.o_done[i]), 1);
-      mbar_init(smem_u32(&bars.o_free[i]), 128);
+      mbar_init(smem_u32(&bars.o_free[i]), kOne ? 256 : 128);
     }
     for (int i = 0; i < kKStages; ++i) {
       mbar_init(smem_u32(&bars.k_full[i]), 1);
@@ -302,8 +327,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
       uint32_t qn[2] = {0, 0};    // items in which tile t was loaded so far
       Item it_;
       for (int it = 0; it < n_waves && ok; ++it) {
-        if (!get_item<kSplit>(it, p, &it_)) continue;
-        for (int t = 0; t < 2 && ok; ++t) {
+        if (!get_item<kMode>(it, p, &it_)) continue;
+        for (int t = 0; t < Rings<kMode>::kQTiles && ok; ++t) {
           if (it_.n_kv[t] == 0) continue;
           if (qn[t] > 0) {  // the previous item's last QK^T of this tile must have read Q_t
             ok = mbar_wait(smem_u32(&bars.q_empty[t]), (qn[t] - 1) & 1, abortp);
@@ -315,7 +340,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
           tma_load_4d(sQ + t * kTileBytes + kHalfBytes, &map_q, bar, 64, it_.h, it_.q0[t], it_.b);
           ++qn[t];
         }
-        for (int j = 0; j < it_.n_max && ok; ++j, ++kc) {
+        const int n_tiles = kOne ? it_.n_kv[0] + it_.n_kv[1] : it_.n_max;
+        for (int j = 0; j < n_tiles && ok; ++j, ++kc) {
           const int st = kc % kKStages;
           const uint32_t use = kc / kKStages;
           if (use > 0) {
@@ -324,8 +350,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
           }
           const uint32_t bar = smem_u32(&bars.k_full[st]);
           mbar_expect_tx(bar, kTileBytes);
-          tma_load_4d(sK + st * kTileBytes, &map_k, bar, 0, it_.h / p.group, ((kSplit ? it_.j0 : 0) + j) * kTile, it_.b);
-          tma_load_4d(sK + st * kTileBytes + kHalfBytes, &map_k, bar, 64, it_.h / p.group, ((kSplit ? it_.j0 : 0) + j) * kTile, it_.b);
+          tma_load_4d(sK + st * kTileBytes, &map_k, bar, 0, it_.h / p.group, ((kMode == kSplit ? it_.j0 : 0) + j) * kTile, it_.b);
+          tma_load_4d(sK + st * kTileBytes + kHalfBytes, &map_k, bar, 64, it_.h / p.group, ((kMode == kSplit ? it_.j0 : 0) + j) * kTile, it_.b);
         }
       }
       if (!ok) {
@@ -343,8 +369,9 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
       uint32_t vc = 0;
       Item it_;
       for (int it = 0; it < n_waves && ok; ++it) {
-        if (!get_item<kSplit>(it, p, &it_)) continue;
-        for (int j = 0; j < it_.n_max && ok; ++j, ++vc) {
+        if (!get_item<kMode>(it, p, &it_)) continue;
+        const int n_tiles = kOne ? it_.n_kv[0] + it_.n_kv[1] : it_.n_max;
+        for (int j = 0; j < n_tiles && ok; ++j, ++vc) {
           const int st = vc % kVStages;
           const uint32_t use = vc / kVStages;
           if (use > 0) {
@@ -353,8 +380,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
           }
           const uint32_t bar = smem_u32(&bars.v_full[st]);
           mbar_expect_tx(bar, kTileBytes);
-          tma_load_4d(sV + st * kTileBytes, &map_v, bar, 0, it_.h / p.group, ((kSplit ? it_.j0 : 0) + j) * kTile, it_.b);
-          tma_load_4d(sV + st * kTileBytes + kHalfBytes, &map_v, bar, 64, it_.h / p.group, ((kSplit ? it_.j0 : 0) + j) * kTile, it_.b);
+          tma_load_4d(sV + st * kTileBytes, &map_v, bar, 0, it_.h / p.group, ((kMode == kSplit ? it_.j0 : 0) + j) * kTile, it_.b);
+          tma_load_4d(sV + st * kTileBytes + kHalfBytes, &map_v, bar, 64, it_.h / p.group, ((kMode == kSplit ? it_.j0 : 0) + j) * kTile, it_.b);
         }
       }
       if (!ok) {
@@ -387,32 +414,47 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
       uint32_t on[2] = {0, 0};      // items of tile t before this one (parity of q_full, o_free)
       Item it_;
       for (int it = 0; it < n_waves && ok; ++it) {
-        if (!get_item<kSplit>(it, p, &it_)) continue;
+        if (!get_item<kMode>(it, p, &it_)) continue;
         const int n_max = it_.n_max;
-        for (int t = 0; t < 2 && ok; ++t) {
+        for (int t = 0; t < Rings<kMode>::kQTiles && ok; ++t) {
           if (it_.n_kv[t] > 0) ok = wait_all(&bars.q_full[t], on[t] & 1, 3);
         }
         for (int j = 0; j <= n_max && ok; ++j) {
           const int jp = j - 1;  // the tile whose P.V is issued in this iteration
           const bool have_k = j < n_max, have_v = jp >= 0;
-          const uint32_t kidx = kc + j, vidx = vc + (have_v ? jp : 0);
-          const int st = kidx % kKStages, stp = vidx % kVStages;
           const bool pv0 = have_v && jp < it_.n_kv[0], pv1 = have_v && jp < it_.n_kv[1];
-          // probe everything this iteration needs at once; fall back to a proper wait on a miss
-          const bool k_hit = !have_k || mbar_try_wait(smem_u32(&bars.k_full[st]), (kidx / kKStages) & 1);
-          const bool v_hit = !have_v || mbar_try_wait(smem_u32(&bars.v_full[stp]), (vidx / kVStages) & 1);
-          const bool p0_hit = !pv0 || mbar_try_wait(smem_u32(&bars.p_ready[0]), (sn[0] + jp) & 1);
-          if (!__all_sync(0xffffffffu, k_hit)) ok = wait_all(&bars.k_full[st], (kidx / kKStages) & 1, 4);
-          if (ok && !__all_sync(0xffffffffu, v_hit)) ok = wait_all(&bars.v_full[stp], (vidx / kVStages) & 1, 5);
-          if (!ok) break;
-          const uint64_t kdesc = umma_smem_desc_sw128(sK + st * kTileBytes, 16, 1024);
-          const uint64_t vdesc = umma_smem_desc_sw128(sV + stp * kTileBytes, kHalfBytes, 1024);
+          uint32_t kidx = kc + j, vidx = vc + (have_v ? jp : 0);
+          bool p0_hit = false;
+          if constexpr (!kOne) {
+            const int st = kidx % kKStages, stp = vidx % kVStages;
+            // probe everything this iteration needs at once; fall back to a proper wait on a miss
+            const bool k_hit = !have_k || mbar_try_wait(smem_u32(&bars.k_full[st]), (kidx / kKStages) & 1);
+            const bool v_hit = !have_v || mbar_try_wait(smem_u32(&bars.v_full[stp]), (vidx / kVStages) & 1);
+            p0_hit = !pv0 || mbar_try_wait(smem_u32(&bars.p_ready[0]), (sn[0] + jp) & 1);
+            if (!__all_sync(0xffffffffu, k_hit)) ok = wait_all(&bars.k_full[st], (kidx / kKStages) & 1, 4);
+            if (ok && !__all_sync(0xffffffffu, v_hit)) ok = wait_all(&bars.v_full[stp], (vidx / kVStages) & 1, 5);
+            if (!ok) break;
+          }
 #pragma unroll
           for (int t = 0; t < 2; ++t) {
             const uint32_t tS = tbase + t * 128;          // S_t, and P_t in its first 64 columns
             const uint32_t tO = tbase + 256 + t * 128;    // O_t
             const bool pv = t == 0 ? pv0 : pv1;
             const bool qk = j < it_.n_kv[t];
+            if constexpr (kOne) {  // every step of either slot has K and V tiles of its own
+              kidx = kc + 2 * j + t;
+              vidx = vc + 2 * (have_v ? jp : 0) + t;
+            }
+            const int st = kidx % kKStages, stp = vidx % kVStages;
+            const uint64_t kdesc = umma_smem_desc_sw128(sK + st * kTileBytes, 16, 1024);
+            const uint64_t vdesc = umma_smem_desc_sw128(sV + stp * kTileBytes, kHalfBytes, 1024);
+            if constexpr (kOne) {
+              const bool k_hit = !qk || mbar_try_wait(smem_u32(&bars.k_full[st]), (kidx / kKStages) & 1);
+              const bool v_hit = !pv || mbar_try_wait(smem_u32(&bars.v_full[stp]), (vidx / kVStages) & 1);
+              if (!__all_sync(0xffffffffu, k_hit)) ok = wait_all(&bars.k_full[st], (kidx / kKStages) & 1, 4);
+              if (ok && !__all_sync(0xffffffffu, v_hit)) ok = wait_all(&bars.v_full[stp], (vidx / kVStages) & 1, 5);
+              if (!ok) break;
+            }
             if (pv) {
               if (t == 1 || !__all_sync(0xffffffffu, p0_hit)) {
                 ok = wait_all(&bars.p_ready[t], (sn[t] + jp) & 1, 6);
@@ -434,10 +476,10 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
                 }
                 // O_t is complete after its last P.V; the V stage is free after the last P.V reading it
                 if (jp == it_.n_kv[t] - 1) umma_commit(smem_u32(&bars.o_done[t]));
-                if (t == 1 || !pv1) umma_commit(smem_u32(&bars.v_empty[stp]));
+                if (kOne || t == 1 || !pv1) umma_commit(smem_u32(&bars.v_empty[stp]));
               }
               if (qk) {
-                const uint64_t qdesc = umma_smem_desc_sw128(sQ + t * kTileBytes, 16, 1024);
+                const uint64_t qdesc = umma_smem_desc_sw128(sQ + (kOne ? 0 : t) * kTileBytes, 16, 1024);
 #pragma unroll
                 for (int kk = 0; kk < 8; ++kk) {
                   const uint64_t off = static_cast<uint64_t>((kk & 3) * 2 + (kk >> 2) * (kHalfBytes >> 4));
@@ -445,15 +487,19 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
                 }
                 umma_commit(smem_u32(&bars.s_full[t]));
                 // the K stage is free after the last QK^T that reads it; Q_t after its last QK^T
-                if (t == 1 || j >= it_.n_kv[1]) umma_commit(smem_u32(&bars.k_empty[st]));
-                if (j == it_.n_kv[t] - 1) umma_commit(smem_u32(&bars.q_empty[t]));
+                if (kOne || t == 1 || j >= it_.n_kv[1]) umma_commit(smem_u32(&bars.k_empty[st]));
+                if (kOne) {
+                  if (2 * j + t == it_.n_kv[0] + it_.n_kv[1] - 1) umma_commit(smem_u32(&bars.q_empty[0]));
+                } else if (j == it_.n_kv[t] - 1) {
+                  umma_commit(smem_u32(&bars.q_empty[t]));
+                }
               }
             }
             __syncwarp();
           }
         }
-        kc += n_max;
-        vc += n_max;
+        kc += kOne ? it_.n_kv[0] + it_.n_kv[1] : n_max;
+        vc += kOne ? it_.n_kv[0] + it_.n_kv[1] : n_max;
         for (int t = 0; t < 2; ++t) {
           sn[t] += it_.n_kv[t];
           if (it_.n_kv[t] > 0) ++on[t];
@@ -476,10 +522,10 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
     uint32_t sn = 0;  // tile steps of this tile before the current item
     uint32_t on = 0;  // items of this tile before the current one
     Item it_;
-    for (int it = 0; it < n_waves && ok; ++it) {
-      if (!get_item<kSplit>(it, p, &it_)) continue;
+    for (int it = 0; it < n_waves && (ok || kOne); ++it) {
+      if (!get_item<kMode>(it, p, &it_)) continue;
       const int n_t = it_.n_kv[t];
-      if (n_t == 0) continue;
+      if (n_t == 0 && !kOne) continue;
       const int row = it_.q0[t] + r_in_tile;
       int lim = p.Skv - 1;
       if (p.causal) lim = min(lim, row + p.diag_off);
@@ -492,7 +538,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
         ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&bars.s_full[t]), (sn + j) & 1, abortp));
         if (!ok) { if (lane == 0) record_timeout(p.status, 7); break; }
         tc_fence_after_sync();
-        const int jk = ((kSplit ? it_.j0 : 0) + j) * kTile;  // first key of this tile
+        const int jk = (kOne ? 2 * j + t : (kMode == kSplit ? it_.j0 : 0) + j) * kTile;  // first key of this tile
         const bool masked_tile = jk + kTile - 1 > tile_min_lim;
         const int thr = lim - jk;  // columns > thr of this tile are masked for this row
 
@@ -634,6 +680,78 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
         tc_fence_before_sync();
         mbar_arrive(smem_u32(&bars.p_ready[t]));
       }
+      if constexpr (kOne) {
+        // ---- epilogue of a one-tile item: the first slot gets the second's exponent reference and row sum
+        // and hands back the factors of both accumulators; each slot writes half of the output columns
+        if (n_t > 0 && ok) {
+          ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&bars.o_done[t]), on & 1, abortp));
+          if (!ok && lane == 0) record_timeout(p.status, 9);
+          tc_fence_after_sync();
+        }
+        // (every softmax warp gets to the barriers for every item, expired waits or not)
+        float f0, f1;
+        if (t == 1) row_s[r_in_tile] = make_float2(l > 0.f ? m_ref : -INFINITY, l);
+        tc_fence_before_sync();
+        named_bar_sync(1, 256);
+        if (t == 0) {
+          const float2 c = row_s[r_in_tile];
+          const float m0 = l > 0.f ? m_ref : -INFINITY;
+          const float mm = fmaxf(m0, c.x);
+          const float w0 = l > 0.f ? ex2(m0 - mm) : 0.f, w1 = c.y > 0.f ? ex2(c.x - mm) : 0.f;
+          const float lsum = l * w0 + c.y * w1;
+          f0 = w0 / lsum;
+          f1 = w1 / lsum;
+          row_s[r_in_tile] = make_float2(f0, f1);
+          if (p.lse2 != nullptr && row < p.Sq)
+            p.lse2[(static_cast<size_t>(it_.b) * p.H + it_.h) * p.Sq + row] = mm + log2f(lsum);
+        }
+        named_bar_sync(1, 256);
+        tc_fence_after_sync();
+        if (t == 1) {
+          f0 = row_s[r_in_tile].x;
+          f1 = row_s[r_in_tile].y;
+        }
+        const bool both = it_.n_kv[1] > 0;
+        uint16_t* orow = static_cast<uint16_t*>(p.out) + static_cast<int64_t>(it_.b) * p.o_sb +
+                         static_cast<int64_t>(row) * p.o_ss + static_cast<int64_t>(it_.h) * p.o_sh + t * 64;
+        const uint32_t tA = tbase + lane_base + 256 + t * 64;
+#pragma unroll
+        for (int c4 = 0; c4 < 2; ++c4) {
+          uint32_t o0[32], o1[32];
+          tmem_ld32(tA + c4 * 32, o0);
+          if (both) tmem_ld32(tA + 128 + c4 * 32, o1);
+          tmem_wait_ld();
+          if (c4 == 1) {
+            // both accumulators are in registers: the next item's first P.V may overwrite them
+            tc_fence_before_sync();
+            mbar_arrive(smem_u32(&bars.o_free[0]));
+            if (both) mbar_arrive(smem_u32(&bars.o_free[1]));
+          }
+          uint32_t w[16];
+#pragma unroll
+          for (int g = 0; g < 16; ++g) {
+            float x = __uint_as_float(o0[2 * g]) * f0, y = __uint_as_float(o0[2 * g + 1]) * f0;
+            if (both) {
+              x = fmaf(__uint_as_float(o1[2 * g]), f1, x);
+              y = fmaf(__uint_as_float(o1[2 * g + 1]), f1, y);
+            }
+            w[g] = pack2<kBF16>(x, y);
+          }
+          if (row < p.Sq) {
+            if (p.out_vec32) {
+              st_global_v8(orow + c4 * 32, *reinterpret_cast<const uint32_t(*)[8]>(&w[0]));
+              st_global_v8(orow + c4 * 32 + 16, *reinterpret_cast<const uint32_t(*)[8]>(&w[8]));
+            } else {
+#pragma unroll
+              for (int g = 0; g < 4; ++g)
+                *reinterpret_cast<uint4*>(orow + c4 * 32 + g * 8) = make_uint4(w[4 * g], w[4 * g + 1], w[4 * g + 2], w[4 * g + 3]);
+            }
+          }
+        }
+        sn += n_t;
+        if (n_t > 0) ++on;
+        continue;
+      }
       if (!ok) break;
 
       // ---- epilogue of the item: O_t / l straight from TMEM to global memory
@@ -641,9 +759,9 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
       if (!ok) { if (lane == 0) record_timeout(p.status, 9); break; }
       tc_fence_after_sync();
 #ifdef ASUKA_REDECODE
-      get_item<kSplit>(it, p, &it_);  // (decoded again rather than kept in registers across the key loop)
+      get_item<kMode>(it, p, &it_);  // (decoded again rather than kept in registers across the key loop)
 #endif
-      if (kSplit && it_.nparts[t] > 1) {
+      if (kMode == kSplit && it_.nparts[t] > 1) {
         // this tile's keys are shared with other items: leave the unnormalised O, the exponent
         // reference and the row sum for the merge (a row that saw no key in this part has l = 0
         // and must not set the scale: its reference goes out as -inf)
@@ -787,14 +905,13 @@ __global__ void __launch_bounds__(kMergeWarps * 32) attn_merge_kernel(const FwdP
 
 }  // namespace
 
-// How many parts the key range of every work item is cut into.  Splitting pays only when the
-// launch has fewer items than SMs and the items are long (measured at head counts of 4 to 32 and
-// S = 1024 to 4096: the partial results cost about as much L2 traffic again as the inputs); it
-// needs workspace for the parts' partial results.
+// How many parts the key range of every two-tile item is cut into (kSplit).  Partial results cost about as
+// much L2 traffic again as the inputs and the merge is a launch of its own, so this is only for launches
+// whose query tiles would leave half of the SMs idle even at one tile per CTA, and long key ranges
+// (measured at head counts of 4 to 32 and S = 1024 to 4096); it needs workspace.
 int attn_fwd_parts(const AttnShape& s, int num_sms, size_t ws_bytes) {
   if (attn_decode_applies(s)) return 1;  // (attn_decode.cu splits the keys itself)
-  const long long nq_blocks = (s.Sq + 2 * kTile - 1) / (2 * kTile);
-  const long long n_items = nq_blocks * s.B * s.H;
+  const long long n_tiles = static_cast<long long>((s.Sq + kTile - 1) / kTile) * s.B * s.H;
   const int max_tiles = (s.Skv + kTile - 1) / kTile;
   int parts = 1;
 #ifdef ASUKA_TUNE_ENV
@@ -804,9 +921,29 @@ int attn_fwd_parts(const AttnShape& s, int num_sms, size_t ws_bytes) {
     return parts;
   }
 #endif
-  if (n_items < num_sms && max_tiles >= 32) parts = 2 * n_items <= num_sms ? 4 : 2;
+  if (2 * n_tiles <= num_sms && max_tiles >= 32) parts = 4;
   while (parts > 1 && attn_fwd_split_bytes(s, parts) > ws_bytes) parts /= 2;
   return parts;
+}
+
+// One query tile per item (kSolo).  Two tiles of an item keep the tensor pipe and the MUFU busy as long as
+// both have keys left, and share every K/V tile; but an item is then as long as its later tile.  One tile
+// whose keys the two slots share is done in half the rounds, at twice the K/V traffic per step: with every
+// SM at work a round takes 1.28 times as long (S = 2048, 64 heads: 80 -> 105 us).  So:
+//   - one tile per SM or fewer, three or more key tiles: always.  Measured (us): 500 rows over 5003 keys,
+//     32/8 heads 86 -> 55; S 1024, 8 heads 22.6 -> 16.7; S 512, 4 heads 15.0 -> 12.4 (a single key tile:
+//     8.9 -> 10.3); unmasked S 2048, 8 heads 35.0 -> 26.7
+//   - up to two tiles per SM, if the launch is a causal square of at least twelve tiles: its late tiles are
+//     twice as long as the mean and the early ones fill in behind them.  S 4096, 8 heads 67.7 -> 47.2;
+//     S 2048, 16 heads 37.6 -> 30.8 (S 1024, 32 heads 22.8 -> 24.7; 1024 rows over 8000 keys 117 -> 148)
+static bool attn_fwd_solo(const AttnShape& s, int num_sms) {
+#ifdef ASUKA_TUNE_ENV
+  if (const char* e = getenv("ASUKA_FWD_SOLO")) return atoi(e) != 0;
+#endif
+  const int nq_tiles = (s.Sq + kTile - 1) / kTile;
+  const long long n_tiles = static_cast<long long>(nq_tiles) * s.B * s.H;
+  if (n_tiles <= num_sms) return s.Skv > 2 * kTile;
+  return s.causal && n_tiles <= 2 * num_sms && nq_tiles >= 12 && 4LL * s.Skv <= 5LL * s.Sq;
 }
 
 size_t attn_fwd_split_bytes(const AttnShape& s, int parts) {
@@ -827,21 +964,14 @@ cudaError_t launch_attn_fwd(const CUtensorMap& mq, const CUtensorMap& mk, const 
   p.diag_off = s.Skv - s.Sq;
   p.nq_blocks = (s.Sq + 2 * kTile - 1) / (2 * kTile);
   p.parts = parts > 1 && split_ws != nullptr ? (parts < kMaxParts ? parts : kMaxParts) : 1;
-  p.n_items = p.nq_blocks * s.B * s.H * p.parts;
   p.nq_tiles = (s.Sq + kTile - 1) / kTile;
+  const bool solo = p.parts == 1 && attn_fwd_solo(s, num_sms);
+  p.n_items = solo ? p.nq_tiles * s.B * s.H : p.nq_blocks * s.B * s.H * p.parts;
   {
     const double kv_bytes = 2.0 * s.B * (s.H / (s.group > 0 ? s.group : 1)) * static_cast<double>(s.Skv) * 128 * 2;
-#ifdef ASUKA_FWD_NO_UNIT_MAJOR
-    p.unit_major = 0;
-#else
     p.unit_major = (p.parts == 1 && p.n_items > num_sms && kv_bytes > 96e6) ? 1 : 0;
-#endif
   }
-#ifdef ASUKA_FWD_NO_PAIR_FAR
-  p.pair_far = 0;
-#else
-  p.pair_far = (p.parts == 1 && s.causal && p.n_items <= num_sms && p.nq_tiles >= 4) ? 1 : 0;
-#endif
+  p.pair_far = (p.parts == 1 && !solo && s.causal && p.n_items <= num_sms && p.nq_tiles >= 4) ? 1 : 0;
   p.group = s.group;
   p.scale_log2 = s.softmax_scale * 1.4426950408889634f;
   p.cap_in = s.softcap > 0.f ? s.softmax_scale / s.softcap : 0.f;
@@ -856,14 +986,14 @@ cudaError_t launch_attn_fwd(const CUtensorMap& mq, const CUtensorMap& mk, const 
   p.part_o = static_cast<float*>(split_ws);
   p.part_ml = p.part_o + static_cast<size_t>(s.B) * s.H * s.Sq * p.parts * 128;
   const dim3 grid(static_cast<unsigned>(p.n_items < num_sms ? p.n_items : num_sms));
-  void (*kern)(CUtensorMap, CUtensorMap, CUtensorMap, FwdParams);
-  if (p.parts > 1) {
-    if (s.softcap > 0.f) kern = s.bf16 ? attn_fwd_kernel<true, true, true> : attn_fwd_kernel<false, true, true>;
-    else kern = s.bf16 ? attn_fwd_kernel<true, false, true> : attn_fwd_kernel<false, false, true>;
-  } else {
-    if (s.softcap > 0.f) kern = s.bf16 ? attn_fwd_kernel<true, true, false> : attn_fwd_kernel<false, true, false>;
-    else kern = s.bf16 ? attn_fwd_kernel<true, false, false> : attn_fwd_kernel<false, false, false>;
-  }
+  auto pick = [&](auto mode) -> void (*)(CUtensorMap, CUtensorMap, CUtensorMap, FwdParams) {
+    constexpr int kMode = decltype(mode)::value;
+    if (s.softcap > 0.f) return s.bf16 ? attn_fwd_kernel<true, true, kMode> : attn_fwd_kernel<false, true, kMode>;
+    return s.bf16 ? attn_fwd_kernel<true, false, kMode> : attn_fwd_kernel<false, false, kMode>;
+  };
+  const auto kern = p.parts > 1 ? pick(std::integral_constant<int, kSplit>())
+                    : solo      ? pick(std::integral_constant<int, kSolo>())
+                                : pick(std::integral_constant<int, kPair>());
   cudaError_t e = ensure_dynamic_smem(reinterpret_cast<const void*>(kern), kSmemBytes);
   if (e != cudaSuccess) return e;
   e = check_register_budget(reinterpret_cast<const void*>(kern), kThreads, 128 * kUtilRegs + 256 * kSoftmaxRegs);
