@@ -392,6 +392,9 @@ int prep_sima(const asuka_sima_params* p, SimaShape* sh) {
   sh->out_f32 = p->out.dtype == ASUKA_F32;
   sh->ea = false;
   if (static_cast<int64_t>(sh->B) * sh->H > (1 << 20)) return ASUKA_ERR_TOO_LARGE;
+  if (static_cast<int64_t>(sh->B) * sh->H * ((sh->S + 127) / 128) > 0x3fffffff) return ASUKA_ERR_TOO_LARGE;
+  const int sms = sm_count();
+  sh->num_sms = sms > 0 ? sms : 148;  // (without a device only the sizes are asked for)
   return ASUKA_OK;
 }
 

@@ -174,6 +174,7 @@ struct SimaShape {
   bool bf16;
   bool out_f32;
   bool ea;  // the EA program (softmax normalisations) instead of SimA (L1 normalisations)
+  int num_sms;
 };
 size_t sima_workspace_bytes(const SimaShape& s);
 cudaError_t launch_sima(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv,

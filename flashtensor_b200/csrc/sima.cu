@@ -19,6 +19,8 @@
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 
+#include <algorithm>
+
 #include "kernels.h"
 #include "sm100_ptx.cuh"
 #include "tma_host.h"
@@ -39,8 +41,8 @@ __device__ __forceinline__ void record_timeout(uint32_t* status, uint32_t site) 
 }
 
 struct SimaWs {
-  float* part_m;     // [BH][nchunks][e][d]  partial (K^T V)^T
-  float* part_c;     // [BH][nchunks][2][128] partial ck, cq
+  float* part_m;     // [BH][max_slots][e][d]  partial (K^T V)^T
+  float* part_c;     // [BH][max_slots][2][128] partial ck, cq
   uint16_t* m16;     // [BH][e][d] scaled M'^T in the input type
   float* inv_scale;  // [BH][4]: one per block of 32 output channels
 };
@@ -52,16 +54,30 @@ constexpr int kStThreads = 384;
 constexpr int kStStages = 2;
 constexpr uint32_t kStSmem = kStStages * 3 * kTileBytes + 1024;
 
+// How the statistics and the output kernel divide their work: the tiles of all units in a row, CTA r takes
+// [r T / G, (r + 1) T / G).  Every CTA gets the same number of tiles to within one, whatever the number of
+// units; a CTA's run crosses from one unit into the next where it falls ("segments").  (A fixed number of
+// slabs per unit left 64 units of 40 tiles in 2.2 waves of CTAs: a quarter of the time for the last one.)
+struct Share {
+  int total, ctas, ntiles;  // T, G, tiles per unit
+  __host__ __device__ int lo(int r) const { return static_cast<int>(static_cast<int64_t>(total) * r / ctas); }
+  __host__ __device__ int owner(int t) const {  // the CTA whose run holds tile t
+    return static_cast<int>((static_cast<int64_t>(t + 1) * ctas - 1) / total);
+  }
+};
+
 struct StatsParams {
   int B, H, S;
-  int nchunks, tiles_per_chunk, ntiles;
+  Share share;
+  int max_slots;     // partial results of a unit in the workspace; slot = CTA - first CTA of the unit
   int ea;            // 1: the EA program (softmax normalisations), 0: SimA (L1 normalisations)
   SimaWs ws;
   uint32_t* status;
 };
 
 struct StBars {
-  uint64_t full[3], empty[3], m_done;  // (two stages in SimA mode, three in EA mode)
+  uint64_t full[3], empty[3];          // (two stages in SimA mode, three in EA mode)
+  uint64_t m_done[2], acc_empty[2];    // accumulators of alternate segments
   uint64_t ktrans[3];                  // EA only: the K tile of the stage has been exponentiated in place
 };
 
@@ -196,11 +212,7 @@ sima_stats_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   volatile uint32_t* abortp = &abort_s;
-  const int chunk = static_cast<int>(blockIdx.x) % p.nchunks;
-  const int bh = static_cast<int>(blockIdx.x) / p.nchunks;
-  const int b = bh / p.H, h = bh % p.H;
-  const int tile0 = chunk * p.tiles_per_chunk;
-  const int ntile = max(0, min(p.tiles_per_chunk, p.ntiles - tile0));
+  const int t_lo = p.share.lo(static_cast<int>(blockIdx.x)), t_hi = p.share.lo(static_cast<int>(blockIdx.x) + 1);
 
   if (tid == 0) {
     abort_s = 0;
@@ -208,7 +220,10 @@ sima_stats_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
       mbar_init(smem_u32(&bars.full[i]), 1);
       mbar_init(smem_u32(&bars.empty[i]), 1 + 8);
     }
-    mbar_init(smem_u32(&bars.m_done), 1);
+    for (int i = 0; i < 2; ++i) {
+      mbar_init(smem_u32(&bars.m_done[i]), 1);
+      mbar_init(smem_u32(&bars.acc_empty[i]), 128);
+    }
     for (int i = 0; i < kSt; ++i) mbar_init(smem_u32(&bars.ktrans[i]), 256);
     mbar_fence_init();
   }
@@ -216,7 +231,7 @@ sima_stats_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
     for (int i = tid; i < 1024; i += kStThreads) ones_s[i] = kBF16 ? 0x3F80 : 0x3C00;
     fence_proxy_async_smem();
   }
-  constexpr uint32_t kTmemCols = kEA ? 256 : 128;  // EA: columns 128.. hold the column sums
+  constexpr uint32_t kTmemCols = 512;  // two accumulators, 256 columns apart; EA: 128.. of each hold the column sums
   if (warp == 1) {
     __syncwarp();
     tmem_alloc(smem_u32(&tmem_base_s), kTmemCols);
@@ -226,12 +241,15 @@ sima_stats_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tbase = tmem_base_s;
+  griddep_wait();               // k, v and q may be the output of the kernel ahead
+  griddep_launch_dependents();
 
-  // stage layout: [K | V | Q] tiles
+  // stage layout: [K | V | Q] tiles; k counts this CTA's tiles through all its segments
   if (warp == 0) {
     if (lane == 0) {
-      for (int i = 0; i < ntile; ++i) {
-        const int k = i;
+      for (int k = 0; k < t_hi - t_lo; ++k) {
+        const int unit = (t_lo + k) / p.share.ntiles;
+        const int b = unit / p.H, h = unit % p.H;
         const int st = k % kSt;
         if (k >= kSt && !mbar_wait(smem_u32(&bars.empty[st]), (k / kSt - 1) & 1, abortp)) {
           record_timeout(p.status, 41);
@@ -239,7 +257,7 @@ sima_stats_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
         }
         const uint32_t bar = smem_u32(&bars.full[st]);
         const uint32_t base = smem_base + st * kStageBytes;
-        const int s0 = (tile0 + i) * kTile;
+        const int s0 = (t_lo + k - unit * p.share.ntiles) * kTile;
         mbar_expect_tx(bar, (kEA ? 2 : 3) * kTileBytes);
         if constexpr (kEA) {
           const uint64_t drop = l2_policy_evict_first();
@@ -265,13 +283,22 @@ sima_stats_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
       constexpr uint32_t kFmt = kBF16 ? UMMA_BF16 : UMMA_F16;
       constexpr uint32_t idesc = umma_idesc_f16(kFmt, UMMA_MN_MAJOR, UMMA_MN_MAJOR, 128, 128);
       bool ok = true;
-      for (int i = 0; i < ntile && ok; ++i) {
-        const int k = i;
+      int seg = 0;
+      uint32_t acc = tbase;
+      for (int k = 0; k < t_hi - t_lo && ok; ++k) {
+        const int i = (t_lo + k) % p.share.ntiles;           // tile within the unit
+        const bool first = k == 0 || i == 0;                 // of the segment
+        const bool last = k == t_hi - t_lo - 1 || i == p.share.ntiles - 1;
         const int st = k % kSt;
+        acc = tbase + (seg & 1) * 256;
+        if (first && seg >= 2) {
+          ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&bars.acc_empty[seg & 1]), ((seg >> 1) - 1) & 1, abortp));
+          if (!ok) { if (lane == 0) record_timeout(p.status, 47); break; }
+        }
         ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&bars.full[st]), (k / kSt) & 1, abortp));
         if (!ok) { if (lane == 0) record_timeout(p.status, 42); break; }
         if constexpr (kEA) {
-          ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&bars.ktrans[i % kSt]), (i / kSt) & 1, abortp));
+          ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&bars.ktrans[st]), (k / kSt) & 1, abortp));
           if (!ok) { if (lane == 0) record_timeout(p.status, 45); break; }
         }
         tc_fence_after_sync();
@@ -283,7 +310,7 @@ sima_stats_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
 #pragma unroll
           for (int kk = 0; kk < 8; ++kk) {
             const uint64_t off = static_cast<uint64_t>(kk * (2048 >> 4));
-            umma_ss(tbase, adesc + off, bdesc + off, idesc, (i > 0 || kk > 0) ? 1u : 0u);
+            umma_ss(acc, adesc + off, bdesc + off, idesc, (!first || kk > 0) ? 1u : 0u);
           }
           if constexpr (kEA) {
             // column sums of the exponentiated (and rounded) K: the same A against 16 columns of ones
@@ -292,15 +319,15 @@ sima_stats_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
 #pragma unroll
             for (int kk = 0; kk < 8; ++kk) {
               const uint64_t off = static_cast<uint64_t>(kk * (2048 >> 4));
-              umma_ss(tbase + 128, adesc + off, odesc, idesc16, (i > 0 || kk > 0) ? 1u : 0u);
+              umma_ss(acc + 128, adesc + off, odesc, idesc16, (!first || kk > 0) ? 1u : 0u);
             }
           }
           umma_commit(smem_u32(&bars.empty[st]));
+          if (last) umma_commit(smem_u32(&bars.m_done[seg & 1]));
         }
         __syncwarp();
+        if (last) ++seg;
       }
-      if (ok && elect_one()) umma_commit(smem_u32(&bars.m_done));
-      __syncwarp();
     }
   } else if (warp >= 4) {
     // warps 4-7: |K| column sums; warps 8-11: |Q| column sums
@@ -308,8 +335,16 @@ sima_stats_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
     const int t128 = tid - 128 - which * 128;
     const int chunk16 = t128 & 15;   // 8 consecutive channels
     const int rg = t128 >> 4;        // rows rg, rg+8, ...
-    float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
     bool ok = true;
+    bool dead = false;  // (EA) a wait has given up: no more work, but every barrier is still taken
+    int seg = 0;
+    for (int t = t_lo, ntile; t < t_hi; t += ntile, ++seg) {
+    const int bh = t / p.share.ntiles, tile0 = t - bh * p.share.ntiles;
+    ntile = min(t_hi - t, p.share.ntiles - tile0);
+    const int k0 = t - t_lo;  // tiles of the segments before this one
+    const size_t part = static_cast<size_t>(bh) * p.max_slots + (static_cast<int>(blockIdx.x) - p.share.owner(bh * p.share.ntiles));
+    const uint32_t tacc = tbase + (seg & 1) * 256;
+    float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
     if constexpr (kEA) {
       // All 256 threads work on the K tile, rows 16 apart per thread: k' = exp(k - ref), rounded to
       // the input type and written back for the MMA; rows past the sequence give 0.  `ref` is a
@@ -322,10 +357,9 @@ sima_stats_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
       const float kL2e = 1.4426950408889634f;
       float2 nref[4] = {};   // -ref * log2(e) of this thread's eight channels
       uint32_t thr[4] = {};  // ref + kEaSlack in the input type, packed
-      bool dead = false;     // a wait has given up: no more work, but every barrier is still taken
       for (int i = 0; i < ntile; ++i) {
-        const int st = i % kSt;
-        if (!__all_sync(0xffffffffu, mbar_wait(smem_u32(&bars.full[st]), (i / kSt) & 1, abortp))) {
+        const int k = k0 + i, st = k % kSt;
+        if (!__all_sync(0xffffffffu, mbar_wait(smem_u32(&bars.full[st]), (k / kSt) & 1, abortp))) {
           if (lane == 0 && !dead) record_timeout(p.status, 43);
           dead = true;
         }
@@ -367,7 +401,7 @@ sima_stats_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
             if (i > 0) {
               // every MMA issued so far has retired once the release of the previous tile's stage
               // has fired (the MMA of this tile waits for the arrivals below)
-              if (!__all_sync(0xffffffffu, mbar_wait(smem_u32(&bars.empty[(i - 1) % kSt]), ((i - 1) / kSt) & 1, abortp))) {
+              if (!__all_sync(0xffffffffu, mbar_wait(smem_u32(&bars.empty[(k - 1) % kSt]), ((k - 1) / kSt) & 1, abortp))) {
                 if (lane == 0 && !dead) record_timeout(p.status, 46);
                 dead = true;
               }
@@ -378,18 +412,18 @@ sima_stats_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
 #pragma unroll
                 for (int c = 0; c < 4; ++c) {
                   uint32_t u[32];
-                  tmem_ld32(tbase + lane_base + c * 32, u);
+                  tmem_ld32(tacc + lane_base + c * 32, u);
                   tmem_wait_ld();
 #pragma unroll
                   for (int x = 0; x < 32; ++x) u[x] = __float_as_uint(__uint_as_float(u[x]) * f);
-                  tmem_st32(tbase + lane_base + c * 32, u);
+                  tmem_st32(tacc + lane_base + c * 32, u);
                 }
                 uint32_t u[16];
-                tmem_ld16(tbase + lane_base + 128, u);
+                tmem_ld16(tacc + lane_base + 128, u);
                 tmem_wait_ld();
 #pragma unroll
                 for (int x = 0; x < 16; ++x) u[x] = __float_as_uint(__uint_as_float(u[x]) * f);
-                tmem_st16(tbase + lane_base + 128, u);
+                tmem_st16(tacc + lane_base + 128, u);
                 tmem_wait_st();
                 tc_fence_before_sync();
               }
@@ -431,9 +465,9 @@ sima_stats_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
       }
       ok = !dead;
     } else {
-      for (int i = 0; i < ntile; ++i) {
-        const int st = i % kSt;
-        ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&bars.full[st]), (i / kSt) & 1, abortp));
+      for (int i = 0; i < ntile && ok; ++i) {
+        const int k = k0 + i, st = k % kSt;
+        ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&bars.full[st]), (k / kSt) & 1, abortp));
         if (!ok) { if (lane == 0) record_timeout(p.status, 43); break; }
         const uint8_t* tile = smem_gen + st * kStageBytes + (which ? 2 * kTileBytes : 0) +
                               (chunk16 >> 3) * kHalfBytes;
@@ -448,52 +482,52 @@ sima_stats_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
       }
     }
     if constexpr (kEA) {
-      // slot 1 of the partial (SimA's sum|Q|): the slab's per-column reference; slot 0 is written below
-      if (which == 1)
-        p.ws.part_c[((static_cast<size_t>(bh) * p.nchunks + chunk) * 2 + 1) * kTile + t128] = ref_s[t128];
+      // slot 1 of the partial (SimA's sum|Q|): the segment's per-column reference; slot 0 is written below
+      if (which == 1) p.ws.part_c[(part * 2 + 1) * kTile + t128] = ref_s[t128];
     } else {
 #pragma unroll
       for (int i = 0; i < 8; ++i) red[which][rg][chunk16 * 8 + i] = acc[i];
       named_bar_sync(1 + which, 128);
-      float s = 0.f;
+      float sum = 0.f;
 #pragma unroll
-      for (int g = 0; g < 8; ++g) s += red[which][g][t128];
-      p.ws.part_c[((static_cast<size_t>(bh) * p.nchunks + chunk) * 2 + which) * kTile + t128] = s;
+      for (int g = 0; g < 8; ++g) sum += red[which][g][t128];
+      p.ws.part_c[(part * 2 + which) * kTile + t128] = sum;
+      named_bar_sync(1 + which, 128);  // (the next segment writes red)
     }
     if (which == 0) {
       // warps 4-7 also drain the accumulator: lane = d, column = e
-      float* dst = p.ws.part_m + (static_cast<size_t>(bh) * p.nchunks + chunk) * kMElems;
+      float* dst = p.ws.part_m + part * kMElems;
       const int wq = warp & 3;
       const int d = wq * 32 + lane;
-      if (ntile > 0) {
-        ok = ok && __all_sync(0xffffffffu, mbar_wait(smem_u32(&bars.m_done), 0, abortp));
-        if (ok) {
-          tc_fence_after_sync();
-#pragma unroll
-          for (int c = 0; c < 4; ++c) {
-            uint32_t u[32];
-            tmem_ld32(tbase + (static_cast<uint32_t>(wq * 32) << 16) + c * 32, u);
-            tmem_wait_ld();
-            // thread d holds M[d][e..]; element (d, e) -> dst[e * 128 + d]: consecutive threads
-            // hit consecutive addresses and the partial is stored transposed, [e][d]
-#pragma unroll
-            for (int i = 0; i < 32; ++i) dst[(c * 32 + i) * kTile + d] = __uint_as_float(u[i]);
-          }
-          if constexpr (kEA) {
-            // slot 0: this slab's part of the softmax denominators (relative to the slab's maxima)
-            uint32_t u[16];
-            tmem_ld16(tbase + (static_cast<uint32_t>(wq * 32) << 16) + 128, u);
-            tmem_wait_ld();
-            p.ws.part_c[((static_cast<size_t>(bh) * p.nchunks + chunk) * 2 + 0) * kTile + d] = __uint_as_float(u[0]);
-          }
-        } else if (lane == 0) {
-          record_timeout(p.status, 44);
-        }
-      } else {
-        for (int i = 0; i < 128; ++i) dst[i * kTile + d] = 0.f;
-        if constexpr (kEA) p.ws.part_c[((static_cast<size_t>(bh) * p.nchunks + chunk) * 2 + 0) * kTile + d] = 0.f;
+      if (ok) {
+        ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&bars.m_done[seg & 1]), (seg >> 1) & 1, abortp));
+        if (!ok && lane == 0) record_timeout(p.status, 44);
       }
+      if (ok) {
+        tc_fence_after_sync();
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+          uint32_t u[32];
+          tmem_ld32(tacc + (static_cast<uint32_t>(wq * 32) << 16) + c * 32, u);
+          tmem_wait_ld();
+          // thread d holds M[d][e..]; element (d, e) -> dst[e * 128 + d]: consecutive threads
+          // hit consecutive addresses and the partial is stored transposed, [e][d]
+#pragma unroll
+          for (int i = 0; i < 32; ++i) dst[(c * 32 + i) * kTile + d] = __uint_as_float(u[i]);
+        }
+        if constexpr (kEA) {
+          // slot 0: this segment's part of the softmax denominators (relative to its references)
+          uint32_t u[16];
+          tmem_ld16(tacc + (static_cast<uint32_t>(wq * 32) << 16) + 128, u);
+          tmem_wait_ld();
+          p.ws.part_c[(part * 2 + 0) * kTile + d] = __uint_as_float(u[0]);
+        }
+        tc_fence_before_sync();
+        mbar_arrive(smem_u32(&bars.acc_empty[seg & 1]));
+      }
+      if constexpr (kEA) dead = dead || !ok;
     }
+    }  // segments
   }
 
   tc_fence_before_sync();
@@ -511,26 +545,29 @@ sima_stats_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
 // One CTA per (head, block of 32 output channels e): 4096 entries of M'^T, its own power-of-two
 // scale (the epilogue of step 3 multiplies each 32-column chunk by the matching inverse).
 constexpr int kRedBlocks = 4;
-constexpr int kMaxChunks = 16;  // slabs per (batch, head) in the three-kernel path
+constexpr int kMaxChunks = 16;  // partial results per (batch, head) in the three-kernel path
 constexpr int kRedElems = kMElems / kRedBlocks;
 template <bool kBF16>
 __global__ void __launch_bounds__(256, 4) sima_reduce_kernel(const StatsParams p) {
-  __shared__ float inv_c[kTile];
-  __shared__ float w_s[kMaxChunks][kTile];  // EA: exp(slab reference - largest reference), per slab and column
+  __shared__ __align__(16) float inv_c[kTile];
+  __shared__ __align__(16) float w_s[kMaxChunks][kTile];  // EA: exp(segment's reference - largest reference), per segment and column
   __shared__ float wmax[8];
   __shared__ float s_scale;
   const int blk = blockIdx.x % kRedBlocks;
   const int bh = blockIdx.x / kRedBlocks, tid = threadIdx.x;
-  const float* pc = p.ws.part_c + static_cast<size_t>(bh) * p.nchunks * 2 * kTile;
-  const float* pm = p.ws.part_m + static_cast<size_t>(bh) * p.nchunks * kMElems + blk * kRedElems;
+  const int nparts = p.share.owner((bh + 1) * p.share.ntiles - 1) - p.share.owner(bh * p.share.ntiles) + 1;
+  const float* pc = p.ws.part_c + static_cast<size_t>(bh) * p.max_slots * 2 * kTile;
+  const float* pm = p.ws.part_m + static_cast<size_t>(bh) * p.max_slots * kMElems + blk * kRedElems;
+  griddep_wait();               // the partial results are the output of the kernel ahead
+  griddep_launch_dependents();
   if (tid < kTile) {
     if (p.ea) {
-      // each slab's exponentials were taken against the slab's own per-column reference (slot 1):
+      // each segment's exponentials were taken against a per-column reference of its own (slot 1):
       // bring them to the largest of these
       float m = -INFINITY;
-      for (int c = 0; c < p.nchunks; ++c) m = fmaxf(m, pc[(c * 2 + 1) * kTile + tid]);
+      for (int c = 0; c < nparts; ++c) m = fmaxf(m, pc[(c * 2 + 1) * kTile + tid]);
       float ck = 0.f;
-      for (int c = 0; c < p.nchunks; ++c) {
+      for (int c = 0; c < nparts; ++c) {
         const float w = __expf(pc[(c * 2 + 1) * kTile + tid] - m);
         w_s[c][tid] = w;
         ck = fmaf(pc[(c * 2 + 0) * kTile + tid], w, ck);
@@ -538,28 +575,57 @@ __global__ void __launch_bounds__(256, 4) sima_reduce_kernel(const StatsParams p
       inv_c[tid] = __fdiv_rn(1.0f, ck);
     } else {
       float ck = 0.f, cq = 0.f;
-      for (int c = 0; c < p.nchunks; ++c) {
+      for (int c = 0; c < nparts; ++c) {
         ck += pc[(c * 2 + 0) * kTile + tid];
         cq += pc[(c * 2 + 1) * kTile + tid];
+        w_s[c][tid] = 1.f;
       }
       inv_c[tid] = __fdiv_rn(1.0f, __fmul_rn(ck, cq));
     }
   }
   __syncthreads();
-  float vals[kRedElems / 256];
-  float amax = 0.f;
+  // sixteen elements a thread, as four float4: all of a part's loads are in flight at once (the kernel is
+  // bound by their latency), parts are added in order
+  constexpr int kVec = kRedElems / 1024;
+  float vals[kVec][4];
+  const int d4 = (tid & 31) * 4;  // first of this thread's four d
 #pragma unroll
-  for (int it = 0; it < kRedElems / 256; ++it) {
-    const int idx = it * 256 + tid;  // = e_local * 128 + d
-    float m = 0.f;
-    if (p.ea) {
-      for (int c = 0; c < p.nchunks; ++c) m = fmaf(pm[static_cast<size_t>(c) * kMElems + idx], w_s[c][idx & 127], m);
-    } else {
-      for (int c = 0; c < p.nchunks; ++c) m += pm[static_cast<size_t>(c) * kMElems + idx];
+  for (int it = 0; it < kVec; ++it)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) vals[it][e] = 0.f;
+  float4 nxt[kVec];
+#pragma unroll
+  for (int it = 0; it < kVec; ++it) nxt[it] = __ldcg(reinterpret_cast<const float4*>(pm + (it * 256 + tid) * 4));
+  for (int c = 0; c < nparts; ++c) {
+    float4 cur[kVec];
+#pragma unroll
+    for (int it = 0; it < kVec; ++it) cur[it] = nxt[it];
+    if (c + 1 < nparts) {
+#pragma unroll
+      for (int it = 0; it < kVec; ++it)
+        nxt[it] = __ldcg(reinterpret_cast<const float4*>(pm + static_cast<size_t>(c + 1) * kMElems + (it * 256 + tid) * 4));
     }
-    m *= inv_c[idx & 127];
-    vals[it] = m;
-    amax = fmaxf(amax, fabsf(m));
+    const float4 w = *reinterpret_cast<const float4*>(&w_s[c][d4]);
+#pragma unroll
+    for (int it = 0; it < kVec; ++it) {
+      vals[it][0] = fmaf(cur[it].x, w.x, vals[it][0]);
+      vals[it][1] = fmaf(cur[it].y, w.y, vals[it][1]);
+      vals[it][2] = fmaf(cur[it].z, w.z, vals[it][2]);
+      vals[it][3] = fmaf(cur[it].w, w.w, vals[it][3]);
+    }
+  }
+  float amax = 0.f;
+  {
+    const float4 ic = *reinterpret_cast<const float4*>(&inv_c[d4]);
+#pragma unroll
+    for (int it = 0; it < kVec; ++it) {
+      vals[it][0] *= ic.x;
+      vals[it][1] *= ic.y;
+      vals[it][2] *= ic.z;
+      vals[it][3] *= ic.w;
+#pragma unroll
+      for (int e = 0; e < 4; ++e) amax = fmaxf(amax, fabsf(vals[it][e]));
+    }
   }
 #pragma unroll
   for (int off = 16; off > 0; off >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, off));
@@ -581,18 +647,11 @@ __global__ void __launch_bounds__(256, 4) sima_reduce_kernel(const StatsParams p
   const float sc = s_scale;
   uint16_t* dst = p.ws.m16 + static_cast<size_t>(bh) * kMElems + blk * kRedElems;
 #pragma unroll
-  for (int it = 0; it < kRedElems / 256; ++it) {
-    const int idx = it * 256 + tid;
-    const float v = vals[it] * sc;
-    uint16_t bits;
-    if constexpr (kBF16) {
-      __nv_bfloat16 hb = __float2bfloat16_rn(v);
-      bits = *reinterpret_cast<uint16_t*>(&hb);
-    } else {
-      __half hh = __float2half_rn(v);
-      bits = *reinterpret_cast<uint16_t*>(&hh);
-    }
-    dst[idx] = bits;
+  for (int it = 0; it < kVec; ++it) {
+    uint2 w;
+    w.x = pack2_16<kBF16>(make_float2(vals[it][0] * sc, vals[it][1] * sc));
+    w.y = pack2_16<kBF16>(make_float2(vals[it][2] * sc, vals[it][3] * sc));
+    *reinterpret_cast<uint2*>(dst + (it * 256 + tid) * 4) = w;
   }
 }
 
@@ -610,7 +669,7 @@ __host__ __device__ constexpr uint32_t out_smem_bytes(bool out_f32, bool ea) {
 
 struct OutParams {
   int B, H, S;
-  int ntiles, tiles_per_cta, nqchunks;
+  Share share;
   const float* inv_scale;
   float* out_f32;  // non-null selects the f32 output path
   int64_t o_sb, o_ss, o_sh;
@@ -618,7 +677,7 @@ struct OutParams {
 };
 
 struct OutBars {
-  uint64_t m_full, q_full[6], q_empty[6], acc_full[2], acc_empty[2];
+  uint64_t m_full, m_empty, q_full[6], q_empty[6], acc_full[2], acc_empty[2];
   uint64_t qtrans[6];     // EA only: the Q tile of the stage has been exponentiated in place
   uint64_t out_ready[6];  // 16-bit output: the result tile has been written into the stage
 };
@@ -647,15 +706,20 @@ sima_out_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   volatile uint32_t* abortp = &abort_s;
-  const int qc = static_cast<int>(blockIdx.x) % p.nqchunks;
-  const int bh = static_cast<int>(blockIdx.x) / p.nqchunks;
-  const int b = bh / p.H, h = bh % p.H;
-  const int tile0 = qc * p.tiles_per_cta;
-  const int ntile = max(0, min(p.tiles_per_cta, p.ntiles - tile0));
+  // this CTA's tiles, in running count i; a change of unit changes M''
+  const int t_lo = p.share.lo(static_cast<int>(blockIdx.x)), ntile = p.share.lo(static_cast<int>(blockIdx.x) + 1) - t_lo;
+  auto place = [&](int i, int* b, int* h, int* s0) {
+    const int unit = (t_lo + i) / p.share.ntiles;
+    *b = unit / p.H;
+    *h = unit % p.H;
+    *s0 = (t_lo + i - unit * p.share.ntiles) * kTile;
+    return unit;
+  };
 
   if (tid == 0) {
     abort_s = 0;
     mbar_init(smem_u32(&bars.m_full), 1);
+    mbar_init(smem_u32(&bars.m_empty), 1);
     for (int i = 0; i < kQ; ++i) {
       mbar_init(smem_u32(&bars.q_full[i]), 1);
       mbar_init(smem_u32(&bars.q_empty[i]), 1);
@@ -686,15 +750,14 @@ sima_out_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
   tc_fence_after_sync();
   const uint32_t tbase = tmem_base_s;
 
+  // Q is no output of the two kernels ahead (and whatever was before them has finished: they waited for
+  // it), so the first tiles are requested at once; only M'' and its scales, and the output, wait.
+  griddep_launch_dependents();
   if (warp == 0) {
-    if (lane == 0 && ntile > 0) {
-      {
-        const uint32_t bar = smem_u32(&bars.m_full);
-        mbar_expect_tx(bar, kTileBytes);
-        tma_load_4d(sM, &map_m, bar, 0, 0, bh * kTile, 0);
-        tma_load_4d(sM + kHalfBytes, &map_m, bar, 64, 0, bh * kTile, 0);
-      }
+    if (lane == 0) {
       for (int i = 0; i < ntile; ++i) {
+        int b, h, s0;
+        place(i, &b, &h, &s0);
         const int st = i % kQ;
         const uint32_t use = static_cast<uint32_t>(i / kQ);
         if (use > 0 && !mbar_wait(smem_u32(&bars.q_empty[st]), (use - 1) & 1, abortp)) {
@@ -703,8 +766,28 @@ sima_out_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
         }
         const uint32_t bar = smem_u32(&bars.q_full[st]);
         mbar_expect_tx(bar, kTileBytes);
-        tma_load_4d(sQ + st * kTileBytes, &map_q, bar, 0, h, (tile0 + i) * kTile, b);
-        tma_load_4d(sQ + st * kTileBytes + kHalfBytes, &map_q, bar, 64, h, (tile0 + i) * kTile, b);
+        tma_load_4d(sQ + st * kTileBytes, &map_q, bar, 0, h, s0, b);
+        tma_load_4d(sQ + st * kTileBytes + kHalfBytes, &map_q, bar, 64, h, s0, b);
+      }
+    }
+  } else if (warp == 3) {
+    // M'' of every unit in turn; the one before it is done with when the last MMA that read it has retired
+    if (lane == 0) {
+      griddep_wait();
+      int loads = 0;
+      for (int i = 0; i < ntile;) {
+        int b, h, s0;
+        const int unit = place(i, &b, &h, &s0);
+        if (loads > 0 && !mbar_wait(smem_u32(&bars.m_empty), (loads - 1) & 1, abortp)) {
+          record_timeout(p.status, 59);
+          break;
+        }
+        const uint32_t bar = smem_u32(&bars.m_full);
+        mbar_expect_tx(bar, kTileBytes);
+        tma_load_4d(sM, &map_m, bar, 0, 0, unit * kTile, 0);
+        tma_load_4d(sM + kHalfBytes, &map_m, bar, 64, 0, unit * kTile, 0);
+        ++loads;
+        i += p.share.ntiles - s0 / kTile;
       }
     }
   } else if (warp == 1) {
@@ -716,11 +799,18 @@ sima_out_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
         if (!good && lane == 0) record_timeout(p.status, site);
         return good;
       };
-      bool ok = wait_all(&bars.m_full, 0, 52);
+      bool ok = true;
+      int seg = 0;
       const uint64_t mdesc = umma_smem_desc_sw128(sM, 16, 1024);
       for (int i = 0; i < ntile && ok; ++i) {
         const int st = i % kQ, buf = i & 1;
-        ok = wait_all(&bars.q_full[st], (i / kQ) & 1, 53);
+        const int in_unit = (t_lo + i) % p.share.ntiles;
+        const bool last = in_unit == p.share.ntiles - 1;
+        if (i == 0 || in_unit == 0) {
+          ok = wait_all(&bars.m_full, seg & 1, 52);
+          ++seg;
+        }
+        if (ok) ok = wait_all(&bars.q_full[st], (i / kQ) & 1, 53);
         if (!ok) break;
         if constexpr (kEA) {
           ok = wait_all(&bars.qtrans[st], (i / kQ) & 1, 56);
@@ -749,6 +839,7 @@ sima_out_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
             }
           }
           umma_commit(smem_u32(&bars.acc_full[buf]));
+          if (last) umma_commit(smem_u32(&bars.m_empty));
           if constexpr (kOutF32) umma_commit(smem_u32(&bars.q_empty[st]));  // (else: the store warp releases it)
         }
         __syncwarp();
@@ -763,7 +854,8 @@ sima_out_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
           record_timeout(p.status, 58);
           break;
         }
-        const int s0 = (tile0 + i) * kTile;
+        int b, h, s0;
+        place(i, &b, &h, &s0);
         tma_store_4d(&map_o, sQ + st * kTileBytes, 0, h, s0, b);
         tma_store_4d(&map_o, sQ + st * kTileBytes + kHalfBytes, 64, h, s0, b);
         tma_store_commit();
@@ -817,12 +909,19 @@ sima_out_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
     const int r = wq * 32 + lane;  // row of the tile
     const uint32_t lane_base = static_cast<uint32_t>(wq * 32) << 16;
     // one inverse scale per block of 32 output channels = per TMEM chunk below
-    const float inv4[4] = {p.inv_scale[bh * 4 + 0], p.inv_scale[bh * 4 + 1], p.inv_scale[bh * 4 + 2],
-                           p.inv_scale[bh * 4 + 3]};
+    float inv4[4] = {1.f, 1.f, 1.f, 1.f};
+    int unit_in = -1;
     bool ok = true;
+    griddep_wait();
     for (int i = 0; i < ntile && ok; ++i) {
       const int buf = i & 1;
-      const int s0 = (tile0 + i) * kTile;
+      int b, h, s0;
+      const int unit = place(i, &b, &h, &s0);
+      if (unit != unit_in) {
+        unit_in = unit;
+#pragma unroll
+        for (int c = 0; c < 4; ++c) inv4[c] = __ldcg(p.inv_scale + unit * 4 + c);
+      }
       ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&bars.acc_full[buf]), (i >> 1) & 1, abortp));
       if (!ok) { if (lane == 0) record_timeout(p.status, 55); break; }
       tc_fence_after_sync();
@@ -1415,35 +1514,30 @@ sima_fused_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
 size_t align256(size_t x) { return (x + 255) & ~static_cast<size_t>(255); }
 
 struct Plan {
-  int ntiles, nchunks, tiles_per_chunk;
+  int ntiles, max_slots;
+  Share share;
   size_t off_pm, off_pc, off_m16, off_sc, off_cnt, total;
 };
-
-// Into how many slabs the sequence of one (batch, head) unit is cut for the statistics and for the
-// output kernel of the three-kernel path: about seven waves of CTAs on a 148-SM part, but at least
-// eight tiles per CTA -- filling and draining the stage ring and loading M'' cost a CTA about as
-// much as four tiles -- unless that would leave SMs without a CTA.
-int slabs_per_unit(int bh, int ntiles) {
-  int want = (1024 + bh - 1) / bh;
-  const int long_enough = ntiles / 8 > 1 ? ntiles / 8 : 1;
-  if (want > long_enough) want = long_enough;
-  const int fill = (148 + bh - 1) / bh;
-  if (want < fill) want = fill;
-  if (want > ntiles) want = ntiles;
-  return want < 1 ? 1 : want;
-}
 
 Plan make_plan(const SimaShape& s) {
   Plan pl;
   const int bh = s.B * s.H;
   pl.ntiles = (s.S + kTile - 1) / kTile;
-  int want = slabs_per_unit(bh, pl.ntiles);
-  if (want > kMaxChunks) want = kMaxChunks;
-  pl.tiles_per_chunk = (pl.ntiles + want - 1) / want;
-  pl.nchunks = (pl.ntiles + pl.tiles_per_chunk - 1) / pl.tiles_per_chunk;
+  // one CTA per SM, but no more than leave every unit kMaxChunks partial results (two CTAs of a unit may
+  // reach over its ends)
+  const int64_t total = static_cast<int64_t>(bh) * pl.ntiles;
+  int64_t ctas = s.num_sms;
+  if (ctas > total) ctas = total;
+  if (ctas > static_cast<int64_t>(bh) * (kMaxChunks - 2)) ctas = static_cast<int64_t>(bh) * (kMaxChunks - 2);
+  pl.share.total = static_cast<int>(total);
+  pl.share.ctas = static_cast<int>(ctas);
+  pl.share.ntiles = pl.ntiles;
+  pl.max_slots = static_cast<int>((static_cast<int64_t>(pl.ntiles) * ctas + total - 1) / total) + 1;
+  if (pl.max_slots > kMaxChunks) pl.max_slots = kMaxChunks;
+  const size_t slots = std::max(static_cast<size_t>(bh) * pl.max_slots, static_cast<size_t>(s.num_sms / kFuGroup) * kFuGroup);
   size_t off = 0;
-  pl.off_pm = off; off = align256(off + static_cast<size_t>(bh) * pl.nchunks * kMElems * 4);
-  pl.off_pc = off; off = align256(off + static_cast<size_t>(bh) * pl.nchunks * 2 * kTile * 4);
+  pl.off_pm = off; off = align256(off + slots * kMElems * 4);
+  pl.off_pc = off; off = align256(off + slots * 2 * kTile * 4);
   pl.off_m16 = off; off = align256(off + static_cast<size_t>(bh) * kMElems * 2);
   pl.off_sc = off; off = align256(off + static_cast<size_t>(bh) * kRedBlocks * 4);
   pl.off_cnt = off; off = align256(off + static_cast<size_t>(bh) * 2 * sizeof(uint32_t));  // fused kernel's counters
@@ -1469,8 +1563,7 @@ cudaError_t launch_sima(const CUtensorMap& mq, const CUtensorMap& mk, const CUte
 #ifdef ASUKA_SIMA_NO_FUSED
   const bool fused = false;
 #else
-  const bool fused = !s.ea && maps64 != nullptr && n_groups > 0 && 2 * bh >= n_groups && pl.ntiles >= kFuGroup &&
-                     static_cast<long long>(bh) * pl.nchunks >= static_cast<long long>(n_groups) * kFuGroup;
+  const bool fused = !s.ea && maps64 != nullptr && n_groups > 0 && 2 * bh >= n_groups && pl.ntiles >= kFuGroup;
 #endif
   if (fused) {
     FusedParams fp;
@@ -1507,7 +1600,8 @@ cudaError_t launch_sima(const CUtensorMap& mq, const CUtensorMap& mk, const CUte
   }
   StatsParams sp;
   sp.B = s.B; sp.H = s.H; sp.S = s.S;
-  sp.nchunks = pl.nchunks; sp.tiles_per_chunk = pl.tiles_per_chunk; sp.ntiles = pl.ntiles;
+  sp.share = pl.share;
+  sp.max_slots = pl.max_slots;
   sp.ws.part_m = reinterpret_cast<float*>(w + pl.off_pm);
   sp.ws.part_c = reinterpret_cast<float*>(w + pl.off_pc);
   sp.ws.m16 = reinterpret_cast<uint16_t*>(w + pl.off_m16);
@@ -1522,15 +1616,15 @@ cudaError_t launch_sima(const CUtensorMap& mq, const CUtensorMap& mk, const CUte
     else kern = s.bf16 ? sima_stats_kernel<true, false> : sima_stats_kernel<false, false>;
     e = ensure_dynamic_smem(reinterpret_cast<const void*>(kern), kStSmem);
     if (e != cudaSuccess) return e;
-    kern<<<static_cast<unsigned>(bh) * pl.nchunks, kStThreads, kStSmem, stream>>>(mq, mk, mv, sp);
+    e = launch_dependent(kern, dim3(static_cast<unsigned>(pl.share.ctas)), dim3(kStThreads), kStSmem, stream, mq, mk, mv, sp);
     count_launch();
-    if ((e = cudaGetLastError()) != cudaSuccess) return e;
+    if (e != cudaSuccess) return e;
   }
   {
     auto kern = s.bf16 ? sima_reduce_kernel<true> : sima_reduce_kernel<false>;
-    kern<<<bh * kRedBlocks, 256, 0, stream>>>(sp);
+    e = launch_dependent(kern, dim3(static_cast<unsigned>(bh) * kRedBlocks), dim3(256), 0, stream, sp);
     count_launch();
-    if ((e = cudaGetLastError()) != cudaSuccess) return e;
+    if (e != cudaSuccess) return e;
   }
   {
     CUtensorMap mm;
@@ -1539,10 +1633,7 @@ cudaError_t launch_sima(const CUtensorMap& mq, const CUtensorMap& mk, const CUte
       return cudaErrorInvalidValue;
     OutParams op;
     op.B = s.B; op.H = s.H; op.S = s.S;
-    op.ntiles = pl.ntiles;
-    const int nq = slabs_per_unit(bh, pl.ntiles);
-    op.tiles_per_cta = (pl.ntiles + nq - 1) / nq;
-    op.nqchunks = (pl.ntiles + op.tiles_per_cta - 1) / op.tiles_per_cta;
+    op.share = pl.share;
     op.inv_scale = sp.ws.inv_scale;
     op.out_f32 = s.out_f32 ? static_cast<float*>(out_ptr) : nullptr;
     op.o_sb = out_stride_b; op.o_ss = out_stride_s; op.o_sh = out_stride_h;
@@ -1558,9 +1649,9 @@ cudaError_t launch_sima(const CUtensorMap& mq, const CUtensorMap& mk, const CUte
     const uint32_t out_smem = out_smem_bytes(s.out_f32, s.ea);
     e = ensure_dynamic_smem(reinterpret_cast<const void*>(kern), static_cast<int>(out_smem));
     if (e != cudaSuccess) return e;
-    kern<<<static_cast<unsigned>(bh) * op.nqchunks, kOutThreads + (s.ea ? 256 : 0), out_smem, stream>>>(mq, mm, s.out_f32 ? mq : mo, op);
+    e = launch_dependent(kern, dim3(static_cast<unsigned>(pl.share.ctas)), dim3(kOutThreads + (s.ea ? 256 : 0)), out_smem, stream,
+                         mq, mm, s.out_f32 ? mq : mo, op);
     count_launch();
-    e = cudaGetLastError();
   }
   return e;
 }
