@@ -13,13 +13,19 @@
 // under the tail and the epilogue of the current one.
 //   warp 0        TMA producer: Q once, then K tiles of 128 keys through a 3-stage ring
 //   warp 2        TMA producer: V tiles through a 2-stage ring
-//   warp 1        issues tcgen05.mma: S_t = Q_t K^T (SMEM x SMEM), O_t += P_t V (TMEM x SMEM)
+//   warp 1        issues the tcgen05.mma of S = Q_t K^T (SMEM x SMEM)
+//   warp 3        issues the tcgen05.mma of O_t += P_t V (TMEM x SMEM)
 //   warps 4-7     softmax of tile 0: one thread per query row, whole row of S in registers
 //   warps 8-11    softmax of tile 1
-// TMEM (512 columns): S_0 | S_1 | O_0 | O_1, 128 f32 columns each; P_t (16-bit, 64 columns)
-// overwrites the front of S_t once S_t is in registers.  The exponent reference of a row is only
-// taken from the first tile's true row maximum and then only moved when a later tile's row sum
-// would overflow the stale one, so O is rescaled (a TMEM round trip) almost never.  The epilogue writes O_t / l from registers straight to global memory.
+// TMEM (512 columns): S | P_0 | P_1 | O_0 | O_1.  A softmax warp takes a whole row of S into registers at
+// once, so ONE S (128 f32 columns) serves both tiles in turn: it is free again 70 clocks after its QK^T,
+// and the next QK^T -- the other tile's -- is issued while this tile is still being exponentiated.  P_t
+// (16-bit, 64 columns each) has columns of its own.  A tile's next S is thus waiting when its softmax
+// comes for it, and P.V is off the chain from one step to the next.  (With P_t over the front of S_t a
+// tile's chain was softmax, P.V, QK^T: of 3180 clk per pair of steps the softmax warps waited 1360.)
+// The exponent reference of a row is only taken from the first tile's true row maximum and moved when a
+// later tile's maximum exceeds it by more than 2^6, so O is rescaled (a TMEM round trip) almost never.
+// The epilogue writes O_t / l from registers straight to global memory.
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 
@@ -53,8 +59,8 @@ constexpr int kThreads = 384;
 constexpr int kUtilRegs = 96;      // 128 * 96 + 256 * 200 = 63488 <= 384 * 168
 constexpr int kSoftmaxRegs = 200;
 constexpr uint32_t kSmemBytes = 7 * kTileBytes + 1024;
-constexpr float kRescaleLimit = 8192.0f;  // largest tile row sum tolerated under a stale reference:
-                                          // bounds every exponential far below fp16's 65504
+constexpr float kRescaleLimit = 6.0f;  // log2 of the largest exponential tolerated under a stale reference:
+                                       // keeps a tile's row sum below 2^13, far from fp16's 65504
 
 struct FwdParams {
   int B, H, Sq, Skv;
@@ -83,7 +89,7 @@ struct Bars {
   uint64_t q_full[2], q_empty[2];
   uint64_t k_full[3], k_empty[3];
   uint64_t v_full[3], v_empty[3];
-  uint64_t s_full[2], p_ready[2], o_done[2], o_free[2];
+  uint64_t s_full[2], s_free, p_ready[2], pv_done[2], o_free[2];
 };
 
 __device__ __forceinline__ float ex2(float x) {
@@ -282,9 +288,10 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
       mbar_init(smem_u32(&bars.q_empty[i]), 1);
       mbar_init(smem_u32(&bars.s_full[i]), 1);
       mbar_init(smem_u32(&bars.p_ready[i]), 128);
-      mbar_init(smem_u32(&bars.o_done[i]), 1);
+      mbar_init(smem_u32(&bars.pv_done[i]), 1);
       mbar_init(smem_u32(&bars.o_free[i]), kOne ? 256 : 128);
     }
+    mbar_init(smem_u32(&bars.s_free), 128);
     for (int i = 0; i < kKStages; ++i) {
       mbar_init(smem_u32(&bars.k_full[i]), 1);
       mbar_init(smem_u32(&bars.k_empty[i]), 1);
@@ -391,17 +398,75 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
       }
     }
   } else if (warp == 1) {
-    // ------------------------------------------------------------------ MMA issuer
-    // One warp issues for both tiles, in the order P.V_0(j-1), QK_0(j), P.V_1(j-1), QK_1(j): the
-    // S/P aliasing of a tile is ordered by program order, and the two tiles are forced to
-    // alternate (their softmax phases share the MUFU, so they must not run in step).  The whole
-    // warp walks the loop (addresses and descriptors stay warp-uniform, waits are converged); one
-    // elected lane issues the tcgen05.mma / commit instructions.  Barriers that are normally
-    // already complete are probed together so that their latencies overlap.
+    // ------------------------------------------------------------------ QK^T issuer
+    // Step j of tile 0, step j of tile 1, step j + 1 of tile 0, ...: each is issued when the softmax warps
+    // have the one before it in registers.  The whole warp walks the loop (addresses and descriptors stay
+    // warp-uniform, waits are converged); one elected lane issues the tcgen05.mma / commit instructions.
+    // Issuing eight MMAs takes as long as they run, and a wait on a barrier that is already complete still
+    // costs 130 clk beside two busy softmax warps: P.V has an issuing warp of its own so that the two
+    // cover for each other (from one warp a pair of steps took 4200 clk), and the barriers of a step are
+    // probed together.
     reg_dealloc<kUtilRegs>();
     {
       constexpr uint32_t kFmt = kBF16 ? UMMA_BF16 : UMMA_F16;
       constexpr uint32_t idesc_qk = umma_idesc_f16(kFmt, UMMA_K_MAJOR, UMMA_K_MAJOR, 128, 128);
+      auto wait_all = [&](uint64_t* bar, uint32_t parity, uint32_t site) -> bool {
+        const bool good = __all_sync(0xffffffffu, mbar_wait(smem_u32(bar), parity, abortp));
+        if (!good && lane == 0) record_timeout(p.status, site);
+        return good;
+      };
+      bool ok = true;
+      uint32_t kc = 0;              // K tiles consumed before this item
+      uint32_t x = 0;               // uses of S so far (parity of s_free)
+      uint32_t on0 = 0, on1 = 0;    // items of either tile before this one (parity of q_full)
+      Item it_;
+      for (int it = 0; it < n_waves && ok; ++it) {
+        if (!get_item<kMode>(it, p, &it_)) continue;
+        const int n0 = it_.n_kv[0], n1 = it_.n_kv[1];
+        for (int j = 0; j < it_.n_max && ok; ++j) {
+#pragma unroll
+          for (int t = 0; t < 2; ++t) {
+            if (j >= (t ? n1 : n0)) continue;
+            const uint32_t kidx = kc + (kOne ? 2 * j + t : j);
+            const int st = kidx % kKStages;
+            const bool k_hit = mbar_try_wait(smem_u32(&bars.k_full[st]), (kidx / kKStages) & 1);
+            const bool s_hit = x == 0 || mbar_try_wait(smem_u32(&bars.s_free), (x - 1) & 1);
+            if (j == 0 && (!kOne || t == 0)) ok = wait_all(&bars.q_full[t], (t ? on1 : on0) & 1, 3);
+            if (ok && !__all_sync(0xffffffffu, k_hit)) ok = wait_all(&bars.k_full[st], (kidx / kKStages) & 1, 4);
+            if (ok && !__all_sync(0xffffffffu, s_hit)) ok = wait_all(&bars.s_free, (x - 1) & 1, 13);
+            if (!ok) break;
+            ++x;
+            tc_fence_after_sync();
+            if (elect_one()) {
+              const uint64_t kdesc = umma_smem_desc_sw128(sK + st * kTileBytes, 16, 1024);
+              const uint64_t qdesc = umma_smem_desc_sw128(sQ + (kOne ? 0 : t) * kTileBytes, 16, 1024);
+#pragma unroll
+              for (int kk = 0; kk < 8; ++kk) {
+                const uint64_t off = static_cast<uint64_t>((kk & 3) * 2 + (kk >> 2) * (kHalfBytes >> 4));
+                umma_ss(tbase, qdesc + off, kdesc + off, idesc_qk, kk > 0 ? 1u : 0u);
+              }
+              umma_commit(smem_u32(&bars.s_full[t]));
+              // the K stage is free after the last QK^T that reads it; Q_t after its last QK^T
+              if (kOne || t == 1 || j >= n1) umma_commit(smem_u32(&bars.k_empty[st]));
+              if (kOne) {
+                if (2 * j + t == n0 + n1 - 1) umma_commit(smem_u32(&bars.q_empty[0]));
+              } else if (j == (t ? n1 : n0) - 1) {
+                umma_commit(smem_u32(&bars.q_empty[t]));
+              }
+            }
+            __syncwarp();
+          }
+        }
+        kc += kOne ? n0 + n1 : it_.n_max;
+        if (n0 > 0) ++on0;
+        if (n1 > 0) ++on1;
+      }
+    }
+  } else if (warp == 3) {
+    // ------------------------------------------------------------------ P.V issuer
+    reg_dealloc<kUtilRegs>();
+    {
+      constexpr uint32_t kFmt = kBF16 ? UMMA_BF16 : UMMA_F16;
       constexpr uint32_t idesc_pv = umma_idesc_f16(kFmt, UMMA_K_MAJOR, UMMA_MN_MAJOR, 128, 128);
       auto wait_all = [&](uint64_t* bar, uint32_t parity, uint32_t site) -> bool {
         const bool good = __all_sync(0xffffffffu, mbar_wait(smem_u32(bar), parity, abortp));
@@ -409,105 +474,48 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
         return good;
       };
       bool ok = true;
-      uint32_t kc = 0, vc = 0;      // K / V tiles consumed before this item
-      uint32_t sn[2] = {0, 0};      // tile steps of tile t before this item (parity of s_full, p_ready)
-      uint32_t on[2] = {0, 0};      // items of tile t before this one (parity of q_full, o_free)
+      uint32_t vc = 0;              // V tiles consumed before this item
+      uint32_t sn0 = 0, sn1 = 0;    // steps of either tile before this item (parity of p_ready)
+      uint32_t on0 = 0, on1 = 0;    // items of either tile before this one (parity of o_free)
       Item it_;
       for (int it = 0; it < n_waves && ok; ++it) {
         if (!get_item<kMode>(it, p, &it_)) continue;
-        const int n_max = it_.n_max;
-        for (int t = 0; t < Rings<kMode>::kQTiles && ok; ++t) {
-          if (it_.n_kv[t] > 0) ok = wait_all(&bars.q_full[t], on[t] & 1, 3);
-        }
-        for (int j = 0; j <= n_max && ok; ++j) {
-          const int jp = j - 1;  // the tile whose P.V is issued in this iteration
-          const bool have_k = j < n_max, have_v = jp >= 0;
-          const bool pv0 = have_v && jp < it_.n_kv[0], pv1 = have_v && jp < it_.n_kv[1];
-          uint32_t kidx = kc + j, vidx = vc + (have_v ? jp : 0);
-          bool p0_hit = false;
-          if constexpr (!kOne) {
-            const int st = kidx % kKStages, stp = vidx % kVStages;
-            // probe everything this iteration needs at once; fall back to a proper wait on a miss
-            const bool k_hit = !have_k || mbar_try_wait(smem_u32(&bars.k_full[st]), (kidx / kKStages) & 1);
-            const bool v_hit = !have_v || mbar_try_wait(smem_u32(&bars.v_full[stp]), (vidx / kVStages) & 1);
-            p0_hit = !pv0 || mbar_try_wait(smem_u32(&bars.p_ready[0]), (sn[0] + jp) & 1);
-            if (!__all_sync(0xffffffffu, k_hit)) ok = wait_all(&bars.k_full[st], (kidx / kKStages) & 1, 4);
-            if (ok && !__all_sync(0xffffffffu, v_hit)) ok = wait_all(&bars.v_full[stp], (vidx / kVStages) & 1, 5);
-            if (!ok) break;
-          }
+        const int n0 = it_.n_kv[0], n1 = it_.n_kv[1];
+        for (int j = 0; j < it_.n_max && ok; ++j) {
 #pragma unroll
           for (int t = 0; t < 2; ++t) {
-            const uint32_t tS = tbase + t * 128;          // S_t, and P_t in its first 64 columns
-            const uint32_t tO = tbase + 256 + t * 128;    // O_t
-            const bool pv = t == 0 ? pv0 : pv1;
-            const bool qk = j < it_.n_kv[t];
-            if constexpr (kOne) {  // every step of either slot has K and V tiles of its own
-              kidx = kc + 2 * j + t;
-              vidx = vc + 2 * (have_v ? jp : 0) + t;
-            }
-            const int st = kidx % kKStages, stp = vidx % kVStages;
-            const uint64_t kdesc = umma_smem_desc_sw128(sK + st * kTileBytes, 16, 1024);
-            const uint64_t vdesc = umma_smem_desc_sw128(sV + stp * kTileBytes, kHalfBytes, 1024);
-            if constexpr (kOne) {
-              const bool k_hit = !qk || mbar_try_wait(smem_u32(&bars.k_full[st]), (kidx / kKStages) & 1);
-              const bool v_hit = !pv || mbar_try_wait(smem_u32(&bars.v_full[stp]), (vidx / kVStages) & 1);
-              if (!__all_sync(0xffffffffu, k_hit)) ok = wait_all(&bars.k_full[st], (kidx / kKStages) & 1, 4);
-              if (ok && !__all_sync(0xffffffffu, v_hit)) ok = wait_all(&bars.v_full[stp], (vidx / kVStages) & 1, 5);
-              if (!ok) break;
-            }
-            if (pv) {
-              if (t == 1 || !__all_sync(0xffffffffu, p0_hit)) {
-                ok = wait_all(&bars.p_ready[t], (sn[t] + jp) & 1, 6);
-                if (!ok) break;
-              }
-              if (jp == 0 && on[t] > 0) {
-                // the first P.V of an item overwrites O_t: the previous item's epilogue must have read it
-                ok = wait_all(&bars.o_free[t], (on[t] - 1) & 1, 12);
-                if (!ok) break;
-              }
-            }
+            if (j >= (t ? n1 : n0)) continue;
+            const uint32_t vidx = vc + (kOne ? 2 * j + t : j);
+            const int st = vidx % kVStages;
+            const uint32_t on = t ? on1 : on0, pn = (t ? sn1 : sn0) + j;
+            ok = wait_all(&bars.v_full[st], (vidx / kVStages) & 1, 5);
+            // the first P.V of an item overwrites O_t: the previous item's epilogue must have read it
+            if (ok && j == 0 && on > 0) ok = wait_all(&bars.o_free[t], (on - 1) & 1, 12);
+            if (ok) ok = wait_all(&bars.p_ready[t], pn & 1, 6);
+            if (!ok) break;
             tc_fence_after_sync();
             if (elect_one()) {
-              if (pv) {
+              const uint64_t vdesc = umma_smem_desc_sw128(sV + st * kTileBytes, kHalfBytes, 1024);
+              const uint32_t tP = tbase + 128 + t * 64, tO = tbase + 256 + t * 128;
 #pragma unroll
-                for (int kk = 0; kk < 8; ++kk) {
-                  umma_ts(tO, tS + kk * 8, vdesc + static_cast<uint64_t>(kk * (2048 >> 4)), idesc_pv,
-                          (jp > 0 || kk > 0) ? 1u : 0u);
-                }
-                // O_t is complete after its last P.V; the V stage is free after the last P.V reading it
-                if (jp == it_.n_kv[t] - 1) umma_commit(smem_u32(&bars.o_done[t]));
-                if (kOne || t == 1 || !pv1) umma_commit(smem_u32(&bars.v_empty[stp]));
+              for (int kk = 0; kk < 8; ++kk) {
+                umma_ts(tO, tP + kk * 8, vdesc + static_cast<uint64_t>(kk * (2048 >> 4)), idesc_pv,
+                        (j > 0 || kk > 0) ? 1u : 0u);
               }
-              if (qk) {
-                const uint64_t qdesc = umma_smem_desc_sw128(sQ + (kOne ? 0 : t) * kTileBytes, 16, 1024);
-#pragma unroll
-                for (int kk = 0; kk < 8; ++kk) {
-                  const uint64_t off = static_cast<uint64_t>((kk & 3) * 2 + (kk >> 2) * (kHalfBytes >> 4));
-                  umma_ss(tS, qdesc + off, kdesc + off, idesc_qk, kk > 0 ? 1u : 0u);
-                }
-                umma_commit(smem_u32(&bars.s_full[t]));
-                // the K stage is free after the last QK^T that reads it; Q_t after its last QK^T
-                if (kOne || t == 1 || j >= it_.n_kv[1]) umma_commit(smem_u32(&bars.k_empty[st]));
-                if (kOne) {
-                  if (2 * j + t == it_.n_kv[0] + it_.n_kv[1] - 1) umma_commit(smem_u32(&bars.q_empty[0]));
-                } else if (j == it_.n_kv[t] - 1) {
-                  umma_commit(smem_u32(&bars.q_empty[t]));
-                }
-              }
+              umma_commit(smem_u32(&bars.pv_done[t]));
+              // the V stage is free after the last P.V that reads it
+              if (kOne || t == 1 || j >= n1) umma_commit(smem_u32(&bars.v_empty[st]));
             }
             __syncwarp();
           }
         }
-        kc += kOne ? it_.n_kv[0] + it_.n_kv[1] : n_max;
-        vc += kOne ? it_.n_kv[0] + it_.n_kv[1] : n_max;
-        for (int t = 0; t < 2; ++t) {
-          sn[t] += it_.n_kv[t];
-          if (it_.n_kv[t] > 0) ++on[t];
-        }
+        vc += kOne ? n0 + n1 : it_.n_max;
+        sn0 += n0;
+        sn1 += n1;
+        if (n0 > 0) ++on0;
+        if (n1 > 0) ++on1;
       }
     }
-  } else if (warp < 4) {
-    reg_dealloc<kUtilRegs>();
   } else {
     // ------------------------------------------------------------------ softmax + epilogue
     reg_alloc<kSoftmaxRegs>();
@@ -515,12 +523,12 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
     const int wq = warp & 3;                     // TMEM lane quarter this warp may touch
     const int r_in_tile = wq * 32 + lane;
     const uint32_t lane_base = static_cast<uint32_t>(wq * 32) << 16;
-    const uint32_t tS = tbase + lane_base + t * 128;
+    const uint32_t tS = tbase + lane_base;
+    const uint32_t tP = tbase + lane_base + 128 + t * 64;
     const uint32_t tO = tbase + lane_base + 256 + t * 128;
-    const float scale = p.scale_log2;
+    const float mul = kCap ? p.cap_out : p.scale_log2;
     bool ok = true;
     uint32_t sn = 0;  // tile steps of this tile before the current item
-    uint32_t on = 0;  // items of this tile before the current one
     Item it_;
     for (int it = 0; it < n_waves && (ok || kOne); ++it) {
       if (!get_item<kMode>(it, p, &it_)) continue;
@@ -542,11 +550,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
         const bool masked_tile = jk + kTile - 1 > tile_min_lim;
         const int thr = lim - jk;  // columns > thr of this tile are masked for this row
 
-        // The whole 128-wide row is exponentiated at once against the reference left by earlier
-        // tiles, so the MUFU starts right after the TMEM load and runs without a gap; the tile's
-        // row sum is looked at afterwards.  If it exceeds 2^13 (or is not finite) the rare path
-        // takes the true maximum, moves the reference up, rescales what was accumulated under the
-        // old one and redoes the tile.
+        // The whole 128-wide row goes to registers at once, and S to the next QK^T.
         float e[128];
         {
           uint32_t(&u)[128] = *reinterpret_cast<uint32_t(*)[128]>(e);
@@ -556,6 +560,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
           tmem_ld32(tS + 96, *reinterpret_cast<uint32_t(*)[32]>(&u[96]));
           tmem_wait_ld();
         }
+        tc_fence_before_sync();
+        mbar_arrive(smem_u32(&bars.s_free));
         if constexpr (kCap) {
           // cap first, mask afterwards (the reference adds the mask to the capped logits)
 #pragma unroll
@@ -565,117 +571,66 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
 #pragma unroll
           for (int i = 0; i < 128; ++i) e[i] = (i > thr) ? -INFINITY : e[i];
         }
-#ifndef ASUKA_NO_SEED
+        // The tile's row maximum is the reference of a first tile; a later one only moves the reference up
+        // (and rescales what was accumulated under the old one) when it exceeds it by too much.
+        float mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+#pragma unroll
+        for (int i = 0; i < 128; i += 8) {
+          mx4[0] = max3(mx4[0], e[i], e[i + 1]);
+          mx4[1] = max3(mx4[1], e[i + 2], e[i + 3]);
+          mx4[2] = max3(mx4[2], e[i + 4], e[i + 5]);
+          mx4[3] = max3(mx4[3], e[i + 6], e[i + 7]);
+        }
+        const float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3])) * mul;
         if (j == 0) {
-          // the first tile of an item has no reference yet: take the tile's true row maximum (the
-          // capped and scaled logit is monotone in the raw one) instead of exponentiating blind
-          float mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+          m_ref = mx > -INFINITY ? mx : 0.f;
+        } else {
+          const bool need = mx > m_ref + kRescaleLimit;
+          if (__any_sync(0xffffffffu, need)) {
+            float alpha = 1.f;
+            if (need) {
+              alpha = ex2(m_ref - mx);
+              m_ref = mx;
+              l *= alpha;
+            }
+            // O_t is the sum over earlier tiles of this item, complete with their last P.V
+            ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&bars.pv_done[t]), (sn + j - 1) & 1, abortp));
+            if (!ok) { if (lane == 0) record_timeout(p.status, 8); break; }
+            tc_fence_after_sync();
 #pragma unroll
-          for (int i = 0; i < 128; i += 8) {
-            mx4[0] = max3(mx4[0], e[i], e[i + 1]);
-            mx4[1] = max3(mx4[1], e[i + 2], e[i + 3]);
-            mx4[2] = max3(mx4[2], e[i + 4], e[i + 5]);
-            mx4[3] = max3(mx4[3], e[i + 6], e[i + 7]);
+            for (int c = 0; c < 8; ++c) {
+              uint32_t o[16];
+              tmem_ld16(tO + c * 16, o);
+              tmem_wait_ld();
+#pragma unroll
+              for (int i = 0; i < 16; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * alpha);
+              tmem_st16(tO + c * 16, o);
+            }
+            tmem_wait_st();
           }
-          const float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3]));
-          m_ref = mx > -INFINITY ? mx * (kCap ? p.cap_out : scale) : 0.f;
         }
-#endif
-        {
-          // two logits per FMA instruction (packed f32x2): the softmax warp of a tile runs alone on
-          // its scheduler and is bound by the number of instructions it has to issue
-          const float mul = kCap ? p.cap_out : scale;
-          const float2 mul2 = make_float2(mul, mul), neg_m2 = make_float2(-m_ref, -m_ref);
-#ifdef ASUKA_NO_PACKED
-          (void)mul2; (void)neg_m2;
-#pragma unroll
-          for (int i = 0; i < 128; ++i) e[i] = ex2(fmaf(e[i], mul, -m_ref));
-#else
-#pragma unroll
-          for (int i = 0; i < 64; ++i) {
-            const float2 x = __ffma2_rn(make_float2(e[2 * i], e[2 * i + 1]), mul2, neg_m2);
-            e[2 * i] = ex2(x.x);
-            e[2 * i + 1] = ex2(x.y);
-          }
-#endif
-        }
-        // The tile's row sum doubles as the overflow probe: it bounds every term from above, and it
-        // is NaN or infinite exactly when some term is.  P is packed
-        // to 16 bits right away (the compiler interleaves it with the exponentials), so that only
-        // the TMEM store is left once the probe has passed.
+        // two logits per FMA instruction (packed f32x2); P is packed to 16 bits right away (the compiler
+        // interleaves it with the exponentials)
+        const float2 mul2 = make_float2(mul, mul), neg_m2 = make_float2(-m_ref, -m_ref);
         float2 ts4[4] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f), make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
         uint32_t pk[64];
 #pragma unroll
         for (int i = 0; i < 64; ++i) {
-          ts4[i & 3] = __fadd2_rn(ts4[i & 3], make_float2(e[2 * i], e[2 * i + 1]));
-          pk[i] = pack2<kBF16>(e[2 * i], e[2 * i + 1]);
+          float2 v = __ffma2_rn(make_float2(e[2 * i], e[2 * i + 1]), mul2, neg_m2);
+          v.x = ex2(v.x);
+          v.y = ex2(v.y);
+          ts4[i & 3] = __fadd2_rn(ts4[i & 3], v);
+          pk[i] = pack2<kBF16>(v.x, v.y);
         }
         const float2 ts2 = __fadd2_rn(__fadd2_rn(ts4[0], ts4[1]), __fadd2_rn(ts4[2], ts4[3]));
-        float tile_sum = ts2.x + ts2.y;
-        const bool need = !(tile_sum <= kRescaleLimit);
-        if (__any_sync(0xffffffffu, need)) {
-          // ---- rare: the raw logits are still intact in TMEM; take their maximum, 32 columns at a time
-          float mx = -INFINITY;
-#pragma unroll
-          for (int c = 0; c < 4; ++c) {
-            uint32_t u[32];
-            tmem_ld32(tS + c * 32, u);
-            tmem_wait_ld();
-#pragma unroll
-            for (int i = 0; i < 32; ++i) {
-              const float v = (masked_tile && c * 32 + i > thr) ? -INFINITY : __uint_as_float(u[i]);
-              mx = fmaxf(mx, v);
-            }
-          }
-          // the scaled (and capped) logit is monotone in the raw one: transform the maximum
-          const float mx2 = kCap ? tanh_approx(mx * p.cap_in) * p.cap_out : mx * scale;
-          float alpha = 1.f;
-          if (need) {
-            alpha = ex2(m_ref - mx2);
-            m_ref = mx2;
-            l *= alpha;
-          }
-          if (j > 0) {
-            // O_t is the sum over earlier tiles of this work item.  P.V of tile j-1 was issued before
-            // QK^T of tile j and the tensor pipe retires in order, so S_t(j) being ready means O_t is
-            // complete.
-#pragma unroll
-            for (int c = 0; c < 4; ++c) {
-              uint32_t o[32];
-              tmem_ld32(tO + c * 32, o);
-              tmem_wait_ld();
-#pragma unroll
-              for (int i = 0; i < 32; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * alpha);
-              tmem_st32(tO + c * 32, o);
-            }
-            tmem_wait_st();
-          }
-          const float mul = kCap ? p.cap_out : scale;
-          const float neg_m = -m_ref;
-#pragma unroll
-          for (int c = 0; c < 4; ++c) {
-            uint32_t u[32];
-            tmem_ld32(tS + c * 32, u);
-            tmem_wait_ld();
-#pragma unroll
-            for (int i = 0; i < 32; ++i) {
-              float v = __uint_as_float(u[i]);
-              if constexpr (kCap) v = tanh_approx(v * p.cap_in);
-              v = (masked_tile && c * 32 + i > thr) ? -INFINITY : v;
-              e[c * 32 + i] = ex2(fmaf(v, mul, neg_m));
-            }
-          }
-          tile_sum = 0.f;
-#pragma unroll
-          for (int i = 0; i < 64; ++i) {
-            tile_sum += e[2 * i] + e[2 * i + 1];
-            pk[i] = pack2<kBF16>(e[2 * i], e[2 * i + 1]);
-          }
+        l += ts2.x + ts2.y;
+        if (j > 0) {  // P_t is free when the last P.V has read it (a new item: its epilogue has waited for that)
+          ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&bars.pv_done[t]), (sn + j - 1) & 1, abortp));
+          if (!ok) { if (lane == 0) record_timeout(p.status, 8); break; }
+          tc_fence_after_sync();
         }
-        l += tile_sum;
-        tmem_st32(tS, *reinterpret_cast<uint32_t(*)[32]>(&pk[0]));
-        tmem_st32(tS + 32, *reinterpret_cast<uint32_t(*)[32]>(&pk[32]));
-        if (!ok) break;
+        tmem_st32(tP, *reinterpret_cast<uint32_t(*)[32]>(&pk[0]));
+        tmem_st32(tP + 32, *reinterpret_cast<uint32_t(*)[32]>(&pk[32]));
         tmem_wait_st();
         tc_fence_before_sync();
         mbar_arrive(smem_u32(&bars.p_ready[t]));
@@ -684,7 +639,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
         // ---- epilogue of a one-tile item: the first slot gets the second's exponent reference and row sum
         // and hands back the factors of both accumulators; each slot writes half of the output columns
         if (n_t > 0 && ok) {
-          ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&bars.o_done[t]), on & 1, abortp));
+          ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&bars.pv_done[t]), (sn + n_t - 1) & 1, abortp));
           if (!ok && lane == 0) record_timeout(p.status, 9);
           tc_fence_after_sync();
         }
@@ -749,18 +704,14 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
           }
         }
         sn += n_t;
-        if (n_t > 0) ++on;
         continue;
       }
       if (!ok) break;
 
       // ---- epilogue of the item: O_t / l straight from TMEM to global memory
-      ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&bars.o_done[t]), on & 1, abortp));
+      ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&bars.pv_done[t]), (sn + n_t - 1) & 1, abortp));
       if (!ok) { if (lane == 0) record_timeout(p.status, 9); break; }
       tc_fence_after_sync();
-#ifdef ASUKA_REDECODE
-      get_item<kMode>(it, p, &it_);  // (decoded again rather than kept in registers across the key loop)
-#endif
       if (kMode == kSplit && it_.nparts[t] > 1) {
         // this tile's keys are shared with other items: leave the unnormalised O, the exponent
         // reference and the row sum for the merge (a row that saw no key in this part has l = 0
@@ -821,7 +772,6 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
         }
       }
       sn += n_t;
-      ++on;
     }
   }
 

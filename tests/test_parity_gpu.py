@@ -411,6 +411,40 @@ def test_logits_that_keep_growing_or_shrinking(ops, dtype, direction):
   no_timeouts(ops)
 
 
+@pytest.mark.parametrize("direction", [1.0, -1.0])
+@pytest.mark.parametrize("shape", [
+    # B, Sq, Skv, H, causal: one tile per item; the early tile of an item with the late one, odd and even
+    # counts; several items per CTA; the unmasked form with a lone last tile; keys cut into parts
+    (1, 513, 1300, 3, True), (1, 650, 650, 40, True), (1, 700, 1000, 30, True), (2, 900, 900, 45, True),
+    (1, 300, 500, 60, False), (1, 4200, 4200, 1, True),
+])
+def test_forward_cuts_with_a_moving_reference(ops, shape, direction):
+  # every way the forward kernel cuts a launch into items, with logits that make the rows' exponent
+  # reference move (up along the keys, in steps on both sides of the 2^6 that is tolerated) or stay
+  B, Sq, Skv, H, causal = shape
+  q, k, v = O.make_inputs("h2o", B, Sq, Skv, H, 128, torch.bfloat16, seed=Sq)
+  k = (k.float() * (1 + direction * torch.arange(Skv).float() / Skv * 6).view(1, Skv, 1, 1)).to(torch.bfloat16)
+  qd, kd, vd = q.cuda(), k.cuda(), v.cuda()
+  out, lse = ops.attn_fwd(qd, kd, vd, causal=causal, return_lse=True)
+
+  # Rows close to one-hot leave outputs as large as single values of V: bf16 rounds each probability and the
+  # result by 2^-8 of itself at most (the row sum is not rounded); tanh.approx is off by 2^-11 of itself,
+  # so a capped logit by cap * 2^-11 and a probability by twice that.
+  def check(got, ref, ref_abs, p_err, what):
+    bound = 2.0 ** -8 * ref.abs() + (2.0 ** -8 + p_err) * ref_abs + 1e-4
+    assert ((got.cpu().float() - ref).abs() <= bound).all(), what
+
+  check(out, O.h2o(q, k, v, causal)[0], O.h2o(q, k, v.abs(), causal)[0], 0.0, "out")
+  s = torch.einsum("bqhd,bkhd->bhqk", q.float(), k.float()) / 128 ** 0.5
+  if causal:
+    s = s + torch.triu(torch.full((Sq, Skv), float("-inf")), diagonal=Skv - Sq + 1)
+  torch.testing.assert_close(lse.cpu(), torch.logsumexp(s, -1) * 1.4426950408889634, rtol=1e-4, atol=2e-3)
+  check(ops.attn_fwd(qd, kd, vd, causal=causal, softcap=30.0), O.gemma2(q, k, v, 30.0, causal),
+        O.gemma2(q, k, v.abs(), 30.0, causal), 2 * 30.0 * 2.0 ** -11, "soft-capped out")
+  assert torch.equal(out, ops.attn_fwd(qd, kd, vd, causal=causal))
+  no_timeouts(ops)
+
+
 @pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
 def test_sibling_cases_vs_oracle(ops, dtype):
   # Gemma-2 soft-capping, SnapKV pooling and CORM thresholds on ragged and rectangular shapes
