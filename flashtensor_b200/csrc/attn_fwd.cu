@@ -891,8 +891,9 @@ __global__ void __launch_bounds__(kMergeWarps * 32) attn_merge_kernel(const FwdP
 
 // How many parts the key range of every two-tile item is cut into (kSplit).  Partial results cost about as
 // much L2 traffic again as the inputs and the merge is a launch of its own, so this is only for launches
-// whose query tiles would leave half of the SMs idle even at one tile per CTA, and long key ranges
-// (measured at head counts of 4 to 32 and S = 1024 to 4096); it needs workspace.
+// whose query tiles would leave half of the SMs idle even at one tile per CTA, and long key ranges (S 4096,
+// 2 heads: 30.9 us with one tile per CTA, 25.5 split; 100 rows over 9000 keys, 16/4 heads 58 and 30; at 1.7
+// tiles per SM S 4096, 8 heads 35 and 66); it needs workspace.
 int attn_fwd_parts(const AttnShape& s, int num_sms, size_t ws_bytes) {
   if (attn_decode_applies(s)) return 1;  // (attn_decode.cu splits the keys itself)
   const long long n_tiles = static_cast<long long>((s.Sq + kTile - 1) / kTile) * s.B * s.H;
@@ -912,14 +913,16 @@ int attn_fwd_parts(const AttnShape& s, int num_sms, size_t ws_bytes) {
 
 // One query tile per item (kSolo).  Two tiles of an item keep the tensor pipe and the MUFU busy as long as
 // both have keys left, and share every K/V tile; but an item is then as long as its later tile.  One tile
-// whose keys the two slots share is done in half the rounds, at twice the K/V traffic per step: with every
-// SM at work a round takes 1.28 times as long (S = 2048, 64 heads: 80 -> 105 us).  So:
-//   - one tile per SM or fewer, three or more key tiles: always.  Measured (us): 500 rows over 5003 keys,
-//     32/8 heads 86 -> 55; S 1024, 8 heads 22.6 -> 16.7; S 512, 4 heads 15.0 -> 12.4 (a single key tile:
-//     8.9 -> 10.3); unmasked S 2048, 8 heads 35.0 -> 26.7
-//   - up to two tiles per SM, if the launch is a causal square of at least twelve tiles: its late tiles are
-//     twice as long as the mean and the early ones fill in behind them.  S 4096, 8 heads 67.7 -> 47.2;
-//     S 2048, 16 heads 37.6 -> 30.8 (S 1024, 32 heads 22.8 -> 24.7; 1024 rows over 8000 keys 117 -> 148)
+// whose keys the two slots share is done in half the rounds, at twice the K/V traffic per step.  So (us, two
+// tiles per item -> one):
+//   - one tile per SM or fewer, three or more key tiles: always.  500 rows over 5003 keys, 32/8 heads
+//     71 -> 44; S 1024, 8 heads 16.3 -> 12.6; S 512, 4 heads 11.2 -> 9.4; unmasked S 2048, 8 heads 29.7 -> 20.4
+//   - with more, if the launch is a causal square, up to a number that grows with its length: the late tiles
+//     are twice as long as the mean, the early ones fill in behind them, and the finer they are the better.
+//     S 1024, 24 heads (1.3 tiles per SM) 18.9 -> 16.7; S 1500, 24 heads (1.9) 23.6 -> 23.4; S 2048, 16 heads
+//     (1.7) 28.1 -> 24.8 and 20 heads (2.2) 32.5 -> 30.6; S 4096, 8 heads (1.7) 45.8 -> 35.1; beyond it
+//     S 1024, 32 heads (1.7) 19.7 -> 20.1; S 8192, 8 heads (3.5) 112 -> 126; and not square, 1024 rows over
+//     8000 keys, 32/8 heads (1.7) 108 -> 118
 static bool attn_fwd_solo(const AttnShape& s, int num_sms) {
 #ifdef ASUKA_TUNE_ENV
   if (const char* e = getenv("ASUKA_FWD_SOLO")) return atoi(e) != 0;
@@ -927,7 +930,7 @@ static bool attn_fwd_solo(const AttnShape& s, int num_sms) {
   const int nq_tiles = (s.Sq + kTile - 1) / kTile;
   const long long n_tiles = static_cast<long long>(nq_tiles) * s.B * s.H;
   if (n_tiles <= num_sms) return s.Skv > 2 * kTile;
-  return s.causal && n_tiles <= 2 * num_sms && nq_tiles >= 12 && 4LL * s.Skv <= 5LL * s.Sq;
+  return s.causal && 4LL * s.Skv <= 5LL * s.Sq && 8 * n_tiles <= static_cast<long long>(num_sms) * ((nq_tiles < 16 ? nq_tiles : 16) + 4);
 }
 
 size_t attn_fwd_split_bytes(const AttnShape& s, int parts) {
