@@ -319,14 +319,17 @@ int col_scores_impl(const asuka_score_params* p, cudaStream_t stream, bool chain
   return map_cuda(launch_col_scores(mq, mk, a, c.s, split_ws, chunks, stream, pending));
 }
 
-int kf_rowstat_impl(const asuka_score_params* p, cudaStream_t stream) {
+int kf_rowstat_impl(const asuka_score_params* p, cudaStream_t stream, bool chained = false) {
   QKV c;
   ScoreArgs a;
   int r = prep_scores(p, true, &c, &a);
   if (r != ASUKA_OK) return r;
   CUtensorMap mq, mk;
   if ((r = make_map(&mq, p->q)) || (r = make_map(&mk, p->k))) return r;
-  return map_cuda(launch_kf_rowstat(mq, mk, a, static_cast<float*>(p->lse.ptr), c.s, stream));
+  a.chained = chained ? 1 : 0;
+  const int sms = sm_count();
+  if (sms <= 0) return ASUKA_ERR_CUDA;
+  return map_cuda(launch_kf_rowstat(mq, mk, a, static_cast<float*>(p->lse.ptr), c.s, sms, stream));
 }
 
 constexpr int kSelectMaxS32 = 32768;  // 4-byte keys in shared memory
@@ -601,7 +604,7 @@ int case_impl(const asuka_case_params* p, CaseKind kind, void* ws, size_t ws_byt
   int r = attn_fwd_impl(&fp, nullptr, stream, extra_bytes > 0 ? extra : nullptr, extra_bytes);
   if (r != ASUKA_OK) return r;
   if (kind == CASE_KF) {
-    if ((r = kf_rowstat_impl(&sp, stream)) != ASUKA_OK) return r;
+    if ((r = kf_rowstat_impl(&sp, stream, true)) != ASUKA_OK) return r;
   }
   // with a selection to follow (and no group mean in between) the selection kernel adds the column
   // pass's partial sums itself: one launch fewer

@@ -28,6 +28,7 @@
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 
+#include <algorithm>
 #include <cstdlib>
 
 #include "../../include/asuka_b200.h"
@@ -66,6 +67,7 @@ struct ColParams {
   uint64_t seed;
   uint32_t unit_off;  // added to the (batch * H + head) index the seeded noise is keyed by
   uint32_t* status;
+  int tail_units;     // (Keyformer row pass) how many of the last units are ordered longest tile first
   int chained;        // the kernel ahead in the stream does not write q or k
   // Query-range split, for launches with too few key blocks to fill the SMs: the query tiles are
   // cut into `n_qchunks` ranges of `q_chunk` tiles, one CTA per (key block, range); every CTA
@@ -866,11 +868,18 @@ kf_col_tma_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
 // what bounds a pass that reads everything once).  The plain variant (direct loads) serves noise
 // tensors whose strides TMA cannot describe.
 // ---------------------------------------------------------------------------------------------
-constexpr int kRsThreads = 320;  // warp 0 producer, warp 1 MMA, warps 2-9 rows (two per 32 rows: columns 0..63 / 64..127)
 constexpr uint32_t kNoiseTileBytes = 128 * 128 * 4;
 constexpr uint32_t kNoiseBoxBytes = kNoiseTileBytes / 4;
+// Warp 0 producer, warp 1 MMA, the others rows: kParts warps per 32 rows, each with its share of every tile's
+// columns.  Two warps per scheduler do not keep the MUFU busy over their chains of load, logarithm, maximum and
+// exponential; the staged variant, one CTA per SM, has four, the seeded one two CTAs of two.
+// With four warps instead of two, the last units' tiles longest first and the start under the forward kernel's
+// tail, the whole case went (us): B1 H16 S1000 58 -> 46, B2 H32 S1000 126 -> 109, B1 H16 S2048 117 -> 92,
+// B2 H32 S2048 356 -> 321, B4 H32 S2048 658 -> 607.
 template <int kNoise> struct RsCfg {  // kNoise 1: two K stages, then eight noise boxes
   static constexpr bool kNoiseTma = kNoise == 1;
+  static constexpr int kParts = kNoiseTma ? 4 : 2;
+  static constexpr int kThreads = (2 + 4 * kParts) * 32;
   static constexpr int kStages = kNoise == 0 ? 4 : 2;  // seeded: small enough for two CTAs per SM
   static constexpr uint32_t kStageBytes = kTileBytes + (kNoiseTma ? kNoiseTileBytes : 0);
   static constexpr uint32_t kSmem = kTileBytes + kStages * kStageBytes + 1024;
@@ -885,12 +894,12 @@ struct RsBars {
 
 // kNoise: 0 noise operand read directly, 1 noise operand staged by TMA, 2 seeded noise
 template <bool kBF16, int kNoise>
-__global__ void __launch_bounds__(kRsThreads, kNoise == 2 ? 2 : 1)
+__global__ void __launch_bounds__(RsCfg<kNoise>::kThreads, kNoise == 2 ? 2 : 1)
 kf_rowstat_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                   const __grid_constant__ CUtensorMap map_n, const ColParams p, float* lse_out) {
   constexpr bool kNoiseTma = kNoise == 1;
   using Cfg = RsCfg<kNoise>;
-  constexpr int kStages = Cfg::kStages;
+  constexpr int kStages = Cfg::kStages, kParts = Cfg::kParts;
   extern __shared__ uint8_t smem_raw[];
   __shared__ __align__(8) RsBars bars;
   __shared__ uint32_t tmem_base_s;
@@ -910,15 +919,25 @@ kf_rowstat_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
   // (measured before the change: 1.65 GB read where 1.27 GB were needed).
   // The seeded variant reads no operand and is bound by its generator: it keeps the order
   // longest tile first over all units, which balances the SMs better.
-  constexpr bool kUnitMajor = kNoise != 2;
-  const int bh = kUnitMajor ? static_cast<int>(blockIdx.x) / p.nq_tiles : static_cast<int>(blockIdx.x) % bh_count;
-  const int qt = p.nq_tiles - 1 - (kUnitMajor ? static_cast<int>(blockIdx.x) % p.nq_tiles
-                                              : static_cast<int>(blockIdx.x) / bh_count);
+  // The last units of the others are ordered that way too, lest the launch end with the long tiles of
+  // its last unit on a few SMs (B1 H32 S2048: the SMs were idle for a quarter of the pass).
+  const int head = (bh_count - p.tail_units) * p.nq_tiles;  // CTAs in unit-major order
+  const int idx = static_cast<int>(blockIdx.x);
+  const bool in_tail = idx >= head;
+  const int bh = in_tail ? bh_count - p.tail_units + (idx - head) % p.tail_units : idx / p.nq_tiles;
+  const int qt = p.nq_tiles - 1 - (in_tail ? (idx - head) / p.tail_units : idx % p.nq_tiles);
   const int b = bh / p.H, h = bh % p.H;
   const int q0 = qt * kTile;
   int last = p.Skv - 1;
   if (p.causal) last = min(last, min(q0 + kTile - 1, p.Sq - 1) + p.diag_off);
   const int n_kv = last / kTile + 1;
+
+  // Chained behind the forward kernel, of which this pass reads nothing: its CTAs start as that kernel's
+  // retire.  They wait for its end before their own, so that whatever waits for this grid waits for both.
+  // (The column pass behind may come up at once where a CTA of this one has the SM to itself, else at the
+  // end: its CTAs, two per SM, should find the SMs equally free.)
+  if (!p.chained) griddep_wait();
+  if (kNoise != 2) griddep_launch_dependents();
 
   if (tid == 0) {
     abort_s = 0;
@@ -935,7 +954,7 @@ kf_rowstat_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
     }
     for (int i = 0; i < 2; ++i) {
       mbar_init(smem_u32(&bars.s_full[i]), 1);
-      mbar_init(smem_u32(&bars.s_empty[i]), 256);
+      mbar_init(smem_u32(&bars.s_empty[i]), kParts * 128);
     }
     mbar_fence_init();
   }
@@ -1024,11 +1043,10 @@ kf_rowstat_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
       }
     }
   } else {
-    // Two warps per 32 rows, each with half of every tile's columns and its own running (maximum,
-    // sum): a row's statistic is a plain merge of the two at the end, so nothing is exchanged per
-    // step, and the scheduler gets twice the warps to hide the noise generator's ALU latency.
-    const int wq = warp & 3;           // TMEM lane quarter (warps 2..9 -> 2,3,0,1,2,3,0,1)
-    const int half = (warp - 2) >> 2;  // columns 0..63 or 64..127 of every tile
+    // kParts warps per 32 rows, each with its columns of every tile and its own running (maximum,
+    // sum): a row's statistic is a plain merge of them at the end, so nothing is exchanged per step.
+    const int wq = warp & 3;           // TMEM lane quarter (warps 2, 3, 4, 5, ... -> 2, 3, 0, 1, ...)
+    const int part = (warp - 2) >> 2;  // which columns of every tile
     const int r_in_tile = wq * 32 + lane;
     const int row = q0 + r_in_tile;
     const uint32_t lane_base = static_cast<uint32_t>(wq * 32) << 16;
@@ -1049,7 +1067,7 @@ kf_rowstat_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
       tc_fence_after_sync();
       const int thr = lim - j * kTile;  // columns > thr are masked
 #pragma unroll
-      for (int c4 = half * 2; c4 < half * 2 + 2; ++c4) {
+      for (int c4 = part * (4 / kParts); c4 < (part + 1) * (4 / kParts); ++c4) {
         uint32_t u[32];
         tmem_ld32(tbase + lane_base + buf * 128 + c4 * 32, u);
         float er[32];
@@ -1101,9 +1119,9 @@ kf_rowstat_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
     }
     // hand-over through the Q tile's shared memory: every MMA that read it has retired (this thread
     // has seen the last S tile), and the variant with the staged noise has no other room left
-    float* part = reinterpret_cast<float*>(smem_gen);  // [m, l][half][row]
-    part[(0 * 2 + half) * kTile + r_in_tile] = m;
-    part[(1 * 2 + half) * kTile + r_in_tile] = l;
+    float* part_s = reinterpret_cast<float*>(smem_gen);  // [m, l][part][row]
+    part_s[part * kTile + r_in_tile] = m;
+    part_s[(kParts + part) * kTile + r_in_tile] = l;
     if (!ok) *abortp = 1u;
   }
 
@@ -1113,17 +1131,24 @@ kf_rowstat_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
     __syncwarp();
     tmem_dealloc(tbase, 256);
   }
+  if (p.chained) griddep_wait();
+  if (kNoise == 2) griddep_launch_dependents();
   if (warp >= 2 && warp < 6 && !*abortp) {
-    // merge the two halves of every row (in column order)
+    // merge the parts of every row (in column order)
     const int r_in_tile = (warp & 3) * 32 + lane;
     const int row = q0 + r_in_tile;
-    const float* part = reinterpret_cast<const float*>(smem_gen);
-    const float m0 = part[0 * kTile + r_in_tile], m1 = part[1 * kTile + r_in_tile];
-    const float m = fmaxf(m0, m1);
+    const float* part_s = reinterpret_cast<const float*>(smem_gen);
+    float m = part_s[r_in_tile];
+#pragma unroll
+    for (int x = 1; x < kParts; ++x) m = fmaxf(m, part_s[x * kTile + r_in_tile]);
     if (row < p.Sq) {
-      // (a half with no visible column has sum 0 and maximum -inf: give it weight 0, not NaN)
-      const float l = part[2 * kTile + r_in_tile] * (m0 > -INFINITY ? ex2(m0 - m) : 0.f) +
-                      part[3 * kTile + r_in_tile] * (m1 > -INFINITY ? ex2(m1 - m) : 0.f);
+      float l = 0.f;
+#pragma unroll
+      for (int x = 0; x < kParts; ++x) {
+        // (a part with no visible column has sum 0 and maximum -inf: give it weight 0, not NaN)
+        const float mx = part_s[x * kTile + r_in_tile];
+        l += part_s[(kParts + x) * kTile + r_in_tile] * (mx > -INFINITY ? ex2(mx - m) : 0.f);
+      }
       lse_out[(static_cast<size_t>(b) * p.H + h) * p.Sq + row] = m + log2f(l);
     }
   }
@@ -1178,6 +1203,7 @@ ColParams make_params(const ScoreArgs& a, const AttnShape& s) {
   p.n_qchunks = 1;
   p.part = nullptr;
   p.part_sq = nullptr;
+  p.tail_units = 0;
   return p;
 }
 
@@ -1275,17 +1301,30 @@ cudaError_t launch_col_scores(const CUtensorMap& mq, const CUtensorMap& mk, cons
 }
 
 cudaError_t launch_kf_rowstat(const CUtensorMap& mq, const CUtensorMap& mk, const ScoreArgs& a,
-                              float* lse2_out, const AttnShape& s, cudaStream_t stream) {
-  const ColParams p = make_params(a, s);
+                              float* lse2_out, const AttnShape& s, int num_sms, cudaStream_t stream) {
+  ColParams p = make_params(a, s);
+  // three waves' worth of tiles, all of them without an operand to read
+  p.tail_units = a.exp_rand == nullptr ? s.B * s.H : std::min(s.B * s.H, (3 * num_sms + p.nq_tiles - 1) / p.nq_tiles);
   const dim3 grid(static_cast<unsigned>(p.nq_tiles) * s.B * s.H);
   cudaError_t e;
   if (a.exp_rand == nullptr) {
     auto kern = s.bf16 ? kf_rowstat_kernel<true, 2> : kf_rowstat_kernel<false, 2>;
     e = ensure_dynamic_smem(reinterpret_cast<const void*>(kern), RsCfg<2>::kSmem);
     if (e != cudaSuccess) return e;
-    kern<<<grid, kRsThreads, RsCfg<2>::kSmem, stream>>>(mq, mk, mq, p, lse2_out);
+    // Two CTAs share an SM.  A launch of half a wave to two waves is balanced by one long and one shorter
+    // tile on each, which is how the CTAs fall when all SMs are free at the start; as the forward kernel's
+    // CTAs retire one by one, the first SM gets the two longest.  Such a launch waits (us, chained / not:
+    // B1 H16 S4096, 1.7 waves, 415 / 402; B2 H16 S2048 225 / 224; B2 H32 S1501, 2.6 waves, 251 / 256; B1 H16
+    // S300, a sixth of a wave, 28 / 36).
+    if (grid.x > static_cast<unsigned>(num_sms) && grid.x < 4u * num_sms) {
+      p.chained = 0;
+      kern<<<grid, RsCfg<2>::kThreads, RsCfg<2>::kSmem, stream>>>(mq, mk, mq, p, lse2_out);
+      e = cudaGetLastError();
+    } else {
+      e = launch_dependent(kern, grid, dim3(RsCfg<2>::kThreads), RsCfg<2>::kSmem, stream, mq, mk, mq, p, lse2_out);
+    }
     count_launch();
-    return cudaGetLastError();
+    return e;
   }
   // TMA needs a 16-byte aligned base and strides that are multiples of 16 bytes
   const bool tma_ok = (reinterpret_cast<uintptr_t>(a.exp_rand) & 15u) == 0 && a.er_stride_q % 4 == 0 &&
@@ -1302,15 +1341,15 @@ cudaError_t launch_kf_rowstat(const CUtensorMap& mq, const CUtensorMap& mk, cons
     auto kern = s.bf16 ? kf_rowstat_kernel<true, 1> : kf_rowstat_kernel<false, 1>;
     e = ensure_dynamic_smem(reinterpret_cast<const void*>(kern), RsCfg<1>::kSmem);
     if (e != cudaSuccess) return e;
-    kern<<<grid, kRsThreads, RsCfg<1>::kSmem, stream>>>(mq, mk, mn, p, lse2_out);
+    e = launch_dependent(kern, grid, dim3(RsCfg<1>::kThreads), RsCfg<1>::kSmem, stream, mq, mk, mn, p, lse2_out);
   } else {
     auto kern = s.bf16 ? kf_rowstat_kernel<true, 0> : kf_rowstat_kernel<false, 0>;
     e = ensure_dynamic_smem(reinterpret_cast<const void*>(kern), RsCfg<0>::kSmem);
     if (e != cudaSuccess) return e;
-    kern<<<grid, kRsThreads, RsCfg<0>::kSmem, stream>>>(mq, mk, mq, p, lse2_out);
+    e = launch_dependent(kern, grid, dim3(RsCfg<0>::kThreads), RsCfg<0>::kSmem, stream, mq, mk, mq, p, lse2_out);
   }
   count_launch();
-  return cudaGetLastError();
+  return e;
 }
 
 }  // namespace asuka

@@ -113,7 +113,7 @@ int col_scores_chunks(const AttnShape& s, int mode, int num_sms, size_t ws_bytes
 size_t col_scores_split_bytes(const AttnShape& s, int mode, int chunks);
 // Keyformer row statistic: writes lse2' [B,H,Sq] of (s + g) / tau
 cudaError_t launch_kf_rowstat(const CUtensorMap& mq, const CUtensorMap& mk, const ScoreArgs& a,
-                              float* lse2_out, const AttnShape& s, cudaStream_t stream);
+                              float* lse2_out, const AttnShape& s, int num_sms, cudaStream_t stream);
 
 struct SelectArgs {
   const float* score;     // [B*H, S] rows, contiguous
