@@ -173,9 +173,11 @@ linattn32_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
 #pragma unroll
             for (int d = 0; d < 4; ++d) acc[e][d] = __fmul2_rn(acc[e][d], ff[d]);
         }
+        // (no value above -inf yet: against 0 the -infs give 0 and a NaN, which the maximum skips, stays one)
+        const float ref = s0 > -INFINITY ? s0 : 0.f;
 #pragma unroll
         for (int u = 0; u < kWarpRows; ++u) {
-          const float e = kv[u] > -INFINITY ? ex2(kv[u] - s0) : 0.f;
+          const float e = ex2(kv[u] - ref);
           s1 += e;
           kt[u * kD + lane] = e;
         }

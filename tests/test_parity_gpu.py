@@ -392,6 +392,23 @@ def test_linear_attention_blocks_at_the_reference_bench_shapes(ops, ea):
   no_timeouts(ops)
 
 
+@pytest.mark.parametrize("n", [40, 333, 784])
+def test_ea_core_with_nan_and_infinite_keys(ops, n):
+  # a NaN key makes its feature's weights NaN, -inf keys weigh nothing (a warp may see nothing else of a
+  # feature, at the front or at the end), a feature of nothing but -inf has no weights
+  g = torch.Generator().manual_seed(3)
+  q, k, v = (torch.randn(2, n, 3, 32, generator=g) for _ in range(3))
+  k[1, n // 2, 2, 5] = float("nan")
+  k[0, :n - 3, 0, 7] = float("-inf")
+  k[0, 8:, 1, 9] = float("-inf")
+  k[1, :, 0, 11] = float("-inf")
+  ref = O.linear_attention_core(q, k, v, True)
+  got = ops.linattn32_fwd(q.cuda(), k.cuda(), v.cuda(), ea=True).cpu()
+  assert torch.equal(got.isnan(), ref.isnan())
+  torch.testing.assert_close(got, ref, rtol=1e-4, atol=1e-5, equal_nan=True)
+  no_timeouts(ops)
+
+
 @pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
 @pytest.mark.parametrize("direction", [1.0, -1.0])
 def test_logits_that_keep_growing_or_shrinking(ops, dtype, direction):
