@@ -14,7 +14,7 @@
 //           for K's row alone, and shared memory was what the kernel waited for).  The statistics are gathered on the way: SimA's
 //           sums of |K| and |Q|; for EA each warp exponentiates K in place against a running
 //           reference of its own per column, raised (with its partial product rescaled) only when
-//           a value exceeds it by more than 8, so no pass over K precedes the product.
+//           a value exceeds it by more than a factor of 2^8, so no pass over K precedes the product.
 //   pass B  Q through a ring of eight tiles; the output row is written over the row of Q it came
 //           from and leaves by TMA.
 // Multiply-adds are the packed two-wide f32 FMAs of sm_100; every sum runs in a fixed order.
@@ -39,6 +39,7 @@ constexpr int kStages = 4;                   // pass A: K, V, Q tiles
 constexpr int kQStages = 8;                  // pass B: Q tiles, in the part of the ring above the partial products
 constexpr uint32_t kPartBytes = kWarps * kD * kD * 4;
 constexpr uint32_t kSmemBytes = kStages * 3 * kTileBytes + 1024;
+constexpr float kSlack = 5.5f;               // EA: by how much a key may exceed its warp's reference (e^5.5 = 2^8)
 static_assert(kPartBytes + kQStages * kTileBytes <= kStages * 3 * kTileBytes, "pass B's ring");
 
 struct Lin32Params {
@@ -51,9 +52,12 @@ struct Lin32Bars {
   uint64_t b_full[kQStages], b_empty[kQStages];
 };
 
-__device__ __forceinline__ float ex2(float x) {
+// e^x of a difference from a reference: the difference is taken first and scaled to powers of two after it.
+// (Scaling the values first rounds each by 2^-24 of itself, not of the difference: with an offset of 100
+// common to all keys the output was off by 1.7e-5 of itself, with -1000 by 1.3e-4; this way by 1.2e-7 with and without.)
+__device__ __forceinline__ float exp_fast(float x) {
   float y;
-  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x * 1.4426950408889634f));
   return y;
 }
 __device__ __forceinline__ float warp_max(float x) {
@@ -84,7 +88,6 @@ linattn32_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
   __shared__ uint32_t abort_s;
   const uint32_t ring = (smem_u32(smem_raw) + 1023u) & ~1023u;
   float* const ring_gen = reinterpret_cast<float*>(smem_raw + (ring - smem_u32(smem_raw)));
-  constexpr float kLog2e = 1.4426950408889634f;
 
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   volatile uint32_t* abortp = &abort_s;
@@ -153,14 +156,14 @@ linattn32_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
 #pragma unroll
         for (int u = 0; u < kWarpRows; ++u) {
           const bool live = t * kRows + warp * kWarpRows + u < p.N;
-          kv[u] = live ? kt[u * kD + lane] * kLog2e : -INFINITY;
+          kv[u] = live ? kt[u * kD + lane] : -INFINITY;
           mx = fmaxf(mx, kv[u]);
         }
         // (a warp whose rows all lie past the end changes nothing)
-        const bool raise = mx > s0 + 8.f;
+        const bool raise = mx > s0 + kSlack;
         if (__any_sync(0xffffffffu, raise)) {
           const float m_new = raise ? mx : s0;
-          const float f = m_new > -INFINITY ? ex2(s0 - m_new) : 1.f;
+          const float f = m_new > -INFINITY ? exp_fast(s0 - m_new) : 1.f;
           s0 = m_new;
           s1 *= f;
           scale_s[warp][lane] = f;
@@ -177,7 +180,7 @@ linattn32_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
         const float ref = s0 > -INFINITY ? s0 : 0.f;
 #pragma unroll
         for (int u = 0; u < kWarpRows; ++u) {
-          const float e = ex2(kv[u] - ref);
+          const float e = exp_fast(kv[u] - ref);
           s1 += e;
           kt[u * kD + lane] = e;
         }
@@ -231,7 +234,7 @@ linattn32_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
         for (int w = 0; w < kWarps; ++w) m = fmaxf(m, stat_s[0][w][d]);
 #pragma unroll
         for (int w = 0; w < kWarps; ++w) {
-          const float f = stat_s[0][w][d] > -INFINITY ? ex2(stat_s[0][w][d] - m) : 0.f;
+          const float f = stat_s[0][w][d] > -INFINITY ? exp_fast(stat_s[0][w][d] - m) : 0.f;
           z = fmaf(f, stat_s[1][w][d], z);
           total = fmaf(f, part[(w * kD + d) * kD + lane], total);
         }
@@ -291,8 +294,8 @@ linattn32_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
       if constexpr (kEA) {
 #pragma unroll
         for (int u = 0; u < kWarpRows; ++u) {
-          const float x = qt[u * kD + lane] * kLog2e;
-          const float e = ex2(x - warp_max(x));
+          const float x = qt[u * kD + lane];
+          const float e = exp_fast(x - warp_max(x));
           qt[u * kD + lane] = e / warp_sum(e);
         }
         __syncwarp();

@@ -409,6 +409,22 @@ def test_ea_core_with_nan_and_infinite_keys(ops, n):
   no_timeouts(ops)
 
 
+@pytest.mark.parametrize("offset", [0.0, 100.0, -1000.0])
+def test_ea_core_keeps_its_accuracy_under_a_common_offset(ops, offset):
+  # softmax does not see an offset common to all its arguments.  Each f32 weight is off by at most
+  # |x - max| (2 + log2 e) 2^-24 (difference, product, rounded log2 e) + 2^-22 (ex2.approx), at |x - max| < 9
+  # 2.1e-6; rounding errors of either sign leave well under half of that in the 2-norm
+  g = torch.Generator().manual_seed(4)
+  q, k, v = (torch.randn(2, 784, 3, 32, generator=g) for _ in range(3))
+  q, k = q + offset, k + offset
+  qd, kd, vd = (t.double().permute(0, 2, 1, 3) for t in (q, k, v))
+  ref = (torch.softmax(qd, 3) @ (torch.softmax(kd, 2).transpose(2, 3) @ vd)).permute(0, 2, 1, 3)
+  got = ops.linattn32_fwd(q.cuda(), k.cuda(), v.cuda(), ea=True).cpu().double()
+  e = ((got - ref).norm() / ref.norm()).item()
+  assert e <= 1e-6
+  no_timeouts(ops)
+
+
 @pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
 @pytest.mark.parametrize("direction", [1.0, -1.0])
 def test_logits_that_keep_growing_or_shrinking(ops, dtype, direction):
