@@ -205,13 +205,13 @@ linattn32_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
 #pragma unroll
           for (int d = 0; d < 4; ++d) acc[e][d] = __ffma2_rn(kk[d], make_float2(ve[e], ve[e]), acc[e][d]);
       }
+      if constexpr (kEA) fence_proxy_async_smem();  // (K' was written over a tile that TMA refills)
       __syncwarp();
       if (lane == 0) mbar_arrive(smem_u32(&bars.a_empty[st]));
     }
     stat_s[0][warp][lane] = s0;
     stat_s[1][warp][lane] = s1;
   }
-  if constexpr (kEA) fence_proxy_async_smem();  // (K' was written over tiles that TMA refills below)
   __syncthreads();
 
   // ---- the warps' partial products to M', in warp order, while the first tiles of pass B arrive
