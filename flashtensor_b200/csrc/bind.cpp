@@ -355,8 +355,16 @@ PyObject* linattn_block(PyObject*, PyObject* const* a, Py_ssize_t n) {
     const at::Tensor x = tensor_arg(a[0]).contiguous(), w_qkv = tensor_arg(a[1]).contiguous(),
                      b_qkv = tensor_arg(a[2]).contiguous(), w_o = tensor_arg(a[3]).contiguous(),
                      b_o = tensor_arg(a[4]).contiguous();
+    // (the core's views of the projection below take its rows to be 3 C long)
+    const int64_t C = x.dim() == 3 ? x.size(2) : -1;
+    if (C < 0 || C % 32 != 0 || !w_qkv.sizes().equals({3 * C, C}) || !b_qkv.sizes().equals({3 * C}) ||
+        !w_o.sizes().equals({C, C}) || !b_o.sizes().equals({C})) {
+      PyErr_SetString(PyExc_RuntimeError,
+                      "expected x [B, N, C], w_qkv [3C, C], b_qkv [3C], w_o [C, C], b_o [C] with C a multiple of 32");
+      throw BadArg();
+    }
     OnDevice on({&x, &w_qkv, &b_qkv, &w_o, &b_o});
-    const int64_t B = x.size(0), N = x.size(1), C = x.size(2);
+    const int64_t B = x.size(0), N = x.size(1);
     const at::Tensor qkv = linear_f32(x.view({B * N, C}), w_qkv, b_qkv, on.stream);
     const at::Tensor core = empty({B, N, C / 32, 32}, at::kFloat, x);
     asuka_linattn32_params p;

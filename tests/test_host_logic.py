@@ -138,6 +138,22 @@ def test_ops_refuse_cpu_tensors(built_lib):
     ops.attn_fwd(q, q, q)
 
 
+@pytest.mark.parametrize("bad", [
+    # index of the operand that does not fit x [2, 40, 64], and its shape
+    (0, (80, 64)), (0, (2, 40, 48)), (1, (64, 64)), (1, (193, 64)), (2, (64,)), (3, (64, 192)), (3, (32, 64)), (4, (63,)),
+])
+def test_the_whole_block_refuses_shapes_its_views_do_not_fit(built_lib, bad):
+  # (before it looks at a device: the core reads the projection's rows as 3 C floats)
+  from flashtensor_b200 import ops
+  shapes = [(2, 40, 64), (192, 64), (192,), (64, 64), (64,)]
+  shapes[bad[0]] = bad[1]
+  with pytest.raises(RuntimeError, match="expected x .B, N, C.*multiple of 32"):
+    ops.linattn_block(*(torch.zeros(s) for s in shapes))
+  shapes = [(2, 40, 64), (192, 64), (192,), (64, 64), (64,)]
+  with pytest.raises(RuntimeError, match="no CPU path"):
+    ops.linattn_block(*(torch.zeros(s) for s in shapes))
+
+
 def test_missing_library_is_loud(tmp_path, monkeypatch):
   monkeypatch.setattr(_lib, "_lib", None)
   monkeypatch.setattr(_lib, "LIB_PATH", str(tmp_path / "nope.so"))
