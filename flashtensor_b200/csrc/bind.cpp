@@ -332,6 +332,13 @@ at::Tensor linear_f32(const at::Tensor& x, const at::Tensor& w, const at::Tensor
   return out;
 }
 
+// `t` as the kernels read it: contiguous from a 16-byte boundary on.  A copy where it is not (a slice of a
+// flat parameter buffer may start anywhere); the caching allocator's blocks start on such a boundary.
+at::Tensor dense(const at::Tensor& t) {
+  const at::Tensor c = t.contiguous().resolve_neg();
+  return (reinterpret_cast<uintptr_t>(c.data_ptr()) & 15u) == 0 ? c : c.clone(at::MemoryFormat::Contiguous);
+}
+
 // (x [M, K], w [N, K], bias [N]) -> out [M, N]
 PyObject* linear(PyObject*, PyObject* const* a, Py_ssize_t n) {
   HANDLE_TH_ERRORS
@@ -352,9 +359,8 @@ PyObject* linattn_block(PyObject*, PyObject* const* a, Py_ssize_t n) {
   HANDLE_TH_ERRORS
   try {
     want_args(n, 6);
-    const at::Tensor x = tensor_arg(a[0]).contiguous(), w_qkv = tensor_arg(a[1]).contiguous(),
-                     b_qkv = tensor_arg(a[2]).contiguous(), w_o = tensor_arg(a[3]).contiguous(),
-                     b_o = tensor_arg(a[4]).contiguous();
+    const at::Tensor x = dense(tensor_arg(a[0])), w_qkv = dense(tensor_arg(a[1])), b_qkv = dense(tensor_arg(a[2])),
+                     w_o = dense(tensor_arg(a[3])), b_o = dense(tensor_arg(a[4]));
     // (the core's views of the projection below take its rows to be 3 C long)
     const int64_t C = x.dim() == 3 ? x.size(2) : -1;
     if (C < 0 || C % 32 != 0 || !w_qkv.sizes().equals({3 * C, C}) || !b_qkv.sizes().equals({3 * C}) ||

@@ -392,6 +392,24 @@ def test_linear_attention_blocks_at_the_reference_bench_shapes(ops, ea):
   no_timeouts(ops)
 
 
+def test_blocks_take_operands_from_anywhere_in_a_buffer(ops):
+  # slices of a flat buffer (contiguous, at no 16-byte boundary), and views that are not contiguous
+  from flashtensor_b200.blocks import EABlock, SimABlock
+  B, N, C = 2, 100, 64
+  shapes = [(B, N, C), (3 * C, C), (3 * C,), (C, C), (C,)]
+  flat = torch.randn(sum(int(np.prod(s)) + 1 for s in shapes), generator=torch.Generator().manual_seed(3)).cuda() / 8
+  args, at = [], 1
+  for s in shapes:
+    args.append(flat[at:at + int(np.prod(s))].view(s))
+    at += int(np.prod(s)) + 1
+  assert sum(a.data_ptr() % 16 != 0 for a in args) >= 3
+  strided = [a.repeat_interleave(2, dim=-1)[..., ::2] for a in args]
+  for block in (EABlock(), SimABlock()):
+    want = block(*(a.clone() for a in args))
+    assert torch.equal(block(*args), want) and torch.equal(block(*strided), want)
+  no_timeouts(ops)
+
+
 @pytest.mark.parametrize("n", [40, 333, 784])
 def test_ea_core_with_nan_and_infinite_keys(ops, n):
   # a NaN key makes its feature's weights NaN, -inf keys weigh nothing (a warp may see nothing else of a
