@@ -170,7 +170,8 @@ LINEAR_MAX_K = 128
 
 def linattn_block(x, w_qkv, b_qkv, w_o, b_o, ea=False):
   """The whole block of bench/sima.mlir (ea=False) or bench/ea.mlir (ea=True), f32: QKV projection,
-  core, output projection in three launches.  x [B, N, C], C a multiple of 32 and at most LINEAR_MAX_K."""
+  core, output projection in three launches.  x [B, N, C], C a multiple of 32 and at most LINEAR_MAX_K.
+  The result has no graph, whatever the operands require (``blocks`` takes another way then)."""
   return _bind().linattn_block(x, w_qkv, b_qkv, w_o, b_o, ea)
 
 

@@ -154,6 +154,42 @@ def test_the_whole_block_refuses_shapes_its_views_do_not_fit(built_lib, bad):
     ops.linattn_block(*(torch.zeros(s) for s in shapes))
 
 
+@pytest.mark.parametrize("ea", [False, True])
+def test_blocks_leave_torch_what_is_more_than_values(monkeypatch, ea):
+  # the output projection gives w_o and b_o gradients, tangents and a batch dimension; only a call that
+  # wants none of it goes to the native block
+  import torch.autograd.forward_ad as fwad
+  from flashtensor_b200 import ops
+  from flashtensor_b200.blocks import EABlock, SimABlock
+  from oracle import attn_oracle as O
+  native = []
+  monkeypatch.setattr(ops, "linattn_block", lambda *a, ea: native.append(ea) or O.linear_attention_block(*a, ea))
+  monkeypatch.setattr(ops, "linattn32_fwd", lambda q, k, v, ea: O.linear_attention_core(q, k, v, ea).contiguous())
+  g = torch.Generator().manual_seed(1)
+  C, B, N = 64, 2, 10
+  x, w_qkv, b_qkv, w_o, b_o = (torch.randn(s, generator=g) for s in ((B, N, C), (3 * C, C), (3 * C,), (C, C), (C,)))
+  block = EABlock() if ea else SimABlock()
+  want = block(x, w_qkv, b_qkv, w_o, b_o)
+  assert native == [ea]
+  w, b = torch.nn.Parameter(w_o.clone()), torch.nn.Parameter(b_o.clone())
+  with torch.no_grad():
+    block(x, w_qkv, b_qkv, w, b)
+  assert native == [ea, ea]
+  out = block(x, w_qkv, b_qkv, w, b)
+  torch.testing.assert_close(out, want)
+  up = torch.randn(out.shape, generator=g)
+  out.backward(up)
+  torch.testing.assert_close(b.grad, up.sum((0, 1)))
+  # (the output is core w_o^T + b_o, so its derivative by w_o along w_o is the output without the bias)
+  torch.testing.assert_close((w.grad * w_o).sum(), (up * (want - b_o)).sum(), rtol=1e-4, atol=1e-4)
+  with fwad.dual_level():
+    dual = block(x, w_qkv, b_qkv, fwad.make_dual(w_o, w_o), b_o)
+    torch.testing.assert_close(fwad.unpack_dual(dual).tangent, want - b_o, rtol=1e-4, atol=1e-4)
+  many = torch.vmap(lambda b: block(x, w_qkv, b_qkv, w_o, b))(torch.stack([b_o, 2 * b_o]))
+  torch.testing.assert_close(many[1], want + b_o)
+  assert native == [ea, ea]
+
+
 def test_missing_library_is_loud(tmp_path, monkeypatch):
   monkeypatch.setattr(_lib, "_lib", None)
   monkeypatch.setattr(_lib, "LIB_PATH", str(tmp_path / "nope.so"))
