@@ -21,8 +21,16 @@
 // to an accumulator, and forty small terms added to a large sum would each leave a bias there
 // (measured at K = 128: 4.1e-7 relative error in the natural order, against 1.5e-7 of an f32 GEMM on
 // the CUDA cores).
-// Measured at B64 N784 C128 (M = 50176, K = 128), bias included: N = 384 (QKV) 32 us, N = 128 (output)
-// 15 us; the f32 GEMM of the BLAS library with its bias pass takes 200 and 64.
+// The split is sound while its terms and products stay clear of both ends of the exponent range.  Infinities
+// and values that round to one have no residual: they, like anything that overflows, leave a sum that is not
+// finite.  Terms and products below 2^-126 are flushed: with weights below 2^20 that costs a sum 2^-98 at most,
+// which is below the rounding of one of 2^-72 or more.  So a sum that is not finite or below 2^-72, and a
+// column with a weight outside [2^-100, 2^20) that is not zero, is computed on the CUDA cores (plain_dot) by
+// the warps that store it; which way a result takes depends on its own row and column.  That is for the odd row
+// or column: all rows at 1e-25 take 1460 us instead of 34, rows of nothing but zeros, which need a look at x only, 91.
+// Measured at B64 N784 C128 (M = 50176, K = 128), calls back to back, bias included: N = 384 (QKV) 33 us,
+// N = 128 (output) 17.7 us (31.5 and 16 without the look at the sums); the f32 GEMM of the BLAS library with its
+// bias pass takes 200 and 64.
 #include <cuda_bf16.h>
 
 #include "kernels.h"
@@ -58,6 +66,83 @@ struct LinParams {
   uint32_t* status;
 };
 
+constexpr float kWeightLow = 7.8886090522101181e-31f, kWeightHigh = 1048576.f;  // 2^-100, 2^20
+constexpr float kSumLow = 2.1175823681357508e-22f;                               // 2^-72
+// (these keep subnormal values, which the build's flags flush elsewhere)
+__device__ __forceinline__ float fma_keep(float a, float b, float c) {
+  float y;
+  asm("fma.rn.f32 %0, %1, %2, %3;" : "=f"(y) : "f"(a), "f"(b), "f"(c));
+  return y;
+}
+__device__ __forceinline__ float add_keep(float a, float b) {
+  float y;
+  asm("add.rn.f32 %0, %1, %2;" : "=f"(y) : "f"(a), "f"(b));
+  return y;
+}
+__device__ __forceinline__ float max3_nan(float a, float b, float c) {
+  float y;
+  asm("max.NaN.f32 %0, %1, %2, %3;" : "=f"(y) : "f"(a), "f"(b), "f"(c));
+  return y;
+}
+__device__ __forceinline__ float min3(float a, float b, float c) {
+  float y;
+  asm("min.f32 %0, %1, %2, %3;" : "=f"(y) : "f"(a), "f"(b), "f"(c));
+  return y;
+}
+
+// largest (NaN if there is one) and smallest magnitude of eight values
+__device__ __forceinline__ void extent8(const float (&v)[8], float* big, float* small) {
+  float a[8];
+#pragma unroll
+  for (int i = 0; i < 8; ++i) a[i] = fabsf(v[i]);
+  *big = max3_nan(max3_nan(a[0], a[1], a[2]), max3_nan(a[3], a[4], a[5]), max3_nan(a[6], a[7], a[7]));
+  *small = min3(min3(a[0], a[1], a[2]), min3(a[3], a[4], a[5]), min3(a[6], a[7], a[7]));
+}
+
+// One row of x against the 32 columns from n_base on, by a whole warp: lane l takes reduction columns 4l to
+// 4l + 3 and returns the sum for output column n_base + l.
+__device__ __noinline__ float plain_dot(const float* __restrict__ x_row, const float* __restrict__ w, int n_base, int N, int K) {
+  const int lane = threadIdx.x & 31;
+  const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+  const bool live = lane * 4 < K;
+  const float4 xv = live ? __ldg(reinterpret_cast<const float4*>(x_row) + lane) : zero;
+  float part[32];
+#pragma unroll
+  for (int c = 0; c < 32; ++c) {
+    const float4 wv = live ? __ldg(reinterpret_cast<const float4*>(w + static_cast<int64_t>(min(n_base + c, N - 1)) * K) + lane) : zero;
+    part[c] = fma_keep(xv.x, wv.x, fma_keep(xv.y, wv.y, fma_keep(xv.z, wv.z, fma_keep(xv.w, wv.w, 0.f))));
+  }
+  // every exchange adds two lanes' sums and halves the columns a lane still holds
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    const bool upper = (lane & o) != 0;
+#pragma unroll
+    for (int c = 0; c < o; ++c)
+      part[c] = add_keep(upper ? part[c + o] : part[c], __shfl_xor_sync(0xffffffffu, upper ? part[c] : part[c + o], o));
+  }
+  return part[0];
+}
+
+// Which of the 32 rows from `x` on (`rows` of them there) have a value other than zero: one bit each.  (Rows
+// of zeros, a batch's padding, have sums of zero that need no second look; eight loads in flight.)
+__device__ __noinline__ uint32_t rows_not_zero(const float* __restrict__ x, int rows, int K) {
+  const int lane = threadIdx.x & 31;
+  uint32_t mask = 0;
+  for (int r0 = 0; r0 < 32; r0 += 8) {
+    float4 v[8];
+#pragma unroll
+    for (int r = 0; r < 8; ++r)
+      v[r] = r0 + r < rows && lane * 4 < K ? __ldg(reinterpret_cast<const float4*>(x + static_cast<int64_t>(r0 + r) * K) + lane)
+                                           : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+    for (int r = 0; r < 8; ++r) {
+      const uint32_t bits = __float_as_uint(v[r].x) | __float_as_uint(v[r].y) | __float_as_uint(v[r].z) | __float_as_uint(v[r].w);
+      if (__any_sync(0xffffffffu, (bits << 1) != 0u)) mask |= 1u << (r0 + r);
+    }
+  }
+  return mask;
+}
+
 struct LinBars {
   uint64_t x_full[2], x_empty[2];
   uint64_t acc_full[2], acc_empty[2];
@@ -78,7 +163,7 @@ __device__ __forceinline__ void split8(const float (&v)[8], uint4 (&t)[3]) {
       const uint32_t p = pack_bf16(a, b);
       w[s][i] = p;
       const float ra = __uint_as_float(p << 16), rb = __uint_as_float(p & 0xffff0000u);
-      a -= ra;  // (exact; infinite values leave NaN, so a row with one gives NaN)
+      a -= ra;  // (exact; an infinity leaves NaN)
       b -= rb;
     }
   }
@@ -129,6 +214,7 @@ __global__ void __launch_bounds__(kThreads, 1) linear_f32_kernel(const __grid_co
   const int wq = warp & 3;  // (epilogue warps) TMEM lane quarter
   const uint32_t lane_base = static_cast<uint32_t>(wq * 32) << 16;
   const int n = n0 + wq * 32 + lane;  // (epilogue warps) this thread's output column
+  float w_big = 0.f, w_small = kWeightHigh;  // (epilogue warps) of that column's weights, the zeros apart
   griddep_wait();
   griddep_launch_dependents();
   if (warp > kSplitWarps) {
@@ -143,6 +229,10 @@ __global__ void __launch_bounds__(kThreads, 1) linear_f32_kernel(const __grid_co
         const float4 lo = live ? __ldg(reinterpret_cast<const float4*>(src + k)) : make_float4(0.f, 0.f, 0.f, 0.f);
         const float4 hi = live ? __ldg(reinterpret_cast<const float4*>(src + k + 4)) : make_float4(0.f, 0.f, 0.f, 0.f);
         const float v[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
+        float big, small;
+        extent8(v, &big, &small);
+        w_big = max3_nan(w_big, big, big);
+        w_small = k < p.K ? fminf(w_small, small) : w_small;
         uint4 q[3];
         split8(v, q);
 #pragma unroll
@@ -157,6 +247,14 @@ __global__ void __launch_bounds__(kThreads, 1) linear_f32_kernel(const __grid_co
       for (int s = 0; s < 3; ++s) tmem_st16(tbase + lane_base + s * kTermCols + k0 / 2, t[s]);
     }
     tmem_wait_st();
+    if (w_small < kWeightLow) {  // a zero, which is no matter, or not: look again
+      w_small = kWeightHigh;
+      if (n < p.N)
+        for (int k = 0; k < p.K; ++k) {
+          const float a = __ldg(src + k);
+          if ((__float_as_uint(a) << 1) != 0u) w_small = fminf(w_small, fabsf(a));  // (a subnormal counts as 0)
+        }
+    }
   }
   tc_fence_before_sync();
   __syncthreads();
@@ -247,6 +345,9 @@ __global__ void __launch_bounds__(kThreads, 1) linear_f32_kernel(const __grid_co
     // ------------------------------------------------------------------ epilogue
     uint8_t* const stage = gX + 2 * kStageBytes + wq * 2 * kOutBytes;
     const float bias = n < p.N ? __ldg(p.bias + n) : 0.f;
+    const bool zero_col = w_big == 0.f;  // a sum of zero is right (with a subnormal weight it is a plain one)
+    const bool plain_col = !(w_big < kWeightHigh) || w_small < kWeightLow;
+    const bool any_plain_col = __any_sync(0xffffffffu, plain_col);
     uint32_t t = 0;
     for (int mt = m_first; mt < p.m_tiles; mt += m_step, ++t) {
       const int st = t & 1;
@@ -256,6 +357,8 @@ __global__ void __launch_bounds__(kThreads, 1) linear_f32_kernel(const __grid_co
       }
       tc_fence_after_sync();
       const int row_t = mt * kTile;
+      float big = 0.f, small = kWeightHigh;  // of this column's sums in the tile
+      bool again = any_plain_col;
 #pragma unroll
       for (int q = 0; q < 4; ++q) {
         uint32_t u[32];
@@ -264,13 +367,27 @@ __global__ void __launch_bounds__(kThreads, 1) linear_f32_kernel(const __grid_co
         if (lane == 0) tma_store_wait_read_n<1>();  // the store before last has left this half of the stage
         __syncwarp();
         tmem_wait_ld();
+        if (row_t + q * 32 + 32 > p.M) {  // (rows past the end, zero as well, are not stored)
+#pragma unroll
+          for (int r = 0; r < 32; ++r) u[r] = row_t + q * 32 + r < p.M ? u[r] : 0x3f800000u;
+        }
+#pragma unroll
+        for (int g = 0; g < 4; ++g) {
+          float b8, s8;
+          extent8(reinterpret_cast<const float(&)[8]>(u[g * 8]), &b8, &s8);
+          big = max3_nan(big, b8, b8);
+          small = fminf(small, s8);
+        }
         if (q == 3) {
-          tc_fence_before_sync();
-          mbar_arrive(smem_u32(&bars.acc_empty[st]));
+          again = __any_sync(0xffffffffu, !(big < INFINITY) || (small < kSumLow && !zero_col)) || again;
+          if (!again) {
+            tc_fence_before_sync();
+            mbar_arrive(smem_u32(&bars.acc_empty[st]));
+          }
         }
 #pragma unroll
         for (int r = 0; r < 32; ++r)
-          *reinterpret_cast<float*>(dst + sw128_offset(r, lane >> 2) + (lane & 3) * 4) = __uint_as_float(u[r]) + bias;
+          *reinterpret_cast<float*>(dst + sw128_offset(r, lane >> 2) + (lane & 3) * 4) = add_keep(__uint_as_float(u[r]), bias);
         const int row_q = row_t + q * 32;
         if (p.tma_out) {
           fence_proxy_async_smem();
@@ -284,6 +401,35 @@ __global__ void __launch_bounds__(kThreads, 1) linear_f32_kernel(const __grid_co
             p.out[static_cast<int64_t>(row_q + r) * p.N + n] =
                 *reinterpret_cast<const float*>(dst + sw128_offset(r, lane >> 2) + (lane & 3) * 4);
         }
+      }
+      if (again) {
+        // results that the sum is not good enough for, over what has just been stored
+        if (lane == 0) tma_store_wait_all();
+        __syncwarp();
+#pragma unroll 1
+        for (int q = 0; q < 4; ++q) {
+          const int row_q = row_t + q * 32;
+          uint32_t u[32];
+          tmem_ld32(tbase + lane_base + kAccCol + st * 128 + q * 32, u);
+          tmem_wait_ld();
+          uint32_t mine = 0;  // this column's rows
+#pragma unroll
+          for (int r = 0; r < 32; ++r) {
+            const float a = fabsf(__uint_as_float(u[r]));
+            if (!(a < INFINITY) || (a < kSumLow && !zero_col)) mine |= 1u << r;
+          }
+          if (plain_col) mine = 0xffffffffu;
+          uint32_t left = __reduce_or_sync(0xffffffffu, mine);
+          if (!any_plain_col && left != 0u) left &= rows_not_zero(p.x + static_cast<int64_t>(row_q) * p.K, p.M - row_q, p.K);
+          for (; left != 0u; left &= left - 1u) {
+            const int r = __ffs(left) - 1;
+            if (row_q + r >= p.M) break;
+            const float y = plain_dot(p.x + static_cast<int64_t>(row_q + r) * p.K, p.w, n0 + wq * 32, p.N, p.K);
+            if (((mine >> r) & 1u) != 0u && n < p.N) p.out[static_cast<int64_t>(row_q + r) * p.N + n] = add_keep(y, bias);
+          }
+        }
+        tc_fence_before_sync();
+        mbar_arrive(smem_u32(&bars.acc_empty[st]));
       }
     }
     if (lane == 0) tma_store_wait_all();

@@ -213,8 +213,9 @@ int asuka_b200_linattn32_fwd(const asuka_linattn32_params* p, asuka_stream strea
 
 /* ---- the projections around that core (bench/sima.mlir:3-5,18-22): out = x w^T + bias in f32 -------
  * x [M, K], w [N, K], bias [N], out [M, N], f32, contiguous; K a multiple of 8, at most
- * ASUKA_LINEAR_MAX_K.  The result has f32 accuracy (products of three-term bf16 splits on the tensor
- * pipe, f32 accumulation). */
+ * ASUKA_LINEAR_MAX_K.  The result has f32 accuracy over f32's whole range, infinities and NaN included
+ * (products of three-term bf16 splits on the tensor pipe, f32 accumulation; results that come out below
+ * 2^-72 or not finite, and columns with weights outside [2^-100, 2^20), by f32 FMA instead). */
 #define ASUKA_LINEAR_MAX_K 128
 typedef struct {
   asuka_tensor x, w, bias, out;

@@ -360,6 +360,49 @@ def test_f32_projection_vs_float64(ops, shape):
   no_timeouts(ops)
 
 
+@pytest.mark.parametrize("shape", [(300, 96, 128), (130, 33, 40), (5, 8, 8), (40000, 384, 64)])
+def test_f32_projection_outside_ordinary_magnitudes(ops, shape):
+  # infinities, NaN, values next to the largest and below the smallest normal number, in rows of x and in
+  # columns: f32's own result, to the bound of the test above plus half the smallest subnormal a rounding;
+  # rows and columns without such a value keep their bits (the last shape: seven row tiles per CTA)
+  M, N, K = shape
+  g = torch.Generator().manual_seed(M)
+  x, w, b = torch.randn(M, K, generator=g), torch.randn(N, K, generator=g), torch.randn(N, generator=g)
+  plain = ops.linear_f32(x.cuda(), w.cuda(), b.cuda()).cpu()
+  inf, nan = float("inf"), float("nan")
+  rows = torch.randperm(M, generator=g)[:max(M // 50, 5)]
+  cols = torch.randperm(N, generator=g)[:6]
+  for n, r in enumerate(rows.tolist()):
+    if n % 5 == 0:
+      x[r, n % K] = (inf, -inf, nan, 3.4e38, -3.3953e38)[n // 5 % 5]
+    else:
+      x[r] *= (1e-35, 1e-39, 1e18, 2.0 ** -60)[n % 5 - 1]
+  b[cols[:4]] = 0.0
+  w[cols[0]] *= 1e-33
+  w[cols[1]] *= 1e-39
+  w[cols[2]] *= 1e18
+  w[cols[3]] = 0.0
+  w[cols[4], K - 1] = -inf
+  w[cols[5]] = w[cols[5]].bfloat16().float()
+  got = ops.linear_f32(x.cuda(), w.cuda(), b.cuda()).cpu()
+  ref = x.double() @ w.double().t() + b.double()
+  # (a value at the edge of overflow may fall on either side of it; a product that overflows against an
+  # infinity is NaN in f32 and infinite in float64)
+  top = torch.finfo(torch.float32).max
+  edge = (ref.abs() - top).abs() < 1e-4 * top
+  edge[:, cols[4]] |= (x.isfinite() & (x.abs() > 1e38)).any(1)
+  want = ref.float()
+  assert torch.equal(got.isnan() & ~edge, want.isnan() & ~edge)
+  assert torch.equal(got.isinf() & ~edge, want.isinf() & ~edge) and torch.equal(got[got.isinf()] > 0, want[got.isinf()] > 0)
+  finite = want.isfinite() & ~edge
+  bound = (K + 2) * (2.0 ** -23 * (x.double().abs() @ w.double().abs().t() + b.double().abs()) + 2.0 ** -149)
+  assert ((got.double() - ref).abs() <= bound)[finite].all()
+  keep_r, keep_c = torch.ones(M, dtype=torch.bool), torch.ones(N, dtype=torch.bool)
+  keep_r[rows], keep_c[cols] = False, False
+  assert torch.equal(got[keep_r][:, keep_c], plain[keep_r][:, keep_c])
+  no_timeouts(ops)
+
+
 @pytest.mark.parametrize("ea", [False, True])
 def test_linear_attention_blocks_at_the_reference_bench_shapes(ops, ea):
   # bench/sima.mlir / bench/ea.mlir: x [B, 784, 128] f32, 4 heads of 32; B reduced from 64 for the CPU oracle
