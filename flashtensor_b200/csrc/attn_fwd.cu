@@ -589,9 +589,15 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
             big |= __float_as_uint(z.x) | __float_as_uint(z.y);
           }
           if (__any_sync(0xffffffffu, (big & 0x40000000u) != 0)) {
-            // (bit 30: some logit of the warp's rows is as large as the cap, infinite or NaN)
+            // (bit 30: some logit of the warp's rows is as large as the cap, infinite or NaN; the others are
+            // treated as below, so that what a logit becomes depends on no other row and no masked key)
 #pragma unroll
-            for (int i = 0; i < 128; ++i) e[i] = tanh_approx(0.5f * e[i]);
+            for (int i = 0; i < 64; ++i) {
+              const float2 z = make_float2(e[2 * i], e[2 * i + 1]);
+              const float2 t = tanh_half2(z);
+              e[2 * i] = fabsf(z.x) < 2.f ? t.x : tanh_approx(0.5f * z.x);
+              e[2 * i + 1] = fabsf(z.y) < 2.f ? t.y : tanh_approx(0.5f * z.y);
+            }
           } else {
 #pragma unroll
             for (int i = 0; i < 64; ++i) {

@@ -539,6 +539,25 @@ def test_forward_cuts_with_a_moving_reference(ops, shape, direction):
   no_timeouts(ops)
 
 
+@pytest.mark.parametrize("shape", [(1, 384, 2), (2, 900, 45), (1, 4200, 1)])
+def test_soft_capped_rows_depend_on_nothing_else(ops, shape):
+  # a masked key and another query row whose logits exceed the cap leave a row's bits alone (one tile per
+  # item, two, keys cut into parts)
+  B, S, H = shape
+  g = torch.Generator(device="cuda").manual_seed(S)
+  q, k, v = (torch.randn(B, S, H, 128, generator=g, device="cuda", dtype=torch.bfloat16) for _ in range(3))
+  base = ops.attn_fwd(q, k, v, softcap=30.0)
+  k2 = k.clone()
+  k2[:, -1] *= 200
+  assert torch.equal(ops.attn_fwd(q, k2, v, softcap=30.0)[:, :-1], base[:, :-1])
+  q2 = q.clone()
+  q2[:, 70] *= 200
+  out = ops.attn_fwd(q2, k, v, softcap=30.0)
+  assert torch.equal(out[:, :70], base[:, :70]) and torch.equal(out[:, 71:], base[:, 71:])
+  assert not torch.equal(out[:, 70], base[:, 70])
+  no_timeouts(ops)
+
+
 @pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
 def test_sibling_cases_vs_oracle(ops, dtype):
   # Gemma-2 soft-capping, SnapKV pooling and CORM thresholds on ragged and rectangular shapes
