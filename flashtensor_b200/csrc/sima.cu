@@ -433,7 +433,9 @@ sima_stats_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
 #pragma unroll
           for (int e = 0; e < 4; ++e) {
             const float r0 = ref_s[chunk16 * 8 + 2 * e], r1 = ref_s[chunk16 * 8 + 2 * e + 1];
-            nref[e] = make_float2(-r0 * kL2e, -r1 * kL2e);
+            // (a column of nothing but -inf so far: against 0 its exponentials are 0; the reference stays -inf,
+            // is raised by the first finite value and weighs nothing in the reduce)
+            nref[e] = make_float2(r0 > -INFINITY ? -r0 * kL2e : 0.f, r1 > -INFINITY ? -r1 * kL2e : 0.f);
             thr[e] = pack2_16<kBF16>(make_float2(r0 + kEaSlack, r1 + kEaSlack));
           }
           dead = dead || *abortp != 0u;

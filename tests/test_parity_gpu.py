@@ -343,6 +343,24 @@ def test_ea_keys_that_grow_along_the_sequence(ops, shape, dtype):
   no_timeouts(ops)
 
 
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("shape", [(1, 1100, 2), (2, 2500, 3), (2, 640, 40)])
+def test_ea_with_infinite_keys(ops, shape, dtype):
+  # keys of -inf weigh nothing, in one feature or in all (padding), though a whole tile, the first tiles or
+  # the last, ragged one of a CTA's run may have nothing else
+  B, S, H = shape
+  g = torch.Generator().manual_seed(S)
+  q, k, v = (torch.randn(B, S, H, 128, generator=g).to(dtype) for _ in range(3))
+  k[:, 128:512, :, 3] = float("-inf")
+  k[:, :384, :, 4] = float("-inf")
+  k[:, S - S % 128:, :, 5] = float("-inf")
+  k[:, S - 40:] = float("-inf")
+  ref = O.ea(q, k, v)
+  close(ops.ea_fwd(q.cuda(), k.cuda(), v.cuda(), out_dtype=torch.float32), ref, "ea f32 out")
+  close(ops.ea_fwd(q.cuda(), k.cuda(), v.cuda()), ref, "ea 16-bit out")
+  no_timeouts(ops)
+
+
 @pytest.mark.parametrize("shape", [(1, 8, 8), (129, 97, 40), (128, 384, 128), (1000, 128, 64), (77, 130, 128), (40000, 96, 32)])
 def test_f32_projection_vs_float64(ops, shape):
   # tile edges in rows and columns, both reduction lengths of a tile, more row tiles than CTAs; f32
