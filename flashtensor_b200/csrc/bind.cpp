@@ -160,8 +160,8 @@ PyObject* attn_fwd(PyObject*, PyObject* const* a, Py_ssize_t n) {
     want_args(n, 8);
     const at::Tensor& q0 = tensor_arg(a[0]);
     const at::Tensor q = as4d(q0), k = as4d(tensor_arg(a[1])), v = as4d(tensor_arg(a[2]));
-    OnDevice on({&q, &k, &v});
     at::Tensor out = optional_tensor(a[6]), lse;
+    OnDevice on({&q, &k, &v, &out});
     if (!out.defined()) out = empty(q.sizes(), q.scalar_type(), q);
     const bool want_lse = bool_arg(a[5]);
     if (want_lse) lse = empty({q.size(0), q.size(2), q.size(1)}, at::kFloat, q);
@@ -204,10 +204,12 @@ PyObject* run_case(PyObject*, PyObject* const* a, Py_ssize_t n) {
     const at::Tensor& q0 = tensor_arg(a[1]);
     const at::Tensor q = as4d(q0), k = as4d(tensor_arg(a[2])), v = as4d(tensor_arg(a[3]));
     const at::Tensor exp_rand = optional_tensor(a[6]);
-    OnDevice on({&q, &k, &v, &exp_rand});
     const int64_t n_idx = static_cast<int64_t>(int_arg(a[11]));
     at::Tensor ws = optional_tensor(a[12]), out = optional_tensor(a[13]), score = optional_tensor(a[14]),
-               score_sq = optional_tensor(a[15]), idx = optional_tensor(a[16]);
+               score_sq = optional_tensor(a[15]), idx = optional_tensor(a[16]), stats[2];
+    for (int i = 0; i < 2; ++i)
+      if (a[17 + i] != Py_True) stats[i] = optional_tensor(a[17 + i]);
+    OnDevice on({&q, &k, &v, &exp_rand, &ws, &out, &score, &score_sq, &idx, &stats[0], &stats[1]});
     // scores and indices are per key/value head (with grouped-query attention: the group mean)
     const int64_t B = k.size(0), Skv = k.size(1), H = k.size(2);
     if (!out.defined()) out = empty(q.sizes(), q.scalar_type(), q);
@@ -230,9 +232,8 @@ PyObject* run_case(PyObject*, PyObject* const* a, Py_ssize_t n) {
     p.causal = bool_arg(a[4]) ? 1 : 0;
     p.k_keep = static_cast<int32_t>(int_arg(a[9]));
     p.recent = static_cast<int32_t>(int_arg(a[10]));
-    at::Tensor stats[2];
     for (int i = 0; i < 2; ++i)
-      stats[i] = a[17 + i] == Py_True ? empty({B, q.size(2), Skv}, at::kFloat, q) : optional_tensor(a[17 + i]);
+      if (a[17 + i] == Py_True) stats[i] = empty({B, q.size(2), Skv}, at::kFloat, q);
     p.roco_mean = desc(stats[0]);
     p.roco_std = desc(stats[1]);
     p.seed_unit_offset = static_cast<uint32_t>(int_arg(a[19]));
@@ -482,8 +483,8 @@ PyObject* select_topk(PyObject*, PyObject* const* a, Py_ssize_t n) {
   try {
     want_args(n, 10);
     const at::Tensor& score = tensor_arg(a[0]);
-    const at::Tensor score_sq = optional_tensor(a[1]);
-    OnDevice on({&score, &score_sq});
+    const at::Tensor score_sq = optional_tensor(a[1]), mean = optional_tensor(a[8]), std = optional_tensor(a[9]);
+    OnDevice on({&score, &score_sq, &mean, &std});
     const at::Tensor idx = empty({score.size(0), score.size(1), static_cast<int64_t>(int_arg(a[5]))}, at::kInt, score);
     asuka_select_params p;
     std::memset(&p, 0, sizeof(p));
@@ -495,8 +496,8 @@ PyObject* select_topk(PyObject*, PyObject* const* a, Py_ssize_t n) {
     p.q_len = static_cast<int32_t>(int_arg(a[6]));
     p.mode = static_cast<int32_t>(int_arg(a[3]));
     p.all_rows = bool_arg(a[7]) ? 1 : 0;
-    p.mean = desc(optional_tensor(a[8]));
-    p.std = desc(optional_tensor(a[9]));
+    p.mean = desc(mean);
+    p.std = desc(std);
     call("asuka_b200_select_topk", [&] { return asuka_b200_select_topk(&p, on.stream); });
     return wrap(idx);
   } catch (const BadArg&) {

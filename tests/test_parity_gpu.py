@@ -808,6 +808,26 @@ def test_errors_raise_and_leave_the_device_usable(ops):
   no_timeouts(ops)
 
 
+def test_buffers_of_the_caller_must_be_on_the_device(ops):
+  # (a host pointer in place of one would be written by a kernel)
+  q = torch.zeros(1, 256, 2, 128, dtype=torch.float16, device="cuda")
+  on_host = lambda *s, dtype=torch.float32: torch.zeros(s, dtype=dtype)
+  calls = [
+      lambda: ops.attn_fwd(q, q, q, out=on_host(1, 256, 2, 128, dtype=torch.float16)),
+      lambda: ops.h2o(q, q, q, out=on_host(1, 256, 2, 128, dtype=torch.float16)),
+      lambda: ops.h2o(q, q, q, score=on_host(1, 2, 256)),
+      lambda: ops.h2o(q, q, q, workspace=on_host(1 << 20, dtype=torch.uint8)),
+      lambda: ops.h2o(q, q, q, k_keep=8, recent=4, idx=on_host(1, 2, 12, dtype=torch.int32)),
+      lambda: ops.roco(q, q, q, score_sq=on_host(1, 2, 256)),
+      lambda: ops.roco(q, q, q, k_keep=8, return_stats=True, roco_mean=on_host(1, 2, 256)),
+      lambda: ops.roco(q, q, q, k_keep=8, return_stats=True, roco_std=on_host(1, 2, 256)),
+  ]
+  for call in calls:
+    with pytest.raises(RuntimeError, match="no CPU path"):
+      call()
+  no_timeouts(ops)
+
+
 class _Banded:
   """Tensors carved out of one pattern-filled device buffer with untouched bands around each, to
   catch stores that land outside an output or a workspace (the ragged ends are the risk)."""
