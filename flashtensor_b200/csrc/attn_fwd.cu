@@ -56,8 +56,15 @@ template <int kMode> struct Rings {
   static constexpr int kV = kMode == kSolo ? 3 : 2;
 };
 constexpr int kThreads = 384;
-constexpr int kUtilRegs = 96;      // 128 * 96 + 256 * 200 = 63488 <= 384 * 168
-constexpr int kSoftmaxRegs = 200;
+// Registers of the utility and of the softmax warps; what a block asks for must fit its 384 * 168 = 64512.
+// The soft-capped one-tile mode has both ways of the tanh beside what its merge keeps: at 200 it spills 464
+// bytes (B1 S1024, 16/8 heads 22 us), at 216 140 (17.6).
+template <bool kCap, int kMode> struct Regs {
+  static constexpr int kUtil = kCap && kMode == kSolo ? 72 : 96;
+  static constexpr int kSoftmax = kCap && kMode == kSolo ? 216 : 200;
+  static constexpr int kBlock = 128 * kUtil + 256 * kSoftmax;
+  static_assert(kBlock <= kThreads * 168, "setmaxnreg would wait for ever");
+};
 constexpr uint32_t kSmemBytes = 7 * kTileBytes + 1024;
 constexpr float kRescaleLimit = 6.0f;  // log2 of the largest exponential tolerated under a stale reference:
                                        // keeps a tile's row sum below 2^13, far from fp16's 65504
@@ -121,8 +128,10 @@ __device__ __forceinline__ float tanh_approx(float x) {
 // tanh(z / 2) for |z| < 2 on the FMA pipe, two at a time: z times a polynomial in z^2, fitted to the smallest
 // relative error on that range (8.2e-5; tanh.approx has 4.9e-4).  The MUFU bounds the soft-capped kernel
 // when it has both the tanh and the exponential of a logit: 8 clk each per warp and scheduler, against 6 of
-// the FMA pipe for this.  bf16 B1 S8192 16/8 heads: 357 us with tanh.approx for all, 358 with it for half,
-// 311 for a quarter, 303 for none; S1024 24.7 -> 16.9.
+// the FMA pipe for this.  Logits beyond the cap keep tanh.approx; a warp's tile that has one pays for both.
+// bf16, 16/8 heads, calls back to back on a cool card: B1 S8192 367 us with tanh.approx for all, 294 with this
+// for all, 417 with both; S1024 (two tiles per item, one, one) 25, 17.6, 22.  In the middle of other work, where
+// the clock is lower, S8192 takes 366 and 340.
 __device__ __forceinline__ float2 tanh_half2(float2 z) {
   const float2 y = __fmul2_rn(z, z);
   float2 p = make_float2(-0.000208044279133901f, -0.000208044279133901f);
@@ -342,7 +351,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
   // 384 threads x 168 registers: the four utility warps hand most of theirs to the softmax warps
   if (warp == 0) {
     // ------------------------------------------------------------------ TMA producer: Q and K
-    reg_dealloc<kUtilRegs>();
+    reg_dealloc<Regs<kCap, kMode>::kUtil>();
     if (lane == 0) {
       bool ok = true;
       uint32_t kc = 0;            // K tiles issued so far
@@ -385,7 +394,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
     }
   } else if (warp == 2) {
     // ------------------------------------------------------------------ TMA producer: V
-    reg_dealloc<kUtilRegs>();
+    reg_dealloc<Regs<kCap, kMode>::kUtil>();
     if (lane == 0) {
       bool ok = true;
       uint32_t vc = 0;
@@ -421,7 +430,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
     // costs 130 clk beside two busy softmax warps: P.V has an issuing warp of its own so that the two
     // cover for each other (from one warp a pair of steps took 4200 clk), and the barriers of a step are
     // probed together.
-    reg_dealloc<kUtilRegs>();
+    reg_dealloc<Regs<kCap, kMode>::kUtil>();
     {
       constexpr uint32_t kFmt = kBF16 ? UMMA_BF16 : UMMA_F16;
       constexpr uint32_t idesc_qk = umma_idesc_f16(kFmt, UMMA_K_MAJOR, UMMA_K_MAJOR, 128, 128);
@@ -479,7 +488,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
     }
   } else if (warp == 3) {
     // ------------------------------------------------------------------ P.V issuer
-    reg_dealloc<kUtilRegs>();
+    reg_dealloc<Regs<kCap, kMode>::kUtil>();
     {
       constexpr uint32_t kFmt = kBF16 ? UMMA_BF16 : UMMA_F16;
       constexpr uint32_t idesc_pv = umma_idesc_f16(kFmt, UMMA_K_MAJOR, UMMA_MN_MAJOR, 128, 128);
@@ -533,7 +542,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
     }
   } else {
     // ------------------------------------------------------------------ softmax + epilogue
-    reg_alloc<kSoftmaxRegs>();
+    reg_alloc<Regs<kCap, kMode>::kSoftmax>();
     const int t = (warp - 4) >> 2;
     const int wq = warp & 3;                     // TMEM lane quarter this warp may touch
     const int r_in_tile = wq * 32 + lane;
@@ -989,7 +998,8 @@ cudaError_t launch_attn_fwd(const CUtensorMap& mq, const CUtensorMap& mk, const 
                                 : pick(std::integral_constant<int, kPair>());
   cudaError_t e = ensure_dynamic_smem(reinterpret_cast<const void*>(kern), kSmemBytes);
   if (e != cudaSuccess) return e;
-  e = check_register_budget(reinterpret_cast<const void*>(kern), kThreads, 128 * kUtilRegs + 256 * kSoftmaxRegs);
+  e = check_register_budget(reinterpret_cast<const void*>(kern), kThreads,
+                            s.softcap > 0.f && solo ? Regs<true, kSolo>::kBlock : Regs<false, kPair>::kBlock);
   if (e != cudaSuccess) return e;
   e = launch_dependent(kern, grid, dim3(kThreads), kSmemBytes, stream, mq, mk, mv, p);
   count_launch();
