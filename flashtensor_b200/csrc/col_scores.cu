@@ -1346,7 +1346,18 @@ cudaError_t launch_kf_rowstat(const CUtensorMap& mq, const CUtensorMap& mk, cons
     auto kern = s.bf16 ? kf_rowstat_kernel<true, 0> : kf_rowstat_kernel<false, 0>;
     e = ensure_dynamic_smem(reinterpret_cast<const void*>(kern), RsCfg<0>::kSmem);
     if (e != cudaSuccess) return e;
-    e = launch_dependent(kern, grid, dim3(RsCfg<0>::kThreads), RsCfg<0>::kSmem, stream, mq, mk, mq, p, lse2_out);
+    // A thread reads its own row of the operand, 4 bytes a load, and lives on L1 holding the sectors meanwhile.
+    // A CTA that comes up under the forward kernel's tail, on an SM whose memory is divided for that kernel (all
+    // of it shared), has next to no L1; a launch that waits gets what its own shared memory leaves.  While half
+    // of the SMs are enough there are idle ones to start on (whole case in us, waiting / chained: B1 H4 S511, 16
+    // tiles, 47.6 / 37.9; H4 S2047, 64 tiles, 129 / 110; H8 S1501, 96 tiles, 107 / 147; B4 H32 S2047 992 / 1825).
+    if (2 * grid.x > static_cast<unsigned>(num_sms)) {
+      p.chained = 0;
+      kern<<<grid, RsCfg<0>::kThreads, RsCfg<0>::kSmem, stream>>>(mq, mk, mq, p, lse2_out);
+      e = cudaGetLastError();
+    } else {
+      e = launch_dependent(kern, grid, dim3(RsCfg<0>::kThreads), RsCfg<0>::kSmem, stream, mq, mk, mq, p, lse2_out);
+    }
   }
   count_launch();
   return e;
