@@ -45,8 +45,18 @@ constexpr int kTile = 128;
 constexpr uint32_t kTileBytes = 128 * 128 * 2;
 constexpr uint32_t kHalfBytes = kTileBytes / 2;
 constexpr int kUtilWarps = 2;                     // producer and MMA issuer
-constexpr int kKeyWarps = 8;                      // col_scores_kernel: two per 32 keys
-constexpr int kColThreads = (kUtilWarps + kKeyWarps) * 32;
+// Key warps of col_scores_kernel, of a CTA that shares its SM with another unless the mode reads an operand per
+// logit (more registers per thread).  Plain loads of the noise live on how many are in flight, so that mode has
+// sixteen warps all the same, each with 32 queries of a tile; Keyformer with a noise operand that TMA cannot
+// describe, whole case in us, eight warps -> sixteen: B1 H16
+// S1001 83.5 -> 80.5, B2 H32 S1501 342 -> 330, B4 H32 S2047 1034 -> 992.
+template <int kMode> struct ColCfg {
+  static constexpr int kKeyWarps = kMode == 2 ? 16 : 8;
+  static constexpr int kSubs = kKeyWarps / 4;      // warps per 32 keys
+  static constexpr int kQueries = 128 / kSubs;     // queries of a tile for each
+  static constexpr int kThreads = (kUtilWarps + kKeyWarps) * 32;
+  static constexpr int kCtas = kMode == 2 || kMode == 4 ? 1 : 2;
+};
 constexpr int kQStages = 2;                       // Q tiles; free again as soon as the MMA has read them
 constexpr int kLseStages = 4;                     // row statistics of the Q tiles; free when the key warps have read them
 constexpr uint32_t kSmemBytes = (1 + kQStages) * kTileBytes + 1024;
@@ -197,13 +207,14 @@ __device__ __forceinline__ void record_timeout(uint32_t* status, uint32_t site) 
 // kMode: 0 sum, 1 sum + sum of squares, 2 perturbed (noise operand), 3 perturbed (seeded noise),
 //        4 CORM: any_i(p_ij >= mask_ij) with a [Sq, Skv] threshold operand (cases/kernels/corm.py:34-37)
 template <bool kBF16, int kMode>
-__global__ void __launch_bounds__(kColThreads, (kMode == 2 || kMode == 4) ? 1 : 2)
+__global__ void __launch_bounds__(ColCfg<kMode>::kThreads, ColCfg<kMode>::kCtas)
 col_scores_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                   const ColParams p) {
   extern __shared__ uint8_t smem_raw[];
   __shared__ __align__(8) ColBars bars;
   __shared__ __align__(16) float lse_s[kLseStages][kTile];  // minus the row statistic
-  __shared__ float part_s[2][2][kTile];  // [sum, sum of squares][query half][key]
+  constexpr int kKeyWarps = ColCfg<kMode>::kKeyWarps, kSubs = ColCfg<kMode>::kSubs, kQueries = ColCfg<kMode>::kQueries;
+  __shared__ float part_s[2][kSubs][kTile];  // [sum, sum of squares][share of the queries][key]
   __shared__ uint32_t tmem_base_s;
   __shared__ uint32_t abort_s;
 
@@ -333,8 +344,8 @@ col_scores_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
       __syncwarp();
     }
   } else {
-    // ------------------------------------------------------------------ one thread per (key, query half)
-    const int hq = (warp - kUtilWarps) >> 2;  // which 64 queries of every query tile
+    // ------------------------------------------------------------------ one thread per (key, share of the queries)
+    const int hq = (warp - kUtilWarps) >> 2;  // which kQueries queries of every query tile
     const int wq = warp & 3;       // TMEM lane quarter this warp may touch (every four consecutive key warps cover all four)
     const int key = kv0 + wq * 32 + lane;
     const uint32_t lane_base = static_cast<uint32_t>(wq * 32) << 16;
@@ -360,15 +371,15 @@ col_scores_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
           ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&bars.s_full[buf]), (c >> 1) & 1, abortp));
           if (!ok) { if (lane == 0) record_timeout(p.status, 26); break; }
           tc_fence_after_sync();
-          const uint32_t tS = tbase + lane_base + buf * 128 + hq * 64;
-          const int q_base = i * kTile + hq * 64;
+          const uint32_t tS = tbase + lane_base + buf * 128 + hq * kQueries;
+          const int q_base = i * kTile + hq * kQueries;
           // query q of this tile sees `key` iff key <= q + diag_off
           const int first_visible = p.causal ? key - p.diag_off - q_base : 0;
           const bool tile_has_mask = p.causal && (kv0 + kTile - 1 - p.diag_off > q_base);
-          const float4* lse4 = reinterpret_cast<const float4*>(lse_s[ls]) + hq * 16;
-          // two chunks of 32 queries: every exponential of a chunk is in flight at once
+          const float4* lse4 = reinterpret_cast<const float4*>(lse_s[ls]) + hq * (kQueries / 4);
+          // chunks of 32 queries: every exponential of a chunk is in flight at once
 #pragma unroll
-          for (int ch = 0; ch < 2; ++ch) {
+          for (int ch = 0; ch < kQueries / 32; ++ch) {
             float s[32];
             tmem_ld32(tS + ch * 32, *reinterpret_cast<uint32_t(*)[32]>(s));
             float noise[(kMode == 2 || kMode == 4) ? 32 : 1];
@@ -389,8 +400,8 @@ col_scores_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
               }
             }
             tmem_wait_ld();
-            if (ch == 1) {
-              // this thread's part of the tile is in registers; when all 256 have said so the MMA
+            if (ch == kQueries / 32 - 1) {
+              // this thread's part of the tile is in registers; when all have said so the MMA
               // warp may overwrite the TMEM buffer
               tc_fence_before_sync();
               mbar_arrive(smem_u32(&bars.s_empty[buf]));
@@ -470,8 +481,8 @@ col_scores_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
         if (lane == 0) mbar_arrive(smem_u32(&bars.lse_empty[ls]));
       }
     }
-    // Both query halves leave their parts in shared memory; after the CTA-wide barrier below the
-    // first half's thread adds the two in a fixed order and stores.
+    // All shares of the queries leave their parts in shared memory; after the CTA-wide barrier below the
+    // first one's thread adds them in a fixed order and stores.
     part_s[0][hq][wq * 32 + lane] = kMode == 4 ? (hit ? 1.f : 0.f) : (acc[0] + acc[1]) + (acc[2] + acc[3]);
     part_s[1][hq][wq * 32 + lane] = (acc2[0] + acc2[1]) + (acc2[2] + acc2[3]);
     if (!ok) *abortp = 1u;
@@ -488,7 +499,8 @@ col_scores_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
     const int key = kv0 + k_in_tile;
     if (key < p.Skv) {
       const size_t o = (static_cast<size_t>(b) * p.H + h) * p.Skv + key;
-      const float v = part_s[0][0][k_in_tile] + part_s[0][1][k_in_tile];
+      float v = part_s[0][0][k_in_tile] + part_s[0][1][k_in_tile];
+      if constexpr (kSubs == 4) v += part_s[0][2][k_in_tile] + part_s[0][3][k_in_tile];
       // with a query-range split the sums of this range go to its slab of the workspace (a range
       // that sees none of the keys leaves zeros there)
       const size_t slab = static_cast<size_t>(qc) * bh_count * p.Skv;
@@ -1281,7 +1293,8 @@ cudaError_t launch_col_scores(const CUtensorMap& mq, const CUtensorMap& mk, cons
   else kern = s.bf16 ? col_scores_kernel<true, 3> : col_scores_kernel<false, 3>;
   e = ensure_dynamic_smem(reinterpret_cast<const void*>(kern), kSmemBytes);
   if (e != cudaSuccess) return e;
-  e = launch_dependent(kern, grid, dim3(kColThreads), kSmemBytes, stream, mq, mk, p);
+  const bool sixteen = a.mode == ASUKA_SCORE_PERTURBED && a.exp_rand != nullptr;  // (mode 2 of the kernel)
+  e = launch_dependent(kern, grid, dim3(sixteen ? ColCfg<2>::kThreads : ColCfg<0>::kThreads), kSmemBytes, stream, mq, mk, p);
   count_launch();
   }
   if (e != cudaSuccess || p.n_qchunks == 1) return e;
