@@ -4,6 +4,7 @@ end of the operator layer over it, flashtensor_b200/_bind.so (csrc/bind.cpp, a C
 Usage: python -m flashtensor_b200.build [--force] [--verbose]
 nvcc cross-compiles without a GPU; the result is loaded with ctypes by flashtensor_b200._lib.
 """
+import importlib.metadata
 import os
 import shutil
 import subprocess
@@ -15,6 +16,7 @@ CSRC = os.path.join(PKG_DIR, "csrc")
 OBJ_DIR = os.path.join(PKG_DIR, "build")
 LIB_PATH = os.path.join(PKG_DIR, "libasuka_b200.so")
 BIND_PATH = os.path.join(PKG_DIR, "_bind.so")
+BIND_STAMP = os.path.join(OBJ_DIR, "_bind.built_against")
 
 SOURCES = ["capi.cu", "attn_fwd.cu", "attn_decode.cu", "col_scores.cu", "select_topk.cu", "score_ops.cu", "sima.cu", "linattn32.cu", "linear_f32.cu"]
 NVCC_FLAGS = [
@@ -80,7 +82,9 @@ def _build_bind(nvcc, force):
   """csrc/bind.cpp against torch's headers and the library above (found beside it at run time)."""
   src = os.path.join(CSRC, "bind.cpp")
   newest = max(os.path.getmtime(f) for f in (src, os.path.join(PKG_DIR, "..", "include", "asuka_b200.h")))
-  if not force and os.path.exists(BIND_PATH) and os.path.getmtime(BIND_PATH) > newest:
+  # torch and Python give a C++ extension no stable interface: built against others it fails at import
+  against = f"torch {importlib.metadata.version('torch')}, Python {sys.version}"
+  if not force and os.path.exists(BIND_PATH) and os.path.getmtime(BIND_PATH) > newest and _read(BIND_STAMP) == against:
     return
   import torch
   root = os.path.dirname(os.path.abspath(torch.__file__))
@@ -95,6 +99,16 @@ def _build_bind(nvcc, force):
   if res.returncode != 0:
     print(res.stdout + res.stderr, file=sys.stderr)
     raise RuntimeError("building the native front end failed")
+  with open(BIND_STAMP, "w") as f:
+    f.write(against)
+
+
+def _read(path):
+  try:
+    with open(path) as f:
+      return f.read()
+  except OSError:
+    return None
 
 
 if __name__ == "__main__":

@@ -190,6 +190,29 @@ def test_blocks_leave_torch_what_is_more_than_values(monkeypatch, ea):
   assert native == [ea, ea]
 
 
+def test_front_end_is_rebuilt_for_another_torch_or_python(built_lib, monkeypatch):
+  import importlib.metadata
+  from flashtensor_b200 import build
+
+  class Rebuild(Exception):
+    pass
+
+  def run(cmd, **kw):
+    assert build.BIND_PATH in cmd
+    raise Rebuild
+
+  monkeypatch.setattr(subprocess, "run", run)
+  build._build_bind("nvcc", force=False)             # as built by the fixture: nothing to do
+  with monkeypatch.context() as m:
+    m.setattr(importlib.metadata, "version", lambda name: "0.0")
+    with pytest.raises(Rebuild):
+      build._build_bind("nvcc", force=False)
+  with monkeypatch.context() as m:
+    m.setattr(sys, "version", "2.7")
+    with pytest.raises(Rebuild):
+      build._build_bind("nvcc", force=False)
+
+
 def test_missing_library_is_loud(tmp_path, monkeypatch):
   monkeypatch.setattr(_lib, "_lib", None)
   monkeypatch.setattr(_lib, "LIB_PATH", str(tmp_path / "nope.so"))
