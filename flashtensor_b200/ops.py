@@ -25,7 +25,11 @@ def _bind():
   global _native
   if _native is None:
     _lib.load()
-    from . import _bind as native
+    try:
+      from . import _bind as native
+    except ImportError as e:
+      raise ImportError(f"the native front end does not load ({e}): build it with `python -m flashtensor_b200.build` "
+                        "(there is no Python fallback)") from e
     _native = native
   return _native
 

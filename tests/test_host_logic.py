@@ -220,6 +220,16 @@ def test_missing_library_is_loud(tmp_path, monkeypatch):
     _lib.load()
 
 
+def test_missing_front_end_is_loud(built_lib, monkeypatch):
+  import flashtensor_b200
+  from flashtensor_b200 import ops
+  monkeypatch.setattr(ops, "_native", None)
+  monkeypatch.delattr(flashtensor_b200, "_bind", raising=False)
+  monkeypatch.setitem(sys.modules, "flashtensor_b200._bind", None)
+  with pytest.raises(ImportError, match="python -m flashtensor_b200.build"):
+    ops.pool_scores(torch.zeros(1, 1, 8), 3)
+
+
 def test_unit_ranges_cover_everything():
   for n_units, ws in ((32, 8), (128, 8), (80, 8), (256, 8), (5, 2), (3, 4)):
     spans = [sharding.unit_range(n_units, r, ws) for r in range(ws)]
