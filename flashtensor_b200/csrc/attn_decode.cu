@@ -18,7 +18,7 @@
 //     matrix instructions (a tcgen05 tile would be 128 rows for at most 16) and a running maximum
 //     and sum of their own, so nothing is exchanged until the end.
 // Measured (bf16, q_len 1, against the 256-row items): B16, 32 query heads on 8 K/V heads, 4001 keys
-// (262 MB) 225 -> 44.5 us = 5.9 TB/s; B16, 32 K/V heads, 4001 keys (1.05 GB) 213 -> 150 us = 7.0 TB/s;
+// (262 MB) 210 -> 45.2 us = 5.8 TB/s; B16, 32 K/V heads, 4001 keys (1.05 GB) 213 -> 150 us = 7.0 TB/s;
 // B1, 8 K/V heads, 4096 keys (17 MB) 80 -> 8.9 us; B1, 8 K/V heads, 300 keys 24.5 -> 6.5 us.
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>

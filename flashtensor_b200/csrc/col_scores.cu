@@ -887,7 +887,8 @@ constexpr uint32_t kNoiseBoxBytes = kNoiseTileBytes / 4;
 // exponential; the staged variant, one CTA per SM, has four, the seeded one two CTAs of two.
 // With four warps instead of two, the last units' tiles longest first and the start under the forward kernel's
 // tail, the whole case went (us): B1 H16 S1000 58 -> 46, B2 H32 S1000 126 -> 109, B1 H16 S2048 117 -> 92,
-// B2 H32 S2048 356 -> 321, B4 H32 S2048 658 -> 607.
+// B2 H32 S2048 356 -> 321, B4 H32 S2048 658 -> 607 (calls back to back on a cool card; among other work, at
+// lower clocks, the last takes 778 and 734).
 template <int kNoise> struct RsCfg {  // kNoise 1: two K stages, then eight noise boxes
   static constexpr bool kNoiseTma = kNoise == 1;
   static constexpr int kParts = kNoiseTma ? 4 : 2;

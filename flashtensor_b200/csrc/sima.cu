@@ -869,8 +869,8 @@ sima_out_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
   } else if (kEA && warp >= 8) {
     // ------------------------------------------------------------- EA: softmax numerators of Q
     // Two threads per row (adjacent lanes, 64 features each) exponentiate every Q tile in place
-    // against the row maximum; the row sums come from the tensor pipe (above).  Half of the
-    // exponentials run on the special-function unit, half on the FMA pipe.
+    // against the row maximum; the row sums come from the tensor pipe (above).  (kEaPolyPairs of every four
+    // pairs of exponentials would go to the FMA pipe; none do.)
     const int t256 = tid - 256;
     const int r = t256 >> 1, half = t256 & 1;
     const float kL2e = 1.4426950408889634f;
@@ -1560,7 +1560,11 @@ cudaError_t launch_sima(const CUtensorMap& mq, const CUtensorMap& mk, const CUte
   const int bh = s.B * s.H;
   uint8_t* w = static_cast<uint8_t*>(ws);
   // One persistent kernel for all three steps when there are enough units to keep most groups of
-  // four CTAs busy (and the partial slots fit the workspace plan above).
+  // four CTAs busy.  The line was drawn against three kernels that cut every unit into slabs.  Against these,
+  // which share the tiles out evenly, it is right below 37 units of 3000 rows and more and wrong above them,
+  // where the groups' last round of units is partial (us, single kernel / three: 24 units, S 700 19.5 / 16.5, S 4096
+  // 33.0 / 34.4; 36 units, S 4096 40.3 / 45.0; 40 units, S 4096 61.6 / 49.3, S 8192 104 / 84; 64 units, S 8192
+  // 125.5 / 125.8; 96 units, S 2000 71.8 / 57.4, S 8192 184 / 180).
   const int n_groups = num_sms / kFuGroup;
 #ifdef ASUKA_SIMA_NO_FUSED
   const bool fused = false;
