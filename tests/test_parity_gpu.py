@@ -265,7 +265,9 @@ def test_keyformer_seeded_noise_vs_oracle(ops, shape, dtype):
 
 
 @pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
-@pytest.mark.parametrize("shape", [(1, 128, 1), (2, 1000, 3), (1, 4096, 2), (1, 77, 2)])
+@pytest.mark.parametrize("shape", [(1, 128, 1), (2, 1000, 3), (1, 4096, 2), (1, 77, 2),
+                                   # runs of tiles that cross from one unit into the next, once and several times
+                                   (3, 1700, 5), (40, 300, 8)])
 def test_sima_vs_oracle(ops, shape, dtype):
   B, S, H = shape
   q, k, v = O.make_inputs("sima", B, S, S, H, 128, dtype, seed=5)
@@ -378,10 +380,27 @@ def test_f32_projection_vs_float64(ops, shape):
   no_timeouts(ops)
 
 
+@pytest.mark.parametrize("shape", [(2048, 384, 128, 0), (2048, 128, 128, 64), (2048, 96, 64, 0)])
+def test_f32_projection_keeps_every_term(ops, shape):
+  # The bound above is a worst case that K >= 64 leaves far below; as a root mean square of error over
+  # sum |x||w| the eight accumulations of h.h, each truncated by at most 2^-23 of a sum about a seventh of that
+  # one, give 8/7 2^-24 (an f32 GEMM 0.24 2^-23).  Without one of the six products it is 2.8 2^-23 and more, with
+  # two terms 4.0 (float64 emulation of these inputs); columns from 64 on alone show the second piece.
+  M, N, K, first = shape
+  g = torch.Generator().manual_seed(1)
+  x, w = torch.randn(M, K, generator=g), torch.randn(N, K, generator=g)
+  x[:, :first] = 0
+  got = ops.linear_f32(x.cuda(), w.cuda(), torch.zeros(N).cuda()).cpu().double()
+  e = (got - x.double() @ w.double().t()) / (x.double().abs() @ w.double().abs().t())
+  rms = e.pow(2).mean().sqrt().item()
+  assert rms <= 2.0 ** -23
+  no_timeouts(ops)
+
+
 @pytest.mark.parametrize("shape", [(300, 96, 128), (130, 33, 40), (5, 8, 8), (40000, 384, 64)])
 def test_f32_projection_outside_ordinary_magnitudes(ops, shape):
   # infinities, NaN, values next to the largest and below the smallest normal number, in rows of x and in
-  # columns: f32's own result, to the bound of the test above plus half the smallest subnormal a rounding;
+  # columns: f32's own result, to the worst-case bound above plus half the smallest subnormal a rounding;
   # rows and columns without such a value keep their bits (the last shape: seven row tiles per CTA)
   M, N, K = shape
   g = torch.Generator().manual_seed(M)
@@ -468,6 +487,24 @@ def test_blocks_take_operands_from_anywhere_in_a_buffer(ops):
   for block in (EABlock(), SimABlock()):
     want = block(*(a.clone() for a in args))
     assert torch.equal(block(*args), want) and torch.equal(block(*strided), want)
+  no_timeouts(ops)
+
+
+@pytest.mark.parametrize("step", [6.0, 2.0, -6.0])
+def test_ea_core_with_keys_that_grow_along_the_sequence(ops, step):
+  # the level of K moves every 64 rows by more than a warp's reference tolerates (raised, with sums already
+  # there, at every stage), by less (every third), or down; one feature goes the other way.  The last levels
+  # carry the weight, so the bound for a common offset (below) holds with the two rescales (2^-22 each) that reach them
+  g = torch.Generator().manual_seed(6)
+  q, k, v = (torch.randn(2, 784, 3, 32, generator=g) for _ in range(3))
+  level = step * (torch.arange(784) // 64).to(torch.float32)
+  k = k + level[None, :, None, None]
+  k[..., 5] -= 2 * level[None, :, None]
+  qd, kd, vd = (t.double().permute(0, 2, 1, 3) for t in (q, k, v))
+  ref = (torch.softmax(qd, 3) @ (torch.softmax(kd, 2).transpose(2, 3) @ vd)).permute(0, 2, 1, 3)
+  got = ops.linattn32_fwd(q.cuda(), k.cuda(), v.cuda(), ea=True).cpu().double()
+  e = ((got - ref).norm() / ref.norm()).item()
+  assert e <= 1e-6 + 2 * 2.0 ** -22
   no_timeouts(ops)
 
 
