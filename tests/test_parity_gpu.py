@@ -777,6 +777,28 @@ def test_selection_with_many_exact_ties(ops):
   assert ops.select_topk(s, 4).cpu().tolist() == [[[1, 2, 3, 4]]]
 
 
+@pytest.mark.parametrize("S", [1, 31, 1024, 1025, 4097, 32768])
+def test_selection_over_any_spread_of_keys(ops, S):
+  # the select looks only at the bits in which a row's keys differ, and stops when a whole bin is kept: keys all
+  # equal, equal but for one, neighbours in the last bits, of both signs, with zeros and infinities, and each
+  # alone in its bin or not; the largest and smallest counts among them
+  from flashtensor_b200 import _lib
+  g = torch.Generator().manual_seed(S)
+  base = torch.rand(S, generator=g)
+  rows = [torch.full((S,), 0.7), base, (base * 40).floor(), base * 2.0 ** -20 + 1.0, torch.randn(S, generator=g) * 1e30,
+          (base - 0.5) * torch.tensor([0.0, 1e-42, 1.0, float("inf")])[torch.randint(0, 4, (S,), generator=g)],
+          torch.cat([base[:1] + 5.0, torch.zeros(S - 1)])]
+  score = torch.stack(rows)[None].nan_to_num(nan=0.0, posinf=float("inf"), neginf=float("-inf")) + 0.0  # (no -0)
+  for k_keep in sorted({1, (S + 1) // 2, max(1, S - 1), S}):
+    idx = ops.select_topk(score.cuda(), k_keep).cpu().numpy()
+    assert np.array_equal(idx, O.keyformer_select(score.numpy(), k_keep)), k_keep
+  if S <= 16384:
+    ssum = torch.where(score < 1e-10, 0.0, score).clamp(max=100)  # (nothing subnormal, nor squared)
+    sq = ssum ** 2 * (1 + torch.rand(score.shape, generator=g).round())
+    idx = ops.select_topk(ssum.cuda(), (S + 1) // 2, mode=_lib.SELECT_ROCO, score_sq=sq.cuda(), q_len=S).cpu().numpy()
+    assert np.array_equal(idx, O.roco_select(ssum.numpy(), sq.numpy(), (S + 1) // 2, S))
+
+
 @pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
 def test_roco_and_keyformer_selection(ops, dtype):
   B, S, H, k_keep = 2, 1024, 3, 128
