@@ -59,6 +59,11 @@ class LinearParams(ctypes.Structure):
   _fields_ = [("x", Tensor), ("w", Tensor), ("bias", Tensor), ("out", Tensor)]
 
 
+class LinAttn32ProjParams(ctypes.Structure):
+  _fields_ = [("q", Tensor), ("k", Tensor), ("v", Tensor), ("w", Tensor), ("bias", Tensor), ("out", Tensor),
+              ("scratch", Tensor), ("ea", ctypes.c_int32)]
+
+
 class GatherParams(ctypes.Structure):
   _fields_ = [("k", Tensor), ("v", Tensor), ("idx", Tensor), ("k_out", Tensor), ("v_out", Tensor)]
 
@@ -97,6 +102,7 @@ SYMBOLS = {
     "asuka_b200_ea_fwd": (ctypes.c_int, [ctypes.POINTER(SimaParams), ctypes.c_void_p, ctypes.c_size_t, ctypes.c_void_p]),
     "asuka_b200_linattn32_fwd": (ctypes.c_int, [ctypes.POINTER(LinAttn32Params), ctypes.c_void_p]),
     "asuka_b200_linear_f32": (ctypes.c_int, [ctypes.POINTER(LinearParams), ctypes.c_void_p]),
+    "asuka_b200_linattn32_proj": (ctypes.c_int, [ctypes.POINTER(LinAttn32ProjParams), ctypes.c_void_p]),
     "asuka_b200_case_workspace_bytes": (ctypes.c_int, [ctypes.POINTER(CaseParams), ctypes.POINTER(ctypes.c_size_t)]),
     "asuka_b200_case_workspace_bytes_split": (ctypes.c_int, [ctypes.POINTER(CaseParams), ctypes.POINTER(ctypes.c_size_t)]),
     "asuka_b200_h2o": (ctypes.c_int, [ctypes.POINTER(CaseParams), ctypes.c_void_p, ctypes.c_size_t, ctypes.c_void_p]),

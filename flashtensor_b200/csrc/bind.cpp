@@ -373,20 +373,23 @@ PyObject* linattn_block(PyObject*, PyObject* const* a, Py_ssize_t n) {
     OnDevice on({&x, &w_qkv, &b_qkv, &w_o, &b_o});
     const int64_t B = x.size(0), N = x.size(1);
     const at::Tensor qkv = linear_f32(x.view({B * N, C}), w_qkv, b_qkv, on.stream);
-    const at::Tensor core = empty({B, N, C / 32, 32}, at::kFloat, x);
-    asuka_linattn32_params p;
-    p.out = desc(core);
-    p.q = p.out;  // the same shape, strided over the fused rows
-    p.q.ptr = qkv.data_ptr();
-    p.q.stride[0] = N * 3 * C;
-    p.q.stride[1] = 3 * C;
+    const at::Tensor out = empty({B, N, C}, at::kFloat, x), scratch = empty({B, C, C}, at::kFloat, x);
+    asuka_linattn32_proj_params p;
+    p.q = desc(qkv);  // [B, N, C / 32, 32], strided over the fused rows
+    p.q.ndim = 4;
+    p.q.shape[0] = B; p.q.shape[1] = N; p.q.shape[2] = C / 32; p.q.shape[3] = 32;
+    p.q.stride[0] = N * 3 * C; p.q.stride[1] = 3 * C; p.q.stride[2] = 32; p.q.stride[3] = 1;
     p.k = p.q;
     p.k.ptr = static_cast<float*>(p.q.ptr) + C;
     p.v = p.q;
     p.v.ptr = static_cast<float*>(p.q.ptr) + 2 * C;
+    p.w = desc(w_o);
+    p.bias = desc(b_o);
+    p.out = desc(out);
+    p.scratch = desc(scratch);
     p.ea = bool_arg(a[5]) ? 1 : 0;
-    call("asuka_b200_linattn32_fwd", [&] { return asuka_b200_linattn32_fwd(&p, on.stream); });
-    return wrap(linear_f32(core.view({B * N, C}), w_o, b_o, on.stream).view({B, N, C}));
+    call("asuka_b200_linattn32_proj", [&] { return asuka_b200_linattn32_proj(&p, on.stream); });
+    return wrap(out);
   } catch (const BadArg&) {
     return nullptr;
   }

@@ -440,6 +440,40 @@ int sima_impl(const asuka_sima_params* p, void* ws, size_t ws_bytes, cudaStream_
                               p->out.stride[2], ws, sh, m64, sms, stream));
 }
 
+// [B, N, H, 32] f32 tensor of q's shape usable as a TMA source/destination
+int check_bnh32(const asuka_tensor& t, const asuka_tensor& q) {
+  if (t.ptr == nullptr) return ASUKA_ERR_NULL_POINTER;
+  if (t.dtype != ASUKA_F32) return ASUKA_ERR_BAD_DTYPE;
+  if (t.ndim != 4 || t.shape[3] != 32) return ASUKA_ERR_BAD_SHAPE;
+  for (int d = 0; d < 4; ++d)
+    if (t.shape[d] <= 0 || t.shape[d] != q.shape[d]) return ASUKA_ERR_BAD_SHAPE;
+  if (t.stride[3] != 1) return ASUKA_ERR_BAD_STRIDE;
+  for (int d = 0; d < 3; ++d)
+    if (t.stride[d] <= 0 || (t.stride[d] % 4) != 0) return ASUKA_ERR_BAD_STRIDE;
+  if ((reinterpret_cast<uintptr_t>(t.ptr) & 15u) != 0) return ASUKA_ERR_MISALIGNED;
+  return ASUKA_OK;
+}
+
+int prep_linattn32(const asuka_tensor& q, const asuka_tensor& k, const asuka_tensor& v, int ea, LinAttn32Args* a) {
+  const asuka_tensor* ts[3] = {&q, &k, &v};
+  for (int i = 0; i < 3; ++i) {
+    const int r = check_bnh32(*ts[i], q);
+    if (r != ASUKA_OK) return r;
+  }
+  if (ea != 0 && ea != 1) return ASUKA_ERR_BAD_ARGUMENT;
+  if (q.shape[0] * q.shape[2] > (1 << 24) || q.shape[1] > (1 << 24)) return ASUKA_ERR_TOO_LARGE;
+  std::memset(a, 0, sizeof(*a));
+  a->q = static_cast<const float*>(q.ptr);
+  a->k = static_cast<const float*>(k.ptr);
+  a->v = static_cast<const float*>(v.ptr);
+  a->B = static_cast<int>(q.shape[0]); a->N = static_cast<int>(q.shape[1]); a->H = static_cast<int>(q.shape[2]);
+  a->ea = ea;
+  a->q_sb = q.stride[0]; a->q_sn = q.stride[1]; a->q_sh = q.stride[2];
+  a->k_sb = k.stride[0]; a->k_sn = k.stride[1]; a->k_sh = k.stride[2];
+  a->v_sb = v.stride[0]; a->v_sn = v.stride[1]; a->v_sh = v.stride[2];
+  return ASUKA_OK;
+}
+
 // forward + column scores (+ selection) on one stream; the row statistic lives in `ws`
 enum CaseKind { CASE_H2O, CASE_ROCO, CASE_KF };
 
@@ -734,35 +768,35 @@ int asuka_b200_pool_scores(const asuka_tensor* score, const asuka_tensor* out, i
 
 int asuka_b200_linattn32_fwd(const asuka_linattn32_params* p, asuka_stream stream) {
   if (p == nullptr) return ASUKA_ERR_NULL_POINTER;
-  const asuka_tensor* ts[4] = {&p->q, &p->k, &p->v, &p->out};
-  for (int i = 0; i < 4; ++i) {
-    const asuka_tensor& t = *ts[i];
-    if (t.ptr == nullptr) return ASUKA_ERR_NULL_POINTER;
-    if (t.dtype != ASUKA_F32) return ASUKA_ERR_BAD_DTYPE;
-    if (t.ndim != 4 || t.shape[3] != 32) return ASUKA_ERR_BAD_SHAPE;
-    for (int d = 0; d < 4; ++d)
-      if (t.shape[d] <= 0 || t.shape[d] != p->q.shape[d]) return ASUKA_ERR_BAD_SHAPE;
-    if (t.stride[3] != 1) return ASUKA_ERR_BAD_STRIDE;
-    for (int d = 0; d < 3; ++d)
-      if (t.stride[d] <= 0 || (t.stride[d] % 4) != 0) return ASUKA_ERR_BAD_STRIDE;
-    if ((reinterpret_cast<uintptr_t>(t.ptr) & 15u) != 0) return ASUKA_ERR_MISALIGNED;
-  }
-  if (p->ea != 0 && p->ea != 1) return ASUKA_ERR_BAD_ARGUMENT;
-  if (p->q.shape[0] * p->q.shape[2] > (1 << 24) || p->q.shape[1] > (1 << 24)) return ASUKA_ERR_TOO_LARGE;
-  int r;
-  if ((r = check_arch()) != ASUKA_OK) return r;
   LinAttn32Args a;
-  a.q = static_cast<const float*>(p->q.ptr);
-  a.k = static_cast<const float*>(p->k.ptr);
-  a.v = static_cast<const float*>(p->v.ptr);
+  int r;
+  if ((r = prep_linattn32(p->q, p->k, p->v, p->ea, &a)) != ASUKA_OK) return r;
+  if ((r = check_bnh32(p->out, p->q)) != ASUKA_OK) return r;
+  if ((r = check_arch()) != ASUKA_OK) return r;
   a.out = static_cast<float*>(p->out.ptr);
-  a.B = static_cast<int>(p->q.shape[0]); a.N = static_cast<int>(p->q.shape[1]); a.H = static_cast<int>(p->q.shape[2]);
-  a.ea = p->ea;
-  a.q_sb = p->q.stride[0]; a.q_sn = p->q.stride[1]; a.q_sh = p->q.stride[2];
-  a.k_sb = p->k.stride[0]; a.k_sn = p->k.stride[1]; a.k_sh = p->k.stride[2];
-  a.v_sb = p->v.stride[0]; a.v_sn = p->v.stride[1]; a.v_sh = p->v.stride[2];
   a.o_sb = p->out.stride[0]; a.o_sn = p->out.stride[1]; a.o_sh = p->out.stride[2];
   return map_cuda(launch_linattn32(a, static_cast<cudaStream_t>(stream)));
+}
+
+int asuka_b200_linattn32_proj(const asuka_linattn32_proj_params* p, asuka_stream stream) {
+  if (p == nullptr) return ASUKA_ERR_NULL_POINTER;
+  LinAttn32Args a;
+  int r;
+  if ((r = prep_linattn32(p->q, p->k, p->v, p->ea, &a)) != ASUKA_OK) return r;
+  if (p->q.stride[2] != 32) return ASUKA_ERR_BAD_STRIDE;
+  const int64_t B = a.B, N = a.N, C = static_cast<int64_t>(a.H) * 32;
+  if (C > ASUKA_LINEAR_MAX_K || B * N > 0x3fffffff) return ASUKA_ERR_TOO_LARGE;
+  const int64_t ws[2] = {C, C}, bs[1] = {C}, os[3] = {B, N, C}, ss[3] = {B, C, C};
+  if ((r = check_dense(p->w, ASUKA_F32, 2, ws)) != ASUKA_OK) return r;
+  if ((r = check_dense(p->bias, ASUKA_F32, 1, bs)) != ASUKA_OK) return r;
+  if ((r = check_dense(p->out, ASUKA_F32, 3, os)) != ASUKA_OK) return r;
+  if ((r = check_dense(p->scratch, ASUKA_F32, 3, ss)) != ASUKA_OK) return r;
+  if ((r = check_arch()) != ASUKA_OK) return r;
+  const int sms = sm_count();
+  if (sms <= 0) return ASUKA_ERR_CUDA;
+  a.out = static_cast<float*>(p->out.ptr);
+  return map_cuda(launch_linattn32_proj(a, static_cast<const float*>(p->w.ptr), static_cast<const float*>(p->bias.ptr),
+                                        static_cast<float*>(p->scratch.ptr), sms, static_cast<cudaStream_t>(stream)));
 }
 
 int asuka_b200_linear_f32(const asuka_linear_params* p, asuka_stream stream) {

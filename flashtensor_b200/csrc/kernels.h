@@ -164,10 +164,17 @@ struct LinAttn32Args {
   int64_t q_sb, q_sn, q_sh, k_sb, k_sn, k_sh, v_sb, v_sn, v_sh, o_sb, o_sn, o_sh;
 };
 cudaError_t launch_linattn32(const LinAttn32Args& a, cudaStream_t stream);
+// ... followed by out[B, N, C] = core w_o[C, C]^T + b_o, C = 32 H <= 128; the heads of q side by side, out dense, w_fold
+// [B, C, C] is scratch (16-byte aligned)
+cudaError_t launch_linattn32_proj(const LinAttn32Args& a, const float* w_o, const float* b_o, float* w_fold, int num_sms,
+                                  cudaStream_t stream);
 
 // out[M, N] = x[M, K] w[N, K]^T + bias[N], contiguous f32, K a multiple of 8 and at most 128
 cudaError_t launch_linear_f32(const float* x, const float* w, const float* bias, float* out, int M, int N, int K,
                               int num_sms, cudaStream_t stream);
+// out[B, M, N] = x[B, M, K] w[B, N, K]^T + bias[N], N and K at most 128; softmax: of every 32 values of x first
+cudaError_t launch_linear_f32_batched(const float* x, int64_t x_sb, int64_t x_sn, const float* w, const float* bias, float* out,
+                                      int B, int M, int N, int K, bool softmax, int num_sms, cudaStream_t stream);
 
 struct SimaShape {
   int B, H, S;

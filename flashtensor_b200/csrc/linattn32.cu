@@ -44,6 +44,8 @@ static_assert(kPartBytes + kQStages * kTileBytes <= kStages * 3 * kTileBytes, "p
 
 struct Lin32Params {
   int N, H;
+  const float* w_o;  // (kFold) output projection [32 H, 32 H], and where its product with every batch's M' goes
+  float* w_fold;     // [B, 32 H, 32 H]
   uint32_t* status;
 };
 
@@ -75,14 +77,14 @@ __device__ __forceinline__ void record_timeout(uint32_t* status, uint32_t site) 
   status[1] = site;
 }
 
-template <bool kEA>
+template <bool kEA, bool kFold>
 __global__ void __launch_bounds__(kThreads, 2)
 linattn32_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                  const __grid_constant__ CUtensorMap map_v, const __grid_constant__ CUtensorMap map_out,
                  const Lin32Params p) {
   extern __shared__ uint8_t smem_raw[];
   __shared__ __align__(8) Lin32Bars bars;
-  __shared__ __align__(16) float m_s[kD][kD];       // M' = normalised K'^T V, [d][e]
+  __shared__ float m_s[kD][kD + 1];                 // M' = normalised K'^T V, [d][e]
   __shared__ __align__(16) float scale_s[kWarps][kD];  // EA: rescale factors of a warp's partial product
   __shared__ float stat_s[2][kWarps][kD];           // SimA: sum|K|, sum|Q|; EA: reference, sum of K'
   __shared__ uint32_t abort_s;
@@ -216,8 +218,15 @@ linattn32_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
 
   // ---- the warps' partial products to M', in warp order, while the first tiles of pass B arrive
   float* const part = ring_gen;
+  float* const w_s = ring_gen + kPartBytes / 4;  // (kFold) this head's columns of the output projection, [c][e]
+  const int C = p.H * kD;
   const uint32_t qring = ring + kPartBytes;
   if (warp < kWarps) {
+    if constexpr (kFold) {  // (the ring is free: nothing is in flight after pass A)
+      for (int i = tid; i < C * (kD / 4); i += kWarps * 32)
+        *reinterpret_cast<float4*>(w_s + i * 4) =
+            __ldg(reinterpret_cast<const float4*>(p.w_o + static_cast<int64_t>(i >> 3) * C + h * kD) + (i & 7));
+    }
 #pragma unroll
     for (int d = 0; d < 4; ++d) {
       *reinterpret_cast<float4*>(part + (warp * kD + d0 + 2 * d) * kD + e0) =
@@ -252,6 +261,27 @@ linattn32_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
       m_s[d][lane] = total * inv;
     }
     named_bar_sync(1, kWarps * 32);
+  }
+
+  if constexpr (kFold) {
+    // ---- out = Qn . blockdiag(M') . w_o^T + b_o: what is left of it after this kernel is one product of the
+    // (EA: normalised) queries with w_fold[b][c][h * 32 + d] = sum_e M'[d][e] w_o[c][h * 32 + e]
+    if (warp < kWarps) {
+      float m[kD];
+#pragma unroll
+      for (int e = 0; e < kD; ++e) m[e] = m_s[lane][e];
+      float* dst = p.w_fold + static_cast<int64_t>(b) * C * C + h * kD + lane;
+      for (int c = warp; c < C; c += kWarps) {
+        float sum = 0.f;
+#pragma unroll
+        for (int i = 0; i < kD / 4; ++i) {
+          const float4 o = *reinterpret_cast<const float4*>(w_s + c * kD + i * 4);
+          sum = fmaf(m[4 * i], o.x, fmaf(m[4 * i + 1], o.y, fmaf(m[4 * i + 2], o.z, fmaf(m[4 * i + 3], o.w, sum))));
+        }
+        dst[static_cast<int64_t>(c) * C] = sum;
+      }
+    }
+    return;
   }
 
   // ---- pass B: out[n][e] = sum_d Qn[n][d] M'[d][e]; a lane keeps its 8 x 4 block of M' in registers,
@@ -341,10 +371,12 @@ linattn32_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
 
 }  // namespace
 
-cudaError_t launch_linattn32(const LinAttn32Args& a, cudaStream_t stream) {
+static cudaError_t launch(const LinAttn32Args& a, const float* w_o, float* w_fold, cudaStream_t stream) {
   Lin32Params p;
   p.N = a.N;
   p.H = a.H;
+  p.w_o = w_o;
+  p.w_fold = w_fold;
   p.status = device_status_words();
   const uint64_t dims[4] = {kD, static_cast<uint64_t>(a.H), static_cast<uint64_t>(a.N), static_cast<uint64_t>(a.B)};
   auto map = [&](CUtensorMap* m, const float* base, int64_t sh, int64_t sn, int64_t sb, uint32_t rows) {
@@ -354,14 +386,29 @@ cudaError_t launch_linattn32(const LinAttn32Args& a, cudaStream_t stream) {
   };
   CUtensorMap mq, mk, mv, mo;
   if (!map(&mq, a.q, a.q_sh, a.q_sn, a.q_sb, kRows) || !map(&mk, a.k, a.k_sh, a.k_sn, a.k_sb, kRows) ||
-      !map(&mv, a.v, a.v_sh, a.v_sn, a.v_sb, kRows) || !map(&mo, a.out, a.o_sh, a.o_sn, a.o_sb, kWarpRows))
+      !map(&mv, a.v, a.v_sh, a.v_sn, a.v_sb, kRows))
     return cudaErrorInvalidValue;
-  auto kern = a.ea ? linattn32_kernel<true> : linattn32_kernel<false>;
+  if (w_o != nullptr) {
+    mo = mq;  // (not used)
+  } else if (!map(&mo, a.out, a.o_sh, a.o_sn, a.o_sb, kWarpRows)) {
+    return cudaErrorInvalidValue;
+  }
+  auto kern = w_o != nullptr ? (a.ea ? linattn32_kernel<true, true> : linattn32_kernel<false, true>)
+                             : (a.ea ? linattn32_kernel<true, false> : linattn32_kernel<false, false>);
   cudaError_t e = ensure_dynamic_smem(reinterpret_cast<const void*>(kern), kSmemBytes);
   if (e != cudaSuccess) return e;
   e = launch_dependent(kern, dim3(static_cast<unsigned>(a.B) * a.H), dim3(kThreads), kSmemBytes, stream, mq, mk, mv, mo, p);
   count_launch();
   return e;
+}
+
+cudaError_t launch_linattn32(const LinAttn32Args& a, cudaStream_t stream) { return launch(a, nullptr, nullptr, stream); }
+
+cudaError_t launch_linattn32_proj(const LinAttn32Args& a, const float* w_o, const float* b_o, float* w_fold, int num_sms,
+                                  cudaStream_t stream) {
+  const cudaError_t e = launch(a, w_o, w_fold, stream);
+  if (e != cudaSuccess) return e;
+  return launch_linear_f32_batched(a.q, a.q_sb, a.q_sn, w_fold, b_o, a.out, a.B, a.N, a.H * kD, a.H * kD, a.ea != 0, num_sms, stream);
 }
 
 }  // namespace asuka

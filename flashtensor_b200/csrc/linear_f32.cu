@@ -15,8 +15,8 @@
 // 38 us instead of the figure below), and an accumulator lane is an output column, so a warp's store
 // is one 128-byte line of an output row.
 //   warps 0-7    load x (a whole tile ahead), split it and store the three terms as swizzled K-major tiles
-//   warp 8       issues tcgen05.mma into one of two accumulators
-//   warps 9-12   split the weights into TMEM; then accumulator + bias to global memory
+//   warps 8-15   split the weights into TMEM; then accumulator + bias to global memory, four warps for either
+//   warp 16      issues tcgen05.mma into one of two accumulators
 // The small products of a tile are accumulated before any h.h: the tensor pipe truncates when it adds
 // to an accumulator, and forty small terms added to a large sum would each leave a bias there
 // (measured at K = 128: 4.1e-7 relative error in the natural order, against 1.5e-7 of an f32 GEMM on
@@ -49,19 +49,31 @@ constexpr uint32_t kTermBytes = kTile * kChunk * 2;  // one bf16 term of a [128 
 constexpr uint32_t kPieceBytes = 3 * kTermBytes;
 constexpr uint32_t kStageBytes = (kMaxK / kChunk) * kPieceBytes;  // a tile of x: 96 KB
 constexpr int kSplitWarps = 8;
-constexpr int kThreads = (kSplitWarps + 1 + 4) * 32;
+constexpr int kEpiWarps = 8;                                      // four for either accumulator
+constexpr int kThreads = (kSplitWarps + kEpiWarps + 4) * 32;      // (the MMA warp and three that idle: setmaxnreg counts in fours)
+constexpr int kSplitRegs = 128, kEpiRegs = 96, kMmaRegs = 32;
+constexpr int kBlockRegs = kSplitWarps * 32 * kSplitRegs + kEpiWarps * 32 * kEpiRegs + 128 * kMmaRegs;
+static_assert(kBlockRegs <= kThreads * 96, "setmaxnreg would wait for ever");
 constexpr uint32_t kOutBytes = 32 * 32 * 4;                       // one TMA store of a warp: 32 rows x 32 columns
-constexpr uint32_t kSmemBytes = 2 * kStageBytes + 4 * 2 * kOutBytes + 1024;
+constexpr uint32_t kSmemBytes = 2 * kStageBytes + kEpiWarps * kOutBytes + 1024;
 constexpr uint32_t kTermCols = kMaxK / 2;  // TMEM columns of one term of the weights
 constexpr uint32_t kAccCol = 3 * kTermCols;
+
+// What a launch multiplies.
+//   kPlain    rows of one matrix with one set of weights
+//   kBatched  every batch's rows with weights of its own (N <= 128); a CTA stays within one batch
+//   kSoftmax  the same, every group of 32 values of a row replaced by its softmax first (EA's queries)
+enum LinMode { kPlain = 0, kBatched = 1, kSoftmax = 2 };
 
 struct LinParams {
   const float* x;
   const float* w;
   const float* bias;
   float* out;
-  int M, N, K;
-  int m_tiles, n_tiles, chunks;
+  int M, N, K;           // M: rows of a batch
+  int64_t x_sn, x_sb;    // strides of x between rows and between batches
+  int n_tiles, chunks;
+  int splits, cta_rows;  // (batched) CTAs per batch, and the rows of each, a multiple of 32
   int tma_out;  // rows of `out` can be described to TMA (N a multiple of 4)
   uint32_t* status;
 };
@@ -99,13 +111,46 @@ __device__ __forceinline__ void extent8(const float (&v)[8], float* big, float* 
   *small = min3(min3(a[0], a[1], a[2]), min3(a[3], a[4], a[5]), min3(a[6], a[7], a[7]));
 }
 
+// e^x of a difference from the maximum (linattn32.cu)
+__device__ __forceinline__ float exp_fast(float x) {
+  float y;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x * 1.4426950408889634f));
+  return y;
+}
+// softmax over the kLanes neighbouring lanes that hold kN values each of a group
+template <int kLanes, int kN>
+__device__ __forceinline__ void softmax_group(float (&v)[kN]) {
+  float m = v[0];
+#pragma unroll
+  for (int i = 1; i < kN; ++i) m = fmaxf(m, v[i]);
+#pragma unroll
+  for (int o = 1; o < kLanes; o <<= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+  float sum = 0.f;
+#pragma unroll
+  for (int i = 0; i < kN; ++i) {
+    v[i] = exp_fast(v[i] - m);
+    sum += v[i];
+  }
+#pragma unroll
+  for (int o = 1; o < kLanes; o <<= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+  const float inv = __frcp_rn(sum);
+#pragma unroll
+  for (int i = 0; i < kN; ++i) v[i] *= inv;
+}
+
 // One row of x against the 32 columns from n_base on, by a whole warp: lane l takes reduction columns 4l to
 // 4l + 3 and returns the sum for output column n_base + l.
+template <bool kSoft>
 __device__ __noinline__ float plain_dot(const float* __restrict__ x_row, const float* __restrict__ w, int n_base, int N, int K) {
   const int lane = threadIdx.x & 31;
   const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
   const bool live = lane * 4 < K;
-  const float4 xv = live ? __ldg(reinterpret_cast<const float4*>(x_row) + lane) : zero;
+  float4 xv = live ? __ldg(reinterpret_cast<const float4*>(x_row) + lane) : zero;
+  if constexpr (kSoft) {
+    float v[4] = {xv.x, xv.y, xv.z, xv.w};
+    softmax_group<8>(v);
+    xv = live ? make_float4(v[0], v[1], v[2], v[3]) : zero;
+  }
   float part[32];
 #pragma unroll
   for (int c = 0; c < 32; ++c) {
@@ -125,14 +170,14 @@ __device__ __noinline__ float plain_dot(const float* __restrict__ x_row, const f
 
 // Which of the 32 rows from `x` on (`rows` of them there) have a value other than zero: one bit each.  (Rows
 // of zeros, a batch's padding, have sums of zero that need no second look; eight loads in flight.)
-__device__ __noinline__ uint32_t rows_not_zero(const float* __restrict__ x, int rows, int K) {
+__device__ __noinline__ uint32_t rows_not_zero(const float* __restrict__ x, int64_t x_sn, int rows, int K) {
   const int lane = threadIdx.x & 31;
   uint32_t mask = 0;
   for (int r0 = 0; r0 < 32; r0 += 8) {
     float4 v[8];
 #pragma unroll
     for (int r = 0; r < 8; ++r)
-      v[r] = r0 + r < rows && lane * 4 < K ? __ldg(reinterpret_cast<const float4*>(x + static_cast<int64_t>(r0 + r) * K) + lane)
+      v[r] = r0 + r < rows && lane * 4 < K ? __ldg(reinterpret_cast<const float4*>(x + (r0 + r) * x_sn) + lane)
                                            : make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
     for (int r = 0; r < 8; ++r) {
@@ -176,9 +221,11 @@ __device__ __forceinline__ void record_timeout(uint32_t* status, uint32_t site) 
   status[1] = site;
 }
 
+template <int kMode>
 __global__ void __launch_bounds__(kThreads, 1) linear_f32_kernel(const __grid_constant__ CUtensorMap map_out, const LinParams p) {
   extern __shared__ uint8_t smem_raw[];
   __shared__ __align__(8) LinBars bars;
+  __shared__ uint8_t w_odd_s[2][kTile];  // of every column, in either half of the reduction: 1 no weight but zeros, 2 one out of range
   __shared__ uint32_t tmem_base_s;
   __shared__ uint32_t abort_s;
   const uint32_t sX = (smem_u32(smem_raw) + 1023u) & ~1023u;
@@ -186,11 +233,23 @@ __global__ void __launch_bounds__(kThreads, 1) linear_f32_kernel(const __grid_co
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   volatile uint32_t* abortp = &abort_s;
-  // CTAs are dealt out over the column blocks; those of one block share its row tiles
-  const int nb = static_cast<int>(blockIdx.x) % p.n_tiles;
-  const int m_first = static_cast<int>(blockIdx.x) / p.n_tiles;
-  const int m_step = (static_cast<int>(gridDim.x) - nb + p.n_tiles - 1) / p.n_tiles;  // CTAs of this column block
+  // This CTA's tiles start at rows row_first, row_first + row_step, ... of batch `batch` and end at row_end.
+  // Plain: CTAs are dealt out over the column blocks; those of one block share its row tiles.
+  int nb = 0, batch = 0, row_first, row_step, row_end;
+  if constexpr (kMode == kPlain) {
+    nb = static_cast<int>(blockIdx.x) % p.n_tiles;
+    row_first = static_cast<int>(blockIdx.x) / p.n_tiles * kTile;
+    row_step = (static_cast<int>(gridDim.x) - nb + p.n_tiles - 1) / p.n_tiles * kTile;  // (CTAs of this column block)
+    row_end = p.M;
+  } else {
+    batch = static_cast<int>(blockIdx.x) / p.splits;
+    row_first = static_cast<int>(blockIdx.x) % p.splits * p.cta_rows;
+    row_step = kTile;
+    row_end = min(p.M, row_first + p.cta_rows);
+  }
   const int n0 = nb * kTile;
+  const float* const x = p.x + batch * p.x_sb;
+  const float* const w = p.w + static_cast<int64_t>(batch) * p.N * p.K;
 
   if (tid == 0) {
     abort_s = 0;
@@ -202,7 +261,7 @@ __global__ void __launch_bounds__(kThreads, 1) linear_f32_kernel(const __grid_co
     }
     mbar_fence_init();
   }
-  if (warp == kSplitWarps) {
+  if (warp == kSplitWarps + kEpiWarps) {
     __syncwarp();
     tmem_alloc(smem_u32(&tmem_base_s), 512);
     tmem_relinquish();
@@ -211,16 +270,19 @@ __global__ void __launch_bounds__(kThreads, 1) linear_f32_kernel(const __grid_co
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tbase = tmem_base_s;
-  const int wq = warp & 3;  // (epilogue warps) TMEM lane quarter
+  const int wq = warp & 3;                    // (epilogue warps) TMEM lane quarter
+  const int eg = (warp - kSplitWarps) >> 2;   // (epilogue warps) which accumulator
   const uint32_t lane_base = static_cast<uint32_t>(wq * 32) << 16;
-  const int n = n0 + wq * 32 + lane;  // (epilogue warps) this thread's output column
-  float w_big = 0.f, w_small = kWeightHigh;  // (epilogue warps) of that column's weights, the zeros apart
+  const int n = n0 + wq * 32 + lane;          // (epilogue warps) this thread's output column
   griddep_wait();
   griddep_launch_dependents();
-  if (warp > kSplitWarps) {
-    // the weights of this block of columns, split once: thread = output column = TMEM lane
-    const float* src = p.w + static_cast<int64_t>(min(n, p.N - 1)) * p.K;
-    for (int k0 = 0; k0 < p.chunks * kChunk; k0 += 32) {
+  if (warp >= kSplitWarps && warp < kSplitWarps + kEpiWarps) {
+    // the weights of this block of columns, split once: thread = output column = TMEM lane, one half of the
+    // reduction columns for either four warps
+    const float* src = w + static_cast<int64_t>(min(n, p.N - 1)) * p.K;
+    float w_big = 0.f, w_small = kWeightHigh;  // of this column's weights, the zeros apart
+    const int k_end = min(p.chunks, eg + 1) * kChunk;
+    for (int k0 = eg * kChunk; k0 < k_end; k0 += 32) {
       uint32_t t[3][16];
 #pragma unroll
       for (int g = 0; g < 4; ++g) {
@@ -250,11 +312,12 @@ __global__ void __launch_bounds__(kThreads, 1) linear_f32_kernel(const __grid_co
     if (w_small < kWeightLow) {  // a zero, which is no matter, or not: look again
       w_small = kWeightHigh;
       if (n < p.N)
-        for (int k = 0; k < p.K; ++k) {
+        for (int k = eg * kChunk; k < min(p.K, k_end); ++k) {
           const float a = __ldg(src + k);
           if ((__float_as_uint(a) << 1) != 0u) w_small = fminf(w_small, fabsf(a));  // (a subnormal counts as 0)
         }
     }
+    w_odd_s[eg][wq * 32 + lane] = (w_big == 0.f ? 1 : 0) | (!(w_big < kWeightHigh) || w_small < kWeightLow ? 2 : 0);
   }
   tc_fence_before_sync();
   __syncthreads();
@@ -264,25 +327,26 @@ __global__ void __launch_bounds__(kThreads, 1) linear_f32_kernel(const __grid_co
     // ------------------------------------------------------------------ load and split x
     // A thread takes 8 columns (32 bytes) of four rows of every 64-column piece; eight threads cover
     // a row's 256 bytes.  The next tile's loads are in flight while this one is split.
+    reg_alloc<kSplitRegs>();
     const int c = tid & 7, row0 = tid >> 3;  // rows row0, +32, +64, +96
     float4 v[2][4][2];
-    auto fetch = [&](int mt) {
+    auto fetch = [&](int row_t) {
 #pragma unroll
       for (int ch = 0; ch < 2; ++ch) {
         const int k = ch * kChunk + c * 8;
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
-          const int row = mt * kTile + row0 + i * 32;
-          const bool live = row < p.M && k < p.K;
-          const float4* src = reinterpret_cast<const float4*>(p.x + static_cast<int64_t>(row) * p.K + k);
+          const int row = row_t + row0 + i * 32;
+          const bool live = row < row_end && k < p.K;
+          const float4* src = reinterpret_cast<const float4*>(x + row * p.x_sn + k);
           v[ch][i][0] = live ? __ldg(src) : make_float4(0.f, 0.f, 0.f, 0.f);
           v[ch][i][1] = live ? __ldg(src + 1) : make_float4(0.f, 0.f, 0.f, 0.f);
         }
       }
     };
     uint32_t t = 0;
-    if (m_first < p.m_tiles) fetch(m_first);
-    for (int mt = m_first; mt < p.m_tiles; mt += m_step, ++t) {
+    if (row_first < row_end) fetch(row_first);
+    for (int row_t = row_first; row_t < row_end; row_t += row_step, ++t) {
       const int st = t & 1;
       if (t >= 2 && !mbar_wait(smem_u32(&bars.x_empty[st]), ((t >> 1) - 1) & 1, abortp)) {
         if (lane == 0) record_timeout(p.status, 81);
@@ -294,7 +358,8 @@ __global__ void __launch_bounds__(kThreads, 1) linear_f32_kernel(const __grid_co
 #pragma unroll
           for (int i = 0; i < 4; ++i) {
             const float4 lo = v[ch][i][0], hi = v[ch][i][1];
-            const float e[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
+            float e[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
+            if constexpr (kMode == kSoftmax) softmax_group<4>(e);  // (past K the weights are zero)
             uint4 q[3];
             split8(e, q);
 #pragma unroll
@@ -304,21 +369,23 @@ __global__ void __launch_bounds__(kThreads, 1) linear_f32_kernel(const __grid_co
           }
         }
       }
-      if (mt + m_step < p.m_tiles) fetch(mt + m_step);
+      if (row_t + row_step < row_end) fetch(row_t + row_step);
       fence_proxy_async_smem();
       mbar_arrive(smem_u32(&bars.x_full[st]));
     }
-  } else if (warp == kSplitWarps) {
+  } else if (warp >= kSplitWarps + kEpiWarps) {
     // ------------------------------------------------------------------ MMA issuer
-    constexpr uint32_t idesc = umma_idesc_f16(UMMA_BF16, UMMA_K_MAJOR, UMMA_K_MAJOR, 128, 128);
+    reg_dealloc<kMmaRegs>();
     auto wait_all = [&](uint64_t* bar, uint32_t parity, uint32_t site) -> bool {
       const bool good = __all_sync(0xffffffffu, mbar_wait(smem_u32(bar), parity, abortp));
       if (!good && lane == 0) record_timeout(p.status, site);
       return good;
     };
     uint32_t t = 0;
-    for (int mt = m_first; mt < p.m_tiles; mt += m_step, ++t) {
+    for (int row_t = row_first; row_t < row_end && warp == kSplitWarps + kEpiWarps; row_t += row_step, ++t) {
       const int st = t & 1;
+      // (the rows of the tile are the N of the MMA: a last tile of few rows costs as much as it has)
+      const uint32_t idesc = umma_idesc_f16(UMMA_BF16, UMMA_K_MAJOR, UMMA_K_MAJOR, 128, min(kTile, (row_end - row_t + 15) & ~15));
       if (t >= 2 && !wait_all(&bars.acc_empty[st], ((t >> 1) - 1) & 1, 82)) break;
       if (!wait_all(&bars.x_full[st], (t >> 1) & 1, 83)) break;
       tc_fence_after_sync();
@@ -343,33 +410,36 @@ __global__ void __launch_bounds__(kThreads, 1) linear_f32_kernel(const __grid_co
     }
   } else {
     // ------------------------------------------------------------------ epilogue
-    uint8_t* const stage = gX + 2 * kStageBytes + wq * 2 * kOutBytes;
+    uint8_t* const dst = gX + 2 * kStageBytes + (warp - kSplitWarps) * kOutBytes;
+    const int odd[2] = {w_odd_s[0][wq * 32 + lane], w_odd_s[1][wq * 32 + lane]};
     const float bias = n < p.N ? __ldg(p.bias + n) : 0.f;
-    const bool zero_col = w_big == 0.f;  // a sum of zero is right (with a subnormal weight it is a plain one)
-    const bool plain_col = !(w_big < kWeightHigh) || w_small < kWeightLow;
+    float* const out = p.out + static_cast<int64_t>(batch) * p.M * p.N;
+    const bool zero_col = (odd[0] & odd[1] & 1) != 0;  // a sum of zero is right (with a subnormal weight it is a plain one)
+    const bool plain_col = ((odd[0] | odd[1]) & 2) != 0;
     const bool any_plain_col = __any_sync(0xffffffffu, plain_col);
     uint32_t t = 0;
-    for (int mt = m_first; mt < p.m_tiles; mt += m_step, ++t) {
+    for (int row_t = row_first; row_t < row_end; row_t += row_step, ++t) {
       const int st = t & 1;
+      if (st != eg) continue;
       if (!__all_sync(0xffffffffu, mbar_wait(smem_u32(&bars.acc_full[st]), (t >> 1) & 1, abortp))) {
         if (lane == 0) record_timeout(p.status, 84);
         break;
       }
       tc_fence_after_sync();
-      const int row_t = mt * kTile;
+      const int nq = min(4, (row_end - row_t + 31) / 32);  // 32-row pieces that have rows
       float big = 0.f, small = kWeightHigh;  // of this column's sums in the tile
       bool again = any_plain_col;
 #pragma unroll
       for (int q = 0; q < 4; ++q) {
+        if (q >= nq) break;
         uint32_t u[32];
         tmem_ld32(tbase + lane_base + kAccCol + st * 128 + q * 32, u);
-        uint8_t* const dst = stage + (q & 1) * kOutBytes;
-        if (lane == 0) tma_store_wait_read_n<1>();  // the store before last has left this half of the stage
+        if (lane == 0) tma_store_wait_read();  // the store before has left the stage
         __syncwarp();
         tmem_wait_ld();
-        if (row_t + q * 32 + 32 > p.M) {  // (rows past the end, zero as well, are not stored)
+        if (row_t + q * 32 + 32 > row_end) {  // (rows past the end, zero as well, are not stored)
 #pragma unroll
-          for (int r = 0; r < 32; ++r) u[r] = row_t + q * 32 + r < p.M ? u[r] : 0x3f800000u;
+          for (int r = 0; r < 32; ++r) u[r] = row_t + q * 32 + r < row_end ? u[r] : 0x3f800000u;
         }
 #pragma unroll
         for (int g = 0; g < 4; ++g) {
@@ -378,7 +448,7 @@ __global__ void __launch_bounds__(kThreads, 1) linear_f32_kernel(const __grid_co
           big = max3_nan(big, b8, b8);
           small = fminf(small, s8);
         }
-        if (q == 3) {
+        if (q == nq - 1) {
           again = __any_sync(0xffffffffu, !(big < INFINITY) || (small < kSumLow && !zero_col)) || again;
           if (!again) {
             tc_fence_before_sync();
@@ -393,12 +463,12 @@ __global__ void __launch_bounds__(kThreads, 1) linear_f32_kernel(const __grid_co
           fence_proxy_async_smem();
           __syncwarp();
           if (lane == 0) {
-            if (row_q < p.M && n < p.N) tma_store_4d(&map_out, smem_u32(dst), n, row_q, 0, 0);  // (lane 0: n is the block's first column)
+            if (n < p.N) tma_store_4d(&map_out, smem_u32(dst), n, row_q, batch, 0);  // (lane 0: n is the block's first column)
             tma_store_commit();
           }
         } else if (n < p.N) {  // (a thread reads back only what it wrote)
-          for (int r = 0; r < 32 && row_q + r < p.M; ++r)
-            p.out[static_cast<int64_t>(row_q + r) * p.N + n] =
+          for (int r = 0; r < 32 && row_q + r < row_end; ++r)
+            out[static_cast<int64_t>(row_q + r) * p.N + n] =
                 *reinterpret_cast<const float*>(dst + sw128_offset(r, lane >> 2) + (lane & 3) * 4);
         }
       }
@@ -407,7 +477,7 @@ __global__ void __launch_bounds__(kThreads, 1) linear_f32_kernel(const __grid_co
         if (lane == 0) tma_store_wait_all();
         __syncwarp();
 #pragma unroll 1
-        for (int q = 0; q < 4; ++q) {
+        for (int q = 0; q < nq; ++q) {
           const int row_q = row_t + q * 32;
           uint32_t u[32];
           tmem_ld32(tbase + lane_base + kAccCol + st * 128 + q * 32, u);
@@ -420,12 +490,12 @@ __global__ void __launch_bounds__(kThreads, 1) linear_f32_kernel(const __grid_co
           }
           if (plain_col) mine = 0xffffffffu;
           uint32_t left = __reduce_or_sync(0xffffffffu, mine);
-          if (!any_plain_col && left != 0u) left &= rows_not_zero(p.x + static_cast<int64_t>(row_q) * p.K, p.M - row_q, p.K);
+          if (kMode != kSoftmax && !any_plain_col && left != 0u) left &= rows_not_zero(x + row_q * p.x_sn, p.x_sn, row_end - row_q, p.K);
           for (; left != 0u; left &= left - 1u) {
             const int r = __ffs(left) - 1;
-            if (row_q + r >= p.M) break;
-            const float y = plain_dot(p.x + static_cast<int64_t>(row_q + r) * p.K, p.w, n0 + wq * 32, p.N, p.K);
-            if (((mine >> r) & 1u) != 0u && n < p.N) p.out[static_cast<int64_t>(row_q + r) * p.N + n] = add_keep(y, bias);
+            if (row_q + r >= row_end) break;
+            const float y = plain_dot<kMode == kSoftmax>(x + (row_q + r) * p.x_sn, w, n0 + wq * 32, p.N, p.K);
+            if (((mine >> r) & 1u) != 0u && n < p.N) out[static_cast<int64_t>(row_q + r) * p.N + n] = add_keep(y, bias);
           }
         }
         tc_fence_before_sync();
@@ -437,7 +507,7 @@ __global__ void __launch_bounds__(kThreads, 1) linear_f32_kernel(const __grid_co
   }
   tc_fence_before_sync();
   __syncthreads();
-  if (warp == kSplitWarps) {
+  if (warp == kSplitWarps + kEpiWarps) {
     __syncwarp();
     tmem_dealloc(tbase, 512);
   }
@@ -445,9 +515,31 @@ __global__ void __launch_bounds__(kThreads, 1) linear_f32_kernel(const __grid_co
 
 }  // namespace
 
+static cudaError_t launch(LinParams& p, int mode, int64_t batches, unsigned grid, cudaStream_t stream) {
+  p.chunks = (p.K + kChunk - 1) / kChunk;
+  p.status = device_status_words();
+  p.tma_out = p.N % 4 == 0 ? 1 : 0;
+  CUtensorMap mo = {};
+  if (p.tma_out) {
+    const uint64_t row_bytes = static_cast<uint64_t>(p.N) * 4, batch_bytes = row_bytes * p.M;
+    const uint64_t dims[4] = {static_cast<uint64_t>(p.N), static_cast<uint64_t>(p.M), static_cast<uint64_t>(batches), 1};
+    const uint64_t strides[3] = {row_bytes, batch_bytes, batch_bytes};
+    const uint32_t box[4] = {32, 32, 1, 1};
+    if (tma_host::make_f32_map_sw128(&mo, p.out, dims, strides, box) != 0) return cudaErrorInvalidValue;
+  }
+  auto kern = mode == kPlain ? linear_f32_kernel<kPlain> : mode == kBatched ? linear_f32_kernel<kBatched> : linear_f32_kernel<kSoftmax>;
+  cudaError_t e = ensure_dynamic_smem(reinterpret_cast<const void*>(kern), kSmemBytes);
+  if (e != cudaSuccess) return e;
+  e = check_register_budget(reinterpret_cast<const void*>(kern), kThreads, kBlockRegs);
+  if (e != cudaSuccess) return e;
+  e = launch_dependent(kern, dim3(grid), dim3(kThreads), kSmemBytes, stream, mo, p);
+  count_launch();
+  return e;
+}
+
 cudaError_t launch_linear_f32(const float* x, const float* w, const float* bias, float* out, int M, int N, int K,
                               int num_sms, cudaStream_t stream) {
-  LinParams p;
+  LinParams p = {};
   p.x = x;
   p.w = w;
   p.bias = bias;
@@ -455,27 +547,40 @@ cudaError_t launch_linear_f32(const float* x, const float* w, const float* bias,
   p.M = M;
   p.N = N;
   p.K = K;
-  p.m_tiles = (M + kTile - 1) / kTile;
+  p.x_sn = K;
   p.n_tiles = (N + kTile - 1) / kTile;
-  p.chunks = (K + kChunk - 1) / kChunk;
-  p.status = device_status_words();
-  p.tma_out = N % 4 == 0 ? 1 : 0;
-  CUtensorMap mo = {};
-  if (p.tma_out) {
-    const uint64_t row_bytes = static_cast<uint64_t>(N) * 4;
-    const uint64_t dims[4] = {static_cast<uint64_t>(N), static_cast<uint64_t>(M), 1, 1};
-    const uint64_t strides[3] = {row_bytes, row_bytes, row_bytes};
-    const uint32_t box[4] = {32, 32, 1, 1};
-    if (tma_host::make_f32_map_sw128(&mo, out, dims, strides, box) != 0) return cudaErrorInvalidValue;
-  }
-  const int64_t tiles = static_cast<int64_t>(p.m_tiles) * p.n_tiles;
+  const int64_t tiles = static_cast<int64_t>((M + kTile - 1) / kTile) * p.n_tiles;
   const int64_t most = num_sms > p.n_tiles ? num_sms : p.n_tiles;  // (every column block needs a CTA)
-  const unsigned grid = static_cast<unsigned>(tiles < most ? tiles : most);
-  cudaError_t e = ensure_dynamic_smem(reinterpret_cast<const void*>(linear_f32_kernel), kSmemBytes);
-  if (e != cudaSuccess) return e;
-  e = launch_dependent(linear_f32_kernel, dim3(grid), dim3(kThreads), kSmemBytes, stream, mo, p);
-  count_launch();
-  return e;
+  return launch(p, kPlain, 1, static_cast<unsigned>(tiles < most ? tiles : most), stream);
+}
+
+cudaError_t launch_linear_f32_batched(const float* x, int64_t x_sb, int64_t x_sn, const float* w, const float* bias, float* out,
+                                      int B, int M, int N, int K, bool softmax, int num_sms, cudaStream_t stream) {
+  LinParams p = {};
+  p.x = x;
+  p.w = w;
+  p.bias = bias;
+  p.out = out;
+  p.M = M;
+  p.N = N;
+  p.K = K;
+  p.x_sn = x_sn;
+  p.x_sb = x_sb;
+  p.n_tiles = 1;
+  // CTAs per batch: the split with the shortest launch, in rows of work per SM; a CTA's set-up (launch, weights
+  // to TMEM, first tile) takes about as long as 160 rows
+  const int pieces = (M + 31) / 32;
+  int64_t best = 0;
+  for (int s = 1; s <= pieces && s <= num_sms; ++s) {
+    const int rows = (pieces + s - 1) / s * 32, splits = (M + rows - 1) / rows;
+    const int64_t cost = (static_cast<int64_t>(B) * splits + num_sms - 1) / num_sms * (rows + 160);
+    if (p.splits == 0 || cost < best) {
+      best = cost;
+      p.cta_rows = rows;
+      p.splits = splits;
+    }
+  }
+  return launch(p, softmax ? kSoftmax : kBatched, B, static_cast<unsigned>(B) * p.splits, stream);
 }
 
 }  // namespace asuka

@@ -222,6 +222,19 @@ typedef struct {
 } asuka_linear_params;
 int asuka_b200_linear_f32(const asuka_linear_params* p, asuka_stream stream);
 
+/* ---- the core and the output projection behind it (bench/sima.mlir:13-22, bench/ea.mlir:13-22) --------
+ * out = core(q, k, v) w^T + bias without the core's output in between: per batch the product of the
+ * core's 32 x 32 matrices with w goes to `scratch`, and out is one projection of q with it.  C = 32 H,
+ * at most ASUKA_LINEAR_MAX_K. */
+typedef struct {
+  asuka_tensor q, k, v;  /* as asuka_linattn32_params; the heads of q side by side (stride[2] = 32) */
+  asuka_tensor w, bias;  /* [C, C], [C] f32, contiguous */
+  asuka_tensor out;      /* [B, N, C] f32, contiguous */
+  asuka_tensor scratch;  /* [B, C, C] f32, contiguous */
+  int32_t ea;
+} asuka_linattn32_proj_params;
+int asuka_b200_linattn32_proj(const asuka_linattn32_proj_params* p, asuka_stream stream);
+
 /* ---- fused cases: forward + column scores (+ selection) enqueued back to back on one stream.
  *      `workspace` holds the row statistics between the kernels: two arrays of B*H*Sq floats
  *      (unperturbed and Keyformer's perturbed one), each rounded up to 256 bytes, plus, when k

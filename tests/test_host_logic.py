@@ -379,6 +379,7 @@ def test_ctypes_structures_match_the_c_header(tmp_path):
       "asuka_sima_params": (_lib.SimaParams, ["q", "out"]),
       "asuka_linattn32_params": (_lib.LinAttn32Params, ["out", "ea"]),
       "asuka_linear_params": (_lib.LinearParams, ["w", "bias", "out"]),
+      "asuka_linattn32_proj_params": (_lib.LinAttn32ProjParams, ["w", "out", "scratch", "ea"]),
       "asuka_gather_params": (_lib.GatherParams, ["idx", "v_out"]),
       "asuka_case_params": (_lib.CaseParams, ["idx", "softmax_scale", "seed", "recent", "roco_mean", "roco_std", "seed_unit_offset"]),
   }

@@ -472,6 +472,65 @@ def test_linear_attention_blocks_at_the_reference_bench_shapes(ops, ea):
   no_timeouts(ops)
 
 
+def block_float64(x, w_qkv, b_qkv, w_o, b_o, ea):
+  """oracle.linear_attention_block in 64 bits"""
+  B, N, C = x.shape
+  qkv = x.double() @ w_qkv.double().t() + b_qkv.double()
+  q, k, v = qkv.reshape(B, N, 3, C // 32, 32).permute(2, 0, 3, 1, 4)
+  if ea:
+    qn, kn = torch.softmax(q, dim=3), torch.softmax(k, dim=2)
+  else:
+    qn, kn = q / q.abs().sum(dim=2, keepdim=True), k / k.abs().sum(dim=2, keepdim=True)
+  return (qn @ (kn.transpose(2, 3) @ v)).permute(0, 2, 1, 3).reshape(B, N, C) @ w_o.double().t() + b_o.double()
+
+
+@pytest.mark.parametrize("ea", [False, True])
+@pytest.mark.parametrize("shape", [(1, 1, 32), (2, 33, 96), (70, 31, 128), (3, 129, 64), (150, 70, 32), (5, 785, 128)])
+def test_block_rows_and_batches_vs_float64(ops, shape, ea):
+  # every batch has weights of its own in the last product, and its rows are cut into CTAs and tiles there:
+  # remainders of a tile, of a 32-row piece and of a 16-row MMA, batches beside one another and in several waves.
+  # Each of the block's three sums (128 terms twice, N once) is off by n 2^-24 of its terms at most
+  B, N, C = shape
+  g = torch.Generator().manual_seed(B + N)
+  args = [torch.randn(B, N, C, generator=g), torch.randn(3 * C, C, generator=g) / C ** 0.5, torch.randn(3 * C, generator=g) * 0.1,
+          torch.randn(C, C, generator=g) / C ** 0.5, torch.randn(C, generator=g) * 0.1]
+  args[0] *= 2.0 ** (torch.arange(B) % 5).view(B, 1, 1)
+  got = ops.linattn_block(*(t.cuda() for t in args), ea=ea).cpu().double()
+  want = block_float64(*args, ea)
+  bound = (2 * 128 + max(N, 128)) * 2.0 ** -24 * want.abs().amax(dim=(1, 2), keepdim=True)
+  assert ((got - want).abs() <= bound).all(), ((got - want).abs() / bound).max()
+  no_timeouts(ops)
+
+
+@pytest.mark.parametrize("ea", [False, True])
+def test_block_batches_keep_to_themselves(ops, ea):
+  # a NaN, an infinity, keys of nothing but zeros and weights of no ordinary size in one batch or column: the
+  # others come out as without them, and the odd ones as the restatement has them
+  B, N, C = 6, 90, 64
+  g = torch.Generator().manual_seed(9)
+  x, w_qkv, b_qkv = torch.randn(B, N, C, generator=g), torch.randn(3 * C, C, generator=g) / 8, torch.zeros(3 * C)
+  w_o, b_o = torch.randn(C, C, generator=g) / 8, torch.randn(C, generator=g)
+  clean = ops.linattn_block(*(t.cuda() for t in (x, w_qkv, b_qkv, w_o, b_o)), ea=ea).cpu()
+  odd = x.clone()
+  odd[1, 40, 3] = float("nan")
+  odd[3, 7, 5] = float("inf")
+  odd[4] = 0.0
+  w_odd = w_o.clone()
+  w_odd[9] *= 1e30
+  w_odd[33] *= 1e-34
+  got = ops.linattn_block(*(t.cuda() for t in (odd, w_qkv, b_qkv, w_odd, b_o)), ea=ea).cpu()
+  keep = [c for c in range(C) if c not in (9, 33)]
+  for b in (0, 2, 5):
+    assert torch.equal(got[b][:, keep], clean[b][:, keep])
+  want = block_float64(odd, w_qkv, b_qkv, w_odd, b_o, ea)
+  assert torch.equal(got.isnan().all(dim=2), want.isnan().all(dim=2)), "rows without a value"
+  for b in (0, 2, 5):
+    for c in (9, 33):
+      scale = want[b, :, c].abs().max()
+      assert ((got[b, :, c].double() - want[b, :, c]).abs() <= 384 * 2.0 ** -24 * scale).all()
+  no_timeouts(ops)
+
+
 def test_blocks_take_operands_from_anywhere_in_a_buffer(ops):
   # slices of a flat buffer (contiguous, at no 16-byte boundary), and views that are not contiguous
   from flashtensor_b200.blocks import EABlock, SimABlock
