@@ -12,7 +12,7 @@
 // cross-thread or cross-CTA reduction exists, and results are bitwise reproducible.
 //   warp 0      producer: one resident K tile (128 keys), Q tiles and their row statistics in two rings
 //   warp 1      tcgen05.mma issuer: S^T[buf] = K Q_i^T into one of two TMEM buffers
-//   warps 2-9   exp2, mask, accumulate; two warps per 32 keys, one for queries 0..63 and one for
+//   warps 2-9   (the perturbed modes: 2-17) exp2, mask, accumulate; two warps per 32 keys, one for queries 0..63 and one for
 //               queries 64..127 of every query tile
 // Two CTAs share an SM (96 KB and 256 TMEM columns each), so sixteen key warps run on it: one warp's
 // stream of FFMA -> MUFU -> FADD chains stalls on its own latencies about half the time, and its loads
@@ -49,9 +49,13 @@ constexpr int kUtilWarps = 2;                     // producer and MMA issuer
 // logit (more registers per thread).  Plain loads of the noise live on how many are in flight, so that mode has
 // sixteen warps all the same, each with 32 queries of a tile; Keyformer with a noise operand that TMA cannot
 // describe, whole case in us, eight warps -> sixteen: B1 H16
-// S1001 83.5 -> 80.5, B2 H32 S1501 342 -> 330, B4 H32 S2047 1034 -> 992.
+// S1001 83.5 -> 80.5, B2 H32 S1501 342 -> 330, B4 H32 S2047 1034 -> 992.  Seeded noise has sixteen too, two CTAs of
+// them on an SM with 16 queries in registers at a time: its long chains of integer mixing and three MUFU operations
+// leave gaps that more warps fill (with the row pass alike, whole case: B1 H16 S600 36.7 -> 34.8, B2 H32 S1501
+// 206 -> 201, B1 H16 S4000 326 -> 318).  The sums of plain probabilities gain nothing by it (H2O S4096 H32 211.4, 212.7).
 template <int kMode> struct ColCfg {
-  static constexpr int kKeyWarps = kMode == 2 ? 16 : 8;
+  static constexpr int kKeyWarps = kMode == 2 || kMode == 3 ? 16 : 8;
+  static constexpr int kChunk = kMode == 3 ? 16 : 32;  // queries that a thread has in registers at once
   static constexpr int kSubs = kKeyWarps / 4;      // warps per 32 keys
   static constexpr int kQueries = 128 / kSubs;     // queries of a tile for each
   static constexpr int kThreads = (kUtilWarps + kKeyWarps) * 32;
@@ -232,6 +236,7 @@ col_scores_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
   extern __shared__ uint8_t smem_raw[];
   __shared__ __align__(8) ColBars bars;
   __shared__ __align__(16) float lse_s[kLseStages][kTile];  // minus the row statistic
+  constexpr int kCh = ColCfg<kMode>::kChunk;
   constexpr int kKeyWarps = ColCfg<kMode>::kKeyWarps, kSubs = ColCfg<kMode>::kSubs, kQueries = ColCfg<kMode>::kQueries;
   __shared__ float part_s[2][kSubs][kTile];  // [sum, sum of squares][share of the queries][key]
   __shared__ uint32_t tmem_base_s;
@@ -397,16 +402,17 @@ col_scores_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
           const int first_visible = p.causal ? key - p.diag_off - q_base : 0;
           const bool tile_has_mask = p.causal && (kv0 + kTile - 1 - p.diag_off > q_base);
           const float4* lse4 = reinterpret_cast<const float4*>(lse_s[ls]) + hq * (kQueries / 4);
-          // chunks of 32 queries: every exponential of a chunk is in flight at once
+          // chunks of queries: every exponential of a chunk is in flight at once
 #pragma unroll
-          for (int ch = 0; ch < kQueries / 32; ++ch) {
-            float s[32];
-            tmem_ld32(tS + ch * 32, *reinterpret_cast<uint32_t(*)[32]>(s));
+          for (int ch = 0; ch < kQueries / kCh; ++ch) {
+            float s[kCh];
+            if constexpr (kCh == 32) tmem_ld32(tS + ch * 32, *reinterpret_cast<uint32_t(*)[32]>(s));
+            else tmem_ld16(tS + ch * 16, *reinterpret_cast<uint32_t(*)[16]>(s));
             float noise[(kMode == 2 || kMode == 4) ? 32 : 1];
             if constexpr (kMode == 2 || kMode == 4) {
 #pragma unroll
               for (int e = 0; e < 32; ++e) {
-                const int qi = min(q_base + ch * 32 + e, p.Sq - 1);
+                const int qi = min(q_base + ch * kCh + e, p.Sq - 1);
                 noise[e] = __ldg(er_col + static_cast<int64_t>(qi) * p.er_sq);
               }
               // the operand is read once, straight from HBM: pull the same chunk of the next query
@@ -414,13 +420,13 @@ col_scores_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
               if (i + 1 < i_end) {
 #pragma unroll
                 for (int e = 0; e < 32; ++e) {
-                  const int qi = min(q_base + kTile + ch * 32 + e, p.Sq - 1);
+                  const int qi = min(q_base + kTile + ch * kCh + e, p.Sq - 1);
                   asm volatile("prefetch.global.L2 [%0];" ::"l"(er_col + static_cast<int64_t>(qi) * p.er_sq));
                 }
               }
             }
             tmem_wait_ld();
-            if (ch == kQueries / 32 - 1) {
+            if (ch == kQueries / kCh - 1) {
               // this thread's part of the tile is in registers; when all have said so the MMA
               // warp may overwrite the TMEM buffer
               tc_fence_before_sync();
@@ -428,12 +434,12 @@ col_scores_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
             }
             uint32_t word_ch = 0;  // (seeded) the chunk's first query and this key after the mix's first xor-shift
             if constexpr (kMode == 3) {
-              word_ch = ((static_cast<uint32_t>(q_base + ch * 32) << 16) ^ static_cast<uint32_t>(key)) ^ head_key;
+              word_ch = ((static_cast<uint32_t>(q_base + ch * kCh) << 16) ^ static_cast<uint32_t>(key)) ^ head_key;
               word_ch ^= word_ch >> 16;
             }
 #pragma unroll
-            for (int g = 0; g < 8; ++g) {
-              const float4 L = lse4[ch * 8 + g];
+            for (int g = 0; g < kCh / 4; ++g) {
+              const float4 L = lse4[ch * (kCh / 4) + g];
               const float lv[4] = {L.x, L.y, L.z, L.w};  // minus the row statistic
               if constexpr (kMode == 2) {
 #pragma unroll
@@ -446,7 +452,7 @@ col_scores_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
 #pragma unroll
                 for (int e = 0; e < 4; e += 2) {
                   const int cc = g * 4 + e;
-                  // (query q0 + cc, cc < 32: the first xor-shift of the mix takes cc << 16 to cc << 16 ^ cc)
+                  // (query q0 + cc, cc < kCh: the first xor-shift of the mix takes cc << 16 to cc << 16 ^ cc)
                   const float2 l2 = seeded_lg2_exp_rand2(word_ch ^ (0x10001u * cc), word_ch ^ (0x10001u * (cc + 1)));
                   const float2 x = __ffma2_rn(make_float2(s[cc], s[cc + 1]), make_float2(scale, scale),
                                               __ffma2_rn(l2, make_float2(-p.inv_tau, -p.inv_tau), make_float2(lv[e], lv[e + 1])));
@@ -483,16 +489,16 @@ col_scores_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
             }
             if (tile_has_mask) {
 #pragma unroll
-              for (int cc = 0; cc < 32; ++cc) s[cc] = (ch * 32 + cc < first_visible) ? 0.f : s[cc];
+              for (int cc = 0; cc < kCh; ++cc) s[cc] = (ch * kCh + cc < first_visible) ? 0.f : s[cc];
             }
             if constexpr (kMode == 4) {
 #pragma unroll
-              for (int cc = 0; cc < 32; ++cc) hit = hit || (s[cc] >= noise[cc] && q_base + ch * 32 + cc < p.Sq);
+              for (int cc = 0; cc < kCh; ++cc) hit = hit || (s[cc] >= noise[cc] && q_base + ch * kCh + cc < p.Sq);
             } else {
               float2 a01 = make_float2(acc[0], acc[1]), a23 = make_float2(acc[2], acc[3]);
               float2 q01 = make_float2(acc2[0], acc2[1]), q23 = make_float2(acc2[2], acc2[3]);
 #pragma unroll
-              for (int cc = 0; cc < 32; cc += 4) {
+              for (int cc = 0; cc < kCh; cc += 4) {
                 const float2 p01 = make_float2(s[cc], s[cc + 1]), p23 = make_float2(s[cc + 2], s[cc + 3]);
                 a01 = __fadd2_rn(a01, p01);
                 a23 = __fadd2_rn(a23, p23);
@@ -921,14 +927,15 @@ constexpr uint32_t kNoiseTileBytes = 128 * 128 * 4;
 constexpr uint32_t kNoiseBoxBytes = kNoiseTileBytes / 4;
 // Warp 0 producer, warp 1 MMA, the others rows: kParts warps per 32 rows, each with its share of every tile's
 // columns.  Two warps per scheduler do not keep the MUFU busy over their chains of load, logarithm, maximum and
-// exponential; the staged variant, one CTA per SM, has four, the seeded one two CTAs of two.
+// exponential; the staged variant, one CTA per SM, has four, the seeded one two CTAs of four (see ColCfg).
 // With four warps instead of two, the last units' tiles longest first and the start under the forward kernel's
 // tail, the whole case went (us): B1 H16 S1000 58 -> 46, B2 H32 S1000 126 -> 109, B1 H16 S2048 117 -> 92,
 // B2 H32 S2048 356 -> 321, B4 H32 S2048 658 -> 607 (calls back to back on a cool card; among other work, at
 // lower clocks, the last takes 778 and 734).
 template <int kNoise> struct RsCfg {  // kNoise 1: two K stages, then eight noise boxes
   static constexpr bool kNoiseTma = kNoise == 1;
-  static constexpr int kParts = kNoiseTma ? 4 : 2;
+  static constexpr int kParts = kNoise == 0 ? 2 : 4;
+  static constexpr int kCols = kNoise == 2 ? 16 : 32;  // columns that a thread has in registers at once
   static constexpr int kThreads = (2 + 4 * kParts) * 32;
   static constexpr int kStages = kNoise == 0 ? 4 : 2;  // seeded: small enough for two CTAs per SM
   static constexpr uint32_t kStageBytes = kTileBytes + (kNoiseTma ? kNoiseTileBytes : 0);
@@ -949,7 +956,7 @@ kf_rowstat_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
                   const __grid_constant__ CUtensorMap map_n, const ColParams p, float* lse_out) {
   constexpr bool kNoiseTma = kNoise == 1;
   using Cfg = RsCfg<kNoise>;
-  constexpr int kStages = Cfg::kStages, kParts = Cfg::kParts;
+  constexpr int kStages = Cfg::kStages, kParts = Cfg::kParts, kW = Cfg::kCols;
   extern __shared__ uint8_t smem_raw[];
   __shared__ __align__(8) RsBars bars;
   __shared__ uint32_t tmem_base_s;
@@ -1118,10 +1125,11 @@ kf_rowstat_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
       tc_fence_after_sync();
       const int thr = lim - j * kTile;  // columns > thr are masked
 #pragma unroll
-      for (int c4 = part * (4 / kParts); c4 < (part + 1) * (4 / kParts); ++c4) {
-        uint32_t u[32];
-        tmem_ld32(tbase + lane_base + buf * 128 + c4 * 32, u);
-        float er[32];
+      for (int c4 = part * (kTile / kW / kParts); c4 < (part + 1) * (kTile / kW / kParts); ++c4) {
+        uint32_t u[kW];
+        if constexpr (kW == 32) tmem_ld32(tbase + lane_base + buf * 128 + c4 * 32, *reinterpret_cast<uint32_t(*)[32]>(u));
+        else tmem_ld16(tbase + lane_base + buf * 128 + c4 * 16, *reinterpret_cast<uint32_t(*)[16]>(u));
+        float er[kW];
         if constexpr (kNoiseTma) {
           const int slot = (j & 1) * 4 + c4;
           ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&bars.n_full[slot]), (j >> 1) & 1, abortp));
@@ -1137,16 +1145,16 @@ kf_rowstat_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
           if (lane == 0) mbar_arrive(smem_u32(&bars.n_empty[slot]));  // in registers: the box may be refilled
         } else if constexpr (kNoise == 0) {
 #pragma unroll
-          for (int e = 0; e < 32; ++e) er[e] = __ldg(er_row + min(j * kTile + c4 * 32 + e, p.Skv - 1));
+          for (int e = 0; e < kW; ++e) er[e] = __ldg(er_row + min(j * kTile + c4 * kW + e, p.Skv - 1));
         }
         tmem_wait_ld();
-        float x[32];
+        float x[kW];
         if constexpr (kNoise == 2) {
-          // (columns j * kTile + c4 * 32 + e, e < 32: the first xor-shift of the mix leaves e where it is)
-          uint32_t word = ((static_cast<uint32_t>(row) << 16) ^ static_cast<uint32_t>(j * kTile + c4 * 32)) ^ head_key;
+          // (columns j * kTile + c4 * kW + e, e < kW: the first xor-shift of the mix leaves e where it is)
+          uint32_t word = ((static_cast<uint32_t>(row) << 16) ^ static_cast<uint32_t>(j * kTile + c4 * kW)) ^ head_key;
           word ^= word >> 16;
 #pragma unroll
-          for (int e = 0; e < 32; e += 2) {
+          for (int e = 0; e < kW; e += 2) {
             const float2 l2 = seeded_lg2_exp_rand2(word ^ e, word ^ (e + 1));
             const float2 v = __ffma2_rn(make_float2(__uint_as_float(u[e]), __uint_as_float(u[e + 1])), make_float2(scale, scale),
                                         __fmul2_rn(l2, make_float2(-p.inv_tau, -p.inv_tau)));
@@ -1155,15 +1163,15 @@ kf_rowstat_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
           }
         } else {
 #pragma unroll
-          for (int e = 0; e < 32; ++e) x[e] = fmaf(__uint_as_float(u[e]), scale, -lg2(er[e]) * p.inv_tau);
+          for (int e = 0; e < kW; ++e) x[e] = fmaf(__uint_as_float(u[e]), scale, -lg2(er[e]) * p.inv_tau);
         }
         if (j * kTile + kTile - 1 > min_lim) {  // (some row of the tile does not see all of these keys)
 #pragma unroll
-          for (int e = 0; e < 32; ++e) x[e] = (c4 * 32 + e > thr) ? -INFINITY : x[e];
+          for (int e = 0; e < kW; ++e) x[e] = (c4 * kW + e > thr) ? -INFINITY : x[e];
         }
         float mt4[4] = {m, -INFINITY, -INFINITY, -INFINITY};
 #pragma unroll
-        for (int e = 0; e < 32; e += 8) {
+        for (int e = 0; e < kW; e += 8) {
 #pragma unroll
           for (int g = 0; g < 4; ++g) mt4[g] = max3(mt4[g], x[e + 2 * g], x[e + 2 * g + 1]);
         }
@@ -1172,7 +1180,7 @@ kf_rowstat_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
           const float2 neg_m2 = make_float2(-m_new, -m_new);
           float2 l01 = make_float2(l * ex2(m - m_new), 0.f), l23 = make_float2(0.f, 0.f);
 #pragma unroll
-          for (int e = 0; e < 32; e += 4) {
+          for (int e = 0; e < kW; e += 4) {
             const float2 a = __fadd2_rn(make_float2(x[e], x[e + 1]), neg_m2), c = __fadd2_rn(make_float2(x[e + 2], x[e + 3]), neg_m2);
             l01 = __fadd2_rn(l01, make_float2(ex2(a.x), ex2(a.y)));
             l23 = __fadd2_rn(l23, make_float2(ex2(c.x), ex2(c.y)));
@@ -1351,8 +1359,7 @@ cudaError_t launch_col_scores(const CUtensorMap& mq, const CUtensorMap& mk, cons
   else kern = s.bf16 ? col_scores_kernel<true, 3> : col_scores_kernel<false, 3>;
   e = ensure_dynamic_smem(reinterpret_cast<const void*>(kern), kSmemBytes);
   if (e != cudaSuccess) return e;
-  const bool sixteen = a.mode == ASUKA_SCORE_PERTURBED && a.exp_rand != nullptr;  // (mode 2 of the kernel)
-  e = launch_dependent(kern, grid, dim3(sixteen ? ColCfg<2>::kThreads : ColCfg<0>::kThreads), kSmemBytes, stream, mq, mk, p);
+  e = launch_dependent(kern, grid, dim3(a.mode == ASUKA_SCORE_PERTURBED ? ColCfg<2>::kThreads : ColCfg<0>::kThreads), kSmemBytes, stream, mq, mk, p);
   count_launch();
   }
   if (e != cudaSuccess || p.n_qchunks == 1) return e;
