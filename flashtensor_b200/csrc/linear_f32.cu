@@ -15,8 +15,8 @@
 // 38 us instead of the figure below), and an accumulator lane is an output column, so a warp's store
 // is one 128-byte line of an output row.
 //   warps 0-7    load x (a whole tile ahead), split it and store the three terms as swizzled K-major tiles
-//   warps 8-15   split the weights into TMEM; then accumulator + bias to global memory, four warps for either
-//   warp 16      issues tcgen05.mma into one of two accumulators
+//   warp 8       issues tcgen05.mma into one of two accumulators
+//   warps 9-12   split the weights into TMEM; then accumulator + bias to global memory
 // The small products of a tile are accumulated before any h.h: the tensor pipe truncates when it adds
 // to an accumulator, and forty small terms added to a large sum would each leave a bias there
 // (measured at K = 128: 4.1e-7 relative error in the natural order, against 1.5e-7 of an f32 GEMM on
@@ -28,9 +28,11 @@
 // column with a weight outside [2^-100, 2^20) that is not zero, is computed on the CUDA cores (plain_dot) by
 // the warps that store it; which way a result takes depends on its own row and column.  That is for the odd row
 // or column: all rows at 1e-25 take 1460 us instead of 34, rows of nothing but zeros, which need a look at x only, 91.
-// Measured at B64 N784 C128 (M = 50176, K = 128), calls back to back, bias included: N = 384 (QKV) 33 us,
-// N = 128 (output) 17.7 us (31.5 and 16 without the look at the sums); the f32 GEMM of the BLAS library with its
-// bias pass takes 200 and 64.
+// Measured at B64 N784 C128 (M = 50176, K = 128), calls back to back, bias included: N = 384 (QKV) 32 us,
+// N = 128 (output) 14.6 us; the f32 GEMM of the BLAS library with its bias pass takes 200 and 64.  A launch is set-up
+// for a third of it, so the warps that split x start while the weights are still being split (whole SimA block
+// 78.5 -> 74 us).  Eight epilogue warps, four to an accumulator, are slower (38 and 17 us: what they and the
+// splitting warps share is the way to shared memory), and so are plain stores instead of TMA's.
 #include <cuda_bf16.h>
 
 #include "kernels.h"
@@ -49,13 +51,9 @@ constexpr uint32_t kTermBytes = kTile * kChunk * 2;  // one bf16 term of a [128 
 constexpr uint32_t kPieceBytes = 3 * kTermBytes;
 constexpr uint32_t kStageBytes = (kMaxK / kChunk) * kPieceBytes;  // a tile of x: 96 KB
 constexpr int kSplitWarps = 8;
-constexpr int kEpiWarps = 8;                                      // four for either accumulator
-constexpr int kThreads = (kSplitWarps + kEpiWarps + 4) * 32;      // (the MMA warp and three that idle: setmaxnreg counts in fours)
-constexpr int kSplitRegs = 128, kEpiRegs = 96, kMmaRegs = 32;
-constexpr int kBlockRegs = kSplitWarps * 32 * kSplitRegs + kEpiWarps * 32 * kEpiRegs + 128 * kMmaRegs;
-static_assert(kBlockRegs <= kThreads * 96, "setmaxnreg would wait for ever");
+constexpr int kThreads = (kSplitWarps + 1 + 4) * 32;
 constexpr uint32_t kOutBytes = 32 * 32 * 4;                       // one TMA store of a warp: 32 rows x 32 columns
-constexpr uint32_t kSmemBytes = 2 * kStageBytes + kEpiWarps * kOutBytes + 1024;
+constexpr uint32_t kSmemBytes = 2 * kStageBytes + 4 * 2 * kOutBytes + 1024;
 constexpr uint32_t kTermCols = kMaxK / 2;  // TMEM columns of one term of the weights
 constexpr uint32_t kAccCol = 3 * kTermCols;
 
@@ -225,7 +223,6 @@ template <int kMode>
 __global__ void __launch_bounds__(kThreads, 1) linear_f32_kernel(const __grid_constant__ CUtensorMap map_out, const LinParams p) {
   extern __shared__ uint8_t smem_raw[];
   __shared__ __align__(8) LinBars bars;
-  __shared__ uint8_t w_odd_s[2][kTile];  // of every column, in either half of the reduction: 1 no weight but zeros, 2 one out of range
   __shared__ uint32_t tmem_base_s;
   __shared__ uint32_t abort_s;
   const uint32_t sX = (smem_u32(smem_raw) + 1023u) & ~1023u;
@@ -261,7 +258,7 @@ __global__ void __launch_bounds__(kThreads, 1) linear_f32_kernel(const __grid_co
     }
     mbar_fence_init();
   }
-  if (warp == kSplitWarps + kEpiWarps) {
+  if (warp == kSplitWarps) {
     __syncwarp();
     tmem_alloc(smem_u32(&tmem_base_s), 512);
     tmem_relinquish();
@@ -270,19 +267,16 @@ __global__ void __launch_bounds__(kThreads, 1) linear_f32_kernel(const __grid_co
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tbase = tmem_base_s;
-  const int wq = warp & 3;                    // (epilogue warps) TMEM lane quarter
-  const int eg = (warp - kSplitWarps) >> 2;   // (epilogue warps) which accumulator
+  const int wq = warp & 3;  // (epilogue warps) TMEM lane quarter
   const uint32_t lane_base = static_cast<uint32_t>(wq * 32) << 16;
-  const int n = n0 + wq * 32 + lane;          // (epilogue warps) this thread's output column
+  const int n = n0 + wq * 32 + lane;  // (epilogue warps) this thread's output column
+  float w_big = 0.f, w_small = kWeightHigh;  // (epilogue warps) of that column's weights, the zeros apart
   griddep_wait();
   griddep_launch_dependents();
-  if (warp >= kSplitWarps && warp < kSplitWarps + kEpiWarps) {
-    // the weights of this block of columns, split once: thread = output column = TMEM lane, one half of the
-    // reduction columns for either four warps
+  if (warp > kSplitWarps) {
+    // the weights of this block of columns, split once: thread = output column = TMEM lane
     const float* src = w + static_cast<int64_t>(min(n, p.N - 1)) * p.K;
-    float w_big = 0.f, w_small = kWeightHigh;  // of this column's weights, the zeros apart
-    const int k_end = min(p.chunks, eg + 1) * kChunk;
-    for (int k0 = eg * kChunk; k0 < k_end; k0 += 32) {
+    for (int k0 = 0; k0 < p.chunks * kChunk; k0 += 32) {
       uint32_t t[3][16];
 #pragma unroll
       for (int g = 0; g < 4; ++g) {
@@ -312,22 +306,22 @@ __global__ void __launch_bounds__(kThreads, 1) linear_f32_kernel(const __grid_co
     if (w_small < kWeightLow) {  // a zero, which is no matter, or not: look again
       w_small = kWeightHigh;
       if (n < p.N)
-        for (int k = eg * kChunk; k < min(p.K, k_end); ++k) {
+        for (int k = 0; k < p.K; ++k) {
           const float a = __ldg(src + k);
           if ((__float_as_uint(a) << 1) != 0u) w_small = fminf(w_small, fabsf(a));  // (a subnormal counts as 0)
         }
     }
-    w_odd_s[eg][wq * 32 + lane] = (w_big == 0.f ? 1 : 0) | (!(w_big < kWeightHigh) || w_small < kWeightLow ? 2 : 0);
   }
-  tc_fence_before_sync();
-  __syncthreads();
-  tc_fence_after_sync();
+  if (warp >= kSplitWarps) {  // (the splitting warps have nothing to do with the weights and are at work already)
+    tc_fence_before_sync();
+    named_bar_sync(1, kThreads - kSplitWarps * 32);
+    tc_fence_after_sync();
+  }
 
   if (warp < kSplitWarps) {
     // ------------------------------------------------------------------ load and split x
     // A thread takes 8 columns (32 bytes) of four rows of every 64-column piece; eight threads cover
     // a row's 256 bytes.  The next tile's loads are in flight while this one is split.
-    reg_alloc<kSplitRegs>();
     const int c = tid & 7, row0 = tid >> 3;  // rows row0, +32, +64, +96
     float4 v[2][4][2];
     auto fetch = [&](int row_t) {
@@ -338,7 +332,7 @@ __global__ void __launch_bounds__(kThreads, 1) linear_f32_kernel(const __grid_co
         for (int i = 0; i < 4; ++i) {
           const int row = row_t + row0 + i * 32;
           const bool live = row < row_end && k < p.K;
-          const float4* src = reinterpret_cast<const float4*>(x + row * p.x_sn + k);
+          const float4* src = reinterpret_cast<const float4*>(x + static_cast<int64_t>(row) * (kMode == kPlain ? p.K : p.x_sn) + k);
           v[ch][i][0] = live ? __ldg(src) : make_float4(0.f, 0.f, 0.f, 0.f);
           v[ch][i][1] = live ? __ldg(src + 1) : make_float4(0.f, 0.f, 0.f, 0.f);
         }
@@ -373,19 +367,19 @@ __global__ void __launch_bounds__(kThreads, 1) linear_f32_kernel(const __grid_co
       fence_proxy_async_smem();
       mbar_arrive(smem_u32(&bars.x_full[st]));
     }
-  } else if (warp >= kSplitWarps + kEpiWarps) {
+  } else if (warp == kSplitWarps) {
     // ------------------------------------------------------------------ MMA issuer
-    reg_dealloc<kMmaRegs>();
     auto wait_all = [&](uint64_t* bar, uint32_t parity, uint32_t site) -> bool {
       const bool good = __all_sync(0xffffffffu, mbar_wait(smem_u32(bar), parity, abortp));
       if (!good && lane == 0) record_timeout(p.status, site);
       return good;
     };
     uint32_t t = 0;
-    for (int row_t = row_first; row_t < row_end && warp == kSplitWarps + kEpiWarps; row_t += row_step, ++t) {
+    for (int row_t = row_first; row_t < row_end; row_t += row_step, ++t) {
       const int st = t & 1;
-      // (the rows of the tile are the N of the MMA: a last tile of few rows costs as much as it has)
-      const uint32_t idesc = umma_idesc_f16(UMMA_BF16, UMMA_K_MAJOR, UMMA_K_MAJOR, 128, min(kTile, (row_end - row_t + 15) & ~15));
+      // (the rows of the tile are the N of the MMA: a batch's last tile of few rows costs as much as it has)
+      const uint32_t idesc = umma_idesc_f16(UMMA_BF16, UMMA_K_MAJOR, UMMA_K_MAJOR, 128,
+                                            kMode == kPlain ? kTile : min(kTile, (row_end - row_t + 15) & ~15));
       if (t >= 2 && !wait_all(&bars.acc_empty[st], ((t >> 1) - 1) & 1, 82)) break;
       if (!wait_all(&bars.x_full[st], (t >> 1) & 1, 83)) break;
       tc_fence_after_sync();
@@ -410,31 +404,28 @@ __global__ void __launch_bounds__(kThreads, 1) linear_f32_kernel(const __grid_co
     }
   } else {
     // ------------------------------------------------------------------ epilogue
-    uint8_t* const dst = gX + 2 * kStageBytes + (warp - kSplitWarps) * kOutBytes;
-    const int odd[2] = {w_odd_s[0][wq * 32 + lane], w_odd_s[1][wq * 32 + lane]};
+    uint8_t* const stage = gX + 2 * kStageBytes + wq * 2 * kOutBytes;
     const float bias = n < p.N ? __ldg(p.bias + n) : 0.f;
     float* const out = p.out + static_cast<int64_t>(batch) * p.M * p.N;
-    const bool zero_col = (odd[0] & odd[1] & 1) != 0;  // a sum of zero is right (with a subnormal weight it is a plain one)
-    const bool plain_col = ((odd[0] | odd[1]) & 2) != 0;
+    const bool zero_col = w_big == 0.f;  // a sum of zero is right (with a subnormal weight it is a plain one)
+    const bool plain_col = !(w_big < kWeightHigh) || w_small < kWeightLow;
     const bool any_plain_col = __any_sync(0xffffffffu, plain_col);
     uint32_t t = 0;
     for (int row_t = row_first; row_t < row_end; row_t += row_step, ++t) {
       const int st = t & 1;
-      if (st != eg) continue;
       if (!__all_sync(0xffffffffu, mbar_wait(smem_u32(&bars.acc_full[st]), (t >> 1) & 1, abortp))) {
         if (lane == 0) record_timeout(p.status, 84);
         break;
       }
       tc_fence_after_sync();
-      const int nq = min(4, (row_end - row_t + 31) / 32);  // 32-row pieces that have rows
       float big = 0.f, small = kWeightHigh;  // of this column's sums in the tile
       bool again = any_plain_col;
 #pragma unroll
       for (int q = 0; q < 4; ++q) {
-        if (q >= nq) break;
         uint32_t u[32];
         tmem_ld32(tbase + lane_base + kAccCol + st * 128 + q * 32, u);
-        if (lane == 0) tma_store_wait_read();  // the store before has left the stage
+        uint8_t* const dst = stage + (q & 1) * kOutBytes;
+        if (lane == 0) tma_store_wait_read_n<1>();  // the store before last has left this half of the stage
         __syncwarp();
         tmem_wait_ld();
         if (row_t + q * 32 + 32 > row_end) {  // (rows past the end, zero as well, are not stored)
@@ -448,7 +439,7 @@ __global__ void __launch_bounds__(kThreads, 1) linear_f32_kernel(const __grid_co
           big = max3_nan(big, b8, b8);
           small = fminf(small, s8);
         }
-        if (q == nq - 1) {
+        if (q == 3) {
           again = __any_sync(0xffffffffu, !(big < INFINITY) || (small < kSumLow && !zero_col)) || again;
           if (!again) {
             tc_fence_before_sync();
@@ -463,7 +454,7 @@ __global__ void __launch_bounds__(kThreads, 1) linear_f32_kernel(const __grid_co
           fence_proxy_async_smem();
           __syncwarp();
           if (lane == 0) {
-            if (n < p.N) tma_store_4d(&map_out, smem_u32(dst), n, row_q, batch, 0);  // (lane 0: n is the block's first column)
+            if (row_q < row_end && n < p.N) tma_store_4d(&map_out, smem_u32(dst), n, row_q, batch, 0);  // (lane 0: n is the block's first column)
             tma_store_commit();
           }
         } else if (n < p.N) {  // (a thread reads back only what it wrote)
@@ -477,7 +468,7 @@ __global__ void __launch_bounds__(kThreads, 1) linear_f32_kernel(const __grid_co
         if (lane == 0) tma_store_wait_all();
         __syncwarp();
 #pragma unroll 1
-        for (int q = 0; q < nq; ++q) {
+        for (int q = 0; q < 4; ++q) {
           const int row_q = row_t + q * 32;
           uint32_t u[32];
           tmem_ld32(tbase + lane_base + kAccCol + st * 128 + q * 32, u);
@@ -507,7 +498,7 @@ __global__ void __launch_bounds__(kThreads, 1) linear_f32_kernel(const __grid_co
   }
   tc_fence_before_sync();
   __syncthreads();
-  if (warp == kSplitWarps + kEpiWarps) {
+  if (warp == kSplitWarps) {
     __syncwarp();
     tmem_dealloc(tbase, 512);
   }
@@ -529,8 +520,6 @@ static cudaError_t launch(LinParams& p, int mode, int64_t batches, unsigned grid
   }
   auto kern = mode == kPlain ? linear_f32_kernel<kPlain> : mode == kBatched ? linear_f32_kernel<kBatched> : linear_f32_kernel<kSoftmax>;
   cudaError_t e = ensure_dynamic_smem(reinterpret_cast<const void*>(kern), kSmemBytes);
-  if (e != cudaSuccess) return e;
-  e = check_register_budget(reinterpret_cast<const void*>(kern), kThreads, kBlockRegs);
   if (e != cudaSuccess) return e;
   e = launch_dependent(kern, dim3(grid), dim3(kThreads), kSmemBytes, stream, mo, p);
   count_launch();
