@@ -840,6 +840,7 @@ kf_col_tma_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
             const int r = sub * 16 + e;
             nz[e] = *reinterpret_cast<const float*>(box + sw128_offset(r, lane >> 2) + (lane & 3) * 4);
           }
+          fence_proxy_async_smem();  // (the reads above before the copy that refills the piece)
           __syncwarp();
           if (lane == 0) mbar_arrive(smem_u32(&bars.n_empty[ns]));
           tmem_wait_ld();
@@ -1141,8 +1142,12 @@ kf_rowstat_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
             const float4 v = *reinterpret_cast<const float4*>(box + sw128_offset(r_in_tile, ch));
             er[ch * 4 + 0] = v.x; er[ch * 4 + 1] = v.y; er[ch * 4 + 2] = v.z; er[ch * 4 + 3] = v.w;
           }
+          // In registers: the box may be refilled.  The refill is the async proxy's: without the fence it can overtake
+          // reads that are still queued (the mask taken out of most steps was enough for that: a handful of rows
+          // in a thousand then had other values in their first boxes).
+          fence_proxy_async_smem();
           __syncwarp();
-          if (lane == 0) mbar_arrive(smem_u32(&bars.n_empty[slot]));  // in registers: the box may be refilled
+          if (lane == 0) mbar_arrive(smem_u32(&bars.n_empty[slot]));
         } else if constexpr (kNoise == 0) {
 #pragma unroll
           for (int e = 0; e < kW; ++e) er[e] = __ldg(er_row + min(j * kTile + c4 * kW + e, p.Skv - 1));
