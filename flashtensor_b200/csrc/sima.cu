@@ -1559,17 +1559,29 @@ cudaError_t launch_sima(const CUtensorMap& mq, const CUtensorMap& mk, const CUte
   const Plan pl = make_plan(s);
   const int bh = s.B * s.H;
   uint8_t* w = static_cast<uint8_t*>(ws);
-  // One persistent kernel for all three steps when there are enough units to keep most groups of
-  // four CTAs busy.  The line was drawn against three kernels that cut every unit into slabs.  Against these,
-  // which share the tiles out evenly, it is right below 37 units of 3000 rows and more and wrong above them,
-  // where the groups' last round of units is partial (us, single kernel / three: 24 units, S 700 19.5 / 16.5, S 4096
-  // 33.0 / 34.4; 36 units, S 4096 40.3 / 45.0; 40 units, S 4096 61.6 / 49.3, S 8192 104 / 84; 64 units, S 8192
-  // 125.5 / 125.8; 96 units, S 2000 71.8 / 57.4, S 8192 184 / 180).
+  // One persistent kernel for all three steps, or three that share the tiles out evenly.  The first reads Q from
+  // L2 the second time and has no gaps between launches; but every round of units costs it a barrier, a reduce
+  // and a fill of 10 us or so however short the sequence is, and its last round may be partial.  So it is for one
+  // round of long sequences, and for several where what it saves, proportional to S, covers that.  Measured in us,
+  // one kernel / three, by units (37 groups) and S; the lines run between 24 units' S 1500 and 4096 and along
+  // (S - 3200) units = 500000:
+  //          700          1500         4096           8192
+  //   24     18.8/15.2    20.7/18.6    30.9/31.5      51.9/55.6
+  //   36     18.8/17.2    22.1/19.7    35.5/43.5      70.0/74.9
+  //   48     30.9/18.1    35.2/23.7    63.6/56.8      107/97.7
+  //   64     32.9/20.1    39.1/31.1    74.1/69.0      125/125
+  //   96     47.2/23.2    57.8/43.6    111/97.4       186/179
+  //   128    59.6/30.9    73.2/55.6    133/126        227/233
+  //   160    73.9/38.5    92.4/67.1    164/156        281/294
+  //   256    111/59.9     132/103      242/241        412/456
   const int n_groups = num_sms / kFuGroup;
 #ifdef ASUKA_SIMA_NO_FUSED
   const bool fused = false;
 #else
-  const bool fused = !s.ea && maps64 != nullptr && n_groups > 0 && 2 * bh >= n_groups && pl.ntiles >= kFuGroup;
+  const bool fused = !s.ea && maps64 != nullptr && n_groups > 0 && 2 * bh >= n_groups &&
+                     (s.out_f32        ? pl.ntiles >= kFuGroup  // (f32 output: the line of before, not measured since)
+                      : bh <= n_groups ? pl.ntiles >= 24
+                                       : static_cast<int64_t>(s.S - 3200) * bh > 500000);
 #endif
   if (fused) {
     FusedParams fp;

@@ -317,6 +317,12 @@ def test_sima_with_many_units_vs_oracle(ops, shape, dtype):
   no_timeouts(ops)
 
 
+@pytest.mark.parametrize("shape", [(1, 2944, 20), (1, 2945, 20), (1, 2950, 37), (1, 2950, 38), (7, 900, 9)])
+def test_sima_on_either_side_of_the_line(ops, shape):
+  # one persistent kernel or three: 24 key tiles or 23 with one round of units, one unit more than a round
+  test_sima_vs_oracle(ops, shape, torch.float16)
+
+
 @pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
 @pytest.mark.parametrize("shape", [(1, 128, 1), (2, 1000, 3), (1, 4096, 4), (3, 2500, 2)])
 def test_ea_vs_oracle(ops, shape, dtype):
