@@ -20,6 +20,9 @@
 // Multiply-adds are the packed two-wide f32 FMAs of sm_100; every sum runs in a fixed order.
 // Measured at B64 H4 N784 (SimA / EA): three passes of plain loads with sixteen rows of a warp in
 // flight 58 / 67 us, this kernel 37 / 47 us.
+// In a whole block (kFold) there is no pass B: the kernel multiplies the 32 x 32 matrices with the output
+// projection, and linear_f32.cu applies the product to the queries (this kernel 23 us then; the block, SimA / EA,
+// 82 / 91.5 -> 70 / 77 us with it and the projections' earlier start).
 #include "kernels.h"
 #include "sm100_ptx.cuh"
 #include "tma_host.h"
@@ -272,13 +275,13 @@ linattn32_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
       for (int e = 0; e < kD; ++e) m[e] = m_s[lane][e];
       float* dst = p.w_fold + static_cast<int64_t>(b) * C * C + h * kD + lane;
       for (int c = warp; c < C; c += kWarps) {
-        float sum = 0.f;
+        float sum[kD / 4];  // (in pairs: one running sum of thirty-two rounds more)
 #pragma unroll
         for (int i = 0; i < kD / 4; ++i) {
           const float4 o = *reinterpret_cast<const float4*>(w_s + c * kD + i * 4);
-          sum = fmaf(m[4 * i], o.x, fmaf(m[4 * i + 1], o.y, fmaf(m[4 * i + 2], o.z, fmaf(m[4 * i + 3], o.w, sum))));
+          sum[i] = fmaf(m[4 * i], o.x, m[4 * i + 1] * o.y) + fmaf(m[4 * i + 2], o.z, m[4 * i + 3] * o.w);
         }
-        dst[static_cast<int64_t>(c) * C] = sum;
+        dst[static_cast<int64_t>(c) * C] = ((sum[0] + sum[1]) + (sum[2] + sum[3])) + ((sum[4] + sum[5]) + (sum[6] + sum[7]));
       }
     }
     return;

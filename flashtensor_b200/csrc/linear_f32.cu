@@ -123,12 +123,10 @@ __device__ __forceinline__ void softmax_group(float (&v)[kN]) {
   for (int i = 1; i < kN; ++i) m = fmaxf(m, v[i]);
 #pragma unroll
   for (int o = 1; o < kLanes; o <<= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
-  float sum = 0.f;
 #pragma unroll
-  for (int i = 0; i < kN; ++i) {
-    v[i] = exp_fast(v[i] - m);
-    sum += v[i];
-  }
+  for (int i = 0; i < kN; ++i) v[i] = exp_fast(v[i] - m);
+  float sum = (v[0] + v[1]) + (v[2] + v[3]);
+  if constexpr (kN == 8) sum += (v[4] + v[5]) + (v[6] + v[7]);
 #pragma unroll
   for (int o = 1; o < kLanes; o <<= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
   const float inv = __frcp_rn(sum);
@@ -271,7 +269,9 @@ __global__ void __launch_bounds__(kThreads, 1) linear_f32_kernel(const __grid_co
   const uint32_t lane_base = static_cast<uint32_t>(wq * 32) << 16;
   const int n = n0 + wq * 32 + lane;  // (epilogue warps) this thread's output column
   float w_big = 0.f, w_small = kWeightHigh;  // (epilogue warps) of that column's weights, the zeros apart
-  griddep_wait();
+  // (batched: the kernel ahead, which writes the weights, reads x itself and has waited for whatever wrote it before
+  // this one could start: the splitting warps need not wait; EA block 79.7 -> 76.8 us)
+  if (kMode == kPlain || warp >= kSplitWarps) griddep_wait();
   griddep_launch_dependents();
   if (warp > kSplitWarps) {
     // the weights of this block of columns, split once: thread = output column = TMEM lane
