@@ -284,6 +284,7 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_const
         mma16816<kBF16>(o[2 * d], pf, vf[0], vf[1]);
         mma16816<kBF16>(o[2 * d + 1], pf, vf[2], vf[3]);
       }
+      fence_proxy_async_smem();  // (the reads above before the copy that refills the stage)
       __syncwarp();
       if (lane == 0) mbar_arrive(smem_u32(&empty[st]));
     }

@@ -210,7 +210,7 @@ linattn32_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
 #pragma unroll
           for (int d = 0; d < 4; ++d) acc[e][d] = __ffma2_rn(kk[d], make_float2(ve[e], ve[e]), acc[e][d]);
       }
-      if constexpr (kEA) fence_proxy_async_smem();  // (K' was written over a tile that TMA refills)
+      fence_proxy_async_smem();  // (the reads above, and EA's K' over the tile, before the copy that refills the stage)
       __syncwarp();
       if (lane == 0) mbar_arrive(smem_u32(&bars.a_empty[st]));
     }

@@ -479,6 +479,7 @@ sima_stats_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
           const uint4 v = *reinterpret_cast<const uint4*>(tile + sw128_offset(row, chunk16 & 7));
           abs_acc8<kBF16>(v, acc);
         }
+        fence_proxy_async_smem();  // (the reads above before the copy that refills the stage)
         __syncwarp();
         if (lane == 0) mbar_arrive(smem_u32(&bars.empty[st]));
       }
@@ -1246,6 +1247,7 @@ sima_fused_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
           const uint4 v = *reinterpret_cast<const uint4*>(tile + sw128_offset(row, chunk16 & 7));
           abs_acc8<kBF16>(v, acc);
         }
+        fence_proxy_async_smem();  // (the reads above before the copy that refills the stage)
         __syncwarp();
         if (lane == 0) mbar_arrive(smem_u32(&bars.empty[st]));
       }
@@ -1491,9 +1493,9 @@ sima_fused_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
           }
         }
       }
-      if constexpr (!kOutF32) {
-        if (tid == 128) tma_store_wait_read();  // phase 1 of the next unit reuses the staging memory
-      }
+      // phase 1 of the next unit reuses the staging memory
+      if constexpr (kOutF32) fence_proxy_async_smem();  // (the copy-out's reads before the copies that fill it)
+      else if (tid == 128) tma_store_wait_read();
       if (!good) *abortp = 1u;
     }
     tc_fence_before_sync();

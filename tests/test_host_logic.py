@@ -398,3 +398,20 @@ def test_ctypes_structures_match_the_c_header(tmp_path):
     assert int(got[name]) == ctypes.sizeof(cls), name
     for f in fields:
       assert int(got[f"{name}.{f}"]) == getattr(cls, f).offset, f"{name}.{f}"
+
+
+def test_stages_go_back_to_tma_behind_a_fence():
+  # A ring's consumers read a stage with ordinary loads; the copy that refills it is the async proxy's, which only
+  # a proxy fence in every reading lane holds back until those loads are done.  (Rings of ordinary stores need none.)
+  plain = {("col_scores.cu", "lse_empty"), ("col_scores.cu", "q_empty")}  # row statistics; what else the stages hold the MMA reads
+  csrc = os.path.join(ROOT, "flashtensor_b200", "csrc")
+  found = 0
+  for name in sorted(os.listdir(csrc)):
+    lines = open(os.path.join(csrc, name)).read().split("\n")
+    for i, line in enumerate(lines):
+      m = re.search(r"if \(lane == 0\) mbar_arrive\(smem_u32\(&(?:bars\.)?(\w*empty)\[", line)
+      if m and (name, m.group(1)) not in plain:
+        found += 1
+        assert any("fence_proxy_async_smem()" in x for x in lines[i - 4:i]), f"{name}:{i + 1}"
+        assert any("__syncwarp()" in x for x in lines[i - 3:i]), f"{name}:{i + 1}"
+  assert found >= 7

@@ -281,6 +281,37 @@ def test_scores_are_the_same_bits_on_every_call(ops, shape):
   no_timeouts(ops)
 
 
+@pytest.mark.parametrize("kind", ["block", "core", "sima", "sima_f32", "ea", "decode"])
+def test_streaming_kernels_give_the_same_bits_on_every_call(ops, kind):
+  # the same of the kernels whose warps read a ring's stages with ordinary loads, each with several rounds of
+  # its ring; SimA by three kernels and by the persistent one, over one round of units and over several
+  g = torch.Generator(device="cuda").manual_seed(2)
+
+  def normal(*shape, dtype=torch.float32):
+    return torch.randn(*shape, generator=g, device="cuda", dtype=dtype)
+
+  calls = []
+  if kind == "block":
+    args = (normal(16, 1500, 128), normal(384, 128) / 11, normal(384), normal(128, 128) / 11, normal(128))
+    calls = [lambda ea=ea: ops.linattn_block(*args, ea=ea) for ea in (False, True)]
+  elif kind == "core":
+    args = [normal(16, 1500, 4, 32) for _ in range(3)]
+    calls = [lambda ea=ea: ops.linattn32_fwd(*args, ea=ea) for ea in (False, True)]
+  elif kind == "decode":
+    q, k, v = (normal(4, s, h, 128, dtype=torch.bfloat16) for s, h in ((1, 32), (4001, 8), (4001, 8)))
+    calls = [lambda: ops.attn_fwd(q, k, v)]
+  else:
+    f = ops.ea_fwd if kind == "ea" else ops.sima_fwd
+    for shape, dtype in [((3, 1700, 16, 128), torch.float16), ((1, 5003, 32, 128), torch.bfloat16), ((2, 7001, 70, 128), torch.float16)]:
+      args = [normal(*shape, dtype=dtype) for _ in range(3)]
+      calls.append(lambda args=args: f(*args, **({"out_dtype": torch.float32} if kind == "sima_f32" else {})))
+  first = [f() for f in calls]
+  for _ in range(10):
+    for f, want in zip(calls, first):
+      assert all(torch.equal(x, y) for x, y in zip(f(), want))
+  no_timeouts(ops)
+
+
 @pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
 @pytest.mark.parametrize("shape", [(1, 128, 1), (2, 1000, 3), (1, 4096, 2), (1, 77, 2),
                                    # runs of tiles that cross from one unit into the next, once and several times
