@@ -301,10 +301,10 @@ def test_streaming_kernels_give_the_same_bits_on_every_call(ops, kind):
     q, k, v = (normal(4, s, h, 128, dtype=torch.bfloat16) for s, h in ((1, 32), (4001, 8), (4001, 8)))
     calls = [lambda: ops.attn_fwd(q, k, v)]
   else:
-    f = ops.ea_fwd if kind == "ea" else ops.sima_fwd
+    op = ops.ea_fwd if kind == "ea" else ops.sima_fwd
     for shape, dtype in [((3, 1700, 16, 128), torch.float16), ((1, 5003, 32, 128), torch.bfloat16), ((2, 7001, 70, 128), torch.float16)]:
       args = [normal(*shape, dtype=dtype) for _ in range(3)]
-      calls.append(lambda args=args: f(*args, **({"out_dtype": torch.float32} if kind == "sima_f32" else {})))
+      calls.append(lambda args=args: op(*args, **({"out_dtype": torch.float32} if kind == "sima_f32" else {})))
   first = [f() for f in calls]
   for _ in range(10):
     for f, want in zip(calls, first):
