@@ -167,6 +167,7 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_const
           ok = false;
           break;
         }
+        if (use > 0) fence_proxy_async_smem();  // (the consumers' reads, behind the wait above, before the copy)
         const uint32_t bar = smem_u32(&full[st]), dst = smem_base + st * kStageBytes;
         mbar_expect_tx(bar, kStageBytes);
         tma_load_4d(dst, &map_k, bar, 0, hk, t * kKeys, b);
@@ -284,7 +285,6 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_const
         mma16816<kBF16>(o[2 * d], pf, vf[0], vf[1]);
         mma16816<kBF16>(o[2 * d + 1], pf, vf[2], vf[3]);
       }
-      fence_proxy_async_smem();  // (the reads above before the copy that refills the stage)
       __syncwarp();
       if (lane == 0) mbar_arrive(smem_u32(&empty[st]));
     }

@@ -255,6 +255,7 @@ sima_stats_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
           record_timeout(p.status, 41);
           break;
         }
+        if (k >= kSt) fence_proxy_async_smem();  // (the consumers' reads, behind the wait above, before the copy)
         const uint32_t bar = smem_u32(&bars.full[st]);
         const uint32_t base = smem_base + st * kStageBytes;
         const int s0 = (t_lo + k - unit * p.share.ntiles) * kTile;
@@ -479,7 +480,6 @@ sima_stats_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
           const uint4 v = *reinterpret_cast<const uint4*>(tile + sw128_offset(row, chunk16 & 7));
           abs_acc8<kBF16>(v, acc);
         }
-        fence_proxy_async_smem();  // (the reads above before the copy that refills the stage)
         __syncwarp();
         if (lane == 0) mbar_arrive(smem_u32(&bars.empty[st]));
       }
@@ -1167,6 +1167,7 @@ sima_fused_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
             record_timeout(p.status, 61);
             break;
           }
+          if (k >= kSt) fence_proxy_async_smem();  // (the consumers' reads, behind the wait above, before the copy)
           const uint32_t bar = smem_u32(&bars.full[st]);
           const uint32_t base = smem_base + st * kStageBytes;
           const int s0 = tile0 * kTile + i * kRows1;
@@ -1188,6 +1189,7 @@ sima_fused_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
         }
         pre2 = 0;
         if (drained) {
+          fence_proxy_async_smem();  // (the consumers' reads, behind the wait above, before the copy)
           for (int i = 0; i < ntile && i < kQ; ++i, ++pre2) {
             const uint32_t k = n2 + i;
             const int st = k % kQ;
@@ -1247,7 +1249,6 @@ sima_fused_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
           const uint4 v = *reinterpret_cast<const uint4*>(tile + sw128_offset(row, chunk16 & 7));
           abs_acc8<kBF16>(v, acc);
         }
-        fence_proxy_async_smem();  // (the reads above before the copy that refills the stage)
         __syncwarp();
         if (lane == 0) mbar_arrive(smem_u32(&bars.empty[st]));
       }

@@ -401,17 +401,24 @@ def test_ctypes_structures_match_the_c_header(tmp_path):
 
 
 def test_stages_go_back_to_tma_behind_a_fence():
-  # A ring's consumers read a stage with ordinary loads; the copy that refills it is the async proxy's, which only
-  # a proxy fence in every reading lane holds back until those loads are done.  (Rings of ordinary stores need none.)
+  # A ring's consumers read a stage with ordinary loads; the copy that refills it is the async proxy's, and only a
+  # proxy fence on the way from one to the other orders them: in the consumers before they hand the stage back, or in
+  # the producer between its wait for them and the copy.  (Rings of ordinary stores need none.)
   plain = {("col_scores.cu", "lse_empty"), ("col_scores.cu", "q_empty")}  # row statistics; what else the stages hold the MMA reads
   csrc = os.path.join(ROOT, "flashtensor_b200", "csrc")
   found = 0
   for name in sorted(os.listdir(csrc)):
-    lines = open(os.path.join(csrc, name)).read().split("\n")
-    for i, line in enumerate(lines):
-      m = re.search(r"if \(lane == 0\) mbar_arrive\(smem_u32\(&(?:bars\.)?(\w*empty)\[", line)
-      if m and (name, m.group(1)) not in plain:
+    text = open(os.path.join(csrc, name)).read()
+    for kernel in text.split("__global__")[1:]:
+      for m in re.finditer(r"if \(lane == 0\) mbar_arrive\(smem_u32\(&((?:bars\.)?(\w*empty))\[", kernel):
+        if (name, m.group(2)) in plain:
+          continue
         found += 1
-        assert any("fence_proxy_async_smem()" in x for x in lines[i - 4:i]), f"{name}:{i + 1}"
-        assert any("__syncwarp()" in x for x in lines[i - 3:i]), f"{name}:{i + 1}"
-  assert found >= 7
+        before = "\n".join(kernel[:m.start()].split("\n")[-5:])
+        assert "__syncwarp()" in before, (name, m.group(1))
+        if "if constexpr" not in before and "fence_proxy_async_smem()" in before:
+          continue
+        waits = [w.end() for w in re.finditer(r"mbar_wait\(smem_u32\(&" + re.escape(m.group(1)) + r"\[", kernel)]
+        to_copy = [kernel[w:kernel.index("tma_load_4d", w)] for w in waits if "tma_load_4d" in kernel[w:]]
+        assert to_copy and all("fence_proxy_async_smem()" in x for x in to_copy), (name, m.group(1))
+  assert found >= 6
