@@ -373,7 +373,7 @@ PyObject* linattn_block(PyObject*, PyObject* const* a, Py_ssize_t n) {
     OnDevice on({&x, &w_qkv, &b_qkv, &w_o, &b_o});
     const int64_t B = x.size(0), N = x.size(1);
     const at::Tensor qkv = linear_f32(x.view({B * N, C}), w_qkv, b_qkv, on.stream);
-    const at::Tensor out = empty({B, N, C}, at::kFloat, x), scratch = empty({B, C, C}, at::kFloat, x);
+    const at::Tensor out = empty({B, N, C}, at::kFloat, x), scratch = empty({B, C + 1, C}, at::kFloat, x);
     asuka_linattn32_proj_params p;
     p.q = desc(qkv);  // [B, N, C / 32, 32], strided over the fused rows
     p.q.ndim = 4;

@@ -786,7 +786,8 @@ int asuka_b200_linattn32_proj(const asuka_linattn32_proj_params* p, asuka_stream
   if (p->q.stride[2] != 32) return ASUKA_ERR_BAD_STRIDE;
   const int64_t B = a.B, N = a.N, C = static_cast<int64_t>(a.H) * 32;
   if (C > ASUKA_LINEAR_MAX_K || B * N > 0x3fffffff) return ASUKA_ERR_TOO_LARGE;
-  const int64_t ws[2] = {C, C}, bs[1] = {C}, os[3] = {B, N, C}, ss[3] = {B, C, C};
+  const int64_t fold_rows = p->scratch.ndim == 3 && p->scratch.shape[1] == C + 1 ? C + 1 : C;
+  const int64_t ws[2] = {C, C}, bs[1] = {C}, os[3] = {B, N, C}, ss[3] = {B, fold_rows, C};
   if ((r = check_dense(p->w, ASUKA_F32, 2, ws)) != ASUKA_OK) return r;
   if ((r = check_dense(p->bias, ASUKA_F32, 1, bs)) != ASUKA_OK) return r;
   if ((r = check_dense(p->out, ASUKA_F32, 3, os)) != ASUKA_OK) return r;
@@ -796,7 +797,8 @@ int asuka_b200_linattn32_proj(const asuka_linattn32_proj_params* p, asuka_stream
   if (sms <= 0) return ASUKA_ERR_CUDA;
   a.out = static_cast<float*>(p->out.ptr);
   return map_cuda(launch_linattn32_proj(a, static_cast<const float*>(p->w.ptr), static_cast<const float*>(p->bias.ptr),
-                                        static_cast<float*>(p->scratch.ptr), sms, static_cast<cudaStream_t>(stream)));
+                                        static_cast<float*>(p->scratch.ptr), static_cast<int>(fold_rows), sms,
+                                        static_cast<cudaStream_t>(stream)));
 }
 
 int asuka_b200_linear_f32(const asuka_linear_params* p, asuka_stream stream) {

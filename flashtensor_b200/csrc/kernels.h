@@ -165,16 +165,30 @@ struct LinAttn32Args {
 };
 cudaError_t launch_linattn32(const LinAttn32Args& a, cudaStream_t stream);
 // ... followed by out[B, N, C] = core w_o[C, C]^T + b_o, C = 32 H <= 128; the heads of q side by side, out dense, w_fold
-// [B, C, C] is scratch (16-byte aligned)
-cudaError_t launch_linattn32_proj(const LinAttn32Args& a, const float* w_o, const float* b_o, float* w_fold, int num_sms,
-                                  cudaStream_t stream);
+// [B, C or C + 1, C] is scratch (16-byte aligned)
+cudaError_t launch_linattn32_proj(const LinAttn32Args& a, const float* w_o, const float* b_o, float* w_fold, int fold_rows,
+                                  int num_sms, cudaStream_t stream);
 
 // out[M, N] = x[M, K] w[N, K]^T + bias[N], contiguous f32, K a multiple of 8 and at most 128
 cudaError_t launch_linear_f32(const float* x, const float* w, const float* bias, float* out, int M, int N, int K,
                               int num_sms, cudaStream_t stream);
-// out[B, M, N] = x[B, M, K] w[B, N, K]^T + bias[N], N and K at most 128; softmax: of every 32 values of x first
-cudaError_t launch_linear_f32_batched(const float* x, int64_t x_sb, int64_t x_sn, const float* w, const float* bias, float* out,
-                                      int B, int M, int N, int K, bool softmax, int num_sms, cudaStream_t stream);
+// How launch_linear_f32_batched cuts M rows of each of B batches.
+struct BatchSplit {
+  int splits, rows;  // CTAs per batch, and the rows of each, a multiple of 32
+};
+BatchSplit linear_f32_split(int B, int M, int num_sms);
+// The exponents of the scales of folded weights (f32_keep.cuh): a row of C words to a batch, or to each CTA of its
+// projection, a byte to a column, the heads one behind the other.  A CTA's may be the first row of `out` that it writes.
+struct FoldScales {
+  uint32_t* ptr;
+  int64_t per_batch, per_cta;  // strides in words
+};
+// out[B, M, N] = x[B, M, K] w[B, N, K]^T + bias[N], N and K at most 128, w (w_rows >= N rows to a batch) as
+// launch_linattn32_proj's first kernel leaves it;
+// softmax: of every 32 values of x first
+cudaError_t launch_linear_f32_batched(const float* x, int64_t x_sb, int64_t x_sn, const float* w, int w_rows, const float* bias, float* out,
+                                      int B, int M, int N, int K, bool softmax, const BatchSplit& split, const FoldScales& scales,
+                                      cudaStream_t stream);
 
 struct SimaShape {
   int B, H, S;

@@ -23,6 +23,7 @@
 // In a whole block (kFold) there is no pass B: the kernel multiplies the 32 x 32 matrices with the output
 // projection, and linear_f32.cu applies the product to the queries (this kernel 23 us then; the block, SimA / EA,
 // 82 / 91.5 -> 70 / 77 us with it and the projections' earlier start).
+#include "f32_keep.cuh"
 #include "kernels.h"
 #include "sm100_ptx.cuh"
 #include "tma_host.h"
@@ -42,13 +43,17 @@ constexpr int kStages = 4;                   // pass A: K, V, Q tiles
 constexpr int kQStages = 8;                  // pass B: Q tiles, in the part of the ring above the partial products
 constexpr uint32_t kPartBytes = kWarps * kD * kD * 4;
 constexpr uint32_t kSmemBytes = kStages * 3 * kTileBytes + 1024;
+constexpr int kFoldLoads = 4;                // (kFold) 16-byte pieces of a thread of a head's 128 columns at most
 constexpr float kSlack = 5.5f;               // EA: by how much a key may exceed its warp's reference (e^5.5 = 2^8)
 static_assert(kPartBytes + kQStages * kTileBytes <= kStages * 3 * kTileBytes, "pass B's ring");
 
 struct Lin32Params {
   int N, H;
   const float* w_o;  // (kFold) output projection [32 H, 32 H], and where its product with every batch's M' goes
-  float* w_fold;     // [B, 32 H, 32 H]
+  float* w_fold;     // [B, fold_rows, 32 H], 32 H rows of it
+  int fold_rows;
+  FoldScales scales;
+  int scale_copies;  // of a batch's words
   uint32_t* status;
 };
 
@@ -90,6 +95,7 @@ linattn32_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
   __shared__ float m_s[kD][kD + 1];                 // M' = normalised K'^T V, [d][e]
   __shared__ __align__(16) float scale_s[kWarps][kD];  // EA: rescale factors of a warp's partial product
   __shared__ float stat_s[2][kWarps][kD];           // SimA: sum|K|, sum|Q|; EA: reference, sum of K'
+  __shared__ __align__(4) uint8_t e_s[4 * kD];      // (kFold) exponents of this head's scales (f32_keep.cuh), by column
   __shared__ uint32_t abort_s;
   const uint32_t ring = (smem_u32(smem_raw) + 1023u) & ~1023u;
   float* const ring_gen = reinterpret_cast<float*>(smem_raw + (ring - smem_u32(smem_raw)));
@@ -132,6 +138,7 @@ linattn32_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
           record_timeout(p.status, 91);
           break;
         }
+        if (t >= kStages) fence_proxy_async_smem();  // (the consumers' reads, behind the wait above, before the copy)
         const uint32_t bar = smem_u32(&bars.a_full[st]), dst = ring + st * 3 * kTileBytes;
         mbar_expect_tx(bar, (kEA ? 2 : 3) * kTileBytes);
         tma_load_4d(dst, &map_k, bar, 0, h, t * kRows, b);
@@ -210,25 +217,40 @@ linattn32_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
 #pragma unroll
           for (int d = 0; d < 4; ++d) acc[e][d] = __ffma2_rn(kk[d], make_float2(ve[e], ve[e]), acc[e][d]);
       }
-      fence_proxy_async_smem();  // (the reads above, and EA's K' over the tile, before the copy that refills the stage)
+      if constexpr (kEA) fence_proxy_async_smem();  // (K' was written over a tile that TMA refills)
       __syncwarp();
       if (lane == 0) mbar_arrive(smem_u32(&bars.a_empty[st]));
     }
     stat_s[0][warp][lane] = s0;
     stat_s[1][warp][lane] = s1;
   }
+  const int C = p.H * kD;
+  float4 o[kFold ? kFoldLoads : 1];  // (kFold) this thread's part of the output projection, on its way during the barrier
+  if constexpr (kFold) {
+#pragma unroll
+    for (int x = 0; x < kFoldLoads; ++x) {
+      const int i = x * kWarps * 32 + tid, c = i >> 3;
+      if (warp < kWarps && c < C) o[x] = __ldg(reinterpret_cast<const float4*>(p.w_o + c * C + h * kD) + (i & 7));
+    }
+  }
   __syncthreads();
 
   // ---- the warps' partial products to M', in warp order, while the first tiles of pass B arrive
   float* const part = ring_gen;
   float* const w_s = ring_gen + kPartBytes / 4;  // (kFold) this head's columns of the output projection, [c][e]
-  const int C = p.H * kD;
   const uint32_t qring = ring + kPartBytes;
   if (warp < kWarps) {
     if constexpr (kFold) {  // (the ring is free: nothing is in flight after pass A)
-      for (int i = tid; i < C * (kD / 4); i += kWarps * 32)
-        *reinterpret_cast<float4*>(w_s + i * 4) =
-            __ldg(reinterpret_cast<const float4*>(p.w_o + static_cast<int64_t>(i >> 3) * C + h * kD) + (i & 7));
+#pragma unroll
+      for (int x = 0; x < kFoldLoads; ++x) {
+        const int i = x * kWarps * 32 + tid, c = i >> 3;
+        if (c < C) {  // (whole warps: C is a multiple of 32)
+          const uint32_t e = fold_scale_exponent(head_max_bits(o[x]));
+          const float s = __uint_as_float(e << 23);
+          *reinterpret_cast<float4*>(w_s + i * 4) = make_float4(mul_keep(o[x].x, s), mul_keep(o[x].y, s), mul_keep(o[x].z, s), mul_keep(o[x].w, s));
+          if ((i & 7) == 0) e_s[c] = static_cast<uint8_t>(e);
+        }
+      }
     }
 #pragma unroll
     for (int d = 0; d < 4; ++d) {
@@ -267,21 +289,29 @@ linattn32_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
   }
 
   if constexpr (kFold) {
+    if (warp == 0 && lane * 4 < C) {
+      const uint32_t e4 = *reinterpret_cast<const uint32_t*>(&e_s[lane * 4]);
+      uint32_t* dst = p.scales.ptr + b * p.scales.per_batch + h * (C / 4) + lane;
+      for (int y = 0; y < p.scale_copies; ++y) dst[y * p.scales.per_cta] = e4;
+    }
     // ---- out = Qn . blockdiag(M') . w_o^T + b_o: what is left of it after this kernel is one product of the
-    // (EA: normalised) queries with w_fold[b][c][h * 32 + d] = sum_e M'[d][e] w_o[c][h * 32 + e]
+    // (EA: normalised) queries with w_fold[b][c][h * 32 + d] = sum_e M'[d][e] w_o[c][h * 32 + e], times the scale of
+    // (c, h) (f32_keep.cuh)
     if (warp < kWarps) {
       float m[kD];
 #pragma unroll
       for (int e = 0; e < kD; ++e) m[e] = m_s[lane][e];
-      float* dst = p.w_fold + static_cast<int64_t>(b) * C * C + h * kD + lane;
+      float* dst = p.w_fold + static_cast<int64_t>(b) * p.fold_rows * C + h * kD + lane;
       for (int c = warp; c < C; c += kWarps) {
         float sum[kD / 4];  // (in pairs: one running sum of thirty-two rounds more)
 #pragma unroll
         for (int i = 0; i < kD / 4; ++i) {
           const float4 o = *reinterpret_cast<const float4*>(w_s + c * kD + i * 4);
-          sum[i] = fmaf(m[4 * i], o.x, m[4 * i + 1] * o.y) + fmaf(m[4 * i + 2], o.z, m[4 * i + 3] * o.w);
+          sum[i] = add_keep(fma_keep(m[4 * i], o.x, mul_keep(m[4 * i + 1], o.y)),
+                            fma_keep(m[4 * i + 2], o.z, mul_keep(m[4 * i + 3], o.w)));
         }
-        dst[static_cast<int64_t>(c) * C] = ((sum[0] + sum[1]) + (sum[2] + sum[3])) + ((sum[4] + sum[5]) + (sum[6] + sum[7]));
+        dst[static_cast<int64_t>(c) * C] = add_keep(add_keep(add_keep(sum[0], sum[1]), add_keep(sum[2], sum[3])),
+                                                    add_keep(add_keep(sum[4], sum[5]), add_keep(sum[6], sum[7])));
       }
     }
     return;
@@ -374,12 +404,11 @@ linattn32_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
 
 }  // namespace
 
-static cudaError_t launch(const LinAttn32Args& a, const float* w_o, float* w_fold, cudaStream_t stream) {
-  Lin32Params p;
+static cudaError_t launch(const LinAttn32Args& a, const Lin32Params& fold, cudaStream_t stream) {
+  const float* const w_o = fold.w_o;
+  Lin32Params p = fold;
   p.N = a.N;
   p.H = a.H;
-  p.w_o = w_o;
-  p.w_fold = w_fold;
   p.status = device_status_words();
   const uint64_t dims[4] = {kD, static_cast<uint64_t>(a.H), static_cast<uint64_t>(a.N), static_cast<uint64_t>(a.B)};
   auto map = [&](CUtensorMap* m, const float* base, int64_t sh, int64_t sn, int64_t sb, uint32_t rows) {
@@ -405,13 +434,26 @@ static cudaError_t launch(const LinAttn32Args& a, const float* w_o, float* w_fol
   return e;
 }
 
-cudaError_t launch_linattn32(const LinAttn32Args& a, cudaStream_t stream) { return launch(a, nullptr, nullptr, stream); }
+cudaError_t launch_linattn32(const LinAttn32Args& a, cudaStream_t stream) { return launch(a, {}, stream); }
 
-cudaError_t launch_linattn32_proj(const LinAttn32Args& a, const float* w_o, const float* b_o, float* w_fold, int num_sms,
-                                  cudaStream_t stream) {
-  const cudaError_t e = launch(a, w_o, w_fold, stream);
+cudaError_t launch_linattn32_proj(const LinAttn32Args& a, const float* w_o, const float* b_o, float* w_fold, int fold_rows,
+                                  int num_sms, cudaStream_t stream) {
+  const int C = a.H * kD;
+  const BatchSplit split = linear_f32_split(a.B, a.N, num_sms);
+  Lin32Params fold = {};
+  fold.w_o = w_o;
+  fold.w_fold = w_fold;
+  fold.fold_rows = fold_rows;
+  if (fold_rows > C) {  // room for the scales behind the folded weights
+    fold.scales = {reinterpret_cast<uint32_t*>(w_fold) + static_cast<int64_t>(C) * C, static_cast<int64_t>(fold_rows) * C, 0};
+    fold.scale_copies = 1;
+  } else {  // in the first row of the output that each CTA of the projection writes, before it does
+    fold.scales = {reinterpret_cast<uint32_t*>(a.out), static_cast<int64_t>(a.N) * C, static_cast<int64_t>(split.rows) * C};
+    fold.scale_copies = split.splits;
+  }
+  const cudaError_t e = launch(a, fold, stream);
   if (e != cudaSuccess) return e;
-  return launch_linear_f32_batched(a.q, a.q_sb, a.q_sn, w_fold, b_o, a.out, a.B, a.N, a.H * kD, a.H * kD, a.ea != 0, num_sms, stream);
+  return launch_linear_f32_batched(a.q, a.q_sb, a.q_sn, w_fold, fold_rows, b_o, a.out, a.B, a.N, C, C, a.ea != 0, split, fold.scales, stream);
 }
 
 }  // namespace asuka

@@ -26,7 +26,9 @@
 // finite.  Terms and products below 2^-126 are flushed: with weights below 2^20 that costs a sum 2^-98 at most,
 // which is below the rounding of one of 2^-72 or more.  So a sum that is not finite or below 2^-72, and a
 // column with a weight outside [2^-100, 2^20) that is not zero, is computed on the CUDA cores (plain_dot) by
-// the warps that store it; which way a result takes depends on its own row and column.  That is for the odd row
+// the warps that store it; which way a result takes depends on its own row and column.  (Folded weights hold the values
+// of a batch, which may be large: there the bounds are 2^100 and, as both of the above grow with the weights, 2^-92
+// of the column's largest for the sum.)  That is for the odd row
 // or column: all rows at 1e-25 take 1460 us instead of 34, rows of nothing but zeros, which need a look at x only, 91.
 // Measured at B64 N784 C128 (M = 50176, K = 128), calls back to back, bias included: N = 384 (QKV) 32 us,
 // N = 128 (output) 14.6 us; the f32 GEMM of the BLAS library with its bias pass takes 200 and 64.  A launch is set-up
@@ -35,6 +37,7 @@
 // splitting warps share is the way to shared memory), and so are plain stores instead of TMA's.
 #include <cuda_bf16.h>
 
+#include "f32_keep.cuh"
 #include "kernels.h"
 #include "sm100_ptx.cuh"
 #include "tma_host.h"
@@ -70,25 +73,18 @@ struct LinParams {
   float* out;
   int M, N, K;           // M: rows of a batch
   int64_t x_sn, x_sb;    // strides of x between rows and between batches
+  int64_t w_sb;          // ... and of w between batches
   int n_tiles, chunks;
   int splits, cta_rows;  // (batched) CTAs per batch, and the rows of each, a multiple of 32
+  FoldScales scales;     // (batched)
   int tma_out;  // rows of `out` can be described to TMA (N a multiple of 4)
   uint32_t* status;
 };
 
-constexpr float kWeightLow = 7.8886090522101181e-31f, kWeightHigh = 1048576.f;  // 2^-100, 2^20
+constexpr float kWeightLow = 7.8886090522101181e-31f;                            // 2^-100
 constexpr float kSumLow = 2.1175823681357508e-22f;                               // 2^-72
-// (these keep subnormal values, which the build's flags flush elsewhere)
-__device__ __forceinline__ float fma_keep(float a, float b, float c) {
-  float y;
-  asm("fma.rn.f32 %0, %1, %2, %3;" : "=f"(y) : "f"(a), "f"(b), "f"(c));
-  return y;
-}
-__device__ __forceinline__ float add_keep(float a, float b) {
-  float y;
-  asm("add.rn.f32 %0, %1, %2;" : "=f"(y) : "f"(a), "f"(b));
-  return y;
-}
+constexpr float kSumPerWeight = 2.0194839173657902e-28f;                         // 2^-92 (folded weights)
+template <int kMode> constexpr float kWeightHighOf = kMode == kPlain ? 1048576.f : 1.2676506002282294e30f;  // 2^20, 2^100
 __device__ __forceinline__ float max3_nan(float a, float b, float c) {
   float y;
   asm("max.NaN.f32 %0, %1, %2, %3;" : "=f"(y) : "f"(a), "f"(b), "f"(c));
@@ -134,15 +130,19 @@ __device__ __forceinline__ void softmax_group(float (&v)[kN]) {
   for (int i = 0; i < kN; ++i) v[i] *= inv;
 }
 
+// a factor of powers of two, kept as the upper half of its bits
+__device__ __forceinline__ float rescale(uint16_t upper) { return __uint_as_float(static_cast<uint32_t>(upper) << 16); }
+
 // One row of x against the 32 columns from n_base on, by a whole warp: lane l takes reduction columns 4l to
-// 4l + 3 and returns the sum for output column n_base + l.
-template <bool kSoft>
-__device__ __noinline__ float plain_dot(const float* __restrict__ x_row, const float* __restrict__ w, int n_base, int N, int K) {
+// 4l + 3 and returns the sum for output column n_base + l.  (Batched: `rescale_rows` holds the factors of these columns.)
+template <int kMode>
+__device__ __noinline__ float plain_dot(const float* __restrict__ x_row, const float* __restrict__ w, const uint16_t (*rescale_rows)[4],
+                                        int n_base, int N, int K) {
   const int lane = threadIdx.x & 31;
   const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
   const bool live = lane * 4 < K;
   float4 xv = live ? __ldg(reinterpret_cast<const float4*>(x_row) + lane) : zero;
-  if constexpr (kSoft) {
+  if constexpr (kMode == kSoftmax) {
     float v[4] = {xv.x, xv.y, xv.z, xv.w};
     softmax_group<8>(v);
     xv = live ? make_float4(v[0], v[1], v[2], v[3]) : zero;
@@ -150,7 +150,11 @@ __device__ __noinline__ float plain_dot(const float* __restrict__ x_row, const f
   float part[32];
 #pragma unroll
   for (int c = 0; c < 32; ++c) {
-    const float4 wv = live ? __ldg(reinterpret_cast<const float4*>(w + static_cast<int64_t>(min(n_base + c, N - 1)) * K) + lane) : zero;
+    float4 wv = live ? __ldg(reinterpret_cast<const float4*>(w + static_cast<int64_t>(min(n_base + c, N - 1)) * K) + lane) : zero;
+    if constexpr (kMode != kPlain) {
+      const float f = rescale(rescale_rows[c][lane >> 3]);
+      wv = make_float4(mul_keep(wv.x, f), mul_keep(wv.y, f), mul_keep(wv.z, f), mul_keep(wv.w, f));
+    }
     part[c] = fma_keep(xv.x, wv.x, fma_keep(xv.y, wv.y, fma_keep(xv.z, wv.z, fma_keep(xv.w, wv.w, 0.f))));
   }
   // every exchange adds two lanes' sums and halves the columns a lane still holds
@@ -219,8 +223,10 @@ __device__ __forceinline__ void record_timeout(uint32_t* status, uint32_t site) 
 
 template <int kMode>
 __global__ void __launch_bounds__(kThreads, 1) linear_f32_kernel(const __grid_constant__ CUtensorMap map_out, const LinParams p) {
+  constexpr float kWeightHigh = kWeightHighOf<kMode>;
   extern __shared__ uint8_t smem_raw[];
   __shared__ __align__(8) LinBars bars;
+  __shared__ __align__(8) uint16_t rescale_s[kMode == kPlain ? 1 : kTile][4];  // (batched) by column: factors of its heads' weights
   __shared__ uint32_t tmem_base_s;
   __shared__ uint32_t abort_s;
   const uint32_t sX = (smem_u32(smem_raw) + 1023u) & ~1023u;
@@ -244,7 +250,7 @@ __global__ void __launch_bounds__(kThreads, 1) linear_f32_kernel(const __grid_co
   }
   const int n0 = nb * kTile;
   const float* const x = p.x + batch * p.x_sb;
-  const float* const w = p.w + static_cast<int64_t>(batch) * p.N * p.K;
+  const float* const w = p.w + batch * p.w_sb;
 
   if (tid == 0) {
     abort_s = 0;
@@ -269,6 +275,7 @@ __global__ void __launch_bounds__(kThreads, 1) linear_f32_kernel(const __grid_co
   const uint32_t lane_base = static_cast<uint32_t>(wq * 32) << 16;
   const int n = n0 + wq * 32 + lane;  // (epilogue warps) this thread's output column
   float w_big = 0.f, w_small = kWeightHigh;  // (epilogue warps) of that column's weights, the zeros apart
+  uint32_t least = 127u;                     // (batched, epilogue warps) exponent of the scale of that column's weights
   // (batched: the kernel ahead, which writes the weights, reads x itself and has waited for whatever wrote it before
   // this one could start: the splitting warps need not wait; EA block 79.7 -> 76.8 us)
   if (kMode == kPlain || warp >= kSplitWarps) griddep_wait();
@@ -276,15 +283,41 @@ __global__ void __launch_bounds__(kThreads, 1) linear_f32_kernel(const __grid_co
   if (warp > kSplitWarps) {
     // the weights of this block of columns, split once: thread = output column = TMEM lane
     const float* src = w + static_cast<int64_t>(min(n, p.N - 1)) * p.K;
+    uint32_t e4 = 0;
+    if (kMode != kPlain && n < p.N) {  // the scales that the column's weights were folded with
+      const uint8_t* e = reinterpret_cast<const uint8_t*>(p.scales.ptr + batch * p.scales.per_batch + static_cast<int>(blockIdx.x) % p.splits * p.scales.per_cta) + n;
+#pragma unroll
+      for (int h = 0; h < 4; ++h)
+        if (h * 32 < p.K) e4 |= static_cast<uint32_t>(__ldcg(e + h * p.K)) << (8 * h);
+    }
+    float4 next[8];  // the next 32 weights
+    auto load = [&](int k0) {
+#pragma unroll
+      for (int i = 0; i < 8; ++i)  // (K is a multiple of 8)
+        next[i] = n < p.N && k0 + i * 4 < p.K ? __ldg(reinterpret_cast<const float4*>(src + k0) + i) : make_float4(0.f, 0.f, 0.f, 0.f);
+    };
+    load(0);
+    if constexpr (kMode != kPlain) {
+      least = 255u;  // all are brought to the scale of the largest
+      for (int h = 0; h * 32 < p.K; ++h) least = min(least, (e4 >> (8 * h)) & 255u);
+#pragma unroll
+      for (int h = 0; h < 4; ++h) {  // 2^-d, subnormal below 2^-126, not less than 2^-133
+        const uint32_t d = max((e4 >> (8 * h)) & 255u, least) - least;
+        rescale_s[wq * 32 + lane][h] = static_cast<uint16_t>(d < 127u ? (127u - d) << 7 : 1u << (133u - min(d, 133u)));
+      }
+    }
     for (int k0 = 0; k0 < p.chunks * kChunk; k0 += 32) {
       uint32_t t[3][16];
+      const float f = kMode == kPlain ? 1.f : rescale(rescale_s[kMode == kPlain ? 0 : wq * 32 + lane][k0 >> 5]);
 #pragma unroll
       for (int g = 0; g < 4; ++g) {
         const int k = k0 + g * 8;
-        const bool live = n < p.N && k < p.K;  // (K is a multiple of 8)
-        const float4 lo = live ? __ldg(reinterpret_cast<const float4*>(src + k)) : make_float4(0.f, 0.f, 0.f, 0.f);
-        const float4 hi = live ? __ldg(reinterpret_cast<const float4*>(src + k + 4)) : make_float4(0.f, 0.f, 0.f, 0.f);
-        const float v[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
+        const float4 lo = next[2 * g], hi = next[2 * g + 1];
+        float v[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
+        if constexpr (kMode != kPlain) {
+#pragma unroll
+          for (int i = 0; i < 8; ++i) v[i] = mul_keep(v[i], f);
+        }
         float big, small;
         extent8(v, &big, &small);
         w_big = max3_nan(w_big, big, big);
@@ -299,6 +332,7 @@ __global__ void __launch_bounds__(kThreads, 1) linear_f32_kernel(const __grid_co
           t[s][g * 4 + 3] = q[s].w;
         }
       }
+      load(k0 + 32);
 #pragma unroll
       for (int s = 0; s < 3; ++s) tmem_st16(tbase + lane_base + s * kTermCols + k0 / 2, t[s]);
     }
@@ -307,7 +341,8 @@ __global__ void __launch_bounds__(kThreads, 1) linear_f32_kernel(const __grid_co
       w_small = kWeightHigh;
       if (n < p.N)
         for (int k = 0; k < p.K; ++k) {
-          const float a = __ldg(src + k);
+          float a = __ldg(src + k);
+          if constexpr (kMode != kPlain) a = mul_keep(a, rescale(rescale_s[wq * 32 + lane][k >> 5]));
           if ((__float_as_uint(a) << 1) != 0u) w_small = fminf(w_small, fabsf(a));  // (a subnormal counts as 0)
         }
     }
@@ -405,8 +440,12 @@ __global__ void __launch_bounds__(kThreads, 1) linear_f32_kernel(const __grid_co
   } else {
     // ------------------------------------------------------------------ epilogue
     uint8_t* const stage = gX + 2 * kStageBytes + wq * 2 * kOutBytes;
+    if (kMode != kPlain && p.scales.per_cta != 0) fence_proxy_async_global();  // (they lay in what this warp now stores by TMA)
     const float bias = n < p.N ? __ldg(p.bias + n) : 0.f;
     float* const out = p.out + static_cast<int64_t>(batch) * p.M * p.N;
+    const float sum_low = kMode == kPlain ? kSumLow : fmaxf(kSumLow, w_big * kSumPerWeight);
+    const float unscale = kMode == kPlain ? 1.f : __uint_as_float((254u - least) << 23);
+    auto result = [&](float sum) { return kMode == kPlain ? add_keep(sum, bias) : fma_keep(sum, unscale, bias); };
     const bool zero_col = w_big == 0.f;  // a sum of zero is right (with a subnormal weight it is a plain one)
     const bool plain_col = !(w_big < kWeightHigh) || w_small < kWeightLow;
     const bool any_plain_col = __any_sync(0xffffffffu, plain_col);
@@ -430,7 +469,7 @@ __global__ void __launch_bounds__(kThreads, 1) linear_f32_kernel(const __grid_co
         tmem_wait_ld();
         if (row_t + q * 32 + 32 > row_end) {  // (rows past the end, zero as well, are not stored)
 #pragma unroll
-          for (int r = 0; r < 32; ++r) u[r] = row_t + q * 32 + r < row_end ? u[r] : 0x3f800000u;
+          for (int r = 0; r < 32; ++r) u[r] = row_t + q * 32 + r < row_end ? u[r] : __float_as_uint(kWeightHigh);
         }
 #pragma unroll
         for (int g = 0; g < 4; ++g) {
@@ -440,7 +479,7 @@ __global__ void __launch_bounds__(kThreads, 1) linear_f32_kernel(const __grid_co
           small = fminf(small, s8);
         }
         if (q == 3) {
-          again = __any_sync(0xffffffffu, !(big < INFINITY) || (small < kSumLow && !zero_col)) || again;
+          again = __any_sync(0xffffffffu, !(big < INFINITY) || (small < sum_low && !zero_col)) || again;
           if (!again) {
             tc_fence_before_sync();
             mbar_arrive(smem_u32(&bars.acc_empty[st]));
@@ -448,7 +487,7 @@ __global__ void __launch_bounds__(kThreads, 1) linear_f32_kernel(const __grid_co
         }
 #pragma unroll
         for (int r = 0; r < 32; ++r)
-          *reinterpret_cast<float*>(dst + sw128_offset(r, lane >> 2) + (lane & 3) * 4) = add_keep(__uint_as_float(u[r]), bias);
+          *reinterpret_cast<float*>(dst + sw128_offset(r, lane >> 2) + (lane & 3) * 4) = result(__uint_as_float(u[r]));
         const int row_q = row_t + q * 32;
         if (p.tma_out) {
           fence_proxy_async_smem();
@@ -477,7 +516,7 @@ __global__ void __launch_bounds__(kThreads, 1) linear_f32_kernel(const __grid_co
 #pragma unroll
           for (int r = 0; r < 32; ++r) {
             const float a = fabsf(__uint_as_float(u[r]));
-            if (!(a < INFINITY) || (a < kSumLow && !zero_col)) mine |= 1u << r;
+            if (!(a < INFINITY) || (a < sum_low && !zero_col)) mine |= 1u << r;
           }
           if (plain_col) mine = 0xffffffffu;
           uint32_t left = __reduce_or_sync(0xffffffffu, mine);
@@ -485,8 +524,8 @@ __global__ void __launch_bounds__(kThreads, 1) linear_f32_kernel(const __grid_co
           for (; left != 0u; left &= left - 1u) {
             const int r = __ffs(left) - 1;
             if (row_q + r >= row_end) break;
-            const float y = plain_dot<kMode == kSoftmax>(x + (row_q + r) * p.x_sn, w, n0 + wq * 32, p.N, p.K);
-            if (((mine >> r) & 1u) != 0u && n < p.N) out[static_cast<int64_t>(row_q + r) * p.N + n] = add_keep(y, bias);
+            const float y = plain_dot<kMode>(x + (row_q + r) * p.x_sn, w, rescale_s + (kMode == kPlain ? 0 : wq * 32), n0 + wq * 32, p.N, p.K);
+            if (((mine >> r) & 1u) != 0u && n < p.N) out[static_cast<int64_t>(row_q + r) * p.N + n] = result(y);
           }
         }
         tc_fence_before_sync();
@@ -543,8 +582,27 @@ cudaError_t launch_linear_f32(const float* x, const float* w, const float* bias,
   return launch(p, kPlain, 1, static_cast<unsigned>(tiles < most ? tiles : most), stream);
 }
 
-cudaError_t launch_linear_f32_batched(const float* x, int64_t x_sb, int64_t x_sn, const float* w, const float* bias, float* out,
-                                      int B, int M, int N, int K, bool softmax, int num_sms, cudaStream_t stream) {
+BatchSplit linear_f32_split(int B, int M, int num_sms) {
+  // the split with the shortest launch, in rows of work per SM; a CTA's set-up (launch, weights to TMEM, first
+  // tile) takes about as long as 160 rows
+  BatchSplit out = {};
+  const int pieces = (M + 31) / 32;
+  int64_t best = 0;
+  for (int s = 1; s <= pieces && s <= num_sms; ++s) {
+    const int rows = (pieces + s - 1) / s * 32, splits = (M + rows - 1) / rows;
+    const int64_t cost = (static_cast<int64_t>(B) * splits + num_sms - 1) / num_sms * (rows + 160);
+    if (out.splits == 0 || cost < best) {
+      best = cost;
+      out.rows = rows;
+      out.splits = splits;
+    }
+  }
+  return out;
+}
+
+cudaError_t launch_linear_f32_batched(const float* x, int64_t x_sb, int64_t x_sn, const float* w, int w_rows, const float* bias, float* out,
+                                      int B, int M, int N, int K, bool softmax, const BatchSplit& split, const FoldScales& scales,
+                                      cudaStream_t stream) {
   LinParams p = {};
   p.x = x;
   p.w = w;
@@ -555,20 +613,11 @@ cudaError_t launch_linear_f32_batched(const float* x, int64_t x_sb, int64_t x_sn
   p.K = K;
   p.x_sn = x_sn;
   p.x_sb = x_sb;
+  p.w_sb = static_cast<int64_t>(w_rows) * K;
   p.n_tiles = 1;
-  // CTAs per batch: the split with the shortest launch, in rows of work per SM; a CTA's set-up (launch, weights
-  // to TMEM, first tile) takes about as long as 160 rows
-  const int pieces = (M + 31) / 32;
-  int64_t best = 0;
-  for (int s = 1; s <= pieces && s <= num_sms; ++s) {
-    const int rows = (pieces + s - 1) / s * 32, splits = (M + rows - 1) / rows;
-    const int64_t cost = (static_cast<int64_t>(B) * splits + num_sms - 1) / num_sms * (rows + 160);
-    if (p.splits == 0 || cost < best) {
-      best = cost;
-      p.cta_rows = rows;
-      p.splits = splits;
-    }
-  }
+  p.splits = split.splits;
+  p.cta_rows = split.rows;
+  p.scales = scales;
   return launch(p, softmax ? kSoftmax : kBatched, B, static_cast<unsigned>(B) * p.splits, stream);
 }
 

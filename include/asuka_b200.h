@@ -230,7 +230,7 @@ typedef struct {
   asuka_tensor q, k, v;  /* as asuka_linattn32_params; the heads of q side by side (stride[2] = 32) */
   asuka_tensor w, bias;  /* [C, C], [C] f32, contiguous */
   asuka_tensor out;      /* [B, N, C] f32, contiguous */
-  asuka_tensor scratch;  /* [B, C, C] f32, contiguous */
+  asuka_tensor scratch;  /* [B, C, C] or (somewhat faster) [B, C + 1, C] f32, contiguous */
   int32_t ea;
 } asuka_linattn32_proj_params;
 int asuka_b200_linattn32_proj(const asuka_linattn32_proj_params* p, asuka_stream stream);

@@ -571,17 +571,68 @@ def test_block_batches_keep_to_themselves(ops, ea):
   odd[4] = 0.0
   w_odd = w_o.clone()
   w_odd[9] *= 1e30
+  w_odd[20] *= 1e-30
   w_odd[33] *= 1e-34
+  b_o[[9, 20, 33]] = 0.0  # (the bound below is of the product alone)
   got = ops.linattn_block(*(t.cuda() for t in (odd, w_qkv, b_qkv, w_odd, b_o)), ea=ea).cpu()
-  keep = [c for c in range(C) if c not in (9, 33)]
+  keep = [c for c in range(C) if c not in (9, 20, 33)]
   for b in (0, 2, 5):
     assert torch.equal(got[b][:, keep], clean[b][:, keep])
   want = block_float64(odd, w_qkv, b_qkv, w_odd, b_o, ea)
   assert torch.equal(got.isnan().all(dim=2), want.isnan().all(dim=2)), "rows without a value"
   for b in (0, 2, 5):
-    for c in (9, 33):
+    for c in (9, 20, 33):
       scale = want[b, :, c].abs().max()
       assert ((got[b, :, c].double() - want[b, :, c]).abs() <= 384 * 2.0 ** -24 * scale).all()
+  no_timeouts(ops)
+
+
+@pytest.mark.parametrize("ea", [False, True])
+@pytest.mark.parametrize("q_size,v_size,o_size,mix", [
+    (1.0, 1e9, 1.0, 1.0), (1.0, 1e20, 1.0, 1.0), (1e-30, 1e5, 1e9, 1.0), (1e4, 1e-25, 1e-6, 1.0), (1.0, 1.0, 1e-36, 1.0),
+    (1.0, 1.0, 1e36, 1.0), (1.0, 1.0, 1.0, 1e12), (1.0, 1e-9, 1.0, 1e20), (1e4, 1e-25, 1e-6, 1e12)])
+def test_block_with_operands_of_any_size(ops, ea, q_size, v_size, o_size, mix):
+  # M' grows with the values over SimA's queries: its product with the output projection leaves f32's range, at either
+  # end, where the block's own sums stay inside.  `mix`: a head of large values under small weights in every other
+  # column, under ordinary ones in the rest.  Bound as in test_block_rows_and_batches_vs_float64, by column
+  B, N, C = 3, 300, 64
+  g = torch.Generator().manual_seed(11)
+  x, w_qkv, w_o = torch.randn(B, N, C, generator=g), torch.randn(3 * C, C, generator=g) / 8, torch.randn(C, C, generator=g) / 8 * o_size
+  if not ea:
+    w_qkv[:C] *= q_size
+  w_qkv[2 * C:] *= v_size
+  w_qkv[2 * C:2 * C + 32] *= mix
+  w_o[::2, :32] /= mix
+  args = (x, w_qkv, torch.zeros(3 * C), w_o, torch.zeros(C))
+  got, want = ops.linattn_block(*(t.cuda() for t in args), ea=ea).cpu().double(), block_float64(*args, ea)
+  bound = (2 * 128 + N) * 2.0 ** -24 * want.abs().amax(dim=1, keepdim=True)
+  assert ((got - want).abs() <= bound).all(), ((got - want).abs() / bound).max()
+  no_timeouts(ops)
+
+
+@pytest.mark.parametrize("ea", [False, True])
+@pytest.mark.parametrize("B,N,H", [(3, 300, 2), (1, 785, 4), (40, 70, 3), (2, 33, 1)])
+def test_core_with_projection_takes_scratch_of_either_size(ops, B, N, H, ea):
+  # the scales of the folded weights have a row of the scratch to themselves, or lie in the output meanwhile
+  import ctypes
+  from flashtensor_b200 import _lib
+  C = 32 * H
+  g = torch.Generator(device="cuda").manual_seed(N)
+  qkv, w, bias = (torch.randn(*s, generator=g, device="cuda") for s in ((B, N, 3, H, 32), (C, C), (C,)))
+  w[::3, :32] *= 1e-20
+  results = []
+  for rows in (C, C + 1):
+    out = torch.full((B, N, C), float("nan"), device="cuda")
+    scratch = torch.full((B, rows, C), float("nan"), device="cuda")
+    p = _lib.LinAttn32ProjParams(*(ops._desc(x) for x in (qkv[:, :, 0], qkv[:, :, 1], qkv[:, :, 2], w, bias, out, scratch)), int(ea))
+    assert _lib.load().asuka_b200_linattn32_proj(ctypes.byref(p), torch.cuda.current_stream().cuda_stream) == 0
+    results.append(out)
+  assert torch.equal(results[0], results[1])
+  core = ops.linattn32_fwd(qkv[:, :, 0], qkv[:, :, 1], qkv[:, :, 2], ea=ea)
+  want = core.double().view(B, N, C) @ w.double().t() + bias.double()
+  # the core's N-term sums and 128 terms of the projection, on either side
+  bound = 2 * (128 + max(N, 128)) * 2.0 ** -24 * (core.double().abs().view(B, N, C) @ w.double().abs().t() + bias.double().abs()).amax(dim=1, keepdim=True)
+  assert ((results[0].double() - want).abs() <= bound).all()
   no_timeouts(ops)
 
 
