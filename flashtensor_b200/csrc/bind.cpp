@@ -5,6 +5,7 @@
 // its selection 39-43 us a call (128 rows, 2 heads, calls back to back).  Here the descriptors are
 // filled from the tensor objects directly and the outputs come straight from the caching
 // allocator: 7.7 and 13-15 us, most of it the launches themselves.  Nothing is cached between calls.  The interpreter lock is released around the C-ABI call, as ctypes does.
+#include <ATen/cuda/CUDAContext.h>
 #include <ATen/cuda/EmptyTensor.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
@@ -354,6 +355,22 @@ PyObject* linear(PyObject*, PyObject* const* a, Py_ssize_t n) {
   END_HANDLE_TH_ERRORS
 }
 
+// From how many rows of a batch on its core is folded into the output projection.  Folding spares the core a pass over
+// the queries and its output, which grow with the rows; it costs C x C weights for every batch, written, read and split
+// by a CTA of the projection that has nothing but that batch's rows, and scratch of that size.  Folded / not, us, SimA at
+// C 128 (B 512 N 16 takes 94 / 55, B 4096 N 49 763 / 402):
+//   N      100        160        192        224        256        320        400        500
+//   B 2    22.4/22.9  24.9/24.5  25.0/24.5  25.1/25.6  25.1/25.5  25.9/26.9  26.8/29.6  27.3/30.8
+//   16     26.4/23.3  27.4/25.1  28.0/26.1  28.7/28.0  31.7/32.4  33.3/34.5  35.6/41.0  37.9/43.7
+//   64     32.0/30.7  34.6/33.9  36.3/34.1  39.2/39.8  38.8/38.9  48.8/47.8  49.3/53.6  59.0/60.9
+//   148    44.0/42.4  50.6/51.4  56.1/56.5  59.4/66.7  62.0/64.5  73.8/79.8  86.2/101   109/117
+//   512    136/100    169/137    180/156    195/175    207/188    237/222    279/282    328/332
+// (C 64: B 64 N 128 22.2/22.0, N 256 27.0/29.0, B 512 N 256 109/108; EA like SimA.)  Above the line the scratch is smaller
+// than the output of the core that the other way needs.
+int64_t fold_from(int64_t B) {
+  return B <= at::cuda::getCurrentDeviceProperties()->multiProcessorCount ? 224 : 384;
+}
+
 // The whole block of bench/sima.mlir / bench/ea.mlir: (x [B, N, C], w_qkv, b_qkv, w_o, b_o, ea) -> [B, N, C];
 // the core reads q, k, v as strided views of the projection's output [B*N, 3, C/32, 32].
 PyObject* linattn_block(PyObject*, PyObject* const* a, Py_ssize_t n) {
@@ -373,7 +390,6 @@ PyObject* linattn_block(PyObject*, PyObject* const* a, Py_ssize_t n) {
     OnDevice on({&x, &w_qkv, &b_qkv, &w_o, &b_o});
     const int64_t B = x.size(0), N = x.size(1);
     const at::Tensor qkv = linear_f32(x.view({B * N, C}), w_qkv, b_qkv, on.stream);
-    const at::Tensor out = empty({B, N, C}, at::kFloat, x), scratch = empty({B, C + 1, C}, at::kFloat, x);
     asuka_linattn32_proj_params p;
     p.q = desc(qkv);  // [B, N, C / 32, 32], strided over the fused rows
     p.q.ndim = 4;
@@ -383,11 +399,23 @@ PyObject* linattn_block(PyObject*, PyObject* const* a, Py_ssize_t n) {
     p.k.ptr = static_cast<float*>(p.q.ptr) + C;
     p.v = p.q;
     p.v.ptr = static_cast<float*>(p.q.ptr) + 2 * C;
+    p.ea = bool_arg(a[5]) ? 1 : 0;
+    if (N < fold_from(B)) {
+      const at::Tensor core = empty({B, N, C / 32, 32}, at::kFloat, x);
+      asuka_linattn32_params c;
+      c.q = p.q;
+      c.k = p.k;
+      c.v = p.v;
+      c.out = desc(core);
+      c.ea = p.ea;
+      call("asuka_b200_linattn32_fwd", [&] { return asuka_b200_linattn32_fwd(&c, on.stream); });
+      return wrap(linear_f32(core.view({B * N, C}), w_o, b_o, on.stream).view({B, N, C}));
+    }
+    const at::Tensor out = empty({B, N, C}, at::kFloat, x), scratch = empty({B, C + 1, C}, at::kFloat, x);
     p.w = desc(w_o);
     p.bias = desc(b_o);
     p.out = desc(out);
     p.scratch = desc(scratch);
-    p.ea = bool_arg(a[5]) ? 1 : 0;
     call("asuka_b200_linattn32_proj", [&] { return asuka_b200_linattn32_proj(&p, on.stream); });
     return wrap(out);
   } catch (const BadArg&) {

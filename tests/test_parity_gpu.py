@@ -539,10 +539,12 @@ def block_float64(x, w_qkv, b_qkv, w_o, b_o, ea):
 
 
 @pytest.mark.parametrize("ea", [False, True])
-@pytest.mark.parametrize("shape", [(1, 1, 32), (2, 33, 96), (70, 31, 128), (3, 129, 64), (150, 70, 32), (5, 785, 128)])
+@pytest.mark.parametrize("shape", [(1, 1, 32), (2, 33, 96), (70, 31, 128), (3, 129, 64), (150, 70, 32), (5, 785, 128),
+                                   (2, 224, 96), (70, 257, 128), (148, 240, 32), (149, 383, 32), (300, 390, 64)])
 def test_block_rows_and_batches_vs_float64(ops, shape, ea):
-  # every batch has weights of its own in the last product, and its rows are cut into CTAs and tiles there:
-  # remainders of a tile, of a 32-row piece and of a 16-row MMA, batches beside one another and in several waves.
+  # from some 224 rows on (384 with more batches than SMs) every batch has weights of its own in the last product, and
+  # its rows are cut into CTAs and tiles there: remainders of a tile, of a 32-row piece and of a 16-row MMA, batches
+  # beside one another and in several waves; below, all rows are those of one product.
   # Each of the block's three sums (128 terms twice, N once) is off by n 2^-24 of its terms at most
   B, N, C = shape
   g = torch.Generator().manual_seed(B + N)
@@ -556,11 +558,12 @@ def test_block_rows_and_batches_vs_float64(ops, shape, ea):
   no_timeouts(ops)
 
 
+@pytest.mark.parametrize("n", [90, 250])
 @pytest.mark.parametrize("ea", [False, True])
-def test_block_batches_keep_to_themselves(ops, ea):
+def test_block_batches_keep_to_themselves(ops, ea, n):
   # a NaN, an infinity, keys of nothing but zeros and weights of no ordinary size in one batch or column: the
   # others come out as without them, and the odd ones as the restatement has them
-  B, N, C = 6, 90, 64
+  B, N, C = 6, n, 64
   g = torch.Generator().manual_seed(9)
   x, w_qkv, b_qkv = torch.randn(B, N, C, generator=g), torch.randn(3 * C, C, generator=g) / 8, torch.zeros(3 * C)
   w_o, b_o = torch.randn(C, C, generator=g) / 8, torch.randn(C, generator=g)
@@ -607,6 +610,20 @@ def test_block_with_operands_of_any_size(ops, ea, q_size, v_size, o_size, mix):
   got, want = ops.linattn_block(*(t.cuda() for t in args), ea=ea).cpu().double(), block_float64(*args, ea)
   bound = (2 * 128 + N) * 2.0 ** -24 * want.abs().amax(dim=1, keepdim=True)
   assert ((got - want).abs() <= bound).all(), ((got - want).abs() / bound).max()
+  no_timeouts(ops)
+
+
+def test_block_of_many_short_batches_takes_no_more_memory_than_its_tensors(ops):
+  # the first projection's output, the core's and the block's; folded weights for every batch would be 64 times the last
+  B, N, C = 8192, 2, 128
+  args = [t.cuda() for t in (torch.randn(B, N, C), torch.randn(3 * C, C) / 11, torch.randn(3 * C), torch.randn(C, C) / 11, torch.randn(C))]
+  ops.linattn_block(*args)
+  torch.cuda.synchronize()
+  torch.cuda.reset_peak_memory_stats()
+  before = torch.cuda.memory_allocated()
+  ops.linattn_block(*args)
+  torch.cuda.synchronize()
+  assert torch.cuda.max_memory_allocated() - before <= 5 * B * N * C * 4 + (1 << 21)
   no_timeouts(ops)
 
 
