@@ -1555,6 +1555,32 @@ Plan make_plan(const SimaShape& s) {
 size_t sima_workspace_bytes(const SimaShape& s) { return make_plan(s).total; }
 
 
+// Whether the persistent kernel is the faster one for 16-bit output.  It reads Q from L2 the second time and has no gaps
+// between launches; but every round of units costs it a barrier, a reduce and a fill of 10 us or so however short the
+// sequence is, and its last round may be partial.  So it is for one round of enough rows in all, and for three rounds
+// and more where what it saves, proportional to S, covers that; two rounds, too few for the groups to get out of step,
+// gain nothing over the three kernels.  Measured in us, one kernel / three, by units (37 groups) and S, inputs cold:
+//         2100       2500       2900       3500       4096       5000
+//   24    26.0/23.6  26.7/26.4  28.8/27.9  30.9/31.1  33.0/34.6  38.0/39.9
+//   32    27.1/26.6  28.8/30.7  31.0/32.2  34.7/37.3  37.7/41.1  43.3/48.1
+//   37    28.8/28.1  30.8/30.8  32.7/34.8  36.9/39.9  41.0/44.7  48.2/52.5
+//         3500       4500       5600       6500       8192
+//   64    68.8/63.5  80.0/75.8  91.9/90.5  103/103    125/126
+//   74    72.3/67.7  83.7/82.2  99.6/97.1  113/111    136/135
+//   96    99.2/86.2  117/107    136/129    154/148    184/180
+//   111   97.0/95.6  114/119    135/144    154/165    191/203
+//   128   120/110    143/138    164/168    186/192    226/236
+//   150   145/126    172/157    198/190    239/233 (S 7000)
+//   170   152/144    182/180    208/218    252/267 (S 7000)
+//   224   207/186    245/229    282/281    313/324    383/400
+//   256   215/212    257/262    304/322    343/368    416/456
+// The lines below are a fit to these and a hundred points between them, none of which but one (5 %, within what its
+// neighbours scatter) loses more than 4 % by it.  With all inputs in L2 the first line would lie some 300 rows higher.
+bool one_kernel_pays(int64_t units, int64_t S, int64_t rounds) {
+  if (rounds == 1) return S * (units - 9) > 58000;
+  return rounds > 2 && S * (units - 20 * rounds - 10) > 60000 * rounds;
+}
+
 cudaError_t launch_sima(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv,
                         const CUtensorMap& mo, void* out_ptr, int64_t out_stride_b,
                         int64_t out_stride_s, int64_t out_stride_h, void* ws, const SimaShape& s,
@@ -1562,29 +1588,14 @@ cudaError_t launch_sima(const CUtensorMap& mq, const CUtensorMap& mk, const CUte
   const Plan pl = make_plan(s);
   const int bh = s.B * s.H;
   uint8_t* w = static_cast<uint8_t*>(ws);
-  // One persistent kernel for all three steps, or three that share the tiles out evenly.  The first reads Q from
-  // L2 the second time and has no gaps between launches; but every round of units costs it a barrier, a reduce
-  // and a fill of 10 us or so however short the sequence is, and its last round may be partial.  So it is for one
-  // round of long sequences, and for several where what it saves, proportional to S, covers that.  Measured in us,
-  // one kernel / three, by units (37 groups) and S; the lines run between 24 units' S 1500 and 4096 and along
-  // (S - 3200) units = 500000:
-  //          700          1500         4096           8192
-  //   24     18.8/15.2    20.7/18.6    30.9/31.5      51.9/55.6
-  //   36     18.8/17.2    22.1/19.7    35.5/43.5      70.0/74.9
-  //   48     30.9/18.1    35.2/23.7    63.6/56.8      107/97.7
-  //   64     32.9/20.1    39.1/31.1    74.1/69.0      125/125
-  //   96     47.2/23.2    57.8/43.6    111/97.4       186/179
-  //   128    59.6/30.9    73.2/55.6    133/126        227/233
-  //   160    73.9/38.5    92.4/67.1    164/156        281/294
-  //   256    111/59.9     132/103      242/241        412/456
+  // One persistent kernel for all three steps, or three that share the tiles out evenly.
   const int n_groups = num_sms / kFuGroup;
 #ifdef ASUKA_SIMA_NO_FUSED
   const bool fused = false;
 #else
   const bool fused = !s.ea && maps64 != nullptr && n_groups > 0 && 2 * bh >= n_groups &&
-                     (s.out_f32        ? pl.ntiles >= kFuGroup  // (f32 output: the line of before, not measured since)
-                      : bh <= n_groups ? pl.ntiles >= 24
-                                       : static_cast<int64_t>(s.S - 3200) * bh > 500000);
+                     (s.out_f32 ? pl.ntiles >= kFuGroup  // (f32 output: the line of before, not measured since)
+                                : one_kernel_pays(bh, s.S, (bh + n_groups - 1) / n_groups));
 #endif
   if (fused) {
     FusedParams fp;

@@ -333,8 +333,9 @@ def test_sima_vs_oracle(ops, shape, dtype):
 @pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
 @pytest.mark.parametrize("shape", [(10, 700, 8), (3, 1000, 32), (80, 512, 1), (2, 1664, 40)])
 def test_sima_with_many_units_vs_oracle(ops, shape, dtype):
-  # enough (batch, head) units that the single persistent kernel runs (groups of four CTAs walk the
-  # units, each CTA a quarter of the sequence); ragged lengths, a quarter with no tile at all
+  # f32 output: enough (batch, head) units that the single persistent kernel runs (groups of four CTAs walk
+  # the units, each CTA a quarter of the sequence); ragged lengths, a quarter with no tile at all.  16-bit
+  # output: the three kernels, these sequences being short
   B, S, H = shape
   q, k, v = O.make_inputs("sima", B, S, S, H, 128, dtype, seed=S)
   ref = O.sima(q, k, v)
@@ -348,10 +349,25 @@ def test_sima_with_many_units_vs_oracle(ops, shape, dtype):
   no_timeouts(ops)
 
 
-@pytest.mark.parametrize("shape", [(1, 2944, 20), (1, 2945, 20), (1, 2950, 37), (1, 2950, 38), (7, 900, 9)])
-def test_sima_on_either_side_of_the_line(ops, shape):
-  # one persistent kernel or three: 24 key tiles or 23 with one round of units, one unit more than a round
-  test_sima_vs_oracle(ops, shape, torch.float16)
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("shape,one_kernel", [
+    ((1, 5272, 20), False), ((1, 5273, 20), True), ((1, 2071, 37), False), ((1, 2072, 37), True), ((1, 9000, 38), False),
+    ((1, 4390, 111), False), ((1, 4391, 111), True), ((2, 7001, 70), True), ((4, 5003, 75), True), ((4, 4417, 37), True), ((7, 900, 9), False)])
+def test_sima_on_either_side_of_the_line(ops, shape, one_kernel, dtype):
+  # one persistent kernel or three (37 groups of four CTAs): one round of units, two, three and more, where the
+  # persistent kernel's stages and staging are used from unit to unit, ragged lengths; the first unit, the last of a
+  # round and those behind it, the last of all
+  B, S, H = shape
+  g = torch.Generator(device="cuda").manual_seed(S)
+  q, k, v = (torch.randn(B, S, H, 128, generator=g, device="cuda").to(dtype) for _ in range(3))
+  out, before = ops.sima_fwd(q, k, v), ops.launch_count()
+  assert torch.equal(out, ops.sima_fwd(q, k, v))
+  assert ops.launch_count() - before == (1 if one_kernel else 3)
+  for u in sorted({0, 36, 37, 73, 74, 111, B * H - 1}):
+    if u < B * H:
+      b, h = u // H, u % H
+      close(out[b:b + 1, :, h:h + 1], O.sima(_unit(q, b, h), _unit(k, b, h), _unit(v, b, h)), f"unit {u}")
+  no_timeouts(ops)
 
 
 @pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
