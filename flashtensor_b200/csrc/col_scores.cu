@@ -1396,9 +1396,10 @@ cudaError_t launch_kf_rowstat(const CUtensorMap& mq, const CUtensorMap& mk, cons
     if (e != cudaSuccess) return e;
     // Two CTAs share an SM.  A launch of half a wave to two waves is balanced by one long and one shorter
     // tile on each, which is how the CTAs fall when all SMs are free at the start; as the forward kernel's
-    // CTAs retire one by one, the first SM gets the two longest.  Such a launch waits (us, chained / not:
-    // B1 H16 S4096, 1.7 waves, 415 / 402; B2 H16 S2048 225 / 224; B2 H32 S1501, 2.6 waves, 251 / 256; B1 H16
-    // S300, a sixth of a wave, 28 / 36).
+    // CTAs retire one by one, the first SM gets the two longest.  Such a launch waits (whole case in us, chained / not:
+    // B1 H16 S2048, 0.9 waves, 141 / 127; B1 H16 S4096, 1.7 waves, 325 / 314; B2 H16 S2048 180 / 179; B2 H40 S1000,
+    // 2.2 waves, 131 / 138; B2 H32 S1501, 2.6 waves, 201 / 209; B1 H16 S300, a sixth of a wave, 24.4 / 32.0; S600
+    // 34.3 / 42.8).
     if (grid.x > static_cast<unsigned>(num_sms) && grid.x < 4u * num_sms) {
       p.chained = 0;
       kern<<<grid, RsCfg<2>::kThreads, RsCfg<2>::kSmem, stream>>>(mq, mk, mq, p, lse2_out);

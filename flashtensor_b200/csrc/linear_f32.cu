@@ -32,8 +32,8 @@
 // or column: all rows at 1e-25 take 1460 us instead of 34, rows of nothing but zeros, which need a look at x only, 91.
 // Measured at B64 N784 C128 (M = 50176, K = 128), calls back to back, bias included: N = 384 (QKV) 32 us,
 // N = 128 (output) 14.6 us; the f32 GEMM of the BLAS library with its bias pass takes 200 and 64.  A launch is set-up
-// for a third of it, so the warps that split x start while the weights are still being split (whole SimA block
-// 78.5 -> 74 us).  Eight epilogue warps, four to an accumulator, are slower (38 and 17 us: what they and the
+// for a third of it, so the warps that split x start while the weights are still being split (4.5 us of a
+// whole SimA block of that size).  Eight epilogue warps, four to an accumulator, are slower (38 and 17 us: what they and the
 // splitting warps share is the way to shared memory), and so are plain stores instead of TMA's.
 #include <cuda_bf16.h>
 
@@ -84,6 +84,11 @@ struct LinParams {
 constexpr float kWeightLow = 7.8886090522101181e-31f;                            // 2^-100
 constexpr float kSumLow = 2.1175823681357508e-22f;                               // 2^-72
 constexpr float kSumPerWeight = 2.0194839173657902e-28f;                         // 2^-92 (folded weights)
+// (softmax) 1 / 32, which the values of a group average.  It is taken off them before they are multiplied and comes back
+// as that share of the sum of the column's weights, in f32: products of values that are all positive have the signs of
+// the weights, and what the tensor pipe truncates of each then adds up.  EA block, error against 64 bits with and without,
+// B64 N784 C128 1.09e-7 and 1.66e-7, B4 N300 1.33e-7 and 1.94e-7 (core and projection apart 1.57e-7 and 1.76e-7).
+constexpr float kShare = 0.03125f;
 template <int kMode> constexpr float kWeightHighOf = kMode == kPlain ? 1048576.f : 1.2676506002282294e30f;  // 2^20, 2^100
 __device__ __forceinline__ float max3_nan(float a, float b, float c) {
   float y;
@@ -275,6 +280,7 @@ __global__ void __launch_bounds__(kThreads, 1) linear_f32_kernel(const __grid_co
   const uint32_t lane_base = static_cast<uint32_t>(wq * 32) << 16;
   const int n = n0 + wq * 32 + lane;  // (epilogue warps) this thread's output column
   float w_big = 0.f, w_small = kWeightHigh;  // (epilogue warps) of that column's weights, the zeros apart
+  float w_sum[4] = {0.f, 0.f, 0.f, 0.f};     // (softmax, epilogue warps) the sum of that column's weights
   uint32_t least = 127u;                     // (batched, epilogue warps) exponent of the scale of that column's weights
   // (batched: the kernel ahead, which writes the weights, reads x itself and has waited for whatever wrote it before
   // this one could start: the splitting warps need not wait; EA block 79.7 -> 76.8 us)
@@ -318,6 +324,7 @@ __global__ void __launch_bounds__(kThreads, 1) linear_f32_kernel(const __grid_co
 #pragma unroll
           for (int i = 0; i < 8; ++i) v[i] = mul_keep(v[i], f);
         }
+        if constexpr (kMode == kSoftmax) w_sum[g] += ((v[0] + v[1]) + (v[2] + v[3])) + ((v[4] + v[5]) + (v[6] + v[7]));
         float big, small;
         extent8(v, &big, &small);
         w_big = max3_nan(w_big, big, big);
@@ -388,7 +395,11 @@ __global__ void __launch_bounds__(kThreads, 1) linear_f32_kernel(const __grid_co
           for (int i = 0; i < 4; ++i) {
             const float4 lo = v[ch][i][0], hi = v[ch][i][1];
             float e[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
-            if constexpr (kMode == kSoftmax) softmax_group<4>(e);  // (past K the weights are zero)
+            if constexpr (kMode == kSoftmax) {  // (past K the weights are zero)
+              softmax_group<4>(e);
+#pragma unroll
+              for (int x = 0; x < 8; ++x) e[x] -= kShare;
+            }
             uint4 q[3];
             split8(e, q);
 #pragma unroll
@@ -445,6 +456,8 @@ __global__ void __launch_bounds__(kThreads, 1) linear_f32_kernel(const __grid_co
     float* const out = p.out + static_cast<int64_t>(batch) * p.M * p.N;
     const float sum_low = kMode == kPlain ? kSumLow : fmaxf(kSumLow, w_big * kSumPerWeight);
     const float unscale = kMode == kPlain ? 1.f : __uint_as_float((254u - least) << 23);
+    // (softmax) what the shares taken off the queries amount to, in every row alike
+    const float shared = kMode != kSoftmax ? 0.f : kShare * ((w_sum[0] + w_sum[1]) + (w_sum[2] + w_sum[3]));
     auto result = [&](float sum) { return kMode == kPlain ? add_keep(sum, bias) : fma_keep(sum, unscale, bias); };
     const bool zero_col = w_big == 0.f;  // a sum of zero is right (with a subnormal weight it is a plain one)
     const bool plain_col = !(w_big < kWeightHigh) || w_small < kWeightLow;
@@ -467,6 +480,10 @@ __global__ void __launch_bounds__(kThreads, 1) linear_f32_kernel(const __grid_co
         if (lane == 0) tma_store_wait_read_n<1>();  // the store before last has left this half of the stage
         __syncwarp();
         tmem_wait_ld();
+        if constexpr (kMode == kSoftmax) {
+#pragma unroll
+          for (int r = 0; r < 32; ++r) u[r] = __float_as_uint(__uint_as_float(u[r]) + shared);
+        }
         if (row_t + q * 32 + 32 > row_end) {  // (rows past the end, zero as well, are not stored)
 #pragma unroll
           for (int r = 0; r < 32; ++r) u[r] = row_t + q * 32 + r < row_end ? u[r] : __float_as_uint(kWeightHigh);
@@ -515,7 +532,7 @@ __global__ void __launch_bounds__(kThreads, 1) linear_f32_kernel(const __grid_co
           uint32_t mine = 0;  // this column's rows
 #pragma unroll
           for (int r = 0; r < 32; ++r) {
-            const float a = fabsf(__uint_as_float(u[r]));
+            const float a = fabsf(__uint_as_float(u[r]) + shared);
             if (!(a < INFINITY) || (a < sum_low && !zero_col)) mine |= 1u << r;
           }
           if (plain_col) mine = 0xffffffffu;

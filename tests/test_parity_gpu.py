@@ -629,6 +629,26 @@ def test_block_with_operands_of_any_size(ops, ea, q_size, v_size, o_size, mix):
   no_timeouts(ops)
 
 
+@pytest.mark.parametrize("ea", [False, True])
+@pytest.mark.parametrize("B,N", [(4, 300), (16, 500), (64, 784)])
+def test_folded_projection_is_no_less_accurate_than_core_and_projection(ops, B, N, ea):
+  # the error against 64 bits beside that of the same block in three calls, which it replaces: what the tensor pipe
+  # truncates must not add up over EA's queries, all of one sign.  (2-norms over half a million results and more: two
+  # such errors that are alike differ by a percent at most)
+  C = 128
+  g = torch.Generator(device="cuda").manual_seed(5)
+  args = [torch.randn(*s, generator=g, device="cuda") * f for s, f in
+          (((B, N, C), 1.0), ((3 * C, C), C ** -0.5), ((3 * C,), 0.1), ((C, C), C ** -0.5), ((C,), 0.1))]
+  x, w_qkv, b_qkv, w_o, b_o = args
+  qkv = ops.linear_f32(x.view(B * N, C), w_qkv, b_qkv).view(B, N, 3, C // 32, 32)
+  core = ops.linattn32_fwd(qkv[:, :, 0], qkv[:, :, 1], qkv[:, :, 2], ea=ea)
+  apart = ops.linear_f32(core.view(B * N, C), w_o, b_o).view(B, N, C)
+  want = block_float64(*args, ea)
+  folded = ops.linattn_block(*args, ea=ea)
+  assert (folded.double() - want).norm() <= 1.02 * (apart.double() - want).norm()
+  no_timeouts(ops)
+
+
 def test_block_of_many_short_batches_takes_no_more_memory_than_its_tensors(ops):
   # the first projection's output, the core's and the block's; folded weights for every batch would be 64 times the last
   B, N, C = 8192, 2, 128
