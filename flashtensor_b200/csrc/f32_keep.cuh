@@ -26,7 +26,7 @@ __device__ __forceinline__ float add_keep(float a, float b) {
 // range where (Q M') w_o^T stays in it.  A head's 32 weights are therefore brought to a largest magnitude of 2^-8 to 2^-7 by
 // a power of two first: 32 products with a finite M' are finite then, and with products that keep their subnormal bits
 // what a folded weight loses at the lower end is below 2^-141 of the weights' size, less than the 2^-126 at which M'
-// itself is flushed.  (Weights beyond 2^119 are scaled by 2^-126, not less.)  The exponents travel with the folded
+// itself is flushed.  (Weights beyond 2^119 are scaled by 2^-126, not less.)  The exponents (1 to 245) travel with the folded
 // weights; the projection brings the heads of a column to the scale of its largest and takes that out of its sums again.
 // Bits of the scale's exponent from those of the largest magnitude; the inverse's are 254 less this.
 __device__ __forceinline__ uint32_t fold_scale_exponent(uint32_t max_bits) {

@@ -289,13 +289,6 @@ __global__ void __launch_bounds__(kThreads, 1) linear_f32_kernel(const __grid_co
   if (warp > kSplitWarps) {
     // the weights of this block of columns, split once: thread = output column = TMEM lane
     const float* src = w + static_cast<int64_t>(min(n, p.N - 1)) * p.K;
-    uint32_t e4 = 0;
-    if (kMode != kPlain && n < p.N) {  // the scales that the column's weights were folded with
-      const uint8_t* e = reinterpret_cast<const uint8_t*>(p.scales.ptr + batch * p.scales.per_batch + static_cast<int>(blockIdx.x) % p.splits * p.scales.per_cta) + n;
-#pragma unroll
-      for (int h = 0; h < 4; ++h)
-        if (h * 32 < p.K) e4 |= static_cast<uint32_t>(__ldcg(e + h * p.K)) << (8 * h);
-    }
     float4 next[8];  // the next 32 weights
     auto load = [&](int k0) {
 #pragma unroll
@@ -304,13 +297,16 @@ __global__ void __launch_bounds__(kThreads, 1) linear_f32_kernel(const __grid_co
     };
     load(0);
     if constexpr (kMode != kPlain) {
-      least = 255u;  // all are brought to the scale of the largest
-      for (int h = 0; h * 32 < p.K; ++h) least = min(least, (e4 >> (8 * h)) & 255u);
+      // the exponents of the scales that the column's heads were folded with: all are brought to that of the largest,
+      // by 2^-126 at most
+      const uint8_t* e_ptr = reinterpret_cast<const uint8_t*>(p.scales.ptr + batch * p.scales.per_batch +
+                                                              static_cast<int>(blockIdx.x) % p.splits * p.scales.per_cta);
+      uint32_t e[4];
 #pragma unroll
-      for (int h = 0; h < 4; ++h) {  // 2^-d, subnormal below 2^-126, not less than 2^-133
-        const uint32_t d = max((e4 >> (8 * h)) & 255u, least) - least;
-        rescale_s[wq * 32 + lane][h] = static_cast<uint16_t>(d < 127u ? (127u - d) << 7 : 1u << (133u - min(d, 133u)));
-      }
+      for (int h = 0; h < 4; ++h) e[h] = n < p.N && h * 32 < p.K ? __ldcg(e_ptr + h * p.K + n) : 254u;
+      least = min(min(e[0], e[1]), min(e[2], e[3]));
+#pragma unroll
+      for (int h = 0; h < 4; ++h) rescale_s[wq * 32 + lane][h] = static_cast<uint16_t>((127u - min(e[h] - least, 126u)) << 7);
     }
     for (int k0 = 0; k0 < p.chunks * kChunk; k0 += 32) {
       uint32_t t[3][16];

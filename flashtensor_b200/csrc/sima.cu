@@ -1574,8 +1574,9 @@ size_t sima_workspace_bytes(const SimaShape& s) { return make_plan(s).total; }
 //   170   152/144    182/180    208/218    252/267 (S 7000)
 //   224   207/186    245/229    282/281    313/324    383/400
 //   256   215/212    257/262    304/322    343/368    416/456
-// The lines below are a fit to these and a hundred points between them, none of which but one (5 %, within what its
-// neighbours scatter) loses more than 4 % by it.  With all inputs in L2 the first line would lie some 300 rows higher.
+// The lines below are a fit to these and a hundred points between them, of which none loses more than 4 % by it, but for 32
+// units just below their line (5 and 6 % at S 2400 and 2500).  With all inputs in L2 the first line would lie some 300
+// rows higher.
 bool one_kernel_pays(int64_t units, int64_t S, int64_t rounds) {
   if (rounds == 1) return S * (units - 9) > 58000;
   return rounds > 2 && S * (units - 20 * rounds - 10) > 60000 * rounds;
