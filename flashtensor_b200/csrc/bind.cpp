@@ -358,15 +358,16 @@ PyObject* linear(PyObject*, PyObject* const* a, Py_ssize_t n) {
 // From how many rows of a batch on its core is folded into the output projection.  Folding spares the core a pass over
 // the queries and its output, which grow with the rows; it costs C x C weights for every batch, written, read and split
 // by a CTA of the projection that has nothing but that batch's rows, and scratch of that size.  Folded / not, us, SimA at
-// C 128 (B 512 N 16 takes 94 / 55, B 4096 N 49 763 / 402):
-//   N      100        160        192        224        256        320        400        500
-//   B 2    22.4/22.9  24.9/24.5  25.0/24.5  25.1/25.6  25.1/25.5  25.9/26.9  26.8/29.6  27.3/30.8
-//   16     26.4/23.3  27.4/25.1  28.0/26.1  28.7/28.0  31.7/32.4  33.3/34.5  35.6/41.0  37.9/43.7
-//   64     32.0/30.7  34.6/33.9  36.3/34.1  39.2/39.8  38.8/38.9  48.8/47.8  49.3/53.6  59.0/60.9
-//   148    44.0/42.4  50.6/51.4  56.1/56.5  59.4/66.7  62.0/64.5  73.8/79.8  86.2/101   109/117
-//   512    136/100    169/137    180/156    195/175    207/188    237/222    279/282    328/332
-// (C 64: B 64 N 128 22.2/22.0, N 256 27.0/29.0, B 512 N 256 109/108; EA like SimA.)  Above the line the scratch is smaller
-// than the output of the core that the other way needs.
+// C 128 (B 512 N 16 takes 93 / 56, B 4096 N 49 777 / 406):
+//   N      100        128        160        192        224        256        320        400        500
+//   B 2    22.0/22.1  22.1/22.4  24.2/23.8  24.2/23.9  24.7/25.1  24.8/25.2  24.9/26.7  26.0/29.3  26.2/30.7
+//   16     25.3/23.1  25.9/23.2  26.7/24.9  27.0/26.3  28.0/28.1  31.7/32.7  32.2/34.4  35.1/40.9  37.1/44.2
+//   64     32.4/31.3  32.5/32.3  33.7/34.9  34.4/34.1  37.3/38.8  38.2/39.1  45.3/47.3  48.8/55.4  53.5/61.9
+//   148    42.2/42.3  47.7/43.5  50.0/51.4  53.5/55.6  59.0/64.2  61.5/67.6  70.2/76.6  92.2/96.3  99.8/116
+//   512    135/105    154/114    168/140    185/151    200/175    206/190    242/224    284/278    328/339
+// (EA: B 16 N 192 28.8/27.4, N 256 33.2/35.4, B 512 N 256 219/213, N 400 294/318.  C 64: B 64 N 128 22.0/22.1, N 256
+// 27.0/28.0, B 512 N 256 108/105.)  Above the line the scratch is smaller than the output of the core that the other way
+// needs.
 int64_t fold_from(int64_t B) {
   return B <= at::cuda::getCurrentDeviceProperties()->multiProcessorCount ? 224 : 384;
 }

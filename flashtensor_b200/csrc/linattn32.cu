@@ -22,7 +22,8 @@
 // flight 58 / 67 us, this kernel 37 / 47 us.
 // In a whole block (kFold) there is no pass B: the kernel multiplies the 32 x 32 matrices with the output
 // projection, and linear_f32.cu applies the product to the queries (this kernel 23 us then; the block, SimA / EA,
-// 82 / 91.5 -> 70 / 77 us with it and the projections' earlier start).
+// 87 / 95 -> 77 / 85 us with it and the projections' earlier start, on one card).  For blocks of some length only, see
+// fold_from in bind.cpp.
 #include "f32_keep.cuh"
 #include "kernels.h"
 #include "sm100_ptx.cuh"
