@@ -87,7 +87,10 @@ constexpr float kSumPerWeight = 2.0194839173657902e-28f;                        
 // (softmax) 1 / 32, which the values of a group average.  It is taken off them before they are multiplied and comes back
 // as that share of the sum of the column's weights, in f32: products of values that are all positive have the signs of
 // the weights, and what the tensor pipe truncates of each then adds up.  EA block, error against 64 bits with and without,
-// B64 N784 C128 1.09e-7 and 1.66e-7, B4 N300 1.33e-7 and 1.94e-7 (core and projection apart 1.57e-7 and 1.76e-7).
+// B64 N784 C128 1.09e-7 and 1.66e-7, B4 N300 1.33e-7 and 1.94e-7 (core and projection apart 1.57e-7 and 1.76e-7); with
+// queries ten times as large, which pick few features, keys five times and values about 3, B4 N300 1.82e-7 and 3.26e-7
+// (1.88e-7).  What the sum of the weights is rounded by stays below 2^-24 of the largest folded weights of the column,
+// also in a row that picks none but small ones.
 constexpr float kShare = 0.03125f;
 template <int kMode> constexpr float kWeightHighOf = kMode == kPlain ? 1048576.f : 1.2676506002282294e30f;  // 2^20, 2^100
 __device__ __forceinline__ float max3_nan(float a, float b, float c) {

@@ -631,7 +631,8 @@ def test_block_with_operands_of_any_size(ops, ea, q_size, v_size, o_size, mix):
 
 @pytest.mark.parametrize("ea", [False, True])
 @pytest.mark.parametrize("B,N", [(4, 300), (16, 500), (64, 784)])
-def test_folded_projection_is_no_less_accurate_than_core_and_projection(ops, B, N, ea):
+@pytest.mark.parametrize("q_size,k_size,v_bias", [(1, 1, 0), (10, 1, 0), (10, 5, 3)])
+def test_folded_projection_is_no_less_accurate_than_core_and_projection(ops, B, N, ea, q_size, k_size, v_bias):
   # the error against 64 bits beside that of the same block in three calls, which it replaces: what the tensor pipe
   # truncates must not add up over EA's queries, all of one sign.  (2-norms over half a million results and more: two
   # such errors that are alike differ by a percent at most)
@@ -640,6 +641,10 @@ def test_folded_projection_is_no_less_accurate_than_core_and_projection(ops, B, 
   args = [torch.randn(*s, generator=g, device="cuda") * f for s, f in
           (((B, N, C), 1.0), ((3 * C, C), C ** -0.5), ((3 * C,), 0.1), ((C, C), C ** -0.5), ((C,), 0.1))]
   x, w_qkv, b_qkv, w_o, b_o = args
+  if ea:  # queries and keys that pick few of the features and rows, values of one sign
+    w_qkv[:C] *= q_size
+    w_qkv[C:2 * C] *= k_size
+    b_qkv[2 * C:] += v_bias
   qkv = ops.linear_f32(x.view(B * N, C), w_qkv, b_qkv).view(B, N, 3, C // 32, 32)
   core = ops.linattn32_fwd(qkv[:, :, 0], qkv[:, :, 1], qkv[:, :, 2], ea=ea)
   apart = ops.linear_f32(core.view(B * N, C), w_o, b_o).view(B, N, C)
