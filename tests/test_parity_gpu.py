@@ -264,6 +264,59 @@ def test_keyformer_seeded_noise_vs_oracle(ops, shape, dtype):
   no_timeouts(ops)
 
 
+@pytest.mark.parametrize("noise", ["dense", "odd", "broadcast", "seeded"])
+@pytest.mark.parametrize("shape", [  # (B, Sq, Skv, H, causal): row blocks and key tiles about one CTA's share and about a cluster's
+    (1, 1, 1, 1, True), (1, 128, 128, 2, True), (2, 129, 129, 3, True), (1, 200, 512, 2, True), (1, 513, 513, 40, False),
+    (1, 1, 700, 3, True), (1, 1024, 1024, 2, True), (1, 1025, 1025, 33, True), (2, 300, 2048, 2, True),
+    (1, 2048, 2048, 2, False), (1, 2049, 2049, 2, True), (1, 4000, 4096, 1, True)])
+def test_keyformer_in_one_pass_vs_two_passes(ops, shape, noise):
+  # the case's kernel against the row pass and the column pass that the library exports one by one, with all of the
+  # workspace it asks for (several pieces of work to a unit) and with what it must have (one)
+  import ctypes
+  from flashtensor_b200 import _lib
+  B, Sq, Skv, H, causal = shape
+  q, k, v = (t.cuda() for t in O.make_inputs("attn", B, Sq, Skv, H, 128, torch.float16, seed=23))
+  g = torch.Generator(device="cuda").manual_seed(3)
+  er = None
+  if noise == "dense":  # rows that TMA can describe
+    er = torch.empty(B, H, Sq, (Skv + 3) // 4 * 4, device="cuda").exponential_(generator=g)[..., :Skv]
+  elif noise == "odd":
+    er = torch.empty(B, H, Sq, Skv // 2 * 2 + 3, device="cuda").exponential_(generator=g)[..., 1:Skv + 1]
+  elif noise == "broadcast":
+    er = torch.empty(1, 1, Sq, Skv, device="cuda").exponential_(generator=g).expand(B, H, Sq, Skv)
+  lse = ops.keyformer_rowstat(q, k, causal=causal, exp_rand=er, tau=1.5, seed=5)
+  want = ops.col_scores(q, k, lse, mode=_lib.SCORE_PERTURBED, causal=causal, exp_rand=er, tau=1.5, seed=5)
+  p = _lib.CaseParams(ops._desc(q), ops._desc(k), ops._desc(v))
+  n = ctypes.c_size_t(0)
+  assert _lib.load().asuka_b200_case_workspace_bytes(ctypes.byref(p), ctypes.byref(n)) == 0
+  for ws in (None, torch.empty(n.value, dtype=torch.uint8, device="cuda")):
+    score = ops.keyformer(q, k, v, er, tau=1.5, seed=5, causal=causal, workspace=ws)[1]
+    # an exponent argument is off by half an ulp of a row statistic of up to 64 (4e-6), twice, and by the
+    # hardware's exponential (2e-7); sums of up to 4000 terms of one sign add about as much again
+    torch.testing.assert_close(score, want, rtol=2e-5, atol=1e-9)
+  no_timeouts(ops)
+
+
+@pytest.mark.parametrize("row_stride", [384, 385])  # by TMA, by plain loads
+def test_keyformer_noise_that_is_not_finite(ops, row_stride):
+  # rows with a zero, a NaN or nothing but infinities among what they see have no distribution: NaN for the keys they
+  # see and no others; a single infinity is a key that the row gives nothing
+  from flashtensor_b200 import _lib
+  q, k, v = (t.cuda() for t in O.make_inputs("attn", 1, 384, 384, 2, 128, torch.float16, seed=29))
+  er = torch.empty(1, 2, 384, row_stride, device="cuda").exponential_()[..., :384]
+  er[0, 0, 40, 11] = 0.
+  er[0, 0, 200, 150] = float("nan")
+  er[0, 1, 20, :21] = float("inf")
+  er[0, 1, 300, 17] = float("inf")
+  er[0, 1, 5, 300] = float("nan")  # (not visible)
+  lse = ops.keyformer_rowstat(q, k, exp_rand=er, tau=1.5)
+  want = ops.col_scores(q, k, lse, mode=_lib.SCORE_PERTURBED, exp_rand=er, tau=1.5)
+  score = ops.keyformer(q, k, v, er, tau=1.5)[1]
+  assert want.isnan()[0, 0, :201].all() and not want.isnan()[0, 0, 201:].any() and want.isnan()[0, 1].sum() == 21
+  torch.testing.assert_close(score, want, rtol=2e-5, atol=1e-9, equal_nan=True)
+  no_timeouts(ops)
+
+
 @pytest.mark.parametrize("shape", [(2, 1000, 16, torch.bfloat16), (1, 2000, 16, torch.float16)])
 def test_scores_are_the_same_bits_on_every_call(ops, shape):
   # sums in a fixed order have no excuse to differ: a box of noise refilled under the reads of its last user gave
