@@ -51,17 +51,18 @@ constexpr uint32_t kHalfBytes = kTileBytes / 2;
 //           merged in the epilogue
 enum FwdMode { kPair = 0, kSplit = 1, kSolo = 2 };
 template <int kMode> struct Rings {
-  static constexpr int kQTiles = kMode == kSolo ? 1 : 2;
+  static constexpr int kQTiles = kMode == kSolo ? 1 : 2;  // of an item
   static constexpr int kK = 3;  // K(j) is needed one iteration before V(j): give it the deeper ring
-  static constexpr int kV = kMode == kSolo ? 3 : 2;
+  static constexpr int kV = 2;
 };
 constexpr int kThreads = 384;
 // Registers of the utility and of the softmax warps; what a block asks for must fit its 384 * 168 = 64512.
 // The soft-capped one-tile mode has both ways of the tanh beside what its merge keeps: at 200 it spills 464
 // bytes (B1 S1024, 16/8 heads 22 us), at 216 140 (17.6).
+// The others at 200 or 208: B1 H32 S1024 18.6 and 17.9.
 template <bool kCap, int kMode> struct Regs {
-  static constexpr int kUtil = kCap && kMode == kSolo ? 72 : 96;
-  static constexpr int kSoftmax = kCap && kMode == kSolo ? 216 : 200;
+  static constexpr int kUtil = kCap && kMode == kSolo ? 72 : 88;
+  static constexpr int kSoftmax = kCap && kMode == kSolo ? 216 : 208;
   static constexpr int kBlock = 128 * kUtil + 256 * kSoftmax;
   static_assert(kBlock <= kThreads * 168, "setmaxnreg would wait for ever");
 };
@@ -69,10 +70,25 @@ constexpr uint32_t kSmemBytes = 7 * kTileBytes + 1024;
 constexpr float kRescaleLimit = 6.0f;  // log2 of the largest exponential tolerated under a stale reference:
                                        // keeps a tile's row sum below 2^13, far from fp16's 65504
 
+// x / d by a multiplication while x * d < 2^32 (the caller's matter), else as it is
+struct FastDiv {
+  uint32_t d, magic;  // magic 0: divide
+  __device__ __forceinline__ int div(int x) const {
+    return static_cast<int>(magic != 0 ? __umulhi(static_cast<uint32_t>(x), magic) : static_cast<uint32_t>(x) / d);
+  }
+};
+FastDiv fast_div(int d, long long x_max) {
+  FastDiv f;
+  f.d = static_cast<uint32_t>(d);
+  f.magic = d > 1 && x_max * d < (1ll << 32) ? static_cast<uint32_t>((1ull << 32) / f.d + 1) : 0u;
+  return f;
+}
+
 struct FwdParams {
   int B, H, Sq, Skv;
   int causal, diag_off;
   int nq_blocks, n_items;
+  FastDiv by_units, by_heads, by_blocks, by_split;  // B * H, H, nq_blocks, B * H * parts: an item is decoded by every role
   int pair_far, nq_tiles;    // pair_far: an item is the query tiles i and nq_tiles - 1 - i (see decode_item)
   int unit_major;            // items are numbered unit by unit instead of heaviest block first
   int group;                 // query heads per key/value head (grouped-query attention)
@@ -194,10 +210,11 @@ template <int kMode>
 __device__ __forceinline__ void decode_item(int idx, const FwdParams& p, Item* item) {
   const int bh_count = p.B * p.H;
   if constexpr (kMode == kSolo) {
-    const int bh = idx % bh_count, n = kv_tiles_for((p.nq_tiles - 1 - idx / bh_count) * kTile, p);
-    item->b = bh / p.H;
-    item->h = bh % p.H;
-    item->q0[0] = item->q0[1] = (p.nq_tiles - 1 - idx / bh_count) * kTile;
+    const int i = p.by_units.div(idx), bh = idx - i * bh_count, b = p.by_heads.div(bh);
+    const int q0 = (p.nq_tiles - 1 - i) * kTile, n = kv_tiles_for(q0, p);
+    item->b = b;
+    item->h = bh - b * p.H;
+    item->q0[0] = item->q0[1] = q0;
     item->j0 = 0;
     item->n_kv[0] = (n + 1) / 2;
     item->n_kv[1] = n / 2;
@@ -211,11 +228,12 @@ __device__ __forceinline__ void decode_item(int idx, const FwdParams& p, Item* i
     // run at about the same time and K/V are in L2 for all but the first of them.  It is used
     // when K and V of the whole launch do not fit L2 (otherwise every wave of blocks would fetch
     // them from DRAM again).
-    const int bh = p.unit_major ? idx / p.nq_blocks : idx % bh_count;
-    item->b = bh / p.H;
-    item->h = bh % p.H;
+    const int i = p.unit_major ? p.by_blocks.div(idx) : p.by_units.div(idx);
+    const int bh = p.unit_major ? i : idx - i * bh_count;
+    item->b = p.by_heads.div(bh);
+    item->h = bh - item->b * p.H;
     if (p.unit_major) {
-      const int qb = p.nq_blocks - 1 - idx % p.nq_blocks;
+      const int qb = p.nq_blocks - 1 - (idx - i * p.nq_blocks);
       item->q0[0] = qb * 2 * kTile;
       item->q0[1] = qb * 2 * kTile + kTile;
     } else if (p.pair_far) {
@@ -223,11 +241,11 @@ __device__ __forceinline__ void decode_item(int idx, const FwdParams& p, Item* i
       // adjacent tiles grow with the block index.  Pairing tile i with tile nq_tiles - 1 - i makes
       // every item nq_tiles + 1 tile steps: the early tile shares the first key tiles with the
       // late one, which then runs on alone.
-      const int i = idx / bh_count, far = p.nq_tiles - 1 - i;
+      const int far = p.nq_tiles - 1 - i;
       item->q0[0] = i * kTile;
       item->q0[1] = far > i ? far * kTile : p.Sq;  // (an odd count leaves the middle tile alone)
     } else {
-      const int qb = p.nq_blocks - 1 - idx / bh_count;
+      const int qb = p.nq_blocks - 1 - i;
       item->q0[0] = qb * 2 * kTile;
       item->q0[1] = qb * 2 * kTile + kTile;
     }
@@ -239,13 +257,12 @@ __device__ __forceinline__ void decode_item(int idx, const FwdParams& p, Item* i
     item->nparts[0] = item->nparts[1] = 1;
     return;
   }
-  const int per_block = bh_count * p.parts;
-  const int qb = p.nq_blocks - 1 - idx / per_block;
-  const int rem = idx % per_block;
-  const int bh = rem % bh_count;
-  item->part = rem / bh_count;
-  item->b = bh / p.H;
-  item->h = bh % p.H;
+  const int block = p.by_split.div(idx), rem = idx - block * bh_count * p.parts;
+  const int qb = p.nq_blocks - 1 - block;
+  item->part = p.by_units.div(rem);
+  const int bh = rem - item->part * bh_count;
+  item->b = p.by_heads.div(bh);
+  item->h = bh - item->b * p.H;
   item->q0[0] = qb * 2 * kTile;
   item->q0[1] = qb * 2 * kTile + kTile;
   const int full0 = kv_tiles_for(item->q0[0], p), full1 = kv_tiles_for(item->q0[1], p);
@@ -295,8 +312,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
   __shared__ uint32_t abort_s;
 
   const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
-  const uint32_t sQ = smem_base;                          // one or two tiles
-  const uint32_t sK = smem_base + Rings<kMode>::kQTiles * kTileBytes;  // kKStages tiles
+  const uint32_t sQ = smem_base;                          // an item's two tiles, or one tile each of two items
+  const uint32_t sK = smem_base + 2 * kTileBytes;         // kKStages tiles
   const uint32_t sV = sK + kKStages * kTileBytes;         // kVStages tiles
 
   const int tid = threadIdx.x;
@@ -338,6 +355,21 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tbase = tmem_base_s;
+  // The first item belongs to the set-up too, and so do its first tiles, on their way from DRAM to L2: more of them get in
+  // the way of the loads behind (B1 H4 S512 18.9 -> 19.2 us for H2O), and so does any in a small launch, which seldom comes
+  // up behind another (there 18.0 -> 18.2).  With the items decoded by multiplications, before -> after: B4 H16 S400
+  // 14.3 -> 12.8, B1 H32 S1024 19.8 -> 17.9 (18.3 without the tiles), S2048 39.1 -> 37.3, S4096 124.3 -> 122.5, 500 rows
+  // over 5003 keys, 32/8 heads, 39.9 -> 39.4.
+  Item it_;
+  const bool has_first = get_item<kMode>(0, p, &it_);
+  if (warp == 4 && lane == 0 && has_first && gridDim.x >= 64) {
+    const int hk = it_.h / p.group, kv0 = (kMode == kSplit ? it_.j0 : 0) * kTile;
+    for (int half = 0; half < 128; half += 64) {
+      for (int t = 0; t < Rings<kMode>::kQTiles; ++t)
+        if (it_.n_kv[t] > 0) tma_prefetch_4d(&map_q, half, it_.h, it_.q0[t], it_.b);
+      tma_prefetch_4d(&map_k, half, hk, kv0, it_.b);
+    }
+  }
   // The set-up above may have run while the kernel ahead in the stream was still draining; q, k and
   // v may be that kernel's outputs and out / lse its inputs, so nothing is read or written before
   // it has finished.  The kernel behind this one (the column pass) may be scheduled from now on:
@@ -355,20 +387,21 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
     if (lane == 0) {
       bool ok = true;
       uint32_t kc = 0;            // K tiles issued so far
-      uint32_t qn[2] = {0, 0};    // items in which tile t was loaded so far
-      Item it_;
+      uint32_t qn[2] = {0, 0};    // items in which tile t was loaded so far (kSolo: loads of either buffer)
+      uint32_t items = 0;
       for (int it = 0; it < n_waves && ok; ++it) {
-        if (!get_item<kMode>(it, p, &it_)) continue;
-        for (int t = 0; t < Rings<kMode>::kQTiles && ok; ++t) {
-          if (it_.n_kv[t] == 0) continue;
+        if (it == 0 ? !has_first : !get_item<kMode>(it, p, &it_)) continue;
+        for (int x = 0; x < Rings<kMode>::kQTiles && ok; ++x) {
+          if (it_.n_kv[x] == 0) continue;
+          const int t = kOne ? static_cast<int>(items++ & 1) : x;
           if (qn[t] > 0) {  // the previous item's last QK^T of this tile must have read Q_t
             ok = mbar_wait(smem_u32(&bars.q_empty[t]), (qn[t] - 1) & 1, abortp);
             if (!ok) { record_timeout(p.status, 11); break; }
           }
           const uint32_t bar = smem_u32(&bars.q_full[t]);
           mbar_expect_tx(bar, kTileBytes);
-          tma_load_4d(sQ + t * kTileBytes, &map_q, bar, 0, it_.h, it_.q0[t], it_.b);
-          tma_load_4d(sQ + t * kTileBytes + kHalfBytes, &map_q, bar, 64, it_.h, it_.q0[t], it_.b);
+          tma_load_4d(sQ + t * kTileBytes, &map_q, bar, 0, it_.h, it_.q0[x], it_.b);
+          tma_load_4d(sQ + t * kTileBytes + kHalfBytes, &map_q, bar, 64, it_.h, it_.q0[x], it_.b);
           ++qn[t];
         }
         const int n_tiles = kOne ? it_.n_kv[0] + it_.n_kv[1] : it_.n_max;
@@ -398,9 +431,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
     if (lane == 0) {
       bool ok = true;
       uint32_t vc = 0;
-      Item it_;
       for (int it = 0; it < n_waves && ok; ++it) {
-        if (!get_item<kMode>(it, p, &it_)) continue;
+        if (it == 0 ? !has_first : !get_item<kMode>(it, p, &it_)) continue;
         const int n_tiles = kOne ? it_.n_kv[0] + it_.n_kv[1] : it_.n_max;
         for (int j = 0; j < n_tiles && ok; ++j, ++vc) {
           const int st = vc % kVStages;
@@ -443,9 +475,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
       uint32_t kc = 0;              // K tiles consumed before this item
       uint32_t x = 0;               // uses of S so far (parity of s_free)
       uint32_t on0 = 0, on1 = 0;    // items of either tile before this one (parity of q_full)
-      Item it_;
       for (int it = 0; it < n_waves && ok; ++it) {
-        if (!get_item<kMode>(it, p, &it_)) continue;
+        if (it == 0 ? !has_first : !get_item<kMode>(it, p, &it_)) continue;
         const int n0 = it_.n_kv[0], n1 = it_.n_kv[1];
         for (int j = 0; j < it_.n_max && ok; ++j) {
 #pragma unroll
@@ -455,7 +486,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
             const int st = kidx % kKStages;
             const bool k_hit = mbar_try_wait(smem_u32(&bars.k_full[st]), (kidx / kKStages) & 1);
             const bool s_hit = x == 0 || mbar_try_wait(smem_u32(&bars.s_free), (x - 1) & 1);
-            if (j == 0 && (!kOne || t == 0)) ok = wait_all(&bars.q_full[t], (t ? on1 : on0) & 1, 3);
+            if (j == 0 && !kOne) ok = wait_all(&bars.q_full[t], (t ? on1 : on0) & 1, 3);
+            if (j == 0 && kOne && t == 0) ok = wait_all(&bars.q_full[on0 & 1], (on0 >> 1) & 1, 3);
             if (ok && !__all_sync(0xffffffffu, k_hit)) ok = wait_all(&bars.k_full[st], (kidx / kKStages) & 1, 4);
             if (ok && !__all_sync(0xffffffffu, s_hit)) ok = wait_all(&bars.s_free, (x - 1) & 1, 13);
             if (!ok) break;
@@ -463,7 +495,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
             tc_fence_after_sync();
             if (elect_one()) {
               const uint64_t kdesc = umma_smem_desc_sw128(sK + st * kTileBytes, 16, 1024);
-              const uint64_t qdesc = umma_smem_desc_sw128(sQ + (kOne ? 0 : t) * kTileBytes, 16, 1024);
+              const uint64_t qdesc = umma_smem_desc_sw128(sQ + (kOne ? (on0 & 1) : t) * kTileBytes, 16, 1024);
 #pragma unroll
               for (int kk = 0; kk < 8; ++kk) {
                 const uint64_t off = static_cast<uint64_t>((kk & 3) * 2 + (kk >> 2) * (kHalfBytes >> 4));
@@ -473,7 +505,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
               // the K stage is free after the last QK^T that reads it; Q_t after its last QK^T
               if (kOne || t == 1 || j >= n1) umma_commit(smem_u32(&bars.k_empty[st]));
               if (kOne) {
-                if (2 * j + t == n0 + n1 - 1) umma_commit(smem_u32(&bars.q_empty[0]));
+                if (2 * j + t == n0 + n1 - 1) umma_commit(smem_u32(&bars.q_empty[on0 & 1]));
               } else if (j == (t ? n1 : n0) - 1) {
                 umma_commit(smem_u32(&bars.q_empty[t]));
               }
@@ -501,9 +533,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
       uint32_t vc = 0;              // V tiles consumed before this item
       uint32_t sn0 = 0, sn1 = 0;    // steps of either tile before this item (parity of p_ready)
       uint32_t on0 = 0, on1 = 0;    // items of either tile before this one (parity of o_free)
-      Item it_;
       for (int it = 0; it < n_waves && ok; ++it) {
-        if (!get_item<kMode>(it, p, &it_)) continue;
+        if (it == 0 ? !has_first : !get_item<kMode>(it, p, &it_)) continue;
         const int n0 = it_.n_kv[0], n1 = it_.n_kv[1];
         for (int j = 0; j < it_.n_max && ok; ++j) {
 #pragma unroll
@@ -553,8 +584,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
     const float mul = kCap ? p.cap_out : p.scale_log2;
     bool ok = true;
     uint32_t sn = 0;  // tile steps of this tile before the current item
-    Item it_;
     for (int it = 0; it < n_waves && (ok || kOne); ++it) {
+      Item it_;  // (the first one again: kept from the set-up it would take registers from the row)
       if (!get_item<kMode>(it, p, &it_)) continue;
       const int n_t = it_.n_kv[t];
       if (n_t == 0 && !kOne) continue;
@@ -934,10 +965,11 @@ int attn_fwd_parts(const AttnShape& s, int num_sms, size_t ws_bytes) {
 //     71 -> 44; S 1024, 8 heads 16.3 -> 12.6; S 512, 4 heads 11.2 -> 9.4; unmasked S 2048, 8 heads 29.7 -> 20.4
 //   - with more, if the launch is a causal square, up to a number that grows with its length: the late tiles
 //     are twice as long as the mean, the early ones fill in behind them, and the finer they are the better.
-//     S 1024, 24 heads (1.3 tiles per SM) 18.9 -> 16.7; S 1500, 24 heads (1.9) 23.6 -> 23.4; S 2048, 16 heads
-//     (1.7) 28.1 -> 24.8 and 20 heads (2.2) 32.5 -> 30.6; S 4096, 8 heads (1.7) 45.8 -> 35.1; beyond it
-//     S 1024, 32 heads (1.7) 19.7 -> 20.1; S 8192, 8 heads (3.5) 112 -> 126; and not square, 1024 rows over
-//     8000 keys, 32/8 heads (1.7) 108 -> 118
+//     Two -> one: S 600, 32 heads (1.1 tiles per SM) 13.3 -> 12.9; S 700, 30 heads (1.2) 14.5 -> 14.2, 32 heads (1.3)
+//     14.8 -> 15.0; S 1024, 25 heads (1.4) 17.4 -> 16.6, 28 heads (1.5) 17.6 -> 18.0; S 1500, 22 heads (1.8) 21.7 -> 21.5,
+//     24 heads (1.9) 21.9 -> 22.2; S 2048, 20 heads (2.2) 31.5 -> 29.9, 22 heads (2.4) 31.6 -> 32.3; S 4096, 11 heads
+//     (2.4) 54.3 -> 49.4; S 8000, 6 heads (2.6) 97 -> 91; beyond it S 8192, 8 heads (3.5) 112 -> 126; and not square,
+//     1024 rows over 8000 keys, 32/8 heads (1.7) 108 -> 118
 static bool attn_fwd_solo(const AttnShape& s, int num_sms) {
 #ifdef ASUKA_TUNE_ENV
   if (const char* e = getenv("ASUKA_FWD_SOLO")) return atoi(e) != 0;
@@ -945,7 +977,8 @@ static bool attn_fwd_solo(const AttnShape& s, int num_sms) {
   const int nq_tiles = (s.Sq + kTile - 1) / kTile;
   const long long n_tiles = static_cast<long long>(nq_tiles) * s.B * s.H;
   if (n_tiles <= num_sms) return s.Skv > 2 * kTile;
-  return s.causal && 4LL * s.Skv <= 5LL * s.Sq && 8 * n_tiles <= static_cast<long long>(num_sms) * ((nq_tiles < 16 ? nq_tiles : 16) + 4);
+  const int length = nq_tiles < 10 ? nq_tiles + 4 : nq_tiles < 16 ? nq_tiles + 3 : nq_tiles < 32 ? 19 : 20;
+  return s.causal && 4LL * s.Skv <= 5LL * s.Sq && 8 * n_tiles <= static_cast<long long>(num_sms) * length;
 }
 
 size_t attn_fwd_split_bytes(const AttnShape& s, int parts) {
@@ -973,6 +1006,11 @@ cudaError_t launch_attn_fwd(const CUtensorMap& mq, const CUtensorMap& mk, const 
     const double kv_bytes = 2.0 * s.B * (s.H / (s.group > 0 ? s.group : 1)) * static_cast<double>(s.Skv) * 128 * 2;
     p.unit_major = (p.parts == 1 && p.n_items > num_sms && kv_bytes > 96e6) ? 1 : 0;
   }
+  const long long x_max = p.n_items;
+  p.by_units = fast_div(s.B * s.H, x_max);
+  p.by_heads = fast_div(s.H, s.B * s.H);
+  p.by_blocks = fast_div(p.nq_blocks, x_max);
+  p.by_split = fast_div(s.B * s.H * p.parts, x_max);
   p.pair_far = (p.parts == 1 && !solo && s.causal && p.n_items <= num_sms && p.nq_tiles >= 4) ? 1 : 0;
   p.group = s.group;
   p.scale_log2 = s.softmax_scale * 1.4426950408889634f;

@@ -123,6 +123,11 @@ __device__ __forceinline__ void tma_load_4d(uint32_t smem_dst, const CUtensorMap
         "r"(c3)
       : "memory");
 }
+// the same box into L2 only: a hint, without an effect on what any later access sees
+__device__ __forceinline__ void tma_prefetch_4d(const CUtensorMap* map, int c0, int c1, int c2, int c3) {
+  asm volatile("cp.async.bulk.prefetch.tensor.4d.L2.global [%0, {%1, %2, %3, %4}];"
+               ::"l"(reinterpret_cast<uint64_t>(map)), "r"(c0), "r"(c1), "r"(c2), "r"(c3) : "memory");
+}
 // L2 eviction priority for data that is read exactly once (streamed operands): such lines are the
 // first to go, which keeps what will be read again resident
 __device__ __forceinline__ uint64_t l2_policy_evict_first() {
