@@ -58,11 +58,11 @@ template <int kMode> struct Rings {
 constexpr int kThreads = 384;
 // Registers of the utility and of the softmax warps; what a block asks for must fit its 384 * 168 = 64512.
 // The soft-capped one-tile mode has both ways of the tanh beside what its merge keeps: at 200 it spills 464
-// bytes (B1 S1024, 16/8 heads 22 us), at 216 140 (17.6).
-// The others at 200 or 208: B1 H32 S1024 18.6 and 17.9.
+// bytes, at 216 156, at 224 84 (S4000, 8 heads 53.6 -> 51.9 us from 216 to 224, 52.5 at 232).  The others at 200 or 208:
+// B1 H32 S1024 18.6 and 17.9.
 template <bool kCap, int kMode> struct Regs {
-  static constexpr int kUtil = kCap && kMode == kSolo ? 72 : 88;
-  static constexpr int kSoftmax = kCap && kMode == kSolo ? 216 : 208;
+  static constexpr int kUtil = kCap && kMode == kSolo ? 56 : 88;
+  static constexpr int kSoftmax = kCap && kMode == kSolo ? 224 : 208;
   static constexpr int kBlock = 128 * kUtil + 256 * kSoftmax;
   static_assert(kBlock <= kThreads * 168, "setmaxnreg would wait for ever");
 };
@@ -585,8 +585,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
     bool ok = true;
     uint32_t sn = 0;  // tile steps of this tile before the current item
     for (int it = 0; it < n_waves && (ok || kOne); ++it) {
-      Item it_;  // (the first one again: kept from the set-up it would take registers from the row)
-      if (!get_item<kMode>(it, p, &it_)) continue;
+      if (it == 0 ? !has_first : !get_item<kMode>(it, p, &it_)) continue;
       const int n_t = it_.n_kv[t];
       if (n_t == 0 && !kOne) continue;
       const int row = it_.q0[t] + r_in_tile;
