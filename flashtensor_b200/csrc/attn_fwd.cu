@@ -32,6 +32,7 @@
 #include <cstdlib>
 #include <type_traits>
 
+#include "fast_div.cuh"
 #include "kernels.h"
 #include "sm100_ptx.cuh"
 
@@ -69,20 +70,6 @@ template <bool kCap, int kMode> struct Regs {
 constexpr uint32_t kSmemBytes = 7 * kTileBytes + 1024;
 constexpr float kRescaleLimit = 6.0f;  // log2 of the largest exponential tolerated under a stale reference:
                                        // keeps a tile's row sum below 2^13, far from fp16's 65504
-
-// x / d by a multiplication while x * d < 2^32 (the caller's matter), else as it is
-struct FastDiv {
-  uint32_t d, magic;  // magic 0: divide
-  __device__ __forceinline__ int div(int x) const {
-    return static_cast<int>(magic != 0 ? __umulhi(static_cast<uint32_t>(x), magic) : static_cast<uint32_t>(x) / d);
-  }
-};
-FastDiv fast_div(int d, long long x_max) {
-  FastDiv f;
-  f.d = static_cast<uint32_t>(d);
-  f.magic = d > 1 && x_max * d < (1ll << 32) ? static_cast<uint32_t>((1ull << 32) / f.d + 1) : 0u;
-  return f;
-}
 
 struct FwdParams {
   int B, H, Sq, Skv;

@@ -316,7 +316,7 @@ int col_scores_impl(const asuka_score_params* p, cudaStream_t stream, bool chain
   size_t usable = 0;
   void* split_ws = align_ws(ws != nullptr ? ws : p->workspace, ws != nullptr ? ws_bytes : p->workspace_bytes, &usable);
   const int chunks = col_scores_chunks(c.s, a.mode, sms, usable);
-  return map_cuda(launch_col_scores(mq, mk, a, c.s, split_ws, chunks, stream, pending));
+  return map_cuda(launch_col_scores(mq, mk, a, c.s, sms, split_ws, chunks, stream, pending));
 }
 
 int kf_rowstat_impl(const asuka_score_params* p, cudaStream_t stream, bool chained = false) {

@@ -32,6 +32,7 @@
 #include <cstdlib>
 
 #include "../../include/asuka_b200.h"
+#include "fast_div.cuh"
 #include "kernels.h"
 #include "score_math.cuh"
 #include "sm100_ptx.cuh"
@@ -61,6 +62,7 @@ template <int kMode> struct ColCfg {
   static constexpr int kQueries = 128 / kSubs;     // queries of a tile for each
   static constexpr int kThreads = (kUtilWarps + kKeyWarps) * 32;
   static constexpr int kCtas = kMode == 2 || kMode == 4 ? 1 : 2;
+  static constexpr bool kLoop = kMode == 0 || kMode == 1;  // a CTA may work through several items
 };
 constexpr int kQStages = 2;                       // Q tiles; free again as soon as the MMA has read them
 constexpr int kLseStages = 4;                     // row statistics of the Q tiles; free when the key warps have read them
@@ -89,12 +91,16 @@ struct ColParams {
   // leaves its partial sums in `part` ([n_qchunks, B*H, Skv], and `part_sq` alike) and
   // sum_chunks_kernel adds them in range order.  n_qchunks = 1: no split, results go to `score`.
   int q_chunk, n_qchunks;
+  FastDiv by_units, by_heads;  // B * H, H
+  int n_items;        // (key tile, query range, unit); as many CTAs, or fewer that take every gridDim.x-th
   float* part;
   float* part_sq;
 };
 
 struct ColBars {
   uint64_t k_full;
+  uint64_t lse_first;  // (chained) the row statistics of the Q tiles that were fetched ahead of them
+  uint64_t part_full;  // an item's partial sums
   uint64_t q_full[kQStages], q_empty[kQStages];
   uint64_t lse_empty[kLseStages];
   uint64_t s_full[2], s_empty[2];
@@ -178,8 +184,9 @@ col_scores_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
   __shared__ __align__(8) ColBars bars;
   __shared__ __align__(16) float lse_s[kLseStages][kTile];  // minus the row statistic
   constexpr int kCh = ColCfg<kMode>::kChunk;
+  constexpr bool kLoop = ColCfg<kMode>::kLoop;
   constexpr int kKeyWarps = ColCfg<kMode>::kKeyWarps, kSubs = ColCfg<kMode>::kSubs, kQueries = ColCfg<kMode>::kQueries;
-  __shared__ float part_s[2][kSubs][kTile];  // [sum, sum of squares][share of the queries][key]
+  __shared__ float part_s[2][2][kSubs][kTile];  // [parity of the item][sum, sum of squares][share of the queries][key]
   __shared__ uint32_t tmem_base_s;
   __shared__ uint32_t abort_s;
 
@@ -192,16 +199,29 @@ col_scores_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
   const int lane = tid & 31;
   volatile uint32_t* abortp = &abort_s;
 
+  // A CTA's items, one key tile of one (batch, head) each: one alone, or (ColParams::n_items) every gridDim.x-th.  Steps
+  // are counted through all of them; ring stages and barrier parities follow from the running counts.
   const int bh_count = p.B * p.H;
-  const int blk = static_cast<int>(blockIdx.x) / bh_count;
-  const int kt = blk / p.n_qchunks;  // low key tiles are the long ones
-  const int qc = p.n_qchunks - 1 - blk % p.n_qchunks;  // (late query ranges see the most keys)
-  const int bh = static_cast<int>(blockIdx.x) % bh_count;
-  const int b = bh / p.H, h = bh % p.H;
-  const int kv0 = kt * kTile;
-  // this CTA's query tiles: its range, from the first tile that can see its first key
-  const int i_begin = max(qc * p.q_chunk, p.causal ? max(0, kv0 - p.diag_off) / kTile : 0);
-  const int i_end = min(p.nq_tiles, (qc + 1) * p.q_chunk);
+  struct Item {
+    int kv0, b, h, bh, qc, i_begin, i_end;  // first key; (batch, head); query range and this item's query tiles of it
+  };
+  auto load_item = [&](int idx, Item& m) -> bool {
+    if (idx >= p.n_items) return false;
+    const int blk = p.by_units.div(idx);
+    const int kt = p.n_qchunks == 1 ? blk : blk / p.n_qchunks;  // low key tiles are the long ones
+    m.qc = p.n_qchunks - 1 - (blk - kt * p.n_qchunks);  // (late query ranges see the most keys)
+    m.bh = idx - blk * bh_count;
+    m.b = p.by_heads.div(m.bh);
+    m.h = m.bh - m.b * p.H;
+    m.kv0 = kt * kTile;
+    // this item's query tiles: its range, from the first tile that can see its first key
+    m.i_begin = max(m.qc * p.q_chunk, p.causal ? max(0, m.kv0 - p.diag_off) / kTile : 0);
+    m.i_end = max(m.i_begin, min(p.nq_tiles, (m.qc + 1) * p.q_chunk));
+    return true;
+  };
+  Item m;
+  const int idx0 = static_cast<int>(blockIdx.x), stride = kLoop ? static_cast<int>(gridDim.x) : p.n_items;
+  load_item(idx0, m);
 
   // Launched as a programmatic dependent: unless the caller vouches for the kernel ahead (the fused
   // case entry points, whose forward kernel writes only the output and the row statistic), q and k
@@ -213,6 +233,8 @@ col_scores_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
   if (tid == 0) {
     abort_s = 0;
     mbar_init(smem_u32(&bars.k_full), 1);
+    mbar_init(smem_u32(&bars.lse_first), 1);
+    mbar_init(smem_u32(&bars.part_full), kKeyWarps);
     for (int i = 0; i < kQStages; ++i) {
       mbar_init(smem_u32(&bars.q_full[i]), 1);
       mbar_init(smem_u32(&bars.q_empty[i]), 1);
@@ -229,8 +251,8 @@ col_scores_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
     // and the CTA-wide barrier below (this thread initialised the barrier it signals)
     const uint32_t bar = smem_u32(&bars.k_full);
     mbar_expect_tx(bar, kTileBytes);
-    tma_load_4d(sK, &map_k, bar, 0, h / p.group, kv0, b);
-    tma_load_4d(sK + kHalfBytes, &map_k, bar, 64, h / p.group, kv0, b);
+    tma_load_4d(sK, &map_k, bar, 0, m.h / p.group, m.kv0, m.b);
+    tma_load_4d(sK + kHalfBytes, &map_k, bar, 64, m.h / p.group, m.kv0, m.b);
   }
   if (warp == 1) {
     __syncwarp();
@@ -244,38 +266,70 @@ col_scores_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
 
   if (warp == 0) {
     // ------------------------------------------------------------------ producer (whole warp)
-    const float* lse_row = p.lse2 + (static_cast<size_t>(b) * p.H + h) * p.Sq;
     const float lse_shift = kMode == 3 ? -kSeededLg2Unit * p.inv_tau : 0.f;  // (seeded_lg2_exp_rand2)
     bool ok = true;
-    if (p.chained) griddep_wait();  // the row statistic is the output of the kernel ahead
-    for (int i = i_begin; i < i_end; ++i) {
-      const int c = i - i_begin;
-      const int st = c % kQStages, ls = c % kLseStages;
-      if (c >= kLseStages)
-        ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&bars.lse_empty[ls]), (c / kLseStages - 1) & 1, abortp));
-      // NEGATED row statistics of this query tile (they are only ever subtracted); rows past the
-      // end get -inf so that exp2 gives 0
-      if (ok) {
-#pragma unroll
-        for (int r = 0; r < 4; ++r) {
-          const int qi = i * kTile + r * 32 + lane;
-          lse_s[ls][r * 32 + lane] = qi < p.Sq ? lse_shift - __ldg(lse_row + qi) : -INFINITY;
-        }
-        if (c >= kQStages)
-          ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&bars.q_empty[st]), (c / kQStages - 1) & 1, abortp));
-      }
-      if (!ok) { if (lane == 0) record_timeout(p.status, 21); break; }
-      __syncwarp();
+    auto load_q = [&](uint32_t c, int i) {
       if (lane == 0) {
+        const int st = c % kQStages;
         const uint32_t bar = smem_u32(&bars.q_full[st]);
         mbar_expect_tx(bar, kTileBytes);
-        tma_load_4d(sQ + st * kTileBytes, &map_q, bar, 0, h, i * kTile, b);
-        tma_load_4d(sQ + st * kTileBytes + kHalfBytes, &map_q, bar, 64, h, i * kTile, b);
+        tma_load_4d(sQ + st * kTileBytes, &map_q, bar, 0, m.h, i * kTile, m.b);
+        tma_load_4d(sQ + st * kTileBytes + kHalfBytes, &map_q, bar, 64, m.h, i * kTile, m.b);
       }
+    };
+    // The row statistic is the output of the kernel ahead, Q is not: the first tiles, and their S, need not wait for it.
+    const int early = p.chained ? min(kQStages, m.i_end - m.i_begin) : 0;
+    for (int x = 0; x < early; ++x) load_q(x, m.i_begin + x);
+    if (p.chained) griddep_wait();
+    uint32_t c = 0;       // steps
+    uint32_t k_loads = 1;
+    bool more = idx0 < p.n_items;
+    for (int idx = idx0; more && ok;) {
+      if (c > 0) {
+        // the K tile of the item before is free once the last MMA that read it has retired
+        const uint32_t last = c - 1;
+        ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&bars.s_full[last & 1]), (last >> 1) & 1, abortp));
+        if (!ok) { if (lane == 0) record_timeout(p.status, 27); break; }
+      }
+      if (idx != idx0) {
+        if (lane == 0) {
+          const uint32_t bar = smem_u32(&bars.k_full);
+          mbar_expect_tx(bar, kTileBytes);
+          tma_load_4d(sK, &map_k, bar, 0, m.h / p.group, m.kv0, m.b);
+          tma_load_4d(sK + kHalfBytes, &map_k, bar, 64, m.h / p.group, m.kv0, m.b);
+        }
+        ++k_loads;
+        __syncwarp();
+      }
+      const float* lse_row = p.lse2 + (static_cast<size_t>(m.b) * p.H + m.h) * p.Sq;
+      for (int i = m.i_begin; i < m.i_end; ++i, ++c) {
+        const int st = c % kQStages, ls = c % kLseStages;
+        if (c >= kLseStages)
+          ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&bars.lse_empty[ls]), (c / kLseStages - 1) & 1, abortp));
+        // NEGATED row statistics of this query tile (they are only ever subtracted); rows past the
+        // end get -inf so that exp2 gives 0
+        if (ok) {
+#pragma unroll
+          for (int r = 0; r < 4; ++r) {
+            const int qi = i * kTile + r * 32 + lane;
+            lse_s[ls][r * 32 + lane] = qi < p.Sq ? lse_shift - __ldg(lse_row + qi) : -INFINITY;
+          }
+          if (c >= kQStages)
+            ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&bars.q_empty[st]), (c / kQStages - 1) & 1, abortp));
+        }
+        if (!ok) { if (lane == 0) record_timeout(p.status, 21); break; }
+        __syncwarp();
+        if (static_cast<int>(c) >= early) load_q(c, i);
+        else if (static_cast<int>(c) == early - 1 && lane == 0) mbar_arrive(smem_u32(&bars.lse_first));
+      }
+      idx += stride;
+      more = kLoop && ok && load_item(idx, m);
     }
-    if (lane == 0 && (!ok || i_begin >= i_end)) {  // nothing else waits for the K tile then
+    if (lane == 0 && (!ok || c == 0)) {  // copies that nothing else waits for then
       volatile uint32_t none = 0;
-      mbar_wait(smem_u32(&bars.k_full), 0, &none);
+      mbar_wait(smem_u32(&bars.k_full), (k_loads - 1) & 1, &none);
+      for (uint32_t x = c > kQStages ? c - kQStages : 0; x < max(c, static_cast<uint32_t>(early)); ++x)
+        mbar_wait(smem_u32(&bars.q_full[x % kQStages]), (x / kQStages) & 1, &none);
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------------ MMA issuer
@@ -288,48 +342,60 @@ col_scores_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
       if (!good && lane == 0) record_timeout(p.status, site);
       return good;
     };
-    bool ok = wait_all(&bars.k_full, 0, 22);
+    bool ok = true;
     const uint64_t kdesc = umma_smem_desc_sw128(sK, 16, 1024);
-    for (int i = i_begin; i < i_end && ok; ++i) {
-      const int c = i - i_begin;
-      const int st = c % kQStages, buf = c & 1;
-      ok = wait_all(&bars.q_full[st], (c / kQStages) & 1, 23);
-      if (ok && c >= 2) ok = wait_all(&bars.s_empty[buf], ((c >> 1) - 1) & 1, 24);
-      if (!ok) break;
-      tc_fence_after_sync();
-      const uint64_t qdesc = umma_smem_desc_sw128(sQ + st * kTileBytes, 16, 1024);
-      if (elect_one()) {
+    uint32_t c = 0, k_loads = 0;
+    bool more = idx0 < p.n_items;
+    for (int idx = idx0; more && ok;) {
+      ok = wait_all(&bars.k_full, k_loads & 1, 22);
+      ++k_loads;
+      for (int i = m.i_begin; i < m.i_end && ok; ++i, ++c) {
+        const int st = c % kQStages, buf = c & 1;
+        ok = wait_all(&bars.q_full[st], (c / kQStages) & 1, 23);
+        if (ok && c >= 2) ok = wait_all(&bars.s_empty[buf], ((c >> 1) - 1) & 1, 24);
+        if (!ok) break;
+        tc_fence_after_sync();
+        const uint64_t qdesc = umma_smem_desc_sw128(sQ + st * kTileBytes, 16, 1024);
+        if (elect_one()) {
 #pragma unroll
-        for (int kk = 0; kk < 8; ++kk) {
-          const uint64_t off = static_cast<uint64_t>((kk & 3) * 2 + (kk >> 2) * (kHalfBytes >> 4));
-          umma_ss(tbase + buf * 128, kdesc + off, qdesc + off, idesc, kk > 0 ? 1u : 0u);
+          for (int kk = 0; kk < 8; ++kk) {
+            const uint64_t off = static_cast<uint64_t>((kk & 3) * 2 + (kk >> 2) * (kHalfBytes >> 4));
+            umma_ss(tbase + buf * 128, kdesc + off, qdesc + off, idesc, kk > 0 ? 1u : 0u);
+          }
+          umma_commit(smem_u32(&bars.s_full[buf]));
+          umma_commit(smem_u32(&bars.q_empty[st]));
         }
-        umma_commit(smem_u32(&bars.s_full[buf]));
-        umma_commit(smem_u32(&bars.q_empty[st]));
+        __syncwarp();
       }
-      __syncwarp();
+      idx += stride;
+      more = kLoop && load_item(idx, m);
     }
   } else {
     // ------------------------------------------------------------------ one thread per (key, share of the queries)
     const int hq = (warp - kUtilWarps) >> 2;  // which kQueries queries of every query tile
     const int wq = warp & 3;       // TMEM lane quarter this warp may touch (every four consecutive key warps cover all four)
-    const int key = kv0 + wq * 32 + lane;
     const uint32_t lane_base = static_cast<uint32_t>(wq * 32) << 16;
     const float scale = p.scale_log2;
-    float acc[4] = {0.f, 0.f, 0.f, 0.f};
-    float acc2[4] = {0.f, 0.f, 0.f, 0.f};
     bool ok = true;
-    const uint32_t head_key = kMode == 3 ? seeded_head_key(p.seed, static_cast<uint32_t>(bh) + p.unit_off) : 0u;
-    const float* er_col = nullptr;
-    if constexpr (kMode == 2 || kMode == 4) {  // mode 4: the threshold operand, strides 0 for b and h
-      er_col = p.exp_rand + static_cast<int64_t>(b) * p.er_sb + static_cast<int64_t>(h) * p.er_sh +
-               min(key, p.Skv - 1);
-    }
-    bool hit = false;
+    uint32_t c = 0, items = 0;
+    // (the first Q tiles did not wait for their row statistics)
+    if (p.chained && m.i_end > m.i_begin) ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&bars.lse_first), 0, abortp));
+    if (!ok && lane == 0) record_timeout(p.status, 29);
+    bool more = ok && idx0 < p.n_items;
+    for (int idx = idx0; more;) {
+      const int kv0 = m.kv0, b = m.b, h = m.h, bh = m.bh;
+      const int key = kv0 + wq * 32 + lane;
+      float acc[4] = {0.f, 0.f, 0.f, 0.f};
+      float acc2[4] = {0.f, 0.f, 0.f, 0.f};
+      const uint32_t head_key = kMode == 3 ? seeded_head_key(p.seed, static_cast<uint32_t>(bh) + p.unit_off) : 0u;
+      const float* er_col = nullptr;
+      if constexpr (kMode == 2 || kMode == 4) {  // mode 4: the threshold operand, strides 0 for b and h
+        er_col = p.exp_rand + static_cast<int64_t>(b) * p.er_sb + static_cast<int64_t>(h) * p.er_sh +
+                 min(key, p.Skv - 1);
+      }
+      bool hit = false;
 
-    {
-      for (int i = i_begin; i < i_end; ++i) {
-        const int c = i - i_begin;
+      for (int i = m.i_begin; i < m.i_end; ++i, ++c) {
         const int ls = c % kLseStages, buf = c & 1;
         {
           // S^T of this step is complete; its MMAs were issued after Q and the row statistics of
@@ -358,7 +424,7 @@ col_scores_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
               }
               // the operand is read once, straight from HBM: pull the same chunk of the next query
               // tile into L2 now, so that its loads find it there one step later
-              if (i + 1 < i_end) {
+              if (i + 1 < m.i_end) {
 #pragma unroll
                 for (int e = 0; e < 32; ++e) {
                   const int qi = min(q_base + kTile + ch * kCh + e, p.Sq - 1);
@@ -456,11 +522,39 @@ col_scores_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
         __syncwarp();
         if (lane == 0) mbar_arrive(smem_u32(&bars.lse_empty[ls]));
       }
+      // All shares of the queries leave their parts in shared memory; the first one's warps add them in a fixed
+      // order and store.  (The other parity's parts may still be read by a warp that is an item behind.)
+      float (*part)[kSubs][kTile] = part_s[items & 1];
+      const int k_in_tile = wq * 32 + lane;
+      part[0][hq][k_in_tile] = kMode == 4 ? (hit ? 1.f : 0.f) : (acc[0] + acc[1]) + (acc[2] + acc[3]);
+      part[1][hq][k_in_tile] = (acc2[0] + acc2[1]) + (acc2[2] + acc2[3]);
+      __syncwarp();
+      if (lane == 0) mbar_arrive(smem_u32(&bars.part_full));
+      if (ok) {
+        ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&bars.part_full), items & 1, abortp));
+        if (!ok && lane == 0) record_timeout(p.status, 28);
+      }
+      if (!ok) break;
+      if (hq == 0 && key < p.Skv) {
+        const size_t o = (static_cast<size_t>(b) * p.H + h) * p.Skv + key;
+        float v = part[0][0][k_in_tile] + part[0][1][k_in_tile];
+        if constexpr (kSubs == 4) v += part[0][2][k_in_tile] + part[0][3][k_in_tile];
+        // with a query-range split the sums of this range go to its slab of the workspace (a range
+        // that sees none of the keys leaves zeros there)
+        const size_t slab = static_cast<size_t>(m.qc) * bh_count * p.Skv;
+        if (items == 0 && p.chained) griddep_wait();
+        if constexpr (kMode == 4) {
+          reinterpret_cast<uint8_t*>(p.score)[o] = v != 0.f ? 1 : 0;
+        } else {
+          (p.n_qchunks > 1 ? p.part + slab : p.score)[o] = v;
+        }
+        if constexpr (kMode == 1)
+          (p.n_qchunks > 1 ? p.part_sq + slab : p.score_sq)[o] = part[1][0][k_in_tile] + part[1][1][k_in_tile];
+      }
+      ++items;
+      idx += stride;
+      more = kLoop && load_item(idx, m);
     }
-    // All shares of the queries leave their parts in shared memory; after the CTA-wide barrier below the
-    // first one's thread adds them in a fixed order and stores.
-    part_s[0][hq][wq * 32 + lane] = kMode == 4 ? (hit ? 1.f : 0.f) : (acc[0] + acc[1]) + (acc[2] + acc[3]);
-    part_s[1][hq][wq * 32 + lane] = (acc2[0] + acc2[1]) + (acc2[2] + acc2[3]);
     if (!ok) *abortp = 1u;
   }
 
@@ -469,25 +563,6 @@ col_scores_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
   if (warp == 1) {
     __syncwarp();
     tmem_dealloc(tbase, 256);
-  }
-  if (warp >= kUtilWarps && warp < kUtilWarps + 4 && !*abortp) {
-    const int k_in_tile = (warp & 3) * 32 + lane;
-    const int key = kv0 + k_in_tile;
-    if (key < p.Skv) {
-      const size_t o = (static_cast<size_t>(b) * p.H + h) * p.Skv + key;
-      float v = part_s[0][0][k_in_tile] + part_s[0][1][k_in_tile];
-      if constexpr (kSubs == 4) v += part_s[0][2][k_in_tile] + part_s[0][3][k_in_tile];
-      // with a query-range split the sums of this range go to its slab of the workspace (a range
-      // that sees none of the keys leaves zeros there)
-      const size_t slab = static_cast<size_t>(qc) * bh_count * p.Skv;
-      if constexpr (kMode == 4) {
-        reinterpret_cast<uint8_t*>(p.score)[o] = v != 0.f ? 1 : 0;
-      } else {
-        (p.n_qchunks > 1 ? p.part + slab : p.score)[o] = v;
-      }
-      if constexpr (kMode == 1)
-        (p.n_qchunks > 1 ? p.part_sq + slab : p.score_sq)[o] = part_s[1][0][k_in_tile] + part_s[1][1][k_in_tile];
-    }
   }
 }
 
@@ -1228,6 +1303,8 @@ ColParams make_params(const ScoreArgs& a, const AttnShape& s) {
   p.part = nullptr;
   p.part_sq = nullptr;
   p.tail_units = 0;
+  p.n_items = 0;
+  p.by_units = p.by_heads = FastDiv{1, 0};
   return p;
 }
 
@@ -1261,7 +1338,7 @@ size_t col_scores_split_bytes(const AttnShape& s, int mode, int chunks) {
 }
 
 cudaError_t launch_col_scores(const CUtensorMap& mq, const CUtensorMap& mk, const ScoreArgs& a,
-                              const AttnShape& s, void* split_ws, int chunks, cudaStream_t stream,
+                              const AttnShape& s, int num_sms, void* split_ws, int chunks, cudaStream_t stream,
                               PendingChunkSum* pending) {
   ColParams p = make_params(a, s);
   if (pending != nullptr) pending->n_chunks = 0;
@@ -1296,7 +1373,17 @@ cudaError_t launch_col_scores(const CUtensorMap& mq, const CUtensorMap& mk, cons
 #endif
   {
   const int n_kt = (s.Skv + kTile - 1) / kTile;
-  const dim3 grid(static_cast<unsigned>(n_kt) * p.n_qchunks * s.B * s.H);
+  p.n_items = n_kt * p.n_qchunks * s.B * s.H;
+  p.by_units = fast_div(s.B * s.H, p.n_items);
+  p.by_heads = fast_div(s.H, s.B * s.H);
+  int ctas = p.n_items;
+  const bool sums = a.mode == ASUKA_SCORE_SUM || a.mode == ASUKA_SCORE_SUM_SQ;
+  // With few query tiles a CTA is set-up for most of its life (barriers, tensor memory, K), and then two CTAs to an SM
+  // that go through all key tiles are faster (H2O, us: 100 rows over 8000 keys, 32/8 heads, 58.3 -> 47.3; 500 over 5003
+  // 72.0 -> 70.0; 2 x 200 over 1500, 16/4 heads 27.3 -> 26.2); with more the order in which SMs become free deals them
+  // out better (1000 over 8000, 16/8 heads 98.7 -> 102.4; B2 H40 S700 37.7 -> 38.7).
+  if (sums && p.n_qchunks == 1 && p.nq_tiles <= 4) ctas = std::min(ctas, 2 * num_sms);
+  const dim3 grid(static_cast<unsigned>(ctas));
   void (*kern)(CUtensorMap, CUtensorMap, ColParams) = nullptr;
   if (a.mode == ASUKA_SCORE_SUM) kern = s.bf16 ? col_scores_kernel<true, 0> : col_scores_kernel<false, 0>;
   else if (a.mode == ASUKA_SCORE_SUM_SQ) kern = s.bf16 ? col_scores_kernel<true, 1> : col_scores_kernel<false, 1>;

@@ -107,7 +107,7 @@ struct PendingChunkSum {
   int n_chunks;          // 0: nothing pending, the scores are final
 };
 cudaError_t launch_col_scores(const CUtensorMap& mq, const CUtensorMap& mk, const ScoreArgs& a,
-                              const AttnShape& s, void* split_ws, int chunks, cudaStream_t stream,
+                              const AttnShape& s, int num_sms, void* split_ws, int chunks, cudaStream_t stream,
                               PendingChunkSum* pending = nullptr);
 int col_scores_chunks(const AttnShape& s, int mode, int num_sms, size_t ws_bytes);
 size_t col_scores_split_bytes(const AttnShape& s, int mode, int chunks);

@@ -264,6 +264,19 @@ def test_keyformer_seeded_noise_vs_oracle(ops, shape, dtype):
   no_timeouts(ops)
 
 
+@pytest.mark.parametrize("shape", [(1, 1, 1300, 32), (2, 128, 1300, 16), (1, 129, 1289, 40), (1, 512, 1920, 32)])
+def test_scores_of_few_rows_over_many_keys_vs_oracle(ops, shape):
+  # more key tiles than CTAs run at once: every CTA of the column pass works through several, one after the other
+  B, Sq, Skv, H = shape
+  q, k, v = O.make_inputs("roco", B, Sq, Skv, H, 128, torch.bfloat16, seed=37)
+  ref = O.roco(q, k, v)
+  got = ops.roco(q.cuda(), k.cuda(), v.cuda())
+  score = ops.h2o(q.cuda(), k.cuda(), v.cuda())[1]
+  for g, r, n in zip(got + (score,), ref + (ref[1],), ("out", "roco_score", "roco_sq_score", "h2o_score")):
+    close(g, r, n)
+  no_timeouts(ops)
+
+
 @pytest.mark.parametrize("noise", ["dense", "odd", "broadcast", "seeded"])
 @pytest.mark.parametrize("shape", [  # (B, Sq, Skv, H, causal): row blocks and key tiles about one CTA's share and about a cluster's
     (1, 1, 1, 1, True), (1, 128, 128, 2, True), (2, 129, 129, 3, True), (1, 200, 512, 2, True), (1, 513, 513, 40, False),
