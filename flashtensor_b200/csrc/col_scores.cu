@@ -62,7 +62,6 @@ template <int kMode> struct ColCfg {
   static constexpr int kQueries = 128 / kSubs;     // queries of a tile for each
   static constexpr int kThreads = (kUtilWarps + kKeyWarps) * 32;
   static constexpr int kCtas = kMode == 2 || kMode == 4 ? 1 : 2;
-  static constexpr bool kLoop = kMode == 0 || kMode == 1;  // a CTA may work through several items
 };
 constexpr int kQStages = 2;                       // Q tiles; free again as soon as the MMA has read them
 constexpr int kLseStages = 4;                     // row statistics of the Q tiles; free when the key warps have read them
@@ -176,7 +175,7 @@ __device__ __forceinline__ float2 ex2_fma_pipe(float2 x) {
 
 // kMode: 0 sum, 1 sum + sum of squares, 2 perturbed (noise operand), 3 perturbed (seeded noise),
 //        4 CORM: any_i(p_ij >= mask_ij) with a [Sq, Skv] threshold operand (cases/kernels/corm.py:34-37)
-template <bool kBF16, int kMode>
+template <bool kBF16, int kMode, bool kLoop = false>
 __global__ void __launch_bounds__(ColCfg<kMode>::kThreads, ColCfg<kMode>::kCtas)
 col_scores_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                   const ColParams p) {
@@ -184,7 +183,6 @@ col_scores_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
   __shared__ __align__(8) ColBars bars;
   __shared__ __align__(16) float lse_s[kLseStages][kTile];  // minus the row statistic
   constexpr int kCh = ColCfg<kMode>::kChunk;
-  constexpr bool kLoop = ColCfg<kMode>::kLoop;
   constexpr int kKeyWarps = ColCfg<kMode>::kKeyWarps, kSubs = ColCfg<kMode>::kSubs, kQueries = ColCfg<kMode>::kQueries;
   __shared__ float part_s[2][2][kSubs][kTile];  // [parity of the item][sum, sum of squares][share of the queries][key]
   __shared__ uint32_t tmem_base_s;
@@ -1382,10 +1380,13 @@ cudaError_t launch_col_scores(const CUtensorMap& mq, const CUtensorMap& mk, cons
   // that go through all key tiles are faster (H2O, us: 100 rows over 8000 keys, 32/8 heads, 58.3 -> 47.3; 500 over 5003
   // 72.0 -> 70.0; 2 x 200 over 1500, 16/4 heads 27.3 -> 26.2); with more the order in which SMs become free deals them
   // out better (1000 over 8000, 16/8 heads 98.7 -> 102.4; B2 H40 S700 37.7 -> 38.7).
-  if (sums && p.n_qchunks == 1 && p.nq_tiles <= 4) ctas = std::min(ctas, 2 * num_sms);
+  const bool loop = sums && p.n_qchunks == 1 && p.nq_tiles <= 4 && ctas > 2 * num_sms;
+  if (loop) ctas = 2 * num_sms;
   const dim3 grid(static_cast<unsigned>(ctas));
   void (*kern)(CUtensorMap, CUtensorMap, ColParams) = nullptr;
-  if (a.mode == ASUKA_SCORE_SUM) kern = s.bf16 ? col_scores_kernel<true, 0> : col_scores_kernel<false, 0>;
+  if (loop && a.mode == ASUKA_SCORE_SUM) kern = s.bf16 ? col_scores_kernel<true, 0, true> : col_scores_kernel<false, 0, true>;
+  else if (loop) kern = s.bf16 ? col_scores_kernel<true, 1, true> : col_scores_kernel<false, 1, true>;
+  else if (a.mode == ASUKA_SCORE_SUM) kern = s.bf16 ? col_scores_kernel<true, 0> : col_scores_kernel<false, 0>;
   else if (a.mode == ASUKA_SCORE_SUM_SQ) kern = s.bf16 ? col_scores_kernel<true, 1> : col_scores_kernel<false, 1>;
   else if (a.mode == ASUKA_SCORE_CORM) kern = s.bf16 ? col_scores_kernel<true, 4> : col_scores_kernel<false, 4>;
   else if (a.exp_rand != nullptr) kern = s.bf16 ? col_scores_kernel<true, 2> : col_scores_kernel<false, 2>;
