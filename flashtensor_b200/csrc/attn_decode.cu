@@ -151,6 +151,16 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_const
     tma_prefetch_desc(&map_k);
     tma_prefetch_desc(&map_v);
   }
+  // What the ring takes first is on its way from DRAM to L2 while the kernel ahead still runs (two stages: B4 H16, 2000 keys,
+  // 15.0 -> 14.5 us, B16 H32/8, 4001 keys, 45.3 -> 45.1; six are slower again).
+  if (warp == kWarps && lane == 0) {
+    for (int t = t_lo; t < min(t_hi, t_lo + 2); ++t) {
+      tma_prefetch_4d(&map_k, 0, hk, t * kKeys, b);
+      tma_prefetch_4d(&map_k, 64, hk, t * kKeys, b);
+      tma_prefetch_4d(&map_v, 0, hk, t * kKeys, b);
+      tma_prefetch_4d(&map_v, 64, hk, t * kKeys, b);
+    }
+  }
   __syncthreads();
   griddep_wait();
   griddep_launch_dependents();

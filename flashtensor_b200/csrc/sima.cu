@@ -241,6 +241,19 @@ sima_stats_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tbase = tmem_base_s;
+  if (warp == 2 && lane == 0) {
+    // what the ring takes first is on its way from DRAM to L2 meanwhile (two tiles: EA B4 H32 S1000 43.6 -> 42.6 us, B2 H32
+    // S5003 76.0 -> 75.4, SimA B1 H16 S1000 16.4 -> 15.9; six are slower, 45.0)
+    for (int k = 0; k < min(2, t_hi - t_lo); ++k) {
+      const int unit = (t_lo + k) / p.share.ntiles, b = unit / p.H, h = unit % p.H;
+      const int s0 = (t_lo + k - unit * p.share.ntiles) * kTile;
+      for (int half = 0; half < 128; half += 64) {
+        tma_prefetch_4d(&map_k, half, h, s0, b);
+        tma_prefetch_4d(&map_v, half, h, s0, b);
+        if (!kEA) tma_prefetch_4d(&map_q, half, h, s0, b);
+      }
+    }
+  }
   griddep_wait();               // k, v and q may be the output of the kernel ahead
   griddep_launch_dependents();
 
