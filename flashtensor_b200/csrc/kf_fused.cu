@@ -69,7 +69,7 @@ struct FusedParams {
   int chunk_tiles;       // query tiles to a chunk
   int n_pieces;          // of a unit; piece i has the chunks from first_chunk[i] to first_chunk[i + 1]
   int first_chunk[kMaxChunks + 1];
-  int n_work;            // pieces of work in all
+  int units, n_work;     // B * H; pieces of work in all
   float* out;            // [n_chunks][B*H][Skv]
   size_t slab;           // B * H * Skv
 };
@@ -129,26 +129,28 @@ __device__ __forceinline__ void tmem_ld_16x256b_x4(uint32_t taddr, uint32_t (&r)
 struct Steps {
   const FusedParams& p;
   uint32_t rank, lnc;  // (lnc: log2 of the cluster's size)
-  int w, bh, chunk;
+  int round, bh, chunk;
+  bool more;
   int qt, qt_end, n_own;
 
   __device__ __forceinline__ Steps(const FusedParams& p_, uint32_t rank_, uint32_t lnc_) : p(p_), rank(rank_), lnc(lnc_) {
-    w = static_cast<int>(blockIdx.x >> lnc);
+    round = 0;
     load_work();
   }
-  __device__ __forceinline__ bool valid() const { return w < p.n_work; }
+  __device__ __forceinline__ bool valid() const { return more; }
   __device__ __forceinline__ bool last_of_chunk() const { return qt == chunk * p.chunk_tiles; }
   // this CTA's t-th key tile: forth and back over the cluster, so that causal row blocks are shared evenly
   __device__ __forceinline__ int key_tile(int t) const {
     return (t << lnc) + static_cast<int>((t & 1) ? (1u << lnc) - 1u - rank : rank);
   }
+  // Pieces are numbered latest (longest) first over all units and dealt out forth and back.
   __device__ __forceinline__ void load_work() {
-    if (!valid()) return;
-    bh = w / p.n_pieces;
-    // (a multiple of the number of pieces of clusters: each gets another piece of its units every round)
-    const int stride = static_cast<int>(gridDim.x >> lnc);
-    const int turn = w - bh * p.n_pieces + (stride % p.n_pieces == 0 ? w / stride : 0);
-    const int piece = p.n_pieces - 1 - turn % p.n_pieces;
+    const int n = static_cast<int>(gridDim.x >> lnc), k = static_cast<int>(blockIdx.x >> lnc);
+    const int w = round * n + ((round & 1) ? n - 1 - k : k);
+    more = w < p.n_work;
+    if (!more) return;
+    const int turn = w / p.units, piece = p.n_pieces - 1 - turn;
+    bh = w - turn * p.units;
     chunk = p.first_chunk[piece + 1] - 1;
     qt = min(p.nq_tiles, (chunk + 1) * p.chunk_tiles) - 1;
     qt_end = p.first_chunk[piece] * p.chunk_tiles;
@@ -165,7 +167,7 @@ struct Steps {
       --qt;
       count_own();
     } else {
-      w += static_cast<int>(gridDim.x >> lnc);
+      ++round;
       load_work();
     }
   }
@@ -778,10 +780,12 @@ FusedPlan kf_fused_plan(const ScoreArgs& a, const AttnShape& s, size_t ws_bytes)
 }
 
 // A unit's chunks to pieces of work: the more pieces, the better they fill the clusters that run at once, `resident`;
-// but a cluster that goes on with the same unit saves what a change costs.  Model, fitted to the times below: 2.2 us for
-// a query tile (exchange, second look), 1.15 us for a key tile of the CTA that has most (2.0 with seeded noise), 2 us
-// for a piece of work.  Whole case in us, 1 / 2 / 4 / 8 pieces: noise operand B1 H4 S2048 106 / 70.8 / 54.6 / 42.8, B4
-// H32 S2048 482 / 482 / 481 / 482, B2 H40 S1500 221 / 199 / 199 / 225; seeded B2 H32 S1501 192 / 196 / 197 / 222.
+// but a cluster that goes on with the same unit saves what a change costs.  The deal is played through with a model of
+// what a cluster does one after the other: 2.2 us for a query tile (exchange, second look), 1.15 us for a key tile of the
+// CTA that has most (2.0 with seeded noise), 2 us for a piece of work.  Whole case in us, 1 / 2 / 4 / 8 pieces: noise
+// operand B1 H4 S2048 106 / 70.8 / 54.6 / 42.8, B4 H32 S2048 482 / 482 / 481 / 482, B2 H40 S1500 221 / 199 / 199 / 225;
+// seeded B2 H32 S1501 192 / 196 / 197 / 222.  Longest pieces first over all units, dealt forth and back, against unit
+// by unit: B2 H16 S1000 60.9 -> 52.6, B1 H8 S2048 60 -> 51, seeded B1 H16 S600 30.1 -> 25.0 (B2 H40 S512 44.8 -> 46.7).
 void cut_pieces(FusedParams& p, int chunks, int noise, int cluster, int resident, long long units) {
   const double per_tile = noise == kNoiseSeeded ? 2.0 : 1.15, per_item = 2.2, per_work = 2.0;
   double chunk[kMaxChunks] = {}, total = 0.;
@@ -794,19 +798,29 @@ void cut_pieces(FusedParams& p, int chunks, int noise, int cluster, int resident
   for (int n = 1; n <= chunks; ++n) {
     // n runs of chunks, each up to its share of the total
     int first[kMaxChunks + 1] = {0};
-    double longest = 0., done = 0.;
+    double run[kMaxChunks], done = 0.;
     for (int x = 0, c = 0; x < n; ++x) {
-      double t = per_work;
+      run[x] = per_work;
       const double until = total * (x + 1) / n;
       do {
-        t += chunk[c];
+        run[x] += chunk[c];
         done += chunk[c++];
       } while (c < chunks - (n - 1 - x) && (x == n - 1 || done + 0.5 * chunk[c] <= until));
       first[x + 1] = c;
-      longest = std::max(longest, t);
     }
-    const long long rounds = (units * n + resident - 1) / resident;
-    const double cost = (rounds - 1) * (total / n + per_work) + longest;
+    // the longest of a few of the clusters, dealt their pieces as Steps does (many rounds: all of them alike)
+    double cost = 0.;
+    const long long works = units * n, rounds = (works + resident - 1) / resident;
+    for (int x = 0; x < 16; ++x) {
+      const long long k = (resident - 1) * x / 15;
+      double t = 0.;
+      for (long long r = 0; r < std::min(rounds, 32ll); ++r) {
+        const long long w = r * resident + ((r & 1) ? resident - 1 - k : k);
+        if (w < works) t += run[n - 1 - w / units];
+      }
+      cost = std::max(cost, t);
+    }
+    if (rounds > 32) cost = (total + n * per_work) * units / resident;
     if (n == 1 || cost < best) {
       best = cost;
       p.n_pieces = n;
@@ -857,7 +871,8 @@ cudaError_t launch_kf_fused(const CUtensorMap& mq, const CUtensorMap& mk, const 
   cudaError_t e = ensure_dynamic_smem(reinterpret_cast<const void*>(kern), static_cast<int>(smem));
   if (e != cudaSuccess) return e;
   cut_pieces(p, plan.chunks, noise, plan.cluster, resident, static_cast<long long>(s.B) * s.H);
-  p.n_work = s.B * s.H * p.n_pieces;
+  p.units = s.B * s.H;
+  p.n_work = p.units * p.n_pieces;
   const int clusters = std::min(p.n_work, resident);
   e = launch_dependent_cluster(kern, dim3(static_cast<unsigned>(clusters * plan.cluster)), dim3(kThreads), smem,
                                static_cast<unsigned>(plan.cluster), stream, mq, mk, mn, p);
