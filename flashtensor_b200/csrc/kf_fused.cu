@@ -773,6 +773,8 @@ FusedPlan kf_fused_plan(const ScoreArgs& a, const AttnShape& s, size_t ws_bytes)
   if (noise == kNoisePlain && a.er_stride_q >= (1ll << 30)) return plan;  // (32-bit row strides in bytes)
   if (cluster == 8 && (noise != kNoiseSeeded || nq < 32 || units > 8)) return plan;
   if (chunks > 1 && static_cast<size_t>(units) * s.Skv * sizeof(float) * chunks > ws_bytes) return plan;
+  // (a device or a partition of one on which such a cluster does not fit)
+  if (resident_clusters(fused_kernel(s.bf16, noise), cluster, fused_smem(noise, cluster)) <= 0) return plan;
   plan.cluster = cluster;
   plan.chunks = chunks;
   plan.chunk_tiles = chunk_tiles;
