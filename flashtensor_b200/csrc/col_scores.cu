@@ -23,6 +23,7 @@
 // rows over 5003 keys, 32/8 heads 45.6 -> 35.8; H2O S4096 H32 110.7 -> 96.8; RoCo B2 H40 S4096
 // 302 -> 272; seeded Keyformer B2 H32 S1501 108.6 -> 99.7.
 //
+// Keyformer takes this and the row pass only where kf_fused.cu does not apply, and through the entry points of their own.
 // The Keyformer row pass (kf_rowstat) is the row-oriented counterpart: S = Q K^T, one thread per
 // query row, online max/sum of the perturbed logits, nothing else.
 #include <cuda_bf16.h>
@@ -944,7 +945,7 @@ constexpr uint32_t kNoiseBoxBytes = kNoiseTileBytes / 4;
 // columns.  Two warps per scheduler do not keep the MUFU busy over their chains of load, logarithm, maximum and
 // exponential; the staged variant, one CTA per SM, has four, the seeded one two CTAs of four (see ColCfg).
 // With four warps instead of two, the last units' tiles longest first and the start under the forward kernel's
-// tail, the whole case went (us): B1 H16 S1000 58 -> 46, B2 H32 S1000 126 -> 109, B1 H16 S2048 117 -> 92,
+// tail, the whole case by two passes went (us): B1 H16 S1000 58 -> 46, B2 H32 S1000 126 -> 109, B1 H16 S2048 117 -> 92,
 // B2 H32 S2048 356 -> 321, B4 H32 S2048 658 -> 607 (calls back to back on a cool card; among other work, at
 // lower clocks, the last takes 778 and 734).
 template <int kNoise> struct RsCfg {  // kNoise 1: two K stages, then eight noise boxes
@@ -1432,7 +1433,7 @@ cudaError_t launch_kf_rowstat(const CUtensorMap& mq, const CUtensorMap& mk, cons
     if (e != cudaSuccess) return e;
     // Two CTAs share an SM.  A launch of half a wave to two waves is balanced by one long and one shorter
     // tile on each, which is how the CTAs fall when all SMs are free at the start; as the forward kernel's
-    // CTAs retire one by one, the first SM gets the two longest.  Such a launch waits (whole case in us, chained / not:
+    // CTAs retire one by one, the first SM gets the two longest.  Such a launch waits (whole case by two passes in us, chained / not:
     // B1 H16 S2048, 0.9 waves, 141 / 127; B1 H16 S4096, 1.7 waves, 325 / 314; B2 H16 S2048 180 / 179; B2 H40 S1000,
     // 2.2 waves, 131 / 138; B2 H32 S1501, 2.6 waves, 201 / 209; B1 H16 S300, a sixth of a wave, 24.4 / 32.0; S600
     // 34.3 / 42.8).
