@@ -927,8 +927,8 @@ int asuka_b200_case_workspace_bytes(const asuka_case_params* p, size_t* bytes) {
 
 int asuka_b200_case_workspace_bytes_split(const asuka_case_params* p, size_t* bytes) {
   const int r = asuka_b200_case_workspace_bytes(p, bytes);
-  // required part + what the work-item splits would like: RoCo's column pass or Keyformer's chunks, whichever asks most
-  if (r == ASUKA_OK) *bytes += std::max(case_split_bytes(p, CASE_ROCO), case_split_bytes(p, CASE_KF));
+  // required part + what the work-item splits would like, RoCo's column pass most, and Keyformer's chunks
+  if (r == ASUKA_OK) *bytes += std::max(case_split_bytes(p, CASE_ROCO), p->tau > 0.f ? case_split_bytes(p, CASE_KF) : 0);
   return r;
 }
 

@@ -302,8 +302,15 @@ def test_keyformer_in_one_pass_vs_two_passes(ops, shape, noise):
   p = _lib.CaseParams(ops._desc(q), ops._desc(k), ops._desc(v))
   n = ctypes.c_size_t(0)
   assert _lib.load().asuka_b200_case_workspace_bytes(ctypes.byref(p), ctypes.byref(n)) == 0
-  for ws in (None, torch.empty(n.value, dtype=torch.uint8, device="cuda")):
-    score = ops.keyformer(q, k, v, er, tau=1.5, seed=5, causal=causal, workspace=ws)[1]
+  required = n.value
+  p = _lib.CaseParams(ops._desc(q), ops._desc(k), ops._desc(v), tau=1.5, causal=int(causal))
+  if er is not None:
+    p.exp_rand = ops._desc(er)
+  assert _lib.load().asuka_b200_case_workspace_bytes_split(ctypes.byref(p), ctypes.byref(n)) == 0
+  mem = _Banded(16 << 20)
+  for ws in (None, mem.take((n.value,), torch.uint8), torch.empty(required, dtype=torch.uint8, device="cuda")):
+    score = ops.keyformer(q, k, v, er, tau=1.5, seed=5, causal=causal, workspace=ws, score=mem.take((B, H, Skv), torch.float32))[1]
+    assert mem.bands_untouched(), "a kernel wrote outside its outputs or workspace"
     # an exponent argument is off by half an ulp of a row statistic of up to 64 (4e-6), twice, and by the
     # hardware's exponential (2e-7); sums of up to 4000 terms of one sign add about as much again
     torch.testing.assert_close(score, want, rtol=2e-5, atol=1e-9)
