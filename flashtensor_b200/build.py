@@ -18,7 +18,7 @@ LIB_PATH = os.path.join(PKG_DIR, "libasuka_b200.so")
 BIND_PATH = os.path.join(PKG_DIR, "_bind.so")
 BIND_STAMP = os.path.join(OBJ_DIR, "_bind.built_against")
 
-SOURCES = ["capi.cu", "attn_fwd.cu", "attn_decode.cu", "col_scores.cu", "kf_fused.cu", "select_topk.cu", "score_ops.cu", "sima.cu", "linattn32.cu", "linear_f32.cu"]
+SOURCES = ["capi.cu", "attn_fwd.cu", "attn_decode.cu", "col_scores.cu", "select_topk.cu", "score_ops.cu", "sima.cu", "linattn32.cu", "linear_f32.cu"]
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a", "-O3", "-lineinfo", "-std=c++17",
     "-Xcompiler", "-fPIC", "--use_fast_math", "-Xptxas", "-v",

@@ -228,7 +228,7 @@ PyObject* run_case(PyObject*, PyObject* const* a, Py_ssize_t n) {
     p.exp_rand = desc(exp_rand);
     p.idx = desc(idx);
     p.softmax_scale = static_cast<float>(float_arg(a[5]));
-    p.tau = kind == 2 ? static_cast<float>(float_arg(a[7])) : 0.f;  // (0: not Keyformer, to the workspace query)
+    p.tau = static_cast<float>(float_arg(a[7]));
     p.seed = int_arg(a[8]);
     p.causal = bool_arg(a[4]) ? 1 : 0;
     p.k_keep = static_cast<int32_t>(int_arg(a[9]));

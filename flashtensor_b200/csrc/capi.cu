@@ -332,25 +332,6 @@ int kf_rowstat_impl(const asuka_score_params* p, cudaStream_t stream, bool chain
   return map_cuda(launch_kf_rowstat(mq, mk, a, static_cast<float*>(p->lse.ptr), c.s, sms, stream));
 }
 
-// behind the forward kernel; `pending` as in col_scores_impl
-int kf_fused_impl(const asuka_score_params* p, const FusedPlan& plan, cudaStream_t stream, void* ws, PendingChunkSum* pending) {
-  QKV c;
-  ScoreArgs a;
-  int r = prep_scores(p, false, &c, &a);
-  if (r != ASUKA_OK) return r;
-  a.chained = 1;
-  CUtensorMap mq, mk;
-  if ((r = make_map(&mq, p->q)) || (r = make_map(&mk, p->k))) return r;
-  PendingChunkSum sum;
-  if ((r = map_cuda(launch_kf_fused(mq, mk, a, c.s, plan, ws, stream, &sum))) != ASUKA_OK) return r;
-  if (pending != nullptr) {
-    *pending = sum;
-    return ASUKA_OK;
-  }
-  if (sum.n_chunks == 0) return ASUKA_OK;
-  return map_cuda(launch_sum_chunks(sum, a.score, nullptr, static_cast<size_t>(c.s.B) * c.s.H * c.s.Skv, stream));
-}
-
 constexpr int kSelectMaxS32 = 32768;  // 4-byte keys in shared memory
 constexpr int kSelectMaxS64 = 16384;  // 8-byte keys (RoCo)
 
@@ -510,19 +491,6 @@ size_t case_ws_bytes(const asuka_case_params* p) {
   return bytes;
 }
 
-// Keyformer's noise as the score kernels take it
-ScoreArgs kf_noise_args(const asuka_case_params* p) {
-  ScoreArgs a;
-  std::memset(&a, 0, sizeof(a));
-  a.mode = ASUKA_SCORE_PERTURBED;
-  a.tau = p->tau;
-  a.exp_rand = static_cast<const float*>(p->exp_rand.ptr);
-  a.er_stride_b = p->exp_rand.stride[0];
-  a.er_stride_h = p->exp_rand.stride[1];
-  a.er_stride_q = p->exp_rand.stride[2];
-  return a;
-}
-
 // what the split of work items would like on top of case_ws_bytes on the current device
 size_t case_split_bytes(const asuka_case_params* p, CaseKind kind) {
   if (p->k.ndim != 4 || p->q.ndim != 4) return 0;
@@ -537,15 +505,7 @@ size_t case_split_bytes(const asuka_case_params* p, CaseKind kind) {
   s.group = p->k.shape[2] > 0 ? static_cast<int>(p->q.shape[2] / p->k.shape[2]) : 1;
   const int mode = kind == CASE_H2O ? ASUKA_SCORE_SUM : kind == CASE_ROCO ? ASUKA_SCORE_SUM_SQ : ASUKA_SCORE_PERTURBED;
   const size_t fwd = attn_fwd_split_bytes(s, attn_fwd_parts(s, sms, ~static_cast<size_t>(0)));
-  size_t col = 0;
-  FusedPlan plan = {0, 0, 0};
-  if (kind == CASE_KF && p->k.shape[1] > 0) {
-    AttnShape kf = s;
-    kf.causal = p->causal;
-    plan = kf_fused_plan(kf_noise_args(p), kf, ~static_cast<size_t>(0));
-  }
-  if (plan.cluster > 0) col = col_scores_split_bytes(s, mode, plan.chunks);
-  else col = col_scores_split_bytes(s, mode, col_scores_chunks(s, mode, sms, ~static_cast<size_t>(0)));
+  const size_t col = col_scores_split_bytes(s, mode, col_scores_chunks(s, mode, sms, ~static_cast<size_t>(0)));
   return ((col + 255) / 256) * 256 + fwd + 256;
 }
 
@@ -657,16 +617,14 @@ int case_impl(const asuka_case_params* p, CaseKind kind, void* ws, size_t ws_byt
   size_t extra_bytes = ws_bytes - case_ws_bytes(p);
   void* col_ws = nullptr;
   size_t col_bytes = 0;
-  FusedPlan plan = {0, 0, 0};
   {
     QKV c; ScoreArgs a;
     if (prep_scores(&sp, false, &c, &a) == ASUKA_OK) {
       const int sms = sm_count();
       size_t usable = 0;
       void* base = align_ws(extra, extra_bytes, &usable);
-      if (kind == CASE_KF) plan = kf_fused_plan(a, c.s, base != nullptr ? usable : 0);
       if (sms > 0 && base != nullptr) {
-        const size_t want = col_scores_split_bytes(c.s, a.mode, plan.cluster > 0 ? plan.chunks : col_scores_chunks(c.s, a.mode, sms, usable));
+        const size_t want = col_scores_split_bytes(c.s, a.mode, col_scores_chunks(c.s, a.mode, sms, usable));
         if (want > 0) {
           col_ws = base;
           col_bytes = want;
@@ -679,16 +637,15 @@ int case_impl(const asuka_case_params* p, CaseKind kind, void* ws, size_t ws_byt
   }
   int r = attn_fwd_impl(&fp, nullptr, stream, extra_bytes > 0 ? extra : nullptr, extra_bytes);
   if (r != ASUKA_OK) return r;
-  if (kind == CASE_KF && plan.cluster == 0) {
+  if (kind == CASE_KF) {
     if ((r = kf_rowstat_impl(&sp, stream, true)) != ASUKA_OK) return r;
   }
   // with a selection to follow (and no group mean in between) the selection kernel adds the column
   // pass's partial sums itself: one launch fewer
   PendingChunkSum pending;
   pending.n_chunks = 0;
-  if (plan.cluster > 0) r = kf_fused_impl(&sp, plan, stream, col_ws, want_idx ? &pending : nullptr);
-  else r = col_scores_impl(&sp, stream, true, col_ws, col_bytes, want_idx && !gqa ? &pending : nullptr);
-  if (r != ASUKA_OK) return r;
+  if ((r = col_scores_impl(&sp, stream, true, col_ws, col_bytes, want_idx && !gqa ? &pending : nullptr)) != ASUKA_OK)
+    return r;
   if (gqa) {
     r = map_cuda(launch_group_mean(head_scores, static_cast<float*>(p->score.ptr), static_cast<int>(B * Hkv),
                                    static_cast<int>(H / Hkv), static_cast<int>(p->k.shape[1]), stream));
@@ -927,8 +884,8 @@ int asuka_b200_case_workspace_bytes(const asuka_case_params* p, size_t* bytes) {
 
 int asuka_b200_case_workspace_bytes_split(const asuka_case_params* p, size_t* bytes) {
   const int r = asuka_b200_case_workspace_bytes(p, bytes);
-  // required part + what the work-item splits would like, RoCo's column pass most, and Keyformer's chunks
-  if (r == ASUKA_OK) *bytes += std::max(case_split_bytes(p, CASE_ROCO), p->tau > 0.f ? case_split_bytes(p, CASE_KF) : 0);
+  // required part + what the work-item splits would like; RoCo's column pass asks most
+  if (r == ASUKA_OK) *bytes += case_split_bytes(p, CASE_ROCO);
   return r;
 }
 

@@ -23,7 +23,6 @@
 // rows over 5003 keys, 32/8 heads 45.6 -> 35.8; H2O S4096 H32 110.7 -> 96.8; RoCo B2 H40 S4096
 // 302 -> 272; seeded Keyformer B2 H32 S1501 108.6 -> 99.7.
 //
-// Keyformer takes this and the row pass only where kf_fused.cu does not apply, and through the entry points of their own.
 // The Keyformer row pass (kf_rowstat) is the row-oriented counterpart: S = Q K^T, one thread per
 // query row, online max/sum of the perturbed logits, nothing else.
 #include <cuda_bf16.h>
@@ -35,7 +34,6 @@
 #include "../../include/asuka_b200.h"
 #include "fast_div.cuh"
 #include "kernels.h"
-#include "score_math.cuh"
 #include "sm100_ptx.cuh"
 #include "tma_host.h"
 
@@ -106,6 +104,21 @@ struct ColBars {
   uint64_t s_full[2], s_empty[2];
 };
 
+__device__ __forceinline__ float ex2(float x) {
+  float y;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+__device__ __forceinline__ float max3(float a, float b, float c) {
+  float y;
+  asm("max.f32 %0, %1, %2, %3;" : "=f"(y) : "f"(a), "f"(b), "f"(c));
+  return y;
+}
+__device__ __forceinline__ float lg2(float x) {
+  float y;
+  asm("lg2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
 // exp2 on the FMA pipe, two logits per instruction (packed f32x2): x = n + f with n = rint(x) taken
 // from the mantissa of x + 1.5 * 2^23, a degree-4 polynomial for 2^f on [-0.5, 0.5] (relative
 // error 2.7e-6), and n added into the exponent field.  The MUFU does 16 exponentials per clock per
@@ -172,6 +185,51 @@ __device__ __forceinline__ float2 ex2_fma_pipe(float2 x) {
   return make_float2(__int_as_float(__float_as_int(p.x) + (__float_as_int(t.x) << 23)),
                      __int_as_float(__float_as_int(p.y) + (__float_as_int(t.y) << 23)));
 #endif
+}
+
+// Seeded Keyformer noise: one bijective 32-bit mix ("lowbias32") per logit.
+//   head_key = hash(seed_lo ^ hash((b*H + h) ^ seed_hi));  word = hash(((q << 16) ^ kv) ^ head_key)
+//   u = ((word >> 9) + 0.5) * 2^-23 in (0,1);  exp_rand = -ln(u);  noise g = -ln(exp_rand) ~ Gumbel(0,1)
+__device__ __forceinline__ uint32_t hash_u32(uint32_t x) {
+  x ^= x >> 16;
+  x *= 0x7feb352du;
+  x ^= x >> 15;
+  x *= 0x846ca68bu;
+  x ^= x >> 16;
+  return x;
+}
+__device__ __forceinline__ uint32_t seeded_head_key(uint64_t seed, uint32_t bh) {
+  return hash_u32(static_cast<uint32_t>(seed) ^ hash_u32(bh ^ static_cast<uint32_t>(seed >> 32)));
+}
+// log2(exp_rand) of two logits less kSeededLg2Unit, from their words after the first xor-shift of the mix.
+// The passes that use it are bound by what they issue beside three MUFU operations per logit (logarithm of u,
+// logarithm of exp_rand, exponential), hence: the first xor-shift is one LOP3 per logit (the words of a thread's
+// neighbouring logits differ in their low bits only), the last one and the conversion to a float in [1, 2) are two
+// shifts and a LOP3, the f32 arithmetic is packed, and the factor ln 2 of exp_rand, a constant after the second
+// logarithm, is left to the row statistic.  17 instructions where the plain restatement takes 25: B2 H32 S1501,
+// row pass 114 -> 88 us, column pass 107 -> 82, whole case 275 -> 217.
+constexpr float kSeededLg2Unit = -0.52876637294489779f;  // log2(ln 2)
+__device__ __forceinline__ float2 seeded_lg2_exp_rand2(uint32_t x0, uint32_t x1) {
+  auto word = [](uint32_t x) {
+    x *= 0x7feb352du;
+    x ^= x >> 15;
+    x *= 0x846ca68bu;
+    return __uint_as_float(((x >> 9) ^ (x >> 25)) | 0x3f800000u);
+  };
+  const float2 u = __fadd2_rn(make_float2(word(x0), word(x1)), make_float2(-1.0f + 5.9604645e-8f, -1.0f + 5.9604645e-8f));  // exact
+  // -log2(u): the hardware log2 has a fixed ABSOLUTE error, useless for u next to 1 (where the
+  // large, row-dominating Gumbel values come from); there use the series in d = 1 - u (exact)
+  const float2 d = __ffma2_rn(u, make_float2(-1.f, -1.f), make_float2(1.f, 1.f));
+  float2 series = __ffma2_rn(d, make_float2(0.48089835f, 0.48089835f), make_float2(0.72134752f, 0.72134752f));
+  series = __ffma2_rn(d, series, make_float2(1.44269504f, 1.44269504f));
+  series = __fmul2_rn(d, series);
+  const float e0 = -lg2(u.x), e1 = -lg2(u.y);
+  return make_float2(lg2(d.x < 0.015625f ? series.x : e0), lg2(d.y < 0.015625f ? series.y : e1));
+}
+
+__device__ __forceinline__ void record_timeout(uint32_t* status, uint32_t site) {
+  atomicAdd(&status[0], 1u);
+  status[1] = site;
 }
 
 // kMode: 0 sum, 1 sum + sum of squares, 2 perturbed (noise operand), 3 perturbed (seeded noise),
@@ -945,7 +1003,7 @@ constexpr uint32_t kNoiseBoxBytes = kNoiseTileBytes / 4;
 // columns.  Two warps per scheduler do not keep the MUFU busy over their chains of load, logarithm, maximum and
 // exponential; the staged variant, one CTA per SM, has four, the seeded one two CTAs of four (see ColCfg).
 // With four warps instead of two, the last units' tiles longest first and the start under the forward kernel's
-// tail, the whole case by two passes went (us): B1 H16 S1000 58 -> 46, B2 H32 S1000 126 -> 109, B1 H16 S2048 117 -> 92,
+// tail, the whole case went (us): B1 H16 S1000 58 -> 46, B2 H32 S1000 126 -> 109, B1 H16 S2048 117 -> 92,
 // B2 H32 S2048 356 -> 321, B4 H32 S2048 658 -> 607 (calls back to back on a cool card; among other work, at
 // lower clocks, the last takes 778 and 734).
 template <int kNoise> struct RsCfg {  // kNoise 1: two K stages, then eight noise boxes
@@ -1406,16 +1464,9 @@ cudaError_t launch_col_scores(const CUtensorMap& mq, const CUtensorMap& mk, cons
     pending->n_chunks = p.n_qchunks;
     return e;
   }
-  PendingChunkSum sum;
-  sum.part = p.part;
-  sum.part_sq = sq ? p.part_sq : nullptr;
-  sum.n_chunks = p.n_qchunks;
-  return launch_sum_chunks(sum, a.score, a.score_sq, n, stream);
-}
-
-cudaError_t launch_sum_chunks(const PendingChunkSum& sum, float* out, float* out_sq, size_t n, cudaStream_t stream) {
-  const cudaError_t e = launch_dependent(sum_chunks_kernel, dim3(static_cast<unsigned>((n + 255) / 256)), dim3(256), 0, stream,
-                                         sum.part, sum.part_sq, out, out_sq, sum.n_chunks, n);
+  e = launch_dependent(sum_chunks_kernel, dim3(static_cast<unsigned>((n + 255) / 256)), dim3(256), 0, stream,
+                       static_cast<const float*>(p.part), static_cast<const float*>(sq ? p.part_sq : nullptr),
+                       a.score, a.score_sq, p.n_qchunks, n);
   count_launch();
   return e;
 }
@@ -1433,7 +1484,7 @@ cudaError_t launch_kf_rowstat(const CUtensorMap& mq, const CUtensorMap& mk, cons
     if (e != cudaSuccess) return e;
     // Two CTAs share an SM.  A launch of half a wave to two waves is balanced by one long and one shorter
     // tile on each, which is how the CTAs fall when all SMs are free at the start; as the forward kernel's
-    // CTAs retire one by one, the first SM gets the two longest.  Such a launch waits (whole case by two passes in us, chained / not:
+    // CTAs retire one by one, the first SM gets the two longest.  Such a launch waits (whole case in us, chained / not:
     // B1 H16 S2048, 0.9 waves, 141 / 127; B1 H16 S4096, 1.7 waves, 325 / 314; B2 H16 S2048 180 / 179; B2 H40 S1000,
     // 2.2 waves, 131 / 138; B2 H32 S1501, 2.6 waves, 201 / 209; B1 H16 S300, a sixth of a wave, 24.4 / 32.0; S600
     // 34.3 / 42.8).

@@ -115,19 +115,6 @@ size_t col_scores_split_bytes(const AttnShape& s, int mode, int chunks);
 cudaError_t launch_kf_rowstat(const CUtensorMap& mq, const CUtensorMap& mk, const ScoreArgs& a,
                               float* lse2_out, const AttnShape& s, int num_sms, cudaStream_t stream);
 
-// Keyformer's score without a row pass of its own (kf_fused.cu): `cluster` CTAs share the keys of a row block, the
-// query tiles of a unit are cut into `chunks` of `chunk_tiles`.  cluster = 0: not for this call.
-struct FusedPlan {
-  int cluster, chunks, chunk_tiles;
-};
-FusedPlan kf_fused_plan(const ScoreArgs& a, const AttnShape& s, size_t ws_bytes);
-// More than one chunk: the score is left as partial sums in `split_ws` (chunks * B * H * Skv floats) for the caller to
-// add, as `pending` says.
-cudaError_t launch_kf_fused(const CUtensorMap& mq, const CUtensorMap& mk, const ScoreArgs& a, const AttnShape& s,
-                            const FusedPlan& plan, void* split_ws, cudaStream_t stream, PendingChunkSum* pending);
-// adds partial sums in order: out[i] = sum_c part[c][i], i < n (and out_sq alike)
-cudaError_t launch_sum_chunks(const PendingChunkSum& sum, float* out, float* out_sq, size_t n, cudaStream_t stream);
-
 struct SelectArgs {
   const float* score;     // [B*H, S] rows, contiguous
   const float* score_sq;  // or null

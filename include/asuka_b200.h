@@ -242,9 +242,7 @@ int asuka_b200_linattn32_proj(const asuka_linattn32_proj_params* p, asuka_stream
  *      group mean.  asuka_b200_case_workspace_bytes gives that figure, which is required.
  *      asuka_b200_case_workspace_bytes_split adds, for launches with too few (batch, head) units
  *      to fill the current device, the scratch that lets the kernels split their work items
- *      further, and for Keyformer (`tau` set) up to 8 * B*H*Skv floats of partial sums, with which its
- *      noise is gone over once instead of twice; a workspace between the two sizes is accepted and used as
- *      far as it goes. ---- */
+ *      further; a workspace between the two sizes is accepted and used as far as it goes. ---- */
 typedef struct {
   asuka_tensor q, k, v, out;
   asuka_tensor score;    /* h2o_score | kf_score | roco_score, [B, H, Skv] f32 */

@@ -278,13 +278,13 @@ def test_scores_of_few_rows_over_many_keys_vs_oracle(ops, shape):
 
 
 @pytest.mark.parametrize("noise", ["dense", "odd", "broadcast", "seeded"])
-@pytest.mark.parametrize("shape", [  # (B, Sq, Skv, H, causal): row blocks and key tiles about one CTA's share and about a cluster's
+@pytest.mark.parametrize("shape", [  # (B, Sq, Skv, H, causal): about the edges of tiles, one key and the longest ranges that are split
     (1, 1, 1, 1, True), (1, 128, 128, 2, True), (2, 129, 129, 3, True), (1, 200, 512, 2, True), (1, 513, 513, 40, False),
     (1, 1, 700, 3, True), (1, 1024, 1024, 2, True), (1, 1025, 1025, 33, True), (2, 300, 2048, 2, True),
     (1, 2048, 2048, 2, False), (1, 2049, 2049, 2, True), (1, 4000, 4096, 1, True)])
-def test_keyformer_in_one_pass_vs_two_passes(ops, shape, noise):
-  # the case's kernel against the row pass and the column pass that the library exports one by one, with all of the
-  # workspace it asks for (several pieces of work to a unit) and with what it must have (one)
+def test_keyformer_case_vs_its_passes_one_by_one(ops, shape, noise):
+  # the case's score against the row pass and the column pass that the library exports one by one, with all of the
+  # workspace it asks for (long query ranges of few units are split) and with what it must have (they are not)
   import ctypes
   from flashtensor_b200 import _lib
   B, Sq, Skv, H, causal = shape
@@ -309,7 +309,11 @@ def test_keyformer_in_one_pass_vs_two_passes(ops, shape, noise):
   assert _lib.load().asuka_b200_case_workspace_bytes_split(ctypes.byref(p), ctypes.byref(n)) == 0
   mem = _Banded(16 << 20)
   for ws in (None, mem.take((n.value,), torch.uint8), torch.empty(required, dtype=torch.uint8, device="cuda")):
+    before = ops.launch_count()
     score = ops.keyformer(q, k, v, er, tau=1.5, seed=5, causal=causal, workspace=ws, score=mem.take((B, H, Skv), torch.float32))[1]
+    launches = ops.launch_count() - before
+    # forward, row pass, column pass; with room for it the forward pass's merge and the sum of the split ranges
+    assert launches == 3 if ws is not None and ws.numel() == required else 3 <= launches <= 5, launches
     assert mem.bands_untouched(), "a kernel wrote outside its outputs or workspace"
     # an exponent argument is off by half an ulp of a row statistic of up to 64 (4e-6), twice, and by the
     # hardware's exponential (2e-7); sums of up to 4000 terms of one sign add about as much again
@@ -1308,6 +1312,24 @@ def test_a_slice_of_the_units_reproduces_the_whole_problem(ops):
     assert torch.equal(part[2], sharding.shard_bhs(whole[2], rank, world))
   parts = [ft.H2O(head_num=3, kv_head_num=3)(*(sharding.shard_bshd(t, r, world) for t in (q, k, v)))[1] for r in range(world)]
   assert torch.equal(sharding.gather_units(parts, B, H), ft.H2O(head_num=H, kv_head_num=H)(q, k, v)[1])
+  no_timeouts(ops)
+
+
+@pytest.mark.parametrize("world", [2])
+def test_a_slice_of_a_long_seeded_problem_has_the_same_scores(ops, world):
+  # 32 query tiles are where the column pass starts to split query ranges by the number of units; ten units and
+  # halves of them are split alike, so a half's scores are the whole problem's to the bit
+  import flashtensor_b200 as ft
+  from flashtensor_b200 import sharding
+  B, S, H, seed, k_keep = 1, 3970, 10, 78, 256
+  q, k, v = (t.cuda() for t in O.make_inputs("attn", B, S, S, H, 128, torch.float16, seed=9))
+  whole = ft.KeyFormer(tau=1.5, head_num=H, kv_head_num=H).seeded(q, k, v, seed, k_keep)
+  for rank in range(world):
+    lo, hi = sharding.unit_range(B * H, rank, world)
+    qs, ks, vs = (sharding.shard_bshd(t, rank, world) for t in (q, k, v))
+    part = ft.KeyFormer(tau=1.5, head_num=hi - lo, kv_head_num=hi - lo).seeded(qs, ks, vs, seed, k_keep, unit_offset=lo)
+    assert torch.equal(part[1], sharding.shard_bhs(whole[1], rank, world))
+    assert torch.equal(part[2], sharding.shard_bhs(whole[2], rank, world))
   no_timeouts(ops)
 
 
