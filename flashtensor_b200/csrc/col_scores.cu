@@ -243,7 +243,7 @@ col_scores_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
   __shared__ __align__(16) float lse_s[kLseStages][kTile];  // minus the row statistic
   constexpr int kCh = ColCfg<kMode>::kChunk;
   constexpr int kKeyWarps = ColCfg<kMode>::kKeyWarps, kSubs = ColCfg<kMode>::kSubs, kQueries = ColCfg<kMode>::kQueries;
-  __shared__ float part_s[2][2][kSubs][kTile];  // [parity of the item][sum, sum of squares][share of the queries][key]
+  __shared__ float part_s[kLoop ? 2 : 1][2][kSubs][kTile];  // [parity of the item][sum, sum of squares][share of the queries][key]
   __shared__ uint32_t tmem_base_s;
   __shared__ uint32_t abort_s;
 
@@ -275,6 +275,23 @@ col_scores_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
     m.i_begin = max(m.qc * p.q_chunk, p.causal ? max(0, m.kv0 - p.diag_off) / kTile : 0);
     m.i_end = max(m.i_begin, min(p.nq_tiles, (m.qc + 1) * p.q_chunk));
     return true;
+  };
+  // the sums of key `k` of item `m` from the shares' parts
+  auto store_sums = [&](const Item& m, const float (*part)[kSubs][kTile], int k) {
+    const int key = m.kv0 + k;
+    if (key >= p.Skv) return;
+    const size_t o = (static_cast<size_t>(m.b) * p.H + m.h) * p.Skv + key;
+    float v = part[0][0][k] + part[0][1][k];
+    if constexpr (kSubs == 4) v += part[0][2][k] + part[0][3][k];
+    // with a query-range split the sums of this range go to its slab of the workspace (a range
+    // that sees none of the keys leaves zeros there)
+    const size_t slab = static_cast<size_t>(m.qc) * bh_count * p.Skv;
+    if constexpr (kMode == 4) {
+      reinterpret_cast<uint8_t*>(p.score)[o] = v != 0.f ? 1 : 0;
+    } else {
+      (p.n_qchunks > 1 ? p.part + slab : p.score)[o] = v;
+    }
+    if constexpr (kMode == 1) (p.n_qchunks > 1 ? p.part_sq + slab : p.score_sq)[o] = part[1][0][k] + part[1][1][k];
   };
   Item m;
   const int idx0 = static_cast<int>(blockIdx.x), stride = kLoop ? static_cast<int>(gridDim.x) : p.n_items;
@@ -434,11 +451,11 @@ col_scores_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
     const uint32_t lane_base = static_cast<uint32_t>(wq * 32) << 16;
     const float scale = p.scale_log2;
     bool ok = true;
-    uint32_t c = 0, items = 0;
+    uint32_t c0 = 0, items = 0;  // steps and items before this one
     // (the first Q tiles did not wait for their row statistics)
     if (p.chained && m.i_end > m.i_begin) ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&bars.lse_first), 0, abortp));
     if (!ok && lane == 0) record_timeout(p.status, 29);
-    bool more = ok && idx0 < p.n_items;
+    bool more = ok;
     for (int idx = idx0; more;) {
       const int kv0 = m.kv0, b = m.b, h = m.h, bh = m.bh;
       const int key = kv0 + wq * 32 + lane;
@@ -452,7 +469,9 @@ col_scores_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
       }
       bool hit = false;
 
-      for (int i = m.i_begin; i < m.i_end; ++i, ++c) {
+      const int i_begin = m.i_begin, i_end = m.i_end;
+      for (int i = i_begin; i < i_end; ++i) {
+        const uint32_t c = c0 + static_cast<uint32_t>(i - i_begin);
         const int ls = c % kLseStages, buf = c & 1;
         {
           // S^T of this step is complete; its MMAs were issued after Q and the row statistics of
@@ -481,7 +500,7 @@ col_scores_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
               }
               // the operand is read once, straight from HBM: pull the same chunk of the next query
               // tile into L2 now, so that its loads find it there one step later
-              if (i + 1 < m.i_end) {
+              if (i + 1 < i_end) {
 #pragma unroll
                 for (int e = 0; e < 32; ++e) {
                   const int qi = min(q_base + kTile + ch * kCh + e, p.Sq - 1);
@@ -579,37 +598,26 @@ col_scores_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
         __syncwarp();
         if (lane == 0) mbar_arrive(smem_u32(&bars.lse_empty[ls]));
       }
-      // All shares of the queries leave their parts in shared memory; the first one's warps add them in a fixed
-      // order and store.  (The other parity's parts may still be read by a warp that is an item behind.)
-      float (*part)[kSubs][kTile] = part_s[items & 1];
-      const int k_in_tile = wq * 32 + lane;
-      part[0][hq][k_in_tile] = kMode == 4 ? (hit ? 1.f : 0.f) : (acc[0] + acc[1]) + (acc[2] + acc[3]);
-      part[1][hq][k_in_tile] = (acc2[0] + acc2[1]) + (acc2[2] + acc2[3]);
-      __syncwarp();
-      if (lane == 0) mbar_arrive(smem_u32(&bars.part_full));
-      if (ok) {
-        ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&bars.part_full), items & 1, abortp));
-        if (!ok && lane == 0) record_timeout(p.status, 28);
-      }
-      if (!ok) break;
-      if (hq == 0 && key < p.Skv) {
-        const size_t o = (static_cast<size_t>(b) * p.H + h) * p.Skv + key;
-        float v = part[0][0][k_in_tile] + part[0][1][k_in_tile];
-        if constexpr (kSubs == 4) v += part[0][2][k_in_tile] + part[0][3][k_in_tile];
-        // with a query-range split the sums of this range go to its slab of the workspace (a range
-        // that sees none of the keys leaves zeros there)
-        const size_t slab = static_cast<size_t>(m.qc) * bh_count * p.Skv;
-        if (items == 0 && p.chained) griddep_wait();
-        if constexpr (kMode == 4) {
-          reinterpret_cast<uint8_t*>(p.score)[o] = v != 0.f ? 1 : 0;
-        } else {
-          (p.n_qchunks > 1 ? p.part + slab : p.score)[o] = v;
+      // All shares of the queries leave their parts in shared memory; the first one's warps add them in a fixed order and
+      // store.  (The other parity's parts may still be read by a warp that is an item behind.)
+      part_s[kLoop ? items & 1 : 0][0][hq][wq * 32 + lane] = kMode == 4 ? (hit ? 1.f : 0.f) : (acc[0] + acc[1]) + (acc[2] + acc[3]);
+      part_s[kLoop ? items & 1 : 0][1][hq][wq * 32 + lane] = (acc2[0] + acc2[1]) + (acc2[2] + acc2[3]);
+      if constexpr (kLoop) {
+        __syncwarp();
+        if (lane == 0) mbar_arrive(smem_u32(&bars.part_full));
+        if (ok) {
+          ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&bars.part_full), items & 1, abortp));
+          if (!ok && lane == 0) record_timeout(p.status, 28);
         }
-        if constexpr (kMode == 1)
-          (p.n_qchunks > 1 ? p.part_sq + slab : p.score_sq)[o] = part[1][0][k_in_tile] + part[1][1][k_in_tile];
+        if (!ok) break;
+        if (hq == 0) {
+          if (items == 0 && p.chained) griddep_wait();
+          store_sums(m, part_s[items & 1], wq * 32 + lane);
+        }
+        c0 += static_cast<uint32_t>(i_end - i_begin);
+        ++items;
+        idx += stride;
       }
-      ++items;
-      idx += stride;
       more = kLoop && load_item(idx, m);
     }
     if (!ok) *abortp = 1u;
@@ -621,6 +629,8 @@ col_scores_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
     __syncwarp();
     tmem_dealloc(tbase, 256);
   }
+  // (one item: the barrier above is the one that its parts wait for)
+  if (!kLoop && warp >= kUtilWarps && warp < kUtilWarps + 4 && !*abortp) store_sums(m, part_s[0], (warp & 3) * 32 + lane);
 }
 
 // ---------------------------------------------------------------------------------------------
