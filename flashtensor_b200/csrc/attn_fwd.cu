@@ -59,11 +59,12 @@ template <int kMode> struct Rings {
 constexpr int kThreads = 384;
 // Registers of the utility and of the softmax warps; what a block asks for must fit its 384 * 168 = 64512.
 // The soft-capped one-tile mode has both ways of the tanh beside what its merge keeps: at 200 it spills 464
-// bytes, at 216 156, at 224 84 (S4000, 8 heads 53.6 -> 51.9 us from 216 to 224, 52.5 at 232).  The others at 200 or 208:
-// B1 H32 S1024 18.6 and 17.9.
+// bytes, at 216 156, at 224 112 (S4000, 8 heads 53.6 -> 51.9 us from 216 to 224, 52.5 at 232).  The others at 200 or 208:
+// B1 H32 S1024 18.6 and 17.9; with split keys 128 rows over 16000, 16/4 heads, 44.3 and 45.1, soft-capped 1000 over 8000, 8/2
+// heads, 50.7 and 51.4.
 template <bool kCap, int kMode> struct Regs {
-  static constexpr int kUtil = kCap && kMode == kSolo ? 56 : 88;
-  static constexpr int kSoftmax = kCap && kMode == kSolo ? 224 : 208;
+  static constexpr int kUtil = kCap && kMode == kSolo ? 56 : kMode == kSplit ? 96 : 88;
+  static constexpr int kSoftmax = kCap && kMode == kSolo ? 224 : kMode == kSplit ? 200 : 208;
   static constexpr int kBlock = 128 * kUtil + 256 * kSoftmax;
   static_assert(kBlock <= kThreads * 168, "setmaxnreg would wait for ever");
 };
@@ -293,6 +294,13 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
   extern __shared__ uint8_t smem_raw[];
   constexpr int kKStages = Rings<kMode>::kK, kVStages = Rings<kMode>::kV;
   constexpr bool kOne = kMode == kSolo;  // one query tile, the two slots share its keys
+  // Which roles take their first item as decoded during the set-up: kept over the fork into roles, an item makes some of
+  // them spill it and reload its fields in their loops, and then decoding it again is cheaper; for the softmax warps that
+  // is not in the way of the first loads.  All roles / issuers only / none, us: split keys, B1 H2 S4096 23.2 / 23.3 / 24.0, 128
+  // rows over 16000 keys, 16/4 heads, 46.3 / 45.1 / 44.8; one tile per item, Keyformer B1 H4 S300 18.6 / 18.7 / 18.4 (where the
+  // other kernels of a build lie moves such a figure by 0.1 to 0.4); two tiles, B1 H32 S1024 16.7 / - / 17.2.
+  constexpr bool kKeepSoftmax = kMode == kPair;
+  constexpr bool kKeepUtil = kMode == kPair || (kMode == kSplit && !kCap);
   __shared__ __align__(8) Bars bars;
   __shared__ float2 row_s[kOne ? kTile : 1];  // (kSolo) second slot's reference and row sum; then both slots' factors
   __shared__ uint32_t tmem_base_s;
@@ -377,7 +385,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
       uint32_t qn[2] = {0, 0};    // items in which tile t was loaded so far (kSolo: loads of either buffer)
       uint32_t items = 0;
       for (int it = 0; it < n_waves && ok; ++it) {
-        if (it == 0 ? !has_first : !get_item<kMode>(it, p, &it_)) continue;
+        if (it == 0 && kKeepUtil ? !has_first : !get_item<kMode>(it, p, &it_)) continue;
         for (int x = 0; x < Rings<kMode>::kQTiles && ok; ++x) {
           if (it_.n_kv[x] == 0) continue;
           const int t = kOne ? static_cast<int>(items++ & 1) : x;
@@ -419,7 +427,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
       bool ok = true;
       uint32_t vc = 0;
       for (int it = 0; it < n_waves && ok; ++it) {
-        if (it == 0 ? !has_first : !get_item<kMode>(it, p, &it_)) continue;
+        if (it == 0 && kKeepUtil ? !has_first : !get_item<kMode>(it, p, &it_)) continue;
         const int n_tiles = kOne ? it_.n_kv[0] + it_.n_kv[1] : it_.n_max;
         for (int j = 0; j < n_tiles && ok; ++j, ++vc) {
           const int st = vc % kVStages;
@@ -463,7 +471,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
       uint32_t x = 0;               // uses of S so far (parity of s_free)
       uint32_t on0 = 0, on1 = 0;    // items of either tile before this one (parity of q_full)
       for (int it = 0; it < n_waves && ok; ++it) {
-        if (it == 0 ? !has_first : !get_item<kMode>(it, p, &it_)) continue;
+        if (it == 0 && kKeepUtil ? !has_first : !get_item<kMode>(it, p, &it_)) continue;
         const int n0 = it_.n_kv[0], n1 = it_.n_kv[1];
         for (int j = 0; j < it_.n_max && ok; ++j) {
 #pragma unroll
@@ -521,7 +529,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
       uint32_t sn0 = 0, sn1 = 0;    // steps of either tile before this item (parity of p_ready)
       uint32_t on0 = 0, on1 = 0;    // items of either tile before this one (parity of o_free)
       for (int it = 0; it < n_waves && ok; ++it) {
-        if (it == 0 ? !has_first : !get_item<kMode>(it, p, &it_)) continue;
+        if (it == 0 && kKeepUtil ? !has_first : !get_item<kMode>(it, p, &it_)) continue;
         const int n0 = it_.n_kv[0], n1 = it_.n_kv[1];
         for (int j = 0; j < it_.n_max && ok; ++j) {
 #pragma unroll
@@ -572,7 +580,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
     bool ok = true;
     uint32_t sn = 0;  // tile steps of this tile before the current item
     for (int it = 0; it < n_waves && (ok || kOne); ++it) {
-      if (it == 0 ? !has_first : !get_item<kMode>(it, p, &it_)) continue;
+      if (it == 0 && kKeepSoftmax ? !has_first : !get_item<kMode>(it, p, &it_)) continue;
       const int n_t = it_.n_kv[t];
       if (n_t == 0 && !kOne) continue;
       const int row = it_.q0[t] + r_in_tile;
