@@ -629,8 +629,17 @@ col_scores_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
     __syncwarp();
     tmem_dealloc(tbase, 256);
   }
-  // (one item: the barrier above is the one that its parts wait for)
-  if (!kLoop && warp >= kUtilWarps && warp < kUtilWarps + 4 && !*abortp) store_sums(m, part_s[0], (warp & 3) * 32 + lane);
+  // One item: the barrier above is the one that its parts wait for.  The modes that are short of registers decode it again
+  // instead of keeping it through the steps (kept -> again, us: RoCo B1 H8 S1500 28.6 -> 28.1, H32 S1501 44.6 -> 44.1; seeded
+  // Keyformer B1 H2 S2048 75.7 -> 75.1, H32 S1501 113.6 -> 112.9; with a noise operand by plain loads 99.8 -> 101.2, H2O as it is).
+  if (!kLoop && warp >= kUtilWarps && warp < kUtilWarps + 4 && !*abortp) {
+    if constexpr (kMode == 1 || kMode == 3) {
+      int idx = idx0;
+      asm volatile("" : "+r"(idx));  // (or the compiler keeps the fields after all)
+      load_item(idx, m);
+    }
+    store_sums(m, part_s[0], (warp & 3) * 32 + lane);
+  }
 }
 
 // ---------------------------------------------------------------------------------------------
