@@ -151,8 +151,10 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_const
     tma_prefetch_desc(&map_k);
     tma_prefetch_desc(&map_v);
   }
-  // What the ring takes first is on its way from DRAM to L2 while the kernel ahead still runs (two stages: B4 H16, 2000 keys,
-  // 15.0 -> 14.5 us, B16 H32/8, 4001 keys, 45.3 -> 45.1; six are slower again).
+  // What the ring takes first is on its way from DRAM to L2 while the kernel ahead still runs: two stages (six are slower
+  // again).  Without and with, us: caches that are not in L2, as in a program with other work between two steps, B4 H16, 2000
+  // keys, 14.2 and 13.7, B8 H32/8, 1000 keys, 10.3 and 9.8, B1 H128/32, 6000 keys, 20.1 and 19.3, B16 H32/8, 4001 keys, 44.2 and
+  // 43.7; caches that are, 9.7 and 10.1, 7.7 and 8.0, 14.6 and 14.5, 44.0 and 43.2.
   if (warp == kWarps && lane == 0) {
     for (int t = t_lo; t < min(t_hi, t_lo + 2); ++t) {
       tma_prefetch_4d(&map_k, 0, hk, t * kKeys, b);

@@ -350,11 +350,11 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tbase = tmem_base_s;
-  // The first item belongs to the set-up too, and so do its first tiles, on their way from DRAM to L2: more of them get in
-  // the way of the loads behind (B1 H4 S512 18.9 -> 19.2 us for H2O), and so does any in a small launch, which seldom comes
-  // up behind another (there 18.0 -> 18.2).  With the items decoded by multiplications, before -> after: B4 H16 S400
-  // 14.3 -> 12.8, B1 H32 S1024 19.8 -> 17.9 (18.3 without the tiles), S2048 39.1 -> 37.3, S4096 124.3 -> 122.5, 500 rows
-  // over 5003 keys, 32/8 heads, 39.9 -> 39.4.
+  // The first item belongs to the set-up too, and so do its first tiles, on their way from DRAM to L2, in launches of 64
+  // CTAs and more.  Without them and with them, us, inputs that are not in L2 / that are: 16 CTAs (B1 H4 S512) 9.00 and
+  // 9.01 / 8.90 and 9.05, 48 (H6 S1024) 12.03 and 12.03 / 11.90 and 12.03, 64 (H8) 12.29 and 12.19 / 12.04 and 12.10, 96 (H12)
+  // 12.79 and 12.60 / 12.26 and 12.28, 148 (H32) 18.01 and 17.52 / 16.95 and 16.95.  More tiles get in the way of the loads
+  // behind (H2O B1 H4 S512, all of the first ring, 18.9 -> 19.2).
   Item it_;
   const bool has_first = get_item<kMode>(0, p, &it_);
   if (warp == 4 && lane == 0 && has_first && gridDim.x >= 64) {

@@ -242,8 +242,9 @@ sima_stats_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
   tc_fence_after_sync();
   const uint32_t tbase = tmem_base_s;
   if (warp == 2 && lane == 0) {
-    // what the ring takes first is on its way from DRAM to L2 meanwhile (two tiles: EA B4 H32 S1000 43.6 -> 42.6 us, B2 H32
-    // S5003 76.0 -> 75.4, SimA B1 H16 S1000 16.4 -> 15.9; six are slower, 45.0)
+    // what the ring takes first is on its way from DRAM to L2 meanwhile: two tiles (six are slower).  Without and with, us:
+    // inputs that are not in L2, EA B4 H32 S1000 42.6 and 40.9, B2 H32 S5003 75.3 and 72.9, SimA B1 H16 S1000 15.6 and 15.2, B2 H32
+    // S1000 26.0 and 25.5; inputs that are, 41.7 and 40.0, 75.2 and 72.8, 14.6 and 14.7, 22.2 and 22.7
     for (int k = 0; k < min(2, t_hi - t_lo); ++k) {
       const int unit = (t_lo + k) / p.share.ntiles, b = unit / p.H, h = unit % p.H;
       const int s0 = (t_lo + k - unit * p.share.ntiles) * kTile;
