@@ -266,7 +266,7 @@ def test_keyformer_seeded_noise_vs_oracle(ops, shape, dtype):
 
 @pytest.mark.parametrize("shape", [(1, 1, 1300, 32), (2, 128, 1300, 16), (1, 129, 1289, 40), (1, 512, 1920, 32)])
 def test_scores_of_few_rows_over_many_keys_vs_oracle(ops, shape):
-  # more key tiles than CTAs run at once: every CTA of the column pass works through several, one after the other
+  # more key tiles than CTAs run at once: CTAs of the column pass go on to a second one
   B, Sq, Skv, H = shape
   q, k, v = O.make_inputs("roco", B, Sq, Skv, H, 128, torch.bfloat16, seed=37)
   ref = O.roco(q, k, v)
@@ -274,6 +274,28 @@ def test_scores_of_few_rows_over_many_keys_vs_oracle(ops, shape):
   score = ops.h2o(q.cuda(), k.cuda(), v.cuda())[1]
   for g, r, n in zip(got + (score,), ref + (ref[1],), ("out", "roco_score", "roco_sq_score", "h2o_score")):
     close(g, r, n)
+  no_timeouts(ops)
+
+
+@pytest.mark.parametrize("case,shape", [  # (B, Sq, Skv, H, Hkv)
+    ("h2o", (1, 130, 5003, 32, 8)), ("h2o", (1, 20, 4200, 40, 20)), ("roco", (1, 130, 3000, 40, 40)), ("roco", (2, 385, 2000, 32, 32))])
+def test_column_pass_with_three_key_tiles_and_more_to_a_cta(ops, case, shape):
+  # from the third on a CTA's barriers are in a phase that they had before and its parts where the first's were;
+  # with several query heads to a key/value head it loads the same K tile again.  (A query tile more than the last
+  # shape has, and the kernel without the loop runs.)
+  B, Sq, Skv, H, Hkv = shape
+  sms = torch.cuda.get_device_properties(0).multi_processor_count
+  assert -(-Skv // 128) * B * H >= 3 * 2 * sms
+  g = torch.Generator().manual_seed(41)
+  q = torch.randn(B, Sq, H, 128, generator=g).to(torch.bfloat16)
+  k, v = (torch.randn(B, Skv, Hkv, 128, generator=g).to(torch.bfloat16) for _ in range(2))
+  ref = O.h2o_gqa(q, k, v) if case == "h2o" else O.roco(q, k, v)
+  f = lambda: getattr(ops, case)(q.cuda(), k.cuda(), v.cuda())  # noqa: E731
+  first = f()
+  for got, want, name in zip(first, ref, ("out", "score", "sq_score")):
+    close(got, want, name)
+  for _ in range(10):
+    assert all(torch.equal(x, y) for x, y in zip(f(), first))
   no_timeouts(ops)
 
 
