@@ -1454,11 +1454,15 @@ cudaError_t launch_col_scores(const CUtensorMap& mq, const CUtensorMap& mk, cons
   p.by_heads = fast_div(s.H, s.B * s.H);
   int ctas = p.n_items;
   const bool sums = a.mode == ASUKA_SCORE_SUM || a.mode == ASUKA_SCORE_SUM_SQ;
-  // With few query tiles a CTA is set-up for most of its life (barriers, tensor memory, K), and then two CTAs to an SM
-  // that go through all key tiles are faster (H2O, us: 100 rows over 8000 keys, 32/8 heads, 58.3 -> 47.3; 500 over 5003
-  // 72.0 -> 70.0; 2 x 200 over 1500, 16/4 heads 27.3 -> 26.2); with more the order in which SMs become free deals them
-  // out better (1000 over 8000, 16/8 heads 98.7 -> 102.4; B2 H40 S700 37.7 -> 38.7).
-  const bool loop = sums && p.n_qchunks == 1 && p.nq_tiles <= 4 && ctas > 2 * num_sms;
+  // With few query tiles a CTA is set-up for most of its life (barriers, tensor memory, K), and then two CTAs to an SM that go
+  // through all key tiles are faster.  H2O, a CTA to an item -> two to an SM, us: 100 rows over 8000 keys, 32/8 heads, 52.7 ->
+  // 45.6; 500 over 5003 69.4 -> 68.5; 2 x 200 over 1500, 16/4 heads, 25.6 -> 25.1; B8 H32 512 over 512 62.6 -> 59.1; one round and
+  // a bit, H40 500 over 1500 (480 items), 36.6 -> 35.9, H16 400 over 2600 (336) 34.2 -> 33.2.  Where the items of such a round
+  // differ in length, the order in which SMs become free deals them out better: B2 H40 512 over 512 (320) 23.6 -> 25.2, B4 H32
+  // 400 over 400 (512) 30.6 -> 31.3, H32 512 over 1200 (320) 24.4 -> 24.8.  So it does with more query tiles (1000 over 8000, 16/8
+  // heads, 98.7 -> 102.4; B2 H40 S700 37.7 -> 38.7).
+  const bool even = !s.causal || static_cast<long long>(s.Skv) >= 3ll * s.Sq;
+  const bool loop = sums && p.n_qchunks == 1 && p.nq_tiles <= 4 && ctas > 2 * num_sms && (even || ctas >= 4 * num_sms);
   if (loop) ctas = 2 * num_sms;
   const dim3 grid(static_cast<unsigned>(ctas));
   void (*kern)(CUtensorMap, CUtensorMap, ColParams) = nullptr;

@@ -46,8 +46,8 @@ __global__ void __launch_bounds__(256) pool_scores_kernel(const float* __restric
 
 // group_mean: grouped-query attention's per-key score, the mean over the query heads of a group
 // (cases/attn_h2o.py:42-46), summed in head order.  Launched as a programmatic dependent of the column pass, and the next
-// call's forward kernel as its (H2O, 32/8 heads, 500 rows over 5003 keys, 69.8 -> 69.2 us; 2 x 200
-// over 1500, 16/4 heads 26.3 -> 25.6).
+// call's forward kernel as its (H2O, 500 rows over 5003 keys, 32/8 heads, 69.3 -> 68.5 us; 2 x 200
+// over 1500, 16/4 heads, 25.8 -> 25.1; 100 over 8000, 32/8 heads, 45.3 -> 45.6).
 __global__ void __launch_bounds__(256) group_mean_kernel(const float* __restrict__ in,
                                                          float* __restrict__ out, int rows, int group,
                                                          int S) {
