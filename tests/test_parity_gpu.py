@@ -1355,6 +1355,20 @@ def test_a_slice_of_a_long_seeded_problem_has_the_same_scores(ops, world):
   no_timeouts(ops)
 
 
+def test_the_workspace_query_asks_for_nothing_that_a_field_of_another_case_would_use(ops):
+  # the parameter block is one for three cases, and a host may fill tau (Keyformer's) for any of them
+  import ctypes
+  from flashtensor_b200 import _lib
+  q, k, v = (torch.empty(2, 2048, 32, 128, device="cuda", dtype=torch.float16) for _ in range(3))
+  sizes = []
+  for tau in (0.0, 1.0):
+    n = ctypes.c_size_t(0)
+    p = _lib.CaseParams(ops._desc(q), ops._desc(k), ops._desc(v), tau=tau, causal=1)
+    assert _lib.load().asuka_b200_case_workspace_bytes_split(ctypes.byref(p), ctypes.byref(n)) == 0
+    sizes.append(n.value)
+  assert sizes[0] == sizes[1]
+
+
 def test_an_expired_wait_is_reported_and_leaves_the_device_usable(ops):
   # a wait that nothing will ever satisfy, with a 2 ms limit: the kernel gives up and returns, the
   # status read reports the time-out once and clears it, and the next call works
